@@ -19,13 +19,44 @@
 // The conv is parallel over rows (each row reads its three predecessors from the launch's own rows or from the pool); the
 // recurrence is sequential over the rows of a segment with the state of one head in the registers of a 256-thread CTA
 // (thread = one p, 32 of the 128 n), so a decode step moves each state once: 2 x 32 KB per (sequence, head).
+#include <type_traits>
 #include "common.cuh"
 
 namespace rx {
 
 constexpr int SSM_P = 64, SSM_N = 128, SSM_HIST = 3;
 constexpr int SCAN_OUT = 1, SCAN_STATE = 2;
-constexpr int SCAN_PF = 4;                        // tokens whose inputs the split scans keep in flight
+
+// two fp32 operations in one instruction (each half rounds as its scalar form): halves the issue slots of the recurrences
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float f2_sum(uint64_t v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// asynchronous copies into shared memory: the inputs of the next tokens arrive while the current ones are computed
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ float ssm_silu(float v) { return v / (1.f + __expf(-v)); }
 __device__ __forceinline__ float ssm_bf(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
@@ -58,7 +89,8 @@ __device__ __forceinline__ void ssm_conv_commit(const float* __restrict__ proj, 
   }
 }
 
-// xbc[r][c] = silu(b[c] + sum_j w[c][j] * in(pos - 3 + j)), grid (M, ceil(C / 256))
+// xbc[r][c] = silu(b[c] + sum_j w[c][j] * in(pos - 3 + j)).  One channel of one row per thread: the form for the few rows of a decode window,
+// where it is latency that counts.  grid (M, ceil(C / 256))
 __global__ void __launch_bounds__(256) ssm_conv_kernel(const float* __restrict__ proj, int ldp, int xoff, int C, const int* __restrict__ row_seq,
                                                       const int* __restrict__ positions, const uint16_t* __restrict__ conv_w,
                                                       const uint16_t* __restrict__ conv_b, const float* __restrict__ pool, float* __restrict__ xbc) {
@@ -70,6 +102,64 @@ __global__ void __launch_bounds__(256) ssm_conv_kernel(const float* __restrict__
 #pragma unroll
   for (int j = 0; j < 4; ++j) acc += ssm_bf(conv_w[c * 4 + j]) * ssm_conv_in(proj, ldp, xoff, pool, C, row_seq, positions, r, 3 - j, c);
   xbc[(size_t)r * C + c] = ssm_silu(acc);
+}
+
+// The same for many rows, bound by memory (one read of the rows, one write): a thread takes two neighbouring channels and walks CONV_RB rows, all
+// loaded before the first is used, with the three rows before them in registers.  The form above reads every input four times through the
+// caches: 137 us for 2048 rows x 10240 channels against 46 us here; the two passes need 26.  grid (ceil(M / CONV_RB), ceil(C / 512)), 256 threads.
+constexpr int CONV_RB = 8;
+__global__ void __launch_bounds__(256) ssm_conv_rows_kernel(const float* __restrict__ proj, int ldp, int xoff, int C, const int* __restrict__ row_seq,
+                                                           const int* __restrict__ positions, const uint16_t* __restrict__ conv_w,
+                                                           const uint16_t* __restrict__ conv_b, const float* __restrict__ pool,
+                                                           float* __restrict__ xbc, int M) {
+  pdl_launch();
+  pdl_wait();
+  const int rb = blockIdx.x * CONV_RB, c = (blockIdx.y * 256 + threadIdx.x) * 2;
+  if (c >= C) return;
+  float x[CONV_RB + 3][2];                          // rows rb - 3 .. rb + CONV_RB - 1
+  int seq[CONV_RB];
+#pragma unroll
+  for (int i = 0; i < CONV_RB; ++i) {
+    const int r = min(rb + i, M - 1);
+    seq[i] = row_seq[r];
+    const float2 v = *reinterpret_cast<const float2*>(proj + (size_t)r * ldp + xoff + c);
+    x[i + 3][0] = v.x, x[i + 3][1] = v.y;
+  }
+  float w[2][4], bias[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    bias[e] = ssm_bf(conv_b[c + e]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[e][j] = ssm_bf(conv_w[(c + e) * 4 + j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) x[j][e] = ssm_conv_in(proj, ldp, xoff, pool, C, row_seq, positions, rb, 3 - j, c + e);
+#pragma unroll
+  for (int i = 0; i < CONV_RB; ++i) {
+    const int r = rb + i;
+    if (r >= M) break;
+    float in[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) in[j][0] = x[i + j][0], in[j][1] = x[i + j][1];
+    const bool near = i >= 3 ? seq[i] != seq[i - 3] : i > 0 && seq[i] != seq[0];
+    if (near) {                                     // another sequence's rows are among the three before: take them where they are kept
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) in[j][e] = ssm_conv_in(proj, ldp, xoff, pool, C, row_seq, positions, r, 3 - j, c + e);
+    }
+    float o[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float acc = bias[e];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc += w[e][j] * in[j][e];
+      o[e] = ssm_silu(acc);
+    }
+    *reinterpret_cast<float2*>(xbc + (size_t)r * C + c) = make_float2(o[0], o[1]);
+  }
 }
 
 // Recurrence.  grid (segments or rows, H).  With a segment table (seg_start != nullptr) block x is segment x; without one block x is
@@ -134,7 +224,9 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const float* __restrict__
 #pragma unroll
     for (int i = 0; i < 32; i += 4) {
       const float4 bb = *reinterpret_cast<const float4*>(sB + nq * 32 + i), cc = *reinterpret_cast<const float4*>(sC + nq * 32 + i);
-      st[i] = st[i] * dA + xdt * bb.x; st[i + 1] = st[i + 1] * dA + xdt * bb.y; st[i + 2] = st[i + 2] * dA + xdt * bb.z; st[i + 3] = st[i + 3] * dA + xdt * bb.w;
+      // (the roundings are spelled out: the split kernel below repeats them, so that a commit leaves the bits of a direct run)
+      st[i] = __fmaf_rn(st[i], dA, __fmul_rn(xdt, bb.x)); st[i + 1] = __fmaf_rn(st[i + 1], dA, __fmul_rn(xdt, bb.y));
+      st[i + 2] = __fmaf_rn(st[i + 2], dA, __fmul_rn(xdt, bb.z)); st[i + 3] = __fmaf_rn(st[i + 3], dA, __fmul_rn(xdt, bb.w));
       a0 += st[i] * cc.x; a1 += st[i + 1] * cc.y; a2 += st[i + 2] * cc.z; a3 += st[i + 3] * cc.w;
     }
     float acc = (a0 + a1) + (a2 + a3);
@@ -148,101 +240,170 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const float* __restrict__
   ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h, (int)gridDim.y);
 }
 
-// Prefill / commit form of the recurrence: a head's 64 state rows p are split over SSM_PS one-warp CTAs (row p only meets x_p, B, C and dt), with
-// the SAME (p, quarter of n) -> lane mapping and arithmetic as ssm_scan_kernel, so states and outputs are bit-identical; one warp per CTA means no
-// block barrier on the per-token path and 8 x more CTAs for a one-sequence prefill.  grid (segments, H, SSM_PS), 32 threads.
-constexpr int SSM_PS = 8;
-__global__ void __launch_bounds__(32) ssm_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
-                                                           int dtoff, int M, int H, int G, const int* __restrict__ row_seq,
-                                                           const int* __restrict__ positions, const int* __restrict__ seg_start,
-                                                           const int* __restrict__ seg_len, const float* __restrict__ dt_bias,
-                                                           const float* __restrict__ a_neg, const float* __restrict__ d_skip,
-                                                           float* __restrict__ ssm_pool, float* conv_pool, float* __restrict__ y, int mode) {
-  pdl_launch();
+// Prefill / commit form of the recurrence, bound by the multiply pipe: three fp32 operations per state value and token, of which the two with three
+// register operands issue at two thirds of the pipe's rate.  A head's 64 state rows p are split over two CTAs of four warps; a thread holds a
+// 4 (p) x 8 (n) tile of the state, so that B and C cost a token four vector loads from shared memory for 96 operations (a 1 x 32 tile needs
+// sixteen; a 4 x 4 tile on twice the warps is bound by those loads again: 506 us).  Products are packed pairs along n.  The inputs of SSM_TC tokens at a
+// time come by cp.async into two buffers, x dt and the decays are made from them by the CTA: two block barriers per SSM_TC tokens, no global load on
+// the per-token path.  State values are rounded exactly as in ssm_scan_kernel (fma(S, dA, (x dt) B)), so both leave the same bits; a token's output
+// is summed over n in this kernel's own fixed order (8 in sequence, then a tree over 16 lanes).  The dependents are released only when the recurrence
+// is done: released at the start, their waiting CTAs (thousands) took the SMs' slots and slowed it by half.
+// One sequence of 2047 tokens, 128 heads: 436 us; 2159 us before (1 x 32 tiles, one warp per CTA, register ring; 3220 us with early release).
+// grid (segments, H, SSM_PS), 128 threads.
+constexpr int SSM_PS = 2, SSM_CP = SSM_P / SSM_PS, SSM_TC = 16;
+struct SsmChunk { float B[SSM_TC][SSM_N], C[SSM_TC][SSM_N], x[SSM_TC][SSM_CP], dt[SSM_TC]; };
+__global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
+                                                            int dtoff, int M, int H, int G, const int* __restrict__ row_seq,
+                                                            const int* __restrict__ positions, const int* __restrict__ seg_start,
+                                                            const int* __restrict__ seg_len, const float* __restrict__ dt_bias,
+                                                            const float* __restrict__ a_neg, const float* __restrict__ d_skip,
+                                                            float* __restrict__ ssm_pool, float* conv_pool, float* __restrict__ y, int mode) {
   pdl_wait();
-  __shared__ __align__(16) float sB[SSM_N], sC[SSM_N];
+  __shared__ __align__(16) SsmChunk buf[2];
+  __shared__ __align__(16) uint64_t xdt2[SSM_TC][SSM_CP], dec2[SSM_TC];      // x dt and the decay of the current chunk, both halves of a pair alike
   const int r0 = seg_start[blockIdx.x], len = seg_len[blockIdx.x];
   if (len <= 0) return;
-  const int h = blockIdx.y, pz = blockIdx.z, lane = threadIdx.x, p = pz * 8 + (lane >> 2), nq = lane & 3;
-  const int seq = row_seq[r0], g = h / (H / G), DI = H * SSM_P;
-  float st[32];
-  float* sp = ssm_pool + (((size_t)seq * H + h) * SSM_P + p) * SSM_N + nq * 32;
-  if (positions[r0] == 0) {
+  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ln = lane & 15, lp = lane >> 4;
+  const int seq = row_seq[r0], g = h / (H / G), DI = H * SSM_P, p0 = blockIdx.z * SSM_CP;
+  // Slot k of a thread is state row pl + (k ^ sel) with sel from lane bits 3 and 2: what a lane passes on in the output sums' tree is then always
+  // its upper slots, without selects.
+  const int pl = warp * 8 + lp * 4, sel = (ln & 8 ? 2 : 0) | (ln & 4 ? 1 : 0);
+  uint64_t st[4][4];                                // [slot][pair of n]: n = 4 ln + {0, 1}, {2, 3}, then 64 more
+  float* sp = ssm_pool + (((size_t)seq * H + h) * SSM_P + p0 + pl) * SSM_N + 4 * ln;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) st[i] = 0.f;
-  } else {
+  for (int p = 0; p < 4; ++p) {
 #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      const float4 v = *reinterpret_cast<const float4*>(sp + i);
-      st[i] = v.x, st[i + 1] = v.y, st[i + 2] = v.z, st[i + 3] = v.w;
+    for (int k = 0; k < 2; ++k) {
+      ulonglong2 v = make_ulonglong2(0ull, 0ull);
+      if (positions[r0] != 0) v = *reinterpret_cast<const ulonglong2*>(sp + (p ^ sel) * SSM_N + 64 * k);
+      st[p][2 * k] = v.x, st[p][2 * k + 1] = v.y;
     }
   }
-  const float A = a_neg[h], Dh = d_skip[h], dtb = dt_bias[h];
-  // a lane's share of a token's inputs: B and C values 32 c + lane (c = 0..3), its row's x, the head's dt; the next token's are in flight while
-  // the current one is computed
-  struct In { float b[4], c[4], x, dt; };
-  auto fetch = [&](int r) {
-    In in;
-    const float* xr = xbc + (size_t)r * C;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      in.b[c] = xr[DI + g * SSM_N + 32 * c + lane];
-      in.c[c] = xr[DI + G * SSM_N + g * SSM_N + 32 * c + lane];
+  auto issue = [&](int c) {                         // tokens c * SSM_TC ..; past the end the last row again (never used)
+    SsmChunk& d = buf[c & 1];
+    for (int t = warp; t < SSM_TC; t += 4) {
+      const float* xr = xbc + (size_t)(r0 + min(c * SSM_TC + t, len - 1)) * C;
+      cp16(&d.B[t][4 * lane], xr + DI + g * SSM_N + 4 * lane);
+      cp16(&d.C[t][4 * lane], xr + DI + (G + g) * SSM_N + 4 * lane);
     }
-    in.x = xr[h * SSM_P + p];
-    in.dt = proj[(size_t)r * ldp + dtoff + h];
-    return in;
+    const int t = tid >> 3;
+    cp16(&d.x[t][4 * (tid & 7)], xbc + (size_t)(r0 + min(c * SSM_TC + t, len - 1)) * C + h * SSM_P + p0 + 4 * (tid & 7));
+    if (tid < SSM_TC) cp4(&d.dt[tid], proj + (size_t)(r0 + min(c * SSM_TC + tid, len - 1)) * ldp + dtoff + h);
+    cp_commit();
   };
-  // a ring of SCAN_PF tokens' inputs in registers: one iteration is far shorter than a trip to memory, so the loads run SCAN_PF tokens ahead
-  In ring[SCAN_PF];
+  const float A = a_neg[h], Dh = d_skip[h], dtb = dt_bias[h];
+  const bool b1 = (ln & 2) != 0, b0 = (ln & 1) != 0;
+  float* yp = y + h * SSM_P + p0 + pl + sel;        // slot 0's row: the one whose sums end in this lane
+  // NT tokens (4, or 1 at the end): the states in turn, then all NT x 4 output sums over the 16 lanes together, each step halving what a lane
+  // carries on.  A sum's tree over the lanes (distances 8, 4, 2, 1) does not depend on NT.
+  auto tokens = [&](const SsmChunk& d, auto n, int t0, int r) {
+    constexpr int NT = decltype(n)::value;
+    float k[NT];
 #pragma unroll
-  for (int k = 0; k < SCAN_PF; ++k)
-    if (k < len) ring[k] = fetch(r0 + k);
-  for (int t0 = 0; t0 < len; t0 += SCAN_PF) {
+    for (int i = 0; i < NT; ++i) {
+      const int t = t0 + i;
+      const ulonglong2 B0 = *reinterpret_cast<const ulonglong2*>(&d.B[t][4 * ln]), B1 = *reinterpret_cast<const ulonglong2*>(&d.B[t][64 + 4 * ln]);
+      const ulonglong2 C0 = *reinterpret_cast<const ulonglong2*>(&d.C[t][4 * ln]), C1 = *reinterpret_cast<const ulonglong2*>(&d.C[t][64 + 4 * ln]);
+      const uint64_t dA2 = dec2[t];
+      float o[4];
 #pragma unroll
-  for (int k = 0; k < SCAN_PF; ++k) {
-    const int t = t0 + k;
-    if (t >= len) break;
-    const int r = r0 + t;
-    const In cur = ring[k];
-    if (t + SCAN_PF < len) ring[k] = fetch(r + SCAN_PF);
-    __syncwarp();
-#pragma unroll
-    for (int c = 0; c < 4; ++c) { sB[32 * c + lane] = cur.b[c]; sC[32 * c + lane] = cur.c[c]; }
-    __syncwarp();
-    float dt = cur.dt + dtb;
-    dt = dt > 20.f ? dt : log1pf(__expf(dt));            // softplus
-    const float dA = __expf(dt * A), xdt = cur.x * dt;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      const float4 bb = *reinterpret_cast<const float4*>(sB + nq * 32 + i), cc = *reinterpret_cast<const float4*>(sC + nq * 32 + i);
-      st[i] = st[i] * dA + xdt * bb.x; st[i + 1] = st[i + 1] * dA + xdt * bb.y; st[i + 2] = st[i + 2] * dA + xdt * bb.z; st[i + 3] = st[i + 3] * dA + xdt * bb.w;
-      a0 += st[i] * cc.x; a1 += st[i + 1] * cc.y; a2 += st[i + 2] * cc.z; a3 += st[i + 3] * cc.w;
+      for (int p = 0; p < 4; ++p) {
+        const uint64_t xd2 = xdt2[t][pl + (p ^ sel)];
+        st[p][0] = f2_fma(st[p][0], dA2, f2_mul(xd2, B0.x));
+        st[p][1] = f2_fma(st[p][1], dA2, f2_mul(xd2, B0.y));
+        st[p][2] = f2_fma(st[p][2], dA2, f2_mul(xd2, B1.x));
+        st[p][3] = f2_fma(st[p][3], dA2, f2_mul(xd2, B1.y));
+        uint64_t a = f2_mul(st[p][0], C0.x);
+        a = f2_fma(st[p][1], C0.y, a);
+        a = f2_fma(st[p][2], C1.x, a);
+        a = f2_fma(st[p][3], C1.y, a);
+        o[p] = f2_sum(a);
+      }
+      const float k0 = o[0] + __shfl_xor_sync(0xffffffffu, o[2], 8), k1 = o[1] + __shfl_xor_sync(0xffffffffu, o[3], 8);
+      k[i] = k0 + __shfl_xor_sync(0xffffffffu, k1, 4);
     }
-    float acc = (a0 + a1) + (a2 + a3);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    if (nq == 0 && (mode & SCAN_OUT)) y[(size_t)r * DI + h * SSM_P + p] = acc + Dh * cur.x;
+    if (!(mode & SCAN_OUT)) return;
+    if constexpr (NT == 4) {                        // lane bits 1 and 0 pick the token
+      const float m0 = (b1 ? k[2] : k[0]) + __shfl_xor_sync(0xffffffffu, b1 ? k[0] : k[2], 2);
+      const float m1 = (b1 ? k[3] : k[1]) + __shfl_xor_sync(0xffffffffu, b1 ? k[1] : k[3], 2);
+      const float m = (b0 ? m1 : m0) + __shfl_xor_sync(0xffffffffu, b0 ? m0 : m1, 1);
+      yp[(size_t)(r + (ln & 3)) * DI] = __fmaf_rn(Dh, d.x[t0 + (ln & 3)][pl + sel], m);
+    } else {
+      float m = k[0];
+      m += __shfl_xor_sync(0xffffffffu, m, 2);
+      m += __shfl_xor_sync(0xffffffffu, m, 1);
+      if ((ln & 3) == 0) yp[(size_t)r * DI] = __fmaf_rn(Dh, d.x[t0][pl + sel], m);
+    }
+  };
+  issue(0);
+  const int nc = (len + SSM_TC - 1) / SSM_TC;
+  for (int c = 0; c < nc; ++c) {
+    cp_wait_all();
+    __syncthreads();                                // chunk c has landed, everybody is done with chunk c - 1
+    if (c + 1 < nc) issue(c + 1);
+    const SsmChunk& d = buf[c & 1];
+    {
+      const int t = tid >> 3, p = 4 * (tid & 7);    // eight threads per token
+      float dt = d.dt[t] + dtb;
+      dt = dt > 20.f ? dt : log1pf(__expf(dt));     // softplus
+      const float dA = __expf(dt * A);
+      const float4 x = *reinterpret_cast<const float4*>(&d.x[t][p]);
+      const float xd[4] = {x.x * dt, x.y * dt, x.z * dt, x.w * dt};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) xdt2[t][p + e] = f2_pack(xd[e], xd[e]);
+      if (p == 0) dec2[t] = f2_pack(dA, dA);
+    }
+    __syncthreads();
+    const int nt = min(SSM_TC, len - c * SSM_TC);
+    int t = 0;
+    for (; t + 4 <= nt; t += 4) tokens(d, std::integral_constant<int, 4>(), t, r0 + c * SSM_TC + t);
+    for (; t < nt; ++t) tokens(d, std::integral_constant<int, 1>(), t, r0 + c * SSM_TC + t);
   }
-  }
+  pdl_launch();
   if (!(mode & SCAN_STATE)) return;
 #pragma unroll
-  for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(sp + i) = make_float4(st[i], st[i + 1], st[i + 2], st[i + 3]);
-  ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h * SSM_PS + pz, (int)(gridDim.y * SSM_PS));
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      *reinterpret_cast<ulonglong2*>(sp + (p ^ sel) * SSM_N + 64 * k) = make_ulonglong2(st[p][2 * k], st[p][2 * k + 1]);
+  ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h * SSM_PS + blockIdx.z, (int)(gridDim.y * SSM_PS));
 }
 
-// out[r][c] = bf16( rmsnorm_group( y * silu(z) )[c] * w[c] ), grid (M, G); the group is d_inner / G channels wide
+// out[r][c] = bf16( rmsnorm_group( y * silu(z) )[c] * w[c] ), grid (M, G); the group is d_inner / G channels wide.  Bound by memory: a thread takes
+// four neighbouring channels at a time and keeps the gated values of the first 1024 channels in registers between the sum and the scaling (read
+// and gated twice, channel by channel, it took 68 us for 2047 rows of 8 x 1024 channels, 46 us now); a wider group is gated again beyond that.
+// VEC: width and alignment allow the vectors; else the four channels are loaded one by one.  A channel is added to the same partial sum either way.
+template <bool VEC>
 __global__ void __launch_bounds__(256) ssm_gate_norm_kernel(const float* __restrict__ y, const float* __restrict__ proj, int ldp, int DI, int G,
                                                            const uint16_t* __restrict__ norm_w, float eps, uint16_t* __restrict__ out) {
   pdl_launch();
   pdl_wait();
   __shared__ float red[8];
   const int r = blockIdx.x, g = blockIdx.y, W = DI / G, c0 = g * W;
-  float ss = 0.f;
-  for (int c = threadIdx.x; c < W; c += 256) {
-    const float v = y[(size_t)r * DI + c0 + c] * ssm_silu(proj[(size_t)r * ldp + c0 + c]);
-    ss += v * v;
+  const float* yr = y + (size_t)r * DI + c0;
+  const float* zr = proj + (size_t)r * ldp + c0;
+  auto gated = [&](int c, float (&v)[4]) {
+    float a[4], z[4];
+    if (VEC) {
+      const float4 p = *reinterpret_cast<const float4*>(yr + c), q = *reinterpret_cast<const float4*>(zr + c);
+      a[0] = p.x, a[1] = p.y, a[2] = p.z, a[3] = p.w, z[0] = q.x, z[1] = q.y, z[2] = q.z, z[3] = q.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = c + e < W ? yr[c + e] : 0.f, z[e] = c + e < W ? zr[c + e] : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = a[e] * ssm_silu(z[e]);
+  };
+  float keep[4] = {0.f, 0.f, 0.f, 0.f}, ss = 0.f;
+  const int c1 = 4 * threadIdx.x;
+  if (c1 < W) gated(c1, keep);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) ss = __fmaf_rn(keep[e], keep[e], ss);
+  for (int c = c1 + 1024; c < W; c += 1024) {
+    float v[4];
+    gated(c, v);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss = __fmaf_rn(v[e], v[e], ss);
   }
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
@@ -251,10 +412,20 @@ __global__ void __launch_bounds__(256) ssm_gate_norm_kernel(const float* __restr
 #pragma unroll
   for (int i = 0; i < 8; ++i) tot += red[i];
   const float rinv = rsqrtf(tot / (float)W + eps);
-  for (int c = threadIdx.x; c < W; c += 256) {
-    const float v = y[(size_t)r * DI + c0 + c] * ssm_silu(proj[(size_t)r * ldp + c0 + c]);
-    __nv_bfloat16 b = __float2bfloat16_rn(v * rinv * ssm_bf(norm_w[c0 + c]));
-    out[(size_t)r * DI + c0 + c] = *reinterpret_cast<uint16_t*>(&b);
+  for (int c = c1; c < W; c += 1024) {
+    float v[4];
+    if (c == c1) v[0] = keep[0], v[1] = keep[1], v[2] = keep[2], v[3] = keep[3];
+    else gated(c, v);
+    uint16_t b[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      __nv_bfloat16 t = __float2bfloat16_rn(v[e] * rinv * (VEC || c + e < W ? ssm_bf(norm_w[c0 + c + e]) : 0.f));
+      b[e] = *reinterpret_cast<uint16_t*>(&t);
+    }
+    uint16_t* op = out + (size_t)r * DI + c0 + c;
+    if (VEC) *reinterpret_cast<uint2*>(op) = make_uint2(b[0] | ((uint32_t)b[1] << 16), b[2] | ((uint32_t)b[3] << 16));
+    else
+      for (int e = 0; e < 4 && c + e < W; ++e) op[e] = b[e];
   }
 }
 
@@ -277,36 +448,46 @@ __global__ void __launch_bounds__(256) ssm_gate_norm_kernel(const float* __restr
 constexpr int GDN_D = 128;
 
 // One token of the delta rule for the 64 state values of a thread (value column j, one half of the keys): decay, S.k (both halves meet in one
-// shuffle), the rank-one write, S.q.  Four partial sums per dot product keep the dependent chains at 16 instead of 64; both scan kernels call
-// this, which is what keeps their states and outputs bit-identical.  sk / sq / sd: this half's 64 keys, queries and (KDA) decays in shared memory,
-// 16-byte aligned.  o is returned before the 1 / |q| factor.
+// shuffle), the rank-one write, S.q.  A dot product is taken over eighths of the keys (16 each, four partial sums), then as a tree
+// over the eighths: the order of gdn_scan_split_kernel, whose threads hold one eighth of two columns, so that both leave the same bits.
+// sk / sq / sd: this half's 64 keys, queries and (KDA) decays in shared memory, 16-byte aligned.  o is returned before the 1 / |q| factor.
 template <bool KDA>
 __device__ __forceinline__ void gdn_token_update(float (&st)[64], const float* sk, const float* sq, const float* sd, float decay, float v, float beta,
                                                  float kinv, float& kv_out, float& o_out) {
-  float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
+  float part[4];
 #pragma unroll
-  for (int i = 0; i < 64; i += 4) {
-    const float4 kk = *reinterpret_cast<const float4*>(sk + i);
-    if (KDA) {
-      const float4 dd = *reinterpret_cast<const float4*>(sd + i);
-      st[i] *= dd.x; st[i + 1] *= dd.y; st[i + 2] *= dd.z; st[i + 3] *= dd.w;
-    } else {
-      st[i] *= decay; st[i + 1] *= decay; st[i + 2] *= decay; st[i + 3] *= decay;
+  for (int u = 0; u < 4; ++u) {
+    float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
+#pragma unroll
+    for (int i = 16 * u; i < 16 * u + 16; i += 4) {
+      const float4 kk = *reinterpret_cast<const float4*>(sk + i);
+      if (KDA) {
+        const float4 dd = *reinterpret_cast<const float4*>(sd + i);
+        st[i] *= dd.x; st[i + 1] *= dd.y; st[i + 2] *= dd.z; st[i + 3] *= dd.w;
+      } else {
+        st[i] *= decay; st[i + 1] *= decay; st[i + 2] *= decay; st[i + 3] *= decay;
+      }
+      k0 = __fmaf_rn(st[i], kk.x, k0); k1 = __fmaf_rn(st[i + 1], kk.y, k1); k2 = __fmaf_rn(st[i + 2], kk.z, k2); k3 = __fmaf_rn(st[i + 3], kk.w, k3);
     }
-    k0 += st[i] * kk.x; k1 += st[i + 1] * kk.y; k2 += st[i + 2] * kk.z; k3 += st[i + 3] * kk.w;
+    part[u] = (k0 + k1) + (k2 + k3);
   }
-  float kv = (k0 + k1) + (k2 + k3);
+  float kv = (part[0] + part[1]) + (part[2] + part[3]);
   kv = (kv + __shfl_xor_sync(0xffffffffu, kv, 1)) * kinv;
-  const float delta = (v - kv) * beta * kinv;          // k enters the update normalised as well
-  float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+  const float delta = __fsub_rn(v, kv) * beta * kinv;          // k enters the update normalised as well
 #pragma unroll
-  for (int i = 0; i < 64; i += 4) {
-    const float4 kk = *reinterpret_cast<const float4*>(sk + i);
-    const float4 qq = *reinterpret_cast<const float4*>(sq + i);
-    st[i] += kk.x * delta; st[i + 1] += kk.y * delta; st[i + 2] += kk.z * delta; st[i + 3] += kk.w * delta;
-    o0 += st[i] * qq.x; o1 += st[i + 1] * qq.y; o2 += st[i + 2] * qq.z; o3 += st[i + 3] * qq.w;
+  for (int u = 0; u < 4; ++u) {
+    float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+#pragma unroll
+    for (int i = 16 * u; i < 16 * u + 16; i += 4) {
+      const float4 kk = *reinterpret_cast<const float4*>(sk + i);
+      const float4 qq = *reinterpret_cast<const float4*>(sq + i);
+      st[i] = __fmaf_rn(kk.x, delta, st[i]); st[i + 1] = __fmaf_rn(kk.y, delta, st[i + 1]);
+      st[i + 2] = __fmaf_rn(kk.z, delta, st[i + 2]); st[i + 3] = __fmaf_rn(kk.w, delta, st[i + 3]);
+      o0 = __fmaf_rn(st[i], qq.x, o0); o1 = __fmaf_rn(st[i + 1], qq.y, o1); o2 = __fmaf_rn(st[i + 2], qq.z, o2); o3 = __fmaf_rn(st[i + 3], qq.w, o3);
+    }
+    part[u] = (o0 + o1) + (o2 + o3);
   }
-  float o = (o0 + o1) + (o2 + o3);
+  float o = (part[0] + part[1]) + (part[2] + part[3]);
   o = o + __shfl_xor_sync(0xffffffffu, o, 1);
   kv_out = kv;
   o_out = o;
@@ -359,7 +540,7 @@ __global__ void __launch_bounds__(256, 2) gdn_scan_kernel(const float* __restric
     __syncthreads();
     const float val = tid < GDN_D ? xr[hk * GDN_D + tid] : xr[(Hk + hk) * GDN_D + (tid - GDN_D)];
     sqk[tid] = val;
-    const float ss = warp_sum(val * val);
+    const float ss = warp_sum(__fmul_rn(val, val));
     if (lane == 0) red[warp] = ss;
     if (KDA && tid < GDN_D) {
       float ai = proj[(size_t)r * ldp + goff + Hv + h * GDN_D + tid] + dt_bias[h * GDN_D + tid];
@@ -380,7 +561,7 @@ __global__ void __launch_bounds__(256, 2) gdn_scan_kernel(const float* __restric
     float kv, o;
     gdn_token_update<KDA>(st, sk, sq, sdec + (KDA ? half * 64 : 0), decay, v, beta, kinv, kv, o);
     o *= qinv;
-    const float ss2 = warp_sum(half == 0 ? o * o : 0.f);
+    const float ss2 = warp_sum(half == 0 ? __fmul_rn(o, o) : 0.f);
     if (lane == 0) red2[warp] = ss2;
     __syncthreads();
     float tot = 0.f;
@@ -399,133 +580,255 @@ __global__ void __launch_bounds__(256, 2) gdn_scan_kernel(const float* __restric
   ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h, (int)gridDim.y);
 }
 
-// ---- prefill form of the delta-rule scan: a head's 128 value columns are split over GDN_JS CTAs (the columns evolve independently: S_j only
-// meets q and k), each ONE warp (no block barrier on the per-token path) with the SAME (column, key half) -> thread mapping and arithmetic as gdn_scan_kernel, so every state value
-// and every output is bit-identical to the unsplit kernel's; the per-head gated norm, which needs all 128 outputs, runs afterwards in
-// gdn_norm_kernel with the unsplit kernel's reduction order.  The inputs of token t + 1 are fetched while token t is computed: a one-sequence
-// prefill was a chain of dependent global loads per token on 48 CTAs; it now runs 192 CTAs with the loads off the critical path.
-constexpr int GDN_JS = 8;
+// ---- prefill / commit form of the delta-rule scan.  A head's 128 value columns evolve independently (S_j only meets q and k): they are split over
+// GDN_JS CTAs of four warps.  A thread holds 2 columns x 16 keys: what bounds the kernel is the way of k and q out of shared memory (a vector
+// load costs four cycles of the SM however many lanes read the same word), and two columns share what is loaded; one column x 32 keys ran at
+// 70 % of that limit and took 811 us where this form takes 549 us (900 + 1148 tokens, 48 heads).  Products are packed pairs; a token's critical path is
+// a 16-key dot product, three shuffles and the rank-one write; the output sums of four tokens go over the lanes together, off that path.  What a
+// token needs besides (1 / |q|, 1 / |k|, decay, write strength) is computed for GDN_TC tokens at a time by the CTA from the inputs that cp.async
+// brought into two buffers (norm sums per token and warp: 40 shuffles, 0.96 us per token, 1105 us).  Every rounding and every order of a sum
+// is gdn_scan_kernel's, so states and outputs are the same bits; the per-head gated norm, which needs all 128 outputs, runs afterwards in
+// gdn_norm_kernel.  The dependents are released at the end (see ssm_scan_split_kernel).  grid (segments, Hv, GDN_JS), 128 threads.
+constexpr int GDN_JS = 4, GDN_PAD = GDN_D + 32;                       // 16 keys every 20 floats: eight lanes' vectors in different banks
+template <bool KDA> struct GdnChunk {
+  static constexpr int TC = KDA ? 8 : 16;
+  float q[TC][GDN_PAD], k[TC][GDN_PAD], d[KDA ? TC : 1][GDN_PAD], v[TC][GDN_D / GDN_JS], a[TC], b[TC];
+};
+__device__ __forceinline__ int gdn_pad(int i) { return i + ((i >> 4) << 2); }
 template <bool KDA>
-__global__ void __launch_bounds__(32) gdn_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
-                                                           int goff, int M, int Hk, int Hv, const int* __restrict__ row_seq,
-                                                           const int* __restrict__ positions, const int* __restrict__ seg_start,
-                                                           const int* __restrict__ seg_len, const float* __restrict__ dt_bias,
-                                                           const float* __restrict__ a_neg, float* __restrict__ s_pool, float* conv_pool,
-                                                           float* __restrict__ y32, int mode) {
-  pdl_launch();
+__global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
+                                                            int goff, int M, int Hk, int Hv, const int* __restrict__ row_seq,
+                                                            const int* __restrict__ positions, const int* __restrict__ seg_start,
+                                                            const int* __restrict__ seg_len, const float* __restrict__ dt_bias,
+                                                            const float* __restrict__ a_neg, float* __restrict__ s_pool, float* conv_pool,
+                                                            float* __restrict__ y32, int mode) {
+  constexpr int TC = GdnChunk<KDA>::TC, JC = GDN_D / GDN_JS;
   pdl_wait();
-  __shared__ __align__(16) float sqk[2 * GDN_D], sdec[KDA ? GDN_D : 4];
+  __shared__ __align__(16) GdnChunk<KDA> buf[2];
+  __shared__ __align__(16) float4 gate[TC];                            // decay, beta, 1 / |k|, 1 / |q| of a token
   const int r0 = seg_start[blockIdx.x], len = seg_len[blockIdx.x];
   if (len <= 0) return;
-  const int h = blockIdx.y, gw = blockIdx.z, lane = threadIdx.x;      // one warp = one of the head's eight state warps
-  const int j = gw * 16 + (lane >> 1), half = lane & 1;
+  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int sub = lane & 3, half = (lane >> 2) & 1, jl = warp * 8 + (lane >> 3) + 4 * (lane & 1), j = blockIdx.z * JC + jl;
+  const int dj = (lane & 1) ? -4 : 4;     // slot 0 is column j, slot 1 column j + dj: of a pair, a lane passes slot 1 on in a sum's tree
   const int seq = row_seq[r0], hk = h / (Hv / Hk), DI = Hv * GDN_D;
-  float st[64];
-  float* sp = s_pool + ((size_t)seq * Hv + h) * (GDN_D * GDN_D) + (size_t)gw * (16 * 128) + lane * 4;
-  if (positions[r0] == 0) {
+  uint64_t st[2][8];                                                   // keys 64 half + 16 sub + (0 .. 15) of the two columns
+  float* sp = s_pool + ((size_t)seq * Hv + h) * (GDN_D * GDN_D) + (size_t)((j >> 4) * 16 + sub * 4) * 128 + (2 * (j & 15) + half) * 4;
+  const bool fresh = positions[r0] == 0;
 #pragma unroll
-    for (int i = 0; i < 64; ++i) st[i] = 0.f;
-  } else {
+  for (int c = 0; c < 2; ++c)
 #pragma unroll
-    for (int i = 0; i < 64; i += 4) {
-      const float4 v = *reinterpret_cast<const float4*>(sp + (i >> 2) * 128);
-      st[i] = v.x, st[i + 1] = v.y, st[i + 2] = v.z, st[i + 3] = v.w;
+    for (int u = 0; u < 4; ++u) {
+      ulonglong2 v = make_ulonglong2(0ull, 0ull);
+      if (!fresh) v = *reinterpret_cast<const ulonglong2*>(sp + u * 128 + c * 8 * dj);
+      st[c][2 * u] = v.x, st[c][2 * u + 1] = v.y;
     }
-  }
-  const float A = a_neg[h], dtb = KDA ? 0.f : dt_bias[h];
-  float kb[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) kb[c] = KDA ? dt_bias[h * GDN_D + 32 * c + lane] : 0.f;
-  const float* sq = sqk + half * 64;
-  const float* sk = sqk + GDN_D + half * 64;
-  // inputs of one token as this lane needs them: q and k values 32 c + lane (c = 0..3), its column's v, the head's gates
-  struct In { float q[4], k[4], ka[4], v, a, b; };
-  auto fetch = [&](int r) {
-    In in;
-    const float* xr = xbc + (size_t)r * C;
-    const float* pr = proj + (size_t)r * ldp + goff;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      in.q[c] = xr[hk * GDN_D + 32 * c + lane];
-      in.k[c] = xr[(Hk + hk) * GDN_D + 32 * c + lane];
-      in.ka[c] = KDA ? pr[Hv + h * GDN_D + 32 * c + lane] : 0.f;
+  const float A = a_neg[h], dtb = KDA ? dt_bias[h * GDN_D + tid] : dt_bias[h];
+  auto issue = [&](int c) {                                            // past the end the last row again (never used)
+    GdnChunk<KDA>& d = buf[c & 1];
+    const int k = tid & 31;
+    for (int t = warp; t < TC; t += 4) {
+      const float* xr = xbc + (size_t)(r0 + min(c * TC + t, len - 1)) * C;
+      cp16(&d.q[t][gdn_pad(4 * k)], xr + hk * GDN_D + 4 * k);
+      cp16(&d.k[t][gdn_pad(4 * k)], xr + (Hk + hk) * GDN_D + 4 * k);
     }
-    in.v = xr[2 * Hk * GDN_D + h * GDN_D + j];
-    in.b = pr[h];
-    in.a = KDA ? 0.f : pr[Hv + h];
-    return in;
+    if (tid < TC * 8) {
+      const int t = tid >> 3, kv = tid & 7;
+      cp16(&d.v[t][4 * kv], xbc + (size_t)(r0 + min(c * TC + t, len - 1)) * C + (2 * Hk + h) * GDN_D + blockIdx.z * JC + 4 * kv);
+    }
+    if (KDA) {
+#pragma unroll
+      for (int t = 0; t < TC; ++t)
+        cp4(&d.d[t][gdn_pad(tid)], proj + (size_t)(r0 + min(c * TC + t, len - 1)) * ldp + goff + Hv + h * GDN_D + tid);
+    }
+    if (tid < TC) {
+      const float* pr = proj + (size_t)(r0 + min(c * TC + tid, len - 1)) * ldp + goff;
+      cp4(&d.b[tid], pr + h);
+      if (!KDA) cp4(&d.a[tid], pr + Hv + h);
+    }
+    cp_commit();
   };
-  In ring[SCAN_PF];                                  // inputs of the next SCAN_PF tokens, in flight while the current one is computed
+  const int kb = (4 * half + sub) * 20;
+  // NT tokens (4, or 1 at the end): the states in turn, then the NT x 2 output sums over the eight lanes of a column pair together
+  auto tokens = [&](const GdnChunk<KDA>& d, auto n, int t0, int r) {
+    constexpr int NT = decltype(n)::value;
+    float o[NT][2];
 #pragma unroll
-  for (int k = 0; k < SCAN_PF; ++k)
-    if (k < len) ring[k] = fetch(r0 + k);
-  for (int t0 = 0; t0 < len; t0 += SCAN_PF) {
+    for (int i = 0; i < NT; ++i) {
+      const int t = t0 + i;
+      const float4 gt = gate[t];
+      const float val = d.v[t][jl];
+      uint64_t kk[8], a[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll
-  for (int k = 0; k < SCAN_PF; ++k) {
-    const int t = t0 + k;
-    if (t >= len) break;
-    const int r = r0 + t;
-    const In cur = ring[k];
-    if (t + SCAN_PF < len) ring[k] = fetch(r + SCAN_PF);
-    __syncwarp();
-    float rq[4], rk[4];                              // the unsplit kernel's eight warp sums: q[32 c .. 32 c + 31], k likewise
+      for (int u = 0; u < 4; ++u) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&d.k[t][kb + 4 * u]);
+        kk[2 * u] = v.x, kk[2 * u + 1] = v.y;
+        ulonglong2 dd;
+        if (KDA) dd = *reinterpret_cast<const ulonglong2*>(&d.d[t][kb + 4 * u]);
+        else dd.x = dd.y = f2_pack(gt.x, gt.x);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      sqk[32 * c + lane] = cur.q[c];
-      sqk[GDN_D + 32 * c + lane] = cur.k[c];
-      rq[c] = warp_sum(cur.q[c] * cur.q[c]);
-      rk[c] = warp_sum(cur.k[c] * cur.k[c]);
-      if (KDA) {
-        float a = cur.ka[c] + kb[c];
-        a = a > 20.f ? a : log1pf(__expf(a));
-        sdec[32 * c + lane] = __expf(A * a);
+        for (int c = 0; c < 2; ++c) {
+          st[c][2 * u] = f2_mul(st[c][2 * u], dd.x);
+          st[c][2 * u + 1] = f2_mul(st[c][2 * u + 1], dd.y);
+          a[c][0] = f2_fma(st[c][2 * u], v.x, a[c][0]);
+          a[c][1] = f2_fma(st[c][2 * u + 1], v.y, a[c][1]);
+        }
+      }
+      float kv = f2_sum(a[0][0]) + f2_sum(a[0][1]);
+      const float kv1 = f2_sum(a[1][0]) + f2_sum(a[1][1]);
+      kv += __shfl_xor_sync(0xffffffffu, kv1, 1);
+      kv += __shfl_xor_sync(0xffffffffu, kv, 2);
+      kv = (kv + __shfl_xor_sync(0xffffffffu, kv, 4)) * gt.z;
+      const float delta = __fsub_rn(val, kv) * gt.y * gt.z, delta1 = __shfl_xor_sync(0xffffffffu, delta, 1);
+      const uint64_t dl[2] = {f2_pack(delta, delta), f2_pack(delta1, delta1)};
+      a[0][0] = a[0][1] = a[1][0] = a[1][1] = 0ull;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(&d.q[t][kb + 4 * u]);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          st[c][2 * u] = f2_fma(kk[2 * u], dl[c], st[c][2 * u]);
+          st[c][2 * u + 1] = f2_fma(kk[2 * u + 1], dl[c], st[c][2 * u + 1]);
+          a[c][0] = f2_fma(st[c][2 * u], qq.x, a[c][0]);
+          a[c][1] = f2_fma(st[c][2 * u + 1], qq.y, a[c][1]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) o[i][c] = f2_sum(a[c][0]) + f2_sum(a[c][1]);
+    }
+    if (!(mode & SCAN_OUT)) return;
+    const bool b1 = (lane & 2) != 0, b2 = (lane & 4) != 0;
+    float m[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) m[i] = o[i][0] + __shfl_xor_sync(0xffffffffu, o[i][1], 1);
+    float* yp = y32 + (size_t)r * DI + h * GDN_D + j;
+    if constexpr (NT == 4) {                                           // bits 1 and 2 pick the token
+      const float n0 = (b1 ? m[2] : m[0]) + __shfl_xor_sync(0xffffffffu, b1 ? m[0] : m[2], 2);
+      const float n1 = (b1 ? m[3] : m[1]) + __shfl_xor_sync(0xffffffffu, b1 ? m[1] : m[3], 2);
+      const float s = (b2 ? n1 : n0) + __shfl_xor_sync(0xffffffffu, b2 ? n0 : n1, 4);
+      const int i = (b1 ? 2 : 0) + (b2 ? 1 : 0);
+      yp[(size_t)i * DI] = s * gate[t0 + i].w;
+    } else {
+      float s = m[0] + __shfl_xor_sync(0xffffffffu, m[0], 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 4);
+      if (!b1 && !b2) yp[0] = s * gate[t0].w;
+    }
+  };
+  issue(0);
+  const int nc = (len + TC - 1) / TC;
+  for (int c = 0; c < nc; ++c) {
+    cp_wait_all();
+    __syncthreads();                                                   // chunk c has landed, everybody is done with chunk c - 1
+    if (c + 1 < nc) issue(c + 1);
+    GdnChunk<KDA>& d = buf[c & 1];
+    // norms: gdn_scan_kernel's warp sums over 32 values (tree over lane distances 16, 8, 4, 2, 1), eight lanes with four values each
+    float rs[TC / 4][2];
+#pragma unroll
+    for (int i = 0; i < TC / 4; ++i)
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        const float* x = (w ? d.k[warp + 4 * i] : d.q[warp + 4 * i]) + (lane >> 3) * 40 + (lane & 7);
+        rs[i][w] = (__fmul_rn(x[0], x[0]) + __fmul_rn(x[20], x[20])) + (__fmul_rn(x[8], x[8]) + __fmul_rn(x[28], x[28]));
+      }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < TC / 4; ++i)
+#pragma unroll
+        for (int w = 0; w < 2; ++w) rs[i][w] += __shfl_xor_sync(0xffffffffu, rs[i][w], o);
+#pragma unroll
+    for (int i = 0; i < TC / 4; ++i) {
+      float tot[2];
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        tot[w] = __shfl_sync(0xffffffffu, rs[i][w], 0);
+#pragma unroll
+        for (int k = 1; k < 4; ++k) tot[w] += __shfl_sync(0xffffffffu, rs[i][w], 8 * k);
+      }
+      const int t = warp + 4 * i;
+      if (lane == i) {
+        float decay = 1.f;
+        if (!KDA) {
+          float al = d.a[t] + dtb;
+          al = al > 20.f ? al : log1pf(__expf(al));
+          decay = __expf(A * al);
+        }
+        gate[t] = make_float4(decay, 1.f / (1.f + __expf(-d.b[t])), rsqrtf(tot[1] + 1e-6f), rsqrtf(tot[0] + 1e-6f) * 0.08838834764831845f);
       }
     }
-    __syncwarp();
-    const float qinv = rsqrtf(rq[0] + rq[1] + rq[2] + rq[3] + 1e-6f) * 0.08838834764831845f;
-    const float kinv = rsqrtf(rk[0] + rk[1] + rk[2] + rk[3] + 1e-6f);
-    float decay = 1.f;
-    if (!KDA) {
-      float a = cur.a + dtb;
-      a = a > 20.f ? a : log1pf(__expf(a));
-      decay = __expf(A * a);
+    if (KDA) {
+#pragma unroll
+      for (int t = 0; t < TC; ++t) {
+        float ai = d.d[t][gdn_pad(tid)] + dtb;
+        ai = ai > 20.f ? ai : log1pf(__expf(ai));
+        d.d[t][gdn_pad(tid)] = __expf(A * ai);
+      }
     }
-    const float beta = 1.f / (1.f + __expf(-cur.b));
-    float kv, o;
-    gdn_token_update<KDA>(st, sk, sq, sdec + (KDA ? half * 64 : 0), decay, cur.v, beta, kinv, kv, o);
-    o *= qinv;
-    if (half == 0 && (mode & SCAN_OUT)) y32[(size_t)r * DI + h * GDN_D + j] = o;
+    __syncthreads();
+    const int nt = min(TC, len - c * TC);
+    int t = 0;
+    for (; t + 4 <= nt; t += 4) tokens(d, std::integral_constant<int, 4>(), t, r0 + c * TC + t);
+    for (; t < nt; ++t) tokens(d, std::integral_constant<int, 1>(), t, r0 + c * TC + t);
   }
-  }
+  pdl_launch();
   if (!(mode & SCAN_STATE)) return;
 #pragma unroll
-  for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(sp + (i >> 2) * 128) = make_float4(st[i], st[i + 1], st[i + 2], st[i + 3]);
-  ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h * GDN_JS + gw, (int)(gridDim.y * GDN_JS));
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) *reinterpret_cast<ulonglong2*>(sp + u * 128 + c * 8 * dj) = make_ulonglong2(st[c][2 * u], st[c][2 * u + 1]);
+  ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h * GDN_JS + blockIdx.z, (int)(gridDim.y * GDN_JS));
 }
 
-// out[r][h][j] = bf16( o * rsqrt(mean_j o^2 + eps) * w[j] * gate(z) ) with the sum of squares taken exactly as gdn_scan_kernel takes it
-// (thread = (j, half), per-warp butterfly over the half == 0 lanes, the eight warp sums added in order).  grid (M, Hv), 256 threads.
+// out[r][h][j] = bf16( o * rsqrt(mean_j o^2 + eps) * w[j] * gate(z) ), bound by memory: one warp per (row, head), four columns per lane.  The sum of
+// squares is taken in gdn_scan_kernel's order: trees over 16 columns (distances 8, 4, 2, 1), the eight sums added in sequence.
+// grid (M, ceil(Hv / 8)), 256 threads.
 template <bool KDA>
 __global__ void __launch_bounds__(256) gdn_norm_kernel(const float* __restrict__ y32, const float* __restrict__ proj, int ldp, int Hv,
                                                       const uint16_t* __restrict__ norm_w, float eps, uint16_t* __restrict__ out) {
   pdl_launch();
   pdl_wait();
-  __shared__ float red2[8];
-  const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j = tid >> 1, half = tid & 1;
-  const int DI = Hv * GDN_D;
-  const float o = y32[(size_t)r * DI + h * GDN_D + j];
-  const float ss2 = warp_sum(half == 0 ? o * o : 0.f);
-  if (lane == 0) red2[warp] = ss2;
-  __syncthreads();
+  const int r = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (h >= Hv) return;
+  const size_t at = ((size_t)r * Hv + h) * GDN_D + 4 * lane;
+  const float* zp = proj + (size_t)r * ldp + h * GDN_D + 4 * lane;
+  const float4 o = *reinterpret_cast<const float4*>(y32 + at);
+  const float z[4] = {zp[0], zp[1], zp[2], zp[3]}, v[4] = {o.x, o.y, o.z, o.w};
+  float s[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s[e] = __fmul_rn(v[e], v[e]);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], 2);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], 1);
+  const float s16 = (s[0] + s[2]) + (s[1] + s[3]);
   float tot = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) tot += red2[i];
-  if (half == 0) {
-    const float z = proj[(size_t)r * ldp + h * GDN_D + j];
-    const float gate = KDA ? 1.f / (1.f + __expf(-z)) : ssm_silu(z);
-    __nv_bfloat16 b = __float2bfloat16_rn(o * rsqrtf(tot / (float)GDN_D + eps) * ssm_bf(norm_w[j]) * gate);
-    out[(size_t)r * DI + h * GDN_D + j] = *reinterpret_cast<uint16_t*>(&b);
+  for (int i = 0; i < 8; ++i) tot += __shfl_sync(0xffffffffu, s16, 4 * i);
+  const float rinv = rsqrtf(tot / (float)GDN_D + eps);
+  uint16_t b[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float gt = KDA ? 1.f / (1.f + __expf(-z[e])) : ssm_silu(z[e]);
+    __nv_bfloat16 t = __float2bfloat16_rn(v[e] * rinv * ssm_bf(norm_w[4 * lane + e]) * gt);
+    b[e] = *reinterpret_cast<uint16_t*>(&t);
   }
+  uint16_t* op = out + at;
+  if ((((uintptr_t)out) & 7) == 0) *reinterpret_cast<uint2*>(op) = make_uint2(b[0] | ((uint32_t)b[1] << 16), b[2] | ((uint32_t)b[3] << 16));
+  else op[0] = b[0], op[1] = b[1], op[2] = b[2], op[3] = b[3];
+}
+
+// The walking form needs pairs of channels (even widths, 8-byte alignment) and enough rows to fill the chip with eighths of them: from about 30
+// rows of 10240 channels on it is the faster one.
+static void launch_conv(const void* proj, int ldp, int xoff, int C, const void* row_seq, const void* positions, const void* conv_w, const void* conv_b,
+                        const void* conv_pool, void* xbc, int M, cudaStream_t st) {
+  const bool pairs = C % 2 == 0 && ldp % 2 == 0 && xoff % 2 == 0 && ((((uintptr_t)proj) | ((uintptr_t)xbc)) & 7) == 0;
+  const int cg = (C + 511) / 512;
+  if (pairs && (long long)(M / CONV_RB) * cg >= 148)
+    launch(ssm_conv_rows_kernel, dim3((M + CONV_RB - 1) / CONV_RB, cg), dim3(256), 0, st, (const float*)proj, ldp, xoff, C, (const int*)row_seq,
+           (const int*)positions, (const uint16_t*)conv_w, (const uint16_t*)conv_b, (const float*)conv_pool, (float*)xbc, M);
+  else
+    launch(ssm_conv_kernel, dim3(M, (C + 255) / 256), dim3(256), 0, st, (const float*)proj, ldp, xoff, C, (const int*)row_seq, (const int*)positions,
+           (const uint16_t*)conv_w, (const uint16_t*)conv_b, (const float*)conv_pool, (float*)xbc);
 }
 
 }  // namespace rx
@@ -545,19 +848,20 @@ RX_API int rx_ssm_mixer(const void* proj, int ldp, int M, int H, int P, int G, i
   if (ldp < dtoff + H) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   if (mode & SCAN_OUT)
-    launch(ssm_conv_kernel, dim3(M, (C + 255) / 256), dim3(256), 0, st, (const float*)proj, ldp, xoff, C, (const int*)row_seq, (const int*)positions,
-           (const uint16_t*)conv_w, (const uint16_t*)conv_b, (const float*)conv_pool, (float*)xbc);
-  if (seg_start != nullptr)
-    launch(ssm_scan_split_kernel, dim3(nseg, H, SSM_PS), dim3(32), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
+    launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
+  if (seg_start != nullptr && (((uintptr_t)xbc) & 15) == 0)     // segments known on the host (prefill, commit); its copies take 16 bytes
+    launch(ssm_scan_split_kernel, dim3(nseg, H, SSM_PS), dim3(128), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
            (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len, (const float*)dt_bias, (const float*)a_neg,
            (const float*)d_skip, (float*)ssm_pool, (float*)conv_pool, (float*)y, mode);
   else
   launch(ssm_scan_kernel, dim3(seg_start ? nseg : M, H), dim3(256), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
          (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len, (const float*)dt_bias, (const float*)a_neg,
          (const float*)d_skip, (float*)ssm_pool, (float*)conv_pool, (float*)y, mode);
-  if (mode & SCAN_OUT)
-    launch(ssm_gate_norm_kernel, dim3(M, G), dim3(256), 0, st, (const float*)y, (const float*)proj, ldp, DI, G, (const uint16_t*)norm_w, eps,
-         (uint16_t*)out_bf16);
+  if (mode & SCAN_OUT) {
+    const bool vec = (DI / G) % 4 == 0 && ldp % 4 == 0 && ((((uintptr_t)y) | ((uintptr_t)proj)) & 15) == 0 && (((uintptr_t)out_bf16) & 7) == 0;
+    launch(vec ? ssm_gate_norm_kernel<true> : ssm_gate_norm_kernel<false>, dim3(M, G), dim3(256), 0, st, (const float*)y, (const float*)proj, ldp, DI, G,
+           (const uint16_t*)norm_w, eps, (uint16_t*)out_bf16);
+  }
   return (int)cudaGetLastError();
 }
 
@@ -575,15 +879,14 @@ RX_API int rx_gdn_mixer(const void* proj, int ldp, int M, int Hk, int Hv, int D,
   if (ldp < goff + Hv + (kda ? Hv * D : Hv)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   if (mode & SCAN_OUT)
-    launch(ssm_conv_kernel, dim3(M, (C + 255) / 256), dim3(256), 0, st, (const float*)proj, ldp, xoff, C, (const int*)row_seq, (const int*)positions,
-           (const uint16_t*)conv_w, (const uint16_t*)conv_b, (const float*)conv_pool, (float*)xbc);
-  if (seg_start != nullptr && y32 != nullptr) {
+    launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
+  if (seg_start != nullptr && y32 != nullptr && ((((uintptr_t)xbc) | ((uintptr_t)y32)) & 15) == 0) {
     // segments known on the host (prefill, commit): the column-split scan with prefetched inputs, then the norm (same bits as the fused kernel)
-    launch(kda ? gdn_scan_split_kernel<true> : gdn_scan_split_kernel<false>, dim3(nseg, Hv, GDN_JS), dim3(32), 0, st, (const float*)xbc, C,
+    launch(kda ? gdn_scan_split_kernel<true> : gdn_scan_split_kernel<false>, dim3(nseg, Hv, GDN_JS), dim3(128), 0, st, (const float*)xbc, C,
            (const float*)proj, ldp, xoff, goff, M, Hk, Hv, (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len,
            (const float*)dt_bias, (const float*)a_neg, (float*)s_pool, (float*)conv_pool, (float*)y32, mode);
     if (mode & SCAN_OUT)
-      launch(kda ? gdn_norm_kernel<true> : gdn_norm_kernel<false>, dim3(M, Hv), dim3(256), 0, st, (const float*)y32, (const float*)proj, ldp, Hv,
+      launch(kda ? gdn_norm_kernel<true> : gdn_norm_kernel<false>, dim3(M, (Hv + 7) / 8), dim3(256), 0, st, (const float*)y32, (const float*)proj, ldp, Hv,
              (const uint16_t*)norm_w, eps, (uint16_t*)out_bf16);
     return (int)cudaGetLastError();
   }
