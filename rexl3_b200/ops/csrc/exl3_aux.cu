@@ -126,11 +126,14 @@ __global__ void __launch_bounds__(1024) norm_rot_in_kernel(const uint16_t* __res
 
 // ------------------------------------------------------------------------------------------------ finish kernels
 // y[row][n] = H_N( sum_s part[s][row][:] )[n] * svh[n] + bias[n] for one 128-block, lane holds 4 consecutive n.
+// ONE: a single plane, known at compile time.  The loop over planes keeps eight loads in registers; a kernel that carries it for nothing holds a
+// third as many warps per SM (100 registers against 32-48), which for the many rows of a prompt is what bounded these kernels.
+template <bool ONE = false>
 __device__ __forceinline__ void finish_block(const float* __restrict__ part, int S, size_t split_stride, size_t off, const __half* svh,
                                              const float* bias, int n0, float (&y)[4]) {
   // loads are issued eight at a time (independent, so their latencies overlap) and added in split order
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (S == 1) acc = __ldg(reinterpret_cast<const float4*>(part + off));
+  if (ONE || S == 1) acc = __ldg(reinterpret_cast<const float4*>(part + off));
   else
   for (int s0 = 0; s0 < S; s0 += 8) {
     float4 p[8];
@@ -149,7 +152,7 @@ __device__ __forceinline__ void finish_block(const float* __restrict__ part, int
   float sv[4];
   load4_f16(svh + n0, sv);
 #pragma unroll
-  for (int r = 0; r < 4; ++r) y[r] *= sv[r];
+  for (int r = 0; r < 4; ++r) y[r] = __fmul_rn(y[r], sv[r]);     // (never contracted into what follows: the variants of a kernel give the same bits)
   if (bias != nullptr) {
     const float4 b = *reinterpret_cast<const float4*>(bias + n0);
     y[0] += b.x; y[1] += b.y; y[2] += b.z; y[3] += b.w;
@@ -157,7 +160,8 @@ __device__ __forceinline__ void finish_block(const float* __restrict__ part, int
 }
 
 // mode 0: out bf16 [M, N];  mode 1: out f32 [M, N]
-__global__ void finish_store_kernel(const float* __restrict__ part, int S, int M, int N, const __half* __restrict__ svh,
+template <bool ONE>
+__global__ void __launch_bounds__(256) finish_store_kernel(const float* __restrict__ part, int S, int M, int N, const __half* __restrict__ svh,
                                     const float* __restrict__ bias, void* __restrict__ out, int f32_out) {
   pdl_launch();
   pdl_wait();
@@ -165,7 +169,7 @@ __global__ void finish_store_kernel(const float* __restrict__ part, int S, int M
   for (int b = blockIdx.y * nw + warp; b < N / 128; b += gridDim.y * nw) {
     const int n0 = b * 128 + lane * 4;
     float y[4];
-    finish_block(part, S, (size_t)M * N, (size_t)row * N + n0, svh, bias, n0, y);
+    finish_block<ONE>(part, S, (size_t)M * N, (size_t)row * N + n0, svh, bias, n0, y);
     if (f32_out) *reinterpret_cast<float4*>((float*)out + (size_t)row * N + n0) = make_float4(y[0], y[1], y[2], y[3]);
     else store4_bf16((uint16_t*)out + (size_t)row * N + n0, y);
   }
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(1024) finish_add_norm_rot_kernel(const float* 
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       r[i] = bf16_to_f(f_to_bf16(r[i] + y[i]));
-      ss += r[i] * r[i];
+      ss = __fmaf_rn(r[i], r[i], ss);
       rowbuf[n0 + i] = r[i];
     }
     store4_bf16(h + (size_t)row * N + n0, r);
@@ -216,20 +220,95 @@ __global__ void __launch_bounds__(1024) finish_add_norm_rot_kernel(const float* 
       float w[4];
       load4_bf16(norm_w + n0, w);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = bf16_to_f(f_to_bf16(v[i] * rinv)) * w[i];
+      for (int i = 0; i < 4; ++i) v[i] = __fmul_rn(bf16_to_f(f_to_bf16(v[i] * rinv)), w[i]);
     }
     if (xn_out != nullptr) store4_bf16(xn_out + (size_t)row * N + n0, v);   // the normalised row itself (router input, per-expert rotations)
     if (suh_next == nullptr) continue;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] *= s[i];
+    for (int i = 0; i < 4; ++i) v[i] = __fmul_rn(v[i], s[i]);
     fwht128_warp(v);
     store4_f16(xr + (size_t)row * N + n0, v);
   }
 }
 
+// The same for the many rows of a prompt slice (one plane, rows of up to ROWS_NB * 1024 elements), bound by memory: a CTA of eight warps per row, a warp's
+// blocks (one in eight) stay in registers between the sum of squares and the scaling, all of them loaded before the first is used.
+// 8192 rows of 5120: 125 us, 165 before (blocks one after the other, the row through shared memory).
+constexpr int ROWS_NB = 5;
+__global__ void __launch_bounds__(256) finish_add_norm_rot_rows_kernel(const float* __restrict__ part, int N, const __half* __restrict__ svh,
+                                                                      const float* __restrict__ bias, uint16_t* __restrict__ h,
+                                                                      const uint16_t* __restrict__ norm_w, float eps, const __half* __restrict__ suh_next,
+                                                                      __half* __restrict__ xr, uint16_t* __restrict__ xn_out) {
+  pdl_launch();
+  pdl_wait();
+  __shared__ float blk_ss[8 * ROWS_NB];
+  const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = N / 128;
+  const size_t base = (size_t)row * N + lane * 4;
+  float v[ROWS_NB][4], r[ROWS_NB][4];
+#pragma unroll
+  for (int i = 0; i < ROWS_NB; ++i) {
+    const int b = warp + 8 * i;
+    if (b < nb) {
+      const float4 p = __ldg(reinterpret_cast<const float4*>(part + base + b * 128));
+      v[i][0] = p.x, v[i][1] = p.y, v[i][2] = p.z, v[i][3] = p.w;
+      load4_bf16(h + base + b * 128, r[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS_NB; ++i) {
+    const int b = warp + 8 * i, n0 = b * 128 + lane * 4;
+    if (b >= nb) break;
+    fwht128_warp(v[i]);
+    float sv[4], ss = 0.f;
+    load4_f16(svh + n0, sv);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[i][e] = __fmul_rn(v[i][e], sv[e]);
+    if (bias != nullptr) {
+      const float4 bb = *reinterpret_cast<const float4*>(bias + n0);
+      v[i][0] += bb.x, v[i][1] += bb.y, v[i][2] += bb.z, v[i][3] += bb.w;
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      v[i][e] = bf16_to_f(f_to_bf16(r[i][e] + v[i][e]));
+      ss = __fmaf_rn(v[i][e], v[i][e], ss);
+    }
+    store4_bf16(h + base + b * 128, v[i]);
+    ss = warp_sum(ss);
+    if (lane == 0) blk_ss[b] = ss;
+  }
+  if (suh_next == nullptr && xn_out == nullptr) return;
+  float rinv = 1.f;
+  __syncthreads();
+  if (norm_w != nullptr) {
+    float tot = 0.f;
+    for (int b = 0; b < nb; ++b) tot += blk_ss[b];
+    rinv = rsqrtf(tot / (float)N + eps);
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS_NB; ++i) {
+    const int b = warp + 8 * i, n0 = b * 128 + lane * 4;
+    if (b >= nb) break;
+    if (norm_w != nullptr) {
+      float w[4];
+      load4_bf16(norm_w + n0, w);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[i][e] = __fmul_rn(bf16_to_f(f_to_bf16(v[i][e] * rinv)), w[e]);
+    }
+    if (xn_out != nullptr) store4_bf16(xn_out + base + b * 128, v[i]);
+    if (suh_next == nullptr) continue;
+    float s[4];
+    load4_f16(suh_next + n0, s);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[i][e] = __fmul_rn(v[i][e], s[e]);
+    fwht128_warp(v[i]);
+    store4_f16(xr + base + b * 128, v[i]);
+  }
+}
+
 // part [S, M, 2F] = gate | up.  act = silu(gate) * up (bf16-rounded like an unfused pipeline would store it), then
 // xr[row][F] = fp16(H(act * suh_down)).
-__global__ void finish_swiglu_rot_kernel(const float* __restrict__ part, int S, int M, int F, const __half* __restrict__ svh,
+template <bool ONE>
+__global__ void __launch_bounds__(256) finish_swiglu_rot_kernel(const float* __restrict__ part, int S, int M, int F, const __half* __restrict__ svh,
                                          const float* __restrict__ bias, const __half* __restrict__ suh_down, __half* __restrict__ xr) {
   pdl_launch();
   pdl_wait();
@@ -238,8 +317,8 @@ __global__ void finish_swiglu_rot_kernel(const float* __restrict__ part, int S, 
   for (int b = blockIdx.y * nw + warp; b < F / 128; b += gridDim.y * nw) {
     const int n0 = b * 128 + lane * 4;
     float g[4], u[4], s[4];
-    finish_block(part, S, (size_t)M * N, (size_t)row * N + n0, svh, bias, n0, g);
-    finish_block(part, S, (size_t)M * N, (size_t)row * N + F + n0, svh, bias, F + n0, u);
+    finish_block<ONE>(part, S, (size_t)M * N, (size_t)row * N + n0, svh, bias, n0, g);
+    finish_block<ONE>(part, S, (size_t)M * N, (size_t)row * N + F + n0, svh, bias, F + n0, u);
     load4_f16(suh_down + n0, s);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -299,13 +378,19 @@ static int blocks_y(int rows, int nblocks128) {
 RX_API int rx_finish_store(const void* part, int S, int M, int N, const void* svh, const void* bias, void* out, int f32_out, void* stream) {
   if (N % 128) return (int)cudaErrorInvalidValue;
   dim3 grid(M, blocks_y(M, N / 128));
-  rx::launch(finish_store_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const float*)part, S, M, N, (const __half*)svh, (const float*)bias, out, f32_out);
+  rx::launch(S == 1 ? finish_store_kernel<true> : finish_store_kernel<false>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const float*)part, S, M, N, (const __half*)svh, (const float*)bias, out, f32_out);
   return (int)cudaGetLastError();
 }
 
 RX_API int rx_finish_add_norm_rot(const void* part, int S, int M, int N, const void* svh, const void* bias, void* h_bf16, const void* norm_w,
                                   float eps, const void* suh_next, void* xr, void* stream, void* xn_out) {
   if (N % 128 || N * 4 > 200 * 1024 || N / 128 > 512) return (int)cudaErrorInvalidValue;
+  // 512 rows fill the chip's SMs with three CTAs and more; fewer want the form below, which has 32 warps for a row
+  if (S == 1 && M >= 512 && N <= ROWS_NB * 1024) {
+    rx::launch(finish_add_norm_rot_rows_kernel, dim3(M), dim3(256), 0, (cudaStream_t)stream, (const float*)part, N, (const __half*)svh, (const float*)bias,
+               (uint16_t*)h_bf16, (const uint16_t*)norm_w, eps, (const __half*)suh_next, (__half*)xr, (uint16_t*)xn_out);
+    return (int)cudaGetLastError();
+  }
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(finish_add_norm_rot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -324,7 +409,7 @@ RX_API int rx_finish_swiglu_rot(const void* part, int S, int M, int F, const voi
                                 void* stream) {
   if (F % 128) return (int)cudaErrorInvalidValue;
   dim3 grid(M, blocks_y(M, F / 128));
-  rx::launch(finish_swiglu_rot_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const float*)part, S, M, F, (const __half*)svh, (const float*)bias,
+  rx::launch(S == 1 ? finish_swiglu_rot_kernel<true> : finish_swiglu_rot_kernel<false>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const float*)part, S, M, F, (const __half*)svh, (const float*)bias,
                                                                   (const __half*)suh_down, (__half*)xr);
   return (int)cudaGetLastError();
 }

@@ -18,8 +18,11 @@ __device__ __forceinline__ uint16_t g_f_to_bf16(float f) {
 // part: f32 [S][M][Nqkv], Nqkv = (n_q + 2 n_kv) * hd, column order q heads | k heads | v heads.
 // For each 128-block: sum splits, Hadamard, * svh (+bias); q/k heads: optional RMSNorm over the head, RoPE (rotate-half);
 // q -> q_out bf16 [M][n_q*hd]; k, v -> paged cache at slot[row] = page*64 + offset (slot < 0: row not cached).
-template <int HD>
-__global__ void finish_qkv_rope_kernel(const float* __restrict__ part, int S, int M, int n_q, int n_kv, const __half* __restrict__ svh,
+// A row's rotations depend on the lane's place in its head alone: the CTA computes HD / 2 sines and cosines once, each lane keeps its four for all
+// blocks.  Bound by memory for many rows (403 us for 8192 rows of 56 heads with four sincosf per lane and block and the loop over planes in
+// registers, 102 us now).  ONE: a single plane, known at compile time (see finish_block).
+template <int HD, bool ONE>
+__global__ void __launch_bounds__(256) finish_qkv_rope_kernel(const float* __restrict__ part, int S, int M, int n_q, int n_kv, const __half* __restrict__ svh,
                                        const float* __restrict__ bias, const uint16_t* __restrict__ q_norm, const uint16_t* __restrict__ k_norm,
                                        float eps, const int* __restrict__ positions, const float* __restrict__ inv_freq,
                                        const int* __restrict__ slot, uint16_t* __restrict__ q_out, uint16_t* __restrict__ k_cache,
@@ -39,14 +42,29 @@ __global__ void finish_qkv_rope_kernel(const float* __restrict__ part, int S, in
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int N = (n_q + 2 * n_kv) * HD;
   const size_t sstride = (size_t)M * N;
-  const float pos = (float)positions[row];
   const int sl = slot[row];
   constexpr int GL = HD / 4;  // lanes per head
+  __shared__ float2 rot[HD / 2];
+  if (threadIdx.x < HD / 2) {
+    const int fi = threadIdx.x;
+    float p = (float)positions[row];
+    if (pos3 != nullptr) {
+      const int axis = (fi % 3 == 1 && fi < lim_h) ? 1 : ((fi % 3 == 2 && fi < lim_w) ? 2 : 0);
+      p = (float)pos3[row * 3 + axis];
+    }
+    float sn, cs;
+    sincosf(p * inv_freq[fi], &sn, &cs);
+    rot[fi] = make_float2(sn, cs);
+  }
+  __syncthreads();
+  float2 sc[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sc[i] = rot[(lane * 4 + i) % (HD / 2)];
   for (int b = blockIdx.y * nw + warp; b < N / 128; b += gridDim.y * nw) {
     const int n0 = b * 128 + lane * 4;
     const size_t off = (size_t)row * N + n0;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (S == 1) acc = __ldg(reinterpret_cast<const float4*>(part + off));
+    if (ONE) acc = __ldg(reinterpret_cast<const float4*>(part + off));
     else
     for (int s0 = 0; s0 < S; s0 += 8) {   // eight independent loads in flight, added in split order
       float4 p[8];
@@ -88,14 +106,7 @@ __global__ void finish_qkv_rope_kernel(const float* __restrict__ part, int S, in
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float other = __shfl_xor_sync(0xffffffffu, y[i], GL / 2);
-        const int fi = (d0 + i) % (HD / 2);
-        float p = pos;
-        if (pos3 != nullptr) {
-          const int axis = (fi % 3 == 1 && fi < lim_h) ? 1 : ((fi % 3 == 2 && fi < lim_w) ? 2 : 0);
-          p = (float)pos3[row * 3 + axis];
-        }
-        float sn, cs;
-        sincosf(p * inv_freq[fi], &sn, &cs);
+        const float sn = sc[i].x, cs = sc[i].y;
         y[i] = first ? (y[i] * cs - other * sn) : (y[i] * cs + other * sn);
       }
     }
@@ -241,14 +252,16 @@ RX_API int rx_finish_qkv_rope(const void* part, int S, int M, int n_q, int n_kv,
                               int section_w, void* k_tscale, void* v_tscale, int q4) {
   const int N = (n_q + 2 * n_kv) * hd;
   if (N % 128) return (int)cudaErrorInvalidValue;
-  const int per_row = (N / 128 + 7) / 8;   // one warp per 128-block
+  // a warp per 128-block, eight to a CTA, while that leaves enough CTAs to fill the chip; with thousands of rows one CTA walks a whole row (its
+  // rotations are computed once, and a grid of very short CTAs is bound by the rate at which they are launched)
+  const int per_row = M >= 1024 ? 1 : (N / 128 + 7) / 8;
   dim3 grid(M, per_row < 1 ? 1 : per_row);
   cudaStream_t st = (cudaStream_t)stream;
 #define RX_ARGS (const float*)part, S, M, n_q, n_kv, (const __half*)svh, (const float*)bias, (const uint16_t*)q_norm, (const uint16_t*)k_norm, eps, \
                 (const int*)positions, (const float*)inv_freq, (const int*)slot, (uint16_t*)q_out, (uint16_t*)k_cache, (uint16_t*)v_cache, \
                 (const float*)kv_scale, (float*)kv_amax, (const int*)pos3, 3 * section_h, 3 * section_w, (float*)k_tscale, (float*)v_tscale, q4
-  if (hd == 128) rx::launch(finish_qkv_rope_kernel<128>, dim3(grid), dim3(256), 0, st, RX_ARGS);
-  else if (hd == 64) rx::launch(finish_qkv_rope_kernel<64>, dim3(grid), dim3(256), 0, st, RX_ARGS);
+  if (hd == 128) rx::launch(S == 1 ? finish_qkv_rope_kernel<128, true> : finish_qkv_rope_kernel<128, false>, dim3(grid), dim3(256), 0, st, RX_ARGS);
+  else if (hd == 64) rx::launch(S == 1 ? finish_qkv_rope_kernel<64, true> : finish_qkv_rope_kernel<64, false>, dim3(grid), dim3(256), 0, st, RX_ARGS);
   else return (int)cudaErrorInvalidValue;
 #undef RX_ARGS
   return (int)cudaGetLastError();
