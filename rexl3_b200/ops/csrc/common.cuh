@@ -228,7 +228,7 @@ __host__ __device__ constexpr uint32_t umma_idesc_f16(int m, int n, int a_fmt, i
 }
 
 // ---------------------------------------------------------------- programmatic dependent launch
-// Every kernel of this library is launched with programmatic stream serialization allowed: a kernel calls pdl_launch() at its
+// The kernels of this library are launched with programmatic stream serialization allowed (exceptions below): a kernel calls pdl_launch() at its
 // start (the next kernel in the stream may begin its prologue, e.g. stream its weights) and pdl_wait() before it touches
 // anything the previous kernel wrote.  pdl_wait() returns once the previous kernel has fully completed and flushed.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -236,16 +236,32 @@ __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.laun
 
 inline int& pdl_enabled() { static int on = 1; return on; }
 
+// Grids of more than PDL_MAX_CTAS CTAs (two per SM) are launched plainly: their CTAs, waiting, hold the slots of a predecessor with several waves or
+// a long tail, which costs more than the launch latency that is saved.  Measured with the limit at 296 / without one: MoE prompt slice of 2100 rows
+// 3.41 / 3.90 ms (the gather's 16,800 CTAs beside the one-CTA plan), verify window of 80 rows 2.20 / 2.27 ms, step of 64 rows 2.14 / 2.18 ms; limits
+// between 600 and 20,000 only helped the first.
+constexpr long long PDL_MAX_CTAS = 296;
+
 template <typename... P, typename... A>
-inline cudaError_t launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+inline cudaError_t launch_pdl(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = early && pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  return launch_pdl((long long)grid.x * grid.y * grid.z <= PDL_MAX_CTAS, kern, grid, block, smem, st, args...);
+}
+// For kernels whose CTAs run long and must be spread evenly over the SMs: begun early they land wherever the predecessor leaves a slot (the Mamba2
+// scan: two CTAs on most SMs when begun alone; a prompt slice of 2047 rows on seven layers takes 12.6 ms, begun early 14.1 ms).
+template <typename... P, typename... A>
+inline cudaError_t launch_alone(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  return launch_pdl(false, kern, grid, block, smem, st, args...);
 }
 
 // ---------------------------------------------------------------- small math helpers

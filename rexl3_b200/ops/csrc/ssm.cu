@@ -850,7 +850,7 @@ RX_API int rx_ssm_mixer(const void* proj, int ldp, int M, int H, int P, int G, i
   if (mode & SCAN_OUT)
     launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
   if (seg_start != nullptr && (((uintptr_t)xbc) & 15) == 0)     // segments known on the host (prefill, commit); its copies take 16 bytes
-    launch(ssm_scan_split_kernel, dim3(nseg, H, SSM_PS), dim3(128), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
+    launch_alone(ssm_scan_split_kernel, dim3(nseg, H, SSM_PS), dim3(128), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
            (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len, (const float*)dt_bias, (const float*)a_neg,
            (const float*)d_skip, (float*)ssm_pool, (float*)conv_pool, (float*)y, mode);
   else
@@ -882,7 +882,7 @@ RX_API int rx_gdn_mixer(const void* proj, int ldp, int M, int Hk, int Hv, int D,
     launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
   if (seg_start != nullptr && y32 != nullptr && ((((uintptr_t)xbc) | ((uintptr_t)y32)) & 15) == 0) {
     // segments known on the host (prefill, commit): the column-split scan with prefetched inputs, then the norm (same bits as the fused kernel)
-    launch(kda ? gdn_scan_split_kernel<true> : gdn_scan_split_kernel<false>, dim3(nseg, Hv, GDN_JS), dim3(128), 0, st, (const float*)xbc, C,
+    launch_alone(kda ? gdn_scan_split_kernel<true> : gdn_scan_split_kernel<false>, dim3(nseg, Hv, GDN_JS), dim3(128), 0, st, (const float*)xbc, C,
            (const float*)proj, ldp, xoff, goff, M, Hk, Hv, (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len,
            (const float*)dt_bias, (const float*)a_neg, (float*)s_pool, (float*)conv_pool, (float*)y32, mode);
     if (mode & SCAN_OUT)
