@@ -225,14 +225,14 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const float* __restrict__
     for (int i = 0; i < 32; i += 4) {
       const float4 bb = *reinterpret_cast<const float4*>(sB + nq * 32 + i), cc = *reinterpret_cast<const float4*>(sC + nq * 32 + i);
       // (the roundings are spelled out: the split kernel below repeats them, so that a commit leaves the bits of a direct run)
-      st[i] = __fmaf_rn(st[i], dA, __fmul_rn(xdt, bb.x)); st[i + 1] = __fmaf_rn(st[i + 1], dA, __fmul_rn(xdt, bb.y));
-      st[i + 2] = __fmaf_rn(st[i + 2], dA, __fmul_rn(xdt, bb.z)); st[i + 3] = __fmaf_rn(st[i + 3], dA, __fmul_rn(xdt, bb.w));
-      a0 += st[i] * cc.x; a1 += st[i + 1] * cc.y; a2 += st[i + 2] * cc.z; a3 += st[i + 3] * cc.w;
+      st[i] = __fmaf_rn(xdt, bb.x, __fmul_rn(st[i], dA)); st[i + 1] = __fmaf_rn(xdt, bb.y, __fmul_rn(st[i + 1], dA));
+      st[i + 2] = __fmaf_rn(xdt, bb.z, __fmul_rn(st[i + 2], dA)); st[i + 3] = __fmaf_rn(xdt, bb.w, __fmul_rn(st[i + 3], dA));
+      a0 = __fmaf_rn(st[i], cc.x, a0); a1 = __fmaf_rn(st[i + 1], cc.y, a1); a2 = __fmaf_rn(st[i + 2], cc.z, a2); a3 = __fmaf_rn(st[i + 3], cc.w, a3);
     }
     float acc = (a0 + a1) + (a2 + a3);
     acc += __shfl_xor_sync(0xffffffffu, acc, 1);
     acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    if (nq == 0 && (mode & SCAN_OUT)) y[(size_t)r * DI + h * SSM_P + p] = acc + Dh * sx[p];
+    if (nq == 0 && (mode & SCAN_OUT)) y[(size_t)r * DI + h * SSM_P + p] = __fmaf_rn(Dh, sx[p], acc);
   }
   if (!(mode & SCAN_STATE)) return;
 #pragma unroll
@@ -240,18 +240,21 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const float* __restrict__
   ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h, (int)gridDim.y);
 }
 
-// Prefill / commit form of the recurrence, bound by the multiply pipe: three fp32 operations per state value and token, of which the two with three
-// register operands issue at two thirds of the pipe's rate.  A head's 64 state rows p are split over two CTAs of four warps; a thread holds a
-// 4 (p) x 8 (n) tile of the state, so that B and C cost a token four vector loads from shared memory for 96 operations (a 1 x 32 tile needs
-// sixteen; a 4 x 4 tile on twice the warps is bound by those loads again: 506 us).  Products are packed pairs along n.  The inputs of SSM_TC tokens at a
-// time come by cp.async into two buffers, x dt and the decays are made from them by the CTA: two block barriers per SSM_TC tokens, no global load on
-// the per-token path.  State values are rounded exactly as in ssm_scan_kernel (fma(S, dA, (x dt) B)), so both leave the same bits; a token's output
-// is summed over n in this kernel's own fixed order (8 in sequence, then a tree over 16 lanes).  The dependents are released only when the recurrence
-// is done: released at the start, their waiting CTAs (thousands) took the SMs' slots and slowed it by half.
-// One sequence of 2047 tokens, 128 heads: 436 us; 2159 us before (1 x 32 tiles, one warp per CTA, register ring; 3220 us with early release).
+// Prefill / commit form of the recurrence, bound by the multiply pipe and by issue: three fp32 operations per state value and token.  A head's 64
+// state rows p are split over two CTAs of four warps; a thread holds four rows of every fourth n of a quarter (n = 32 nq + 4 m + k, m = 0 .. 7), so
+// that B and C cost a token four vector loads from shared memory for 96 operations (a 1 x 32 tile needs sixteen) and a thread's share of an
+// output is one of the sixteen chains that ssm_scan_kernel adds up.  Every rounding and every order of a sum is that kernel's: states and outputs
+// are the same bits.  (Packed pairs along n took 436 us, 463 us this way: what they save in issue slots is small, two of the three operations
+// read three registers, which the packed form issues every third cycle; a 4 x 4 tile on twice the warps is bound by the loads again: 506 us.)
+// The inputs of SSM_TC tokens at a time come by cp.async into two buffers, x dt and the decays are made from them by the CTA: two block barriers per
+// SSM_TC tokens, no global load on the per-token path.  The dependents are released only when the recurrence is done: released at the start, their
+// waiting CTAs (thousands) took the SMs' slots and slowed it by half.
+// One sequence of 2047 tokens, 128 heads: 463 us; 2159 us before (1 x 32 tiles, one warp per CTA, register ring; 3220 us with early release).
 // grid (segments, H, SSM_PS), 128 threads.
 constexpr int SSM_PS = 2, SSM_CP = SSM_P / SSM_PS, SSM_TC = 16;
 struct SsmChunk { float B[SSM_TC][SSM_N], C[SSM_TC][SSM_N], x[SSM_TC][SSM_CP], dt[SSM_TC]; };
+// where n stands in a token's B and C: the eight values of a thread (nq, k) as two vectors, sixteen threads' vectors side by side
+__device__ __forceinline__ int ssm_place(int n) { return ((n >> 4) & 1) * 64 + ((n >> 5) * 4 + (n & 3)) * 4 + ((n >> 2) & 3); }
 __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
                                                             int dtoff, int M, int H, int G, const int* __restrict__ row_seq,
                                                             const int* __restrict__ positions, const int* __restrict__ seg_start,
@@ -260,31 +263,30 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
                                                             float* __restrict__ ssm_pool, float* conv_pool, float* __restrict__ y, int mode) {
   pdl_wait();
   __shared__ __align__(16) SsmChunk buf[2];
-  __shared__ __align__(16) uint64_t xdt2[SSM_TC][SSM_CP], dec2[SSM_TC];      // x dt and the decay of the current chunk, both halves of a pair alike
+  __shared__ float xdt[SSM_TC][SSM_CP], dec[SSM_TC];                         // x dt and the decay of the current chunk
   const int r0 = seg_start[blockIdx.x], len = seg_len[blockIdx.x];
   if (len <= 0) return;
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ln = lane & 15, lp = lane >> 4;
   const int seq = row_seq[r0], g = h / (H / G), DI = H * SSM_P, p0 = blockIdx.z * SSM_CP;
-  // Slot k of a thread is state row pl + (k ^ sel) with sel from lane bits 3 and 2: what a lane passes on in the output sums' tree is then always
-  // its upper slots, without selects.
-  const int pl = warp * 8 + lp * 4, sel = (ln & 8 ? 2 : 0) | (ln & 4 ? 1 : 0);
-  uint64_t st[4][4];                                // [slot][pair of n]: n = 4 ln + {0, 1}, {2, 3}, then 64 more
-  float* sp = ssm_pool + (((size_t)seq * H + h) * SSM_P + p0 + pl) * SSM_N + 4 * ln;
+  // Slot i of a thread is state row pl + (i ^ sel) with sel from lane bits 0 and 1: what a lane passes on in the output sums' tree is then always its
+  // upper slots, without selects.
+  const int pl = warp * 8 + lp * 4, sel = (ln & 1 ? 2 : 0) | (ln & 2 ? 1 : 0);
+  float st[4][8];
+  float* sp = ssm_pool + (((size_t)seq * H + h) * SSM_P + p0 + pl) * SSM_N + (ln >> 2) * 32 + (ln & 3);
+  const bool fresh = positions[r0] == 0;
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
+  for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      ulonglong2 v = make_ulonglong2(0ull, 0ull);
-      if (positions[r0] != 0) v = *reinterpret_cast<const ulonglong2*>(sp + (p ^ sel) * SSM_N + 64 * k);
-      st[p][2 * k] = v.x, st[p][2 * k + 1] = v.y;
-    }
-  }
+    for (int m = 0; m < 8; ++m) st[p][m] = fresh ? 0.f : sp[(p ^ sel) * SSM_N + 4 * m];
+  const int place = ssm_place(tid);
   auto issue = [&](int c) {                         // tokens c * SSM_TC ..; past the end the last row again (never used)
     SsmChunk& d = buf[c & 1];
-    for (int t = warp; t < SSM_TC; t += 4) {
-      const float* xr = xbc + (size_t)(r0 + min(c * SSM_TC + t, len - 1)) * C;
-      cp16(&d.B[t][4 * lane], xr + DI + g * SSM_N + 4 * lane);
-      cp16(&d.C[t][4 * lane], xr + DI + (G + g) * SSM_N + 4 * lane);
+    const float* src = xbc + DI + g * SSM_N + tid;
+#pragma unroll
+    for (int t = 0; t < SSM_TC; ++t) {
+      const float* xr = src + (size_t)(r0 + min(c * SSM_TC + t, len - 1)) * C;
+      cp4(&d.B[t][place], xr);
+      cp4(&d.C[t][place], xr + G * SSM_N);
     }
     const int t = tid >> 3;
     cp16(&d.x[t][4 * (tid & 7)], xbc + (size_t)(r0 + min(c * SSM_TC + t, len - 1)) * C + h * SSM_P + p0 + 4 * (tid & 7));
@@ -292,47 +294,45 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
     cp_commit();
   };
   const float A = a_neg[h], Dh = d_skip[h], dtb = dt_bias[h];
-  const bool b1 = (ln & 2) != 0, b0 = (ln & 1) != 0;
+  const bool b2 = (ln & 4) != 0, b3 = (ln & 8) != 0;
   float* yp = y + h * SSM_P + p0 + pl + sel;        // slot 0's row: the one whose sums end in this lane
   // NT tokens (4, or 1 at the end): the states in turn, then all NT x 4 output sums over the 16 lanes together, each step halving what a lane
-  // carries on.  A sum's tree over the lanes (distances 8, 4, 2, 1) does not depend on NT.
+  // carries on.  A sum's tree over the lanes (distances 1, 2, 4, 8) does not depend on NT.
   auto tokens = [&](const SsmChunk& d, auto n, int t0, int r) {
     constexpr int NT = decltype(n)::value;
     float k[NT];
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       const int t = t0 + i;
-      const ulonglong2 B0 = *reinterpret_cast<const ulonglong2*>(&d.B[t][4 * ln]), B1 = *reinterpret_cast<const ulonglong2*>(&d.B[t][64 + 4 * ln]);
-      const ulonglong2 C0 = *reinterpret_cast<const ulonglong2*>(&d.C[t][4 * ln]), C1 = *reinterpret_cast<const ulonglong2*>(&d.C[t][64 + 4 * ln]);
-      const uint64_t dA2 = dec2[t];
-      float o[4];
+      const float4 B0 = *reinterpret_cast<const float4*>(&d.B[t][4 * ln]), B1 = *reinterpret_cast<const float4*>(&d.B[t][64 + 4 * ln]);
+      const float4 C0 = *reinterpret_cast<const float4*>(&d.C[t][4 * ln]), C1 = *reinterpret_cast<const float4*>(&d.C[t][64 + 4 * ln]);
+      const float b[8] = {B0.x, B0.y, B0.z, B0.w, B1.x, B1.y, B1.z, B1.w}, c[8] = {C0.x, C0.y, C0.z, C0.w, C1.x, C1.y, C1.z, C1.w};
+      const float dA = dec[t];
+      float xd[4], o[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const uint64_t xd2 = xdt2[t][pl + (p ^ sel)];
-        st[p][0] = f2_fma(st[p][0], dA2, f2_mul(xd2, B0.x));
-        st[p][1] = f2_fma(st[p][1], dA2, f2_mul(xd2, B0.y));
-        st[p][2] = f2_fma(st[p][2], dA2, f2_mul(xd2, B1.x));
-        st[p][3] = f2_fma(st[p][3], dA2, f2_mul(xd2, B1.y));
-        uint64_t a = f2_mul(st[p][0], C0.x);
-        a = f2_fma(st[p][1], C0.y, a);
-        a = f2_fma(st[p][2], C1.x, a);
-        a = f2_fma(st[p][3], C1.y, a);
-        o[p] = f2_sum(a);
-      }
-      const float k0 = o[0] + __shfl_xor_sync(0xffffffffu, o[2], 8), k1 = o[1] + __shfl_xor_sync(0xffffffffu, o[3], 8);
-      k[i] = k0 + __shfl_xor_sync(0xffffffffu, k1, 4);
+      for (int p = 0; p < 4; ++p) xd[p] = xdt[t][pl + (p ^ sel)];
+#pragma unroll
+      for (int m = 0; m < 8; ++m)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          st[p][m] = __fmaf_rn(xd[p], b[m], __fmul_rn(st[p][m], dA));
+          o[p] = __fmaf_rn(st[p][m], c[m], o[p]);
+        }
+      const float k0 = o[0] + __shfl_xor_sync(0xffffffffu, o[2], 1), k1 = o[1] + __shfl_xor_sync(0xffffffffu, o[3], 1);
+      k[i] = k0 + __shfl_xor_sync(0xffffffffu, k1, 2);
     }
     if (!(mode & SCAN_OUT)) return;
-    if constexpr (NT == 4) {                        // lane bits 1 and 0 pick the token
-      const float m0 = (b1 ? k[2] : k[0]) + __shfl_xor_sync(0xffffffffu, b1 ? k[0] : k[2], 2);
-      const float m1 = (b1 ? k[3] : k[1]) + __shfl_xor_sync(0xffffffffu, b1 ? k[1] : k[3], 2);
-      const float m = (b0 ? m1 : m0) + __shfl_xor_sync(0xffffffffu, b0 ? m0 : m1, 1);
-      yp[(size_t)(r + (ln & 3)) * DI] = __fmaf_rn(Dh, d.x[t0 + (ln & 3)][pl + sel], m);
+    if constexpr (NT == 4) {                        // lane bits 2 and 3 pick the token
+      const float m0 = (b2 ? k[2] : k[0]) + __shfl_xor_sync(0xffffffffu, b2 ? k[0] : k[2], 4);
+      const float m1 = (b2 ? k[3] : k[1]) + __shfl_xor_sync(0xffffffffu, b2 ? k[1] : k[3], 4);
+      const float m = (b3 ? m1 : m0) + __shfl_xor_sync(0xffffffffu, b3 ? m0 : m1, 8);
+      const int t = (b2 ? 2 : 0) + (b3 ? 1 : 0);
+      yp[(size_t)(r + t) * DI] = __fmaf_rn(Dh, d.x[t0 + t][pl + sel], m);
     } else {
       float m = k[0];
-      m += __shfl_xor_sync(0xffffffffu, m, 2);
-      m += __shfl_xor_sync(0xffffffffu, m, 1);
-      if ((ln & 3) == 0) yp[(size_t)r * DI] = __fmaf_rn(Dh, d.x[t0][pl + sel], m);
+      m += __shfl_xor_sync(0xffffffffu, m, 4);
+      m += __shfl_xor_sync(0xffffffffu, m, 8);
+      if (!b2 && !b3) yp[(size_t)r * DI] = __fmaf_rn(Dh, d.x[t0][pl + sel], m);
     }
   };
   issue(0);
@@ -346,12 +346,9 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
       const int t = tid >> 3, p = 4 * (tid & 7);    // eight threads per token
       float dt = d.dt[t] + dtb;
       dt = dt > 20.f ? dt : log1pf(__expf(dt));     // softplus
-      const float dA = __expf(dt * A);
       const float4 x = *reinterpret_cast<const float4*>(&d.x[t][p]);
-      const float xd[4] = {x.x * dt, x.y * dt, x.z * dt, x.w * dt};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) xdt2[t][p + e] = f2_pack(xd[e], xd[e]);
-      if (p == 0) dec2[t] = f2_pack(dA, dA);
+      xdt[t][p] = x.x * dt, xdt[t][p + 1] = x.y * dt, xdt[t][p + 2] = x.z * dt, xdt[t][p + 3] = x.w * dt;
+      if (p == 0) dec[t] = __expf(dt * A);
     }
     __syncthreads();
     const int nt = min(SSM_TC, len - c * SSM_TC);
@@ -364,16 +361,14 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
 #pragma unroll
   for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-      *reinterpret_cast<ulonglong2*>(sp + (p ^ sel) * SSM_N + 64 * k) = make_ulonglong2(st[p][2 * k], st[p][2 * k + 1]);
+    for (int m = 0; m < 8; ++m) sp[(p ^ sel) * SSM_N + 4 * m] = st[p][m];
   ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h * SSM_PS + blockIdx.z, (int)(gridDim.y * SSM_PS));
 }
 
-// out[r][c] = bf16( rmsnorm_group( y * silu(z) )[c] * w[c] ), grid (M, G); the group is d_inner / G channels wide.  Bound by memory: a thread takes
-// four neighbouring channels at a time and keeps the gated values of the first 1024 channels in registers between the sum and the scaling (read
-// and gated twice, channel by channel, it took 68 us for 2047 rows of 8 x 1024 channels, 46 us now); a wider group is gated again beyond that.
-// VEC: width and alignment allow the vectors; else the four channels are loaded one by one.  A channel is added to the same partial sum either way.
-template <bool VEC>
+// out[r][c] = bf16( rmsnorm_group( y * silu(z) )[c] * w[c] ), grid (M, G); the group is d_inner / G channels wide.  Bound by memory: a thread's
+// first GN_KEEP channels stay in registers between the sum and the scaling (loaded together; read and gated twice, one after the other, it took
+// 68 us for 2047 rows of 8 x 1024 channels, 46 us now); a wider group is gated again beyond that.
+constexpr int GN_KEEP = 4;
 __global__ void __launch_bounds__(256) ssm_gate_norm_kernel(const float* __restrict__ y, const float* __restrict__ proj, int ldp, int DI, int G,
                                                            const uint16_t* __restrict__ norm_w, float eps, uint16_t* __restrict__ out) {
   pdl_launch();
@@ -382,28 +377,21 @@ __global__ void __launch_bounds__(256) ssm_gate_norm_kernel(const float* __restr
   const int r = blockIdx.x, g = blockIdx.y, W = DI / G, c0 = g * W;
   const float* yr = y + (size_t)r * DI + c0;
   const float* zr = proj + (size_t)r * ldp + c0;
-  auto gated = [&](int c, float (&v)[4]) {
-    float a[4], z[4];
-    if (VEC) {
-      const float4 p = *reinterpret_cast<const float4*>(yr + c), q = *reinterpret_cast<const float4*>(zr + c);
-      a[0] = p.x, a[1] = p.y, a[2] = p.z, a[3] = p.w, z[0] = q.x, z[1] = q.y, z[2] = q.z, z[3] = q.w;
-    } else {
+  float keep[GN_KEEP], z[GN_KEEP], ss = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) a[e] = c + e < W ? yr[c + e] : 0.f, z[e] = c + e < W ? zr[c + e] : 0.f;
-    }
+  for (int i = 0; i < GN_KEEP; ++i) {
+    const int c = threadIdx.x + 256 * i;
+    keep[i] = c < W ? yr[c] : 0.f;
+    z[i] = c < W ? zr[c] : 0.f;
+  }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = a[e] * ssm_silu(z[e]);
-  };
-  float keep[4] = {0.f, 0.f, 0.f, 0.f}, ss = 0.f;
-  const int c1 = 4 * threadIdx.x;
-  if (c1 < W) gated(c1, keep);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) ss = __fmaf_rn(keep[e], keep[e], ss);
-  for (int c = c1 + 1024; c < W; c += 1024) {
-    float v[4];
-    gated(c, v);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) ss = __fmaf_rn(v[e], v[e], ss);
+  for (int i = 0; i < GN_KEEP; ++i) {
+    keep[i] = __fmul_rn(keep[i], ssm_silu(z[i]));
+    ss = __fmaf_rn(keep[i], keep[i], ss);
+  }
+  for (int c = threadIdx.x + 256 * GN_KEEP; c < W; c += 256) {
+    const float v = __fmul_rn(yr[c], ssm_silu(zr[c]));
+    ss = __fmaf_rn(v, v, ss);
   }
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
@@ -412,21 +400,14 @@ __global__ void __launch_bounds__(256) ssm_gate_norm_kernel(const float* __restr
 #pragma unroll
   for (int i = 0; i < 8; ++i) tot += red[i];
   const float rinv = rsqrtf(tot / (float)W + eps);
-  for (int c = c1; c < W; c += 1024) {
-    float v[4];
-    if (c == c1) v[0] = keep[0], v[1] = keep[1], v[2] = keep[2], v[3] = keep[3];
-    else gated(c, v);
-    uint16_t b[4];
+  auto put = [&](int c, float v) {
+    __nv_bfloat16 b = __float2bfloat16_rn(v * rinv * ssm_bf(norm_w[c0 + c]));
+    out[(size_t)r * DI + c0 + c] = *reinterpret_cast<uint16_t*>(&b);
+  };
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      __nv_bfloat16 t = __float2bfloat16_rn(v[e] * rinv * (VEC || c + e < W ? ssm_bf(norm_w[c0 + c + e]) : 0.f));
-      b[e] = *reinterpret_cast<uint16_t*>(&t);
-    }
-    uint16_t* op = out + (size_t)r * DI + c0 + c;
-    if (VEC) *reinterpret_cast<uint2*>(op) = make_uint2(b[0] | ((uint32_t)b[1] << 16), b[2] | ((uint32_t)b[3] << 16));
-    else
-      for (int e = 0; e < 4 && c + e < W; ++e) op[e] = b[e];
-  }
+  for (int i = 0; i < GN_KEEP; ++i)
+    if (threadIdx.x + 256 * i < W) put(threadIdx.x + 256 * i, keep[i]);
+  for (int c = threadIdx.x + 256 * GN_KEEP; c < W; c += 256) put(c, yr[c] * ssm_silu(zr[c]));
 }
 
 // ------------------------------------------------------------------------------------------------ gated delta net
@@ -857,11 +838,9 @@ RX_API int rx_ssm_mixer(const void* proj, int ldp, int M, int H, int P, int G, i
   launch(ssm_scan_kernel, dim3(seg_start ? nseg : M, H), dim3(256), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
          (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len, (const float*)dt_bias, (const float*)a_neg,
          (const float*)d_skip, (float*)ssm_pool, (float*)conv_pool, (float*)y, mode);
-  if (mode & SCAN_OUT) {
-    const bool vec = (DI / G) % 4 == 0 && ldp % 4 == 0 && ((((uintptr_t)y) | ((uintptr_t)proj)) & 15) == 0 && (((uintptr_t)out_bf16) & 7) == 0;
-    launch(vec ? ssm_gate_norm_kernel<true> : ssm_gate_norm_kernel<false>, dim3(M, G), dim3(256), 0, st, (const float*)y, (const float*)proj, ldp, DI, G,
-           (const uint16_t*)norm_w, eps, (uint16_t*)out_bf16);
-  }
+  if (mode & SCAN_OUT)
+    launch(ssm_gate_norm_kernel, dim3(M, G), dim3(256), 0, st, (const float*)y, (const float*)proj, ldp, DI, G, (const uint16_t*)norm_w, eps,
+           (uint16_t*)out_bf16);
   return (int)cudaGetLastError();
 }
 

@@ -1,4 +1,4 @@
-"""The prefill forms of the recurrent mixers against the per-row forms: the same bits of states (and, for the delta nets, of outputs)."""
+"""The prefill forms of the recurrent mixers against the per-row forms: the same bits of states and outputs."""
 import pytest
 import torch
 
@@ -56,11 +56,8 @@ def test_mamba_prefill_equals_row_form(lens, H, G, pad):
         conv, pool, out = conv0.clone(), s0.clone(), torch.zeros(M, DI, dtype=torch.bfloat16, device="cuda")
         K.ssm_mixer(proj, M, H, P, G, N, seq, pos, *seg, *args, 1e-6, conv, pool, torch.empty(M * C, device="cuda"), torch.empty(M * DI, device="cuda"), out)
         got.append((out.float(), conv, pool))
-    assert torch.equal(got[0][1], got[1][1]) and torch.equal(got[0][2], got[1][2])
-    # outputs: two fp32 sums of 128 terms in different orders (128 x 2^-24 of the terms' size), rounded to bf16: one unit in the last place (2^-7)
-    # of an output, or of the terms that cancelled in it (rows are normed, so terms are of size one)
-    a, b = got[0][0], got[1][0]
-    assert torch.isfinite(a).all() and ((a - b).abs() <= 2.0 ** -7 * b.abs() + 1e-4).all()
+    for a, b in zip(*got):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
 
 
 def test_conv_walking_rows_equals_one_row_per_thread():
