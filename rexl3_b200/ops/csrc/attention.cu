@@ -74,8 +74,8 @@ __device__ __forceinline__ void load_kv_page(uint8_t* kdst, uint8_t* vdst, const
   }
 }
 
-// FP8 (E4M3) cache: a page of one KV head is 64 x HD bytes, loaded unswizzled, then expanded by the whole CTA to an fp16 tile in the
-// swizzled layout the fragment loads expect.  E4M3 -> fp16 is exact; the per-head scale is applied to the scores / the output.
+// FP8 (E4M3) cache: a page of one KV head is 64 x HD bytes; outside the decode kernel for it (attn_decode_f8_kernel) it is expanded by the whole CTA
+// to an fp16 tile in the swizzled layout the fragment loads expect.  E4M3 -> fp16 is exact; the per-head scale is applied to the scores / the output.
 template <int HD>
 __device__ __forceinline__ void load_kv_page8(uint8_t* kdst, uint8_t* vdst, const CUtensorMap* tk, const CUtensorMap* tv, int page, int kvh,
                                               int n_kv, uint64_t* bar) {
@@ -107,6 +107,10 @@ __device__ __forceinline__ void load_kv_page_i8(uint8_t* kdst, uint8_t* vdst, fl
   bulk_g2s(sc + PAGE, v_ts + (size_t)y, PAGE * 4, bar);
 }
 
+// Where the 16 bytes of chunk j of a key stand in a byte page: rows of 128 bytes are loaded with the 128-byte swizzle (rx_make_kv_tmap8).
+template <int HD>
+__device__ __forceinline__ int byte_chunk(int key, int j) { return key * HD + ((HD == 128 ? j ^ (key & 7) : j) << 4); }
+
 // sc != nullptr: the bytes are int8 and sc[key] is the key's scale (else: E4M3 bytes)
 template <int HD>
 __device__ __forceinline__ void expand_page8(const uint8_t* src, uint8_t* dst, const float* sc = nullptr) {
@@ -114,7 +118,7 @@ __device__ __forceinline__ void expand_page8(const uint8_t* src, uint8_t* dst, c
   const uint32_t dbase = smem_u32(dst);
   for (int c = threadIdx.x; c < CHUNKS; c += blockDim.x) {
     const int key = c / (HD / 16), j = c % (HD / 16);
-    const uint4 r = *reinterpret_cast<const uint4*>(src + (size_t)c * 16);
+    const uint4 r = *reinterpret_cast<const uint4*>(src + byte_chunk<HD>(key, j));
     const uint32_t w[4] = {r.x, r.y, r.z, r.w};
     uint32_t h[8];
     if (sc != nullptr) {
@@ -272,10 +276,64 @@ __device__ __forceinline__ void attn_step(const uint32_t (&qa)[HD / 16][4], uint
 }
 
 
+// Scores of one m16 tile against 16 keys -> probabilities as the A fragment of P.V.  valid_lo / valid_hi: keys the lane's two rows may see.  A row's
+// running maximum is only moved when the new scores exceed it by more than 2^8 (the sums and accumulators are then rescaled; otherwise the stale
+// maximum stays and P holds values up to 256, well inside bf16 / fp16 range), so the 64 multiplies of the rescale are skipped for most pages.
+template <bool F16, int NO>
+__device__ __forceinline__ void attn_softmax16(float (&s)[2][4], int valid_lo, int valid_hi, float scale_log2, float (&m)[2], float (&l)[2],
+                                               float (&o)[NO][4], uint32_t (&pa)[4]) {
+  const int lane = threadIdx.x & 31;
+  float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int kk = j * 8 + 2 * (lane & 3) + (e & 1);
+      const float v = (kk < (e < 2 ? valid_lo : valid_hi)) ? s[j][e] * scale_log2 : -INFINITY;
+      s[j][e] = v;
+      mx[e >> 1] = fmaxf(mx[e >> 1], v);
+    }
+  }
+  float corr[2];
+  bool moved = false;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+    mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+    corr[r] = 1.f;
+    if (mx[r] > m[r] + 8.f) {                      // also the first valid keys of a row (m = -inf)
+      corr[r] = (m[r] == -INFINITY) ? 1.f : exp2f(m[r] - mx[r]);
+      m[r] = mx[r];
+      moved = moved || corr[r] != 1.f;
+    }
+  }
+  float rs[2] = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    float p[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float mm = m[e >> 1];
+      p[e] = (mm == -INFINITY) ? 0.f : exp2f(s[j][e] - mm);
+      rs[e >> 1] += p[e];
+    }
+    pa[j * 2 + 0] = F16 ? pack_f16(p[0], p[1]) : pack_bf16(p[0], p[1]);
+    pa[j * 2 + 1] = F16 ? pack_f16(p[2], p[3]) : pack_bf16(p[2], p[3]);
+  }
+  if (__any_sync(0xffffffffu, moved)) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) l[r] *= corr[r];
+#pragma unroll
+    for (int d = 0; d < NO; ++d) {
+      o[d][0] *= corr[0]; o[d][1] *= corr[0]; o[d][2] *= corr[1]; o[d][3] *= corr[1];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) l[r] += rs[r];
+}
+
 // The decode kernel's step: like attn_step for MT tiles at once over the same 16 keys.  Each K / V fragment is fetched from shared memory once
-// and feeds every tile's MMA; a row's running maximum is only moved when the new scores exceed it by more than 2^8 (the accumulators are then
-// rescaled; otherwise the stale maximum stays and P holds values up to 256, well inside bf16 / fp16 range), so the 64 multiplies of the
-// rescale are skipped for most pages.  `ntiles` (uniform) = tiles that hold a live row.
+// and feeds every tile's MMA.  `ntiles` (uniform) = tiles that hold a live row.
 template <int HD, int MT, bool F16>
 __device__ __forceinline__ void attn_step_mt(const uint32_t (&qa)[MT][HD / 16][4], uint32_t ksm, uint32_t vsm, int key0, const int (&valid)[MT][2],
                                              int ntiles, float scale_log2, float (&m)[MT][2], float (&l)[MT][2], float (&o)[MT][HD / 8][4]) {
@@ -303,58 +361,8 @@ __device__ __forceinline__ void attn_step_mt(const uint32_t (&qa)[MT][HD / 16][4
   }
   uint32_t pa[MT][4];
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    if (mt < ntiles) {
-      // mask + row max
-      float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int kk = j * 8 + 2 * (lane & 3) + (e & 1);
-          const float v = (kk < valid[mt][e >> 1]) ? s[mt][j][e] * scale_log2 : -INFINITY;
-          s[mt][j][e] = v;
-          mx[e >> 1] = fmaxf(mx[e >> 1], v);
-        }
-      }
-      float corr[2];
-      bool moved = false;
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-        corr[r] = 1.f;
-        if (mx[r] > m[mt][r] + 8.f) {              // also the first valid keys of a row (m = -inf)
-          corr[r] = (m[mt][r] == -INFINITY) ? 1.f : exp2f(m[mt][r] - mx[r]);
-          m[mt][r] = mx[r];
-          moved = moved || corr[r] != 1.f;
-        }
-      }
-      float rs[2] = {0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        float p[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float mm = m[mt][e >> 1];
-          p[e] = (mm == -INFINITY) ? 0.f : exp2f(s[mt][j][e] - mm);
-          rs[e >> 1] += p[e];
-        }
-        pa[mt][j * 2 + 0] = F16 ? pack_f16(p[0], p[1]) : pack_bf16(p[0], p[1]);
-        pa[mt][j * 2 + 1] = F16 ? pack_f16(p[2], p[3]) : pack_bf16(p[2], p[3]);
-      }
-      if (__any_sync(0xffffffffu, moved)) {
-#pragma unroll
-        for (int r = 0; r < 2; ++r) l[mt][r] *= corr[r];
-#pragma unroll
-        for (int d = 0; d < HD / 8; ++d) {
-          o[mt][d][0] *= corr[0]; o[mt][d][1] *= corr[0]; o[mt][d][2] *= corr[1]; o[mt][d][3] *= corr[1];
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 2; ++r) l[mt][r] += rs[r];
-    }
-  }
+  for (int mt = 0; mt < MT; ++mt)
+    if (mt < ntiles) attn_softmax16<F16>(s[mt], valid[mt][0], valid[mt][1], scale_log2, m[mt], l[mt], o[mt], pa[mt]);
   {
     const int mi = lane >> 3;
     const int key = key0 + (mi & 1) * 8 + (lane & 7);
@@ -673,6 +681,252 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
   }
 }
 
+// E4M3 cache with 128-wide heads.  Same work items and masks as attn_decode_kernel, bound by HBM instead of by the expansion (that kernel turns every page
+// into fp16 tiles in shared memory, between two block barriers per page: 182 us for 6 sequences x 32,100 keys, 394 MB, where this one takes
+// 87 us).  A warp takes one whole page of the item's four: it is its own producer (two tiles, K and V; the next item's page is fetched into a
+// tile as soon as the warp has read it), needs no block barrier before the merge and no running maximum, and its MMAs run in eight
+// and more independent chains (one 16-key slice of every page per warp left it waiting for MMA latencies: 143 us).  The bytes go straight
+// into the fragments: the order of the head's 128 values along the MMAs' k (scores) and n (outputs) is free, so a lane takes 32 neighbouring bytes of
+// a K row and 16 of a V row, and a conversion of two bytes is a fragment register (V: after a byte permute that pairs two keys).  A block of
+// more than 16 (row, head) pairs goes over the page once per m16 tile, with the same instructions for every tile: a row's bits depend on
+// neither its tile nor its block mates.  A failed wait does not leave the loop (warps meet at barriers): every later wait then returns at once.
+constexpr int F8_TILE = PAGE * 128, F8_HDP = 128 + 8;
+constexpr int F8_SMEM = 8 * F8_TILE + 4 * 16 * F8_HDP * 4 + 2 * 4 * 16 * 2 * 4 + 8 * 8 + 16 + 1024;
+// four bytes -> two fp16 pairs
+__device__ __forceinline__ void f8x4_to_f16x4(uint32_t b, uint32_t& lo, uint32_t& hi) {
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}" : "=r"(lo), "=r"(hi) : "r"(b));
+}
+__global__ void __launch_bounds__(ATT_THREADS, 2)
+attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const uint16_t* __restrict__ q,
+                      const int* __restrict__ block_table, int max_blocks, const int* __restrict__ ctx_len, float* __restrict__ part_o,
+                      float* __restrict__ part_ml, int n_q, int n_kv, int max_chunks, float scale_log2_in, int* status,
+                      const float* __restrict__ kv_scale, const int* __restrict__ plan, const int* __restrict__ vbt) {
+  constexpr int HD = 128, HDP = F8_HDP;
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  uint8_t *ktile = smem + warp * 2 * F8_TILE, *vtile = ktile + F8_TILE;
+  float* sm_o = (float*)(smem + 8 * F8_TILE);                           // [page][16][HDP]: one tile's partial outputs
+  float* sm_ml2 = sm_o + 4 * 16 * HDP;                                  // two of [page][16][2], tiles in turn
+  uint64_t* bars = (uint64_t*)(sm_ml2 + 2 * 4 * 16 * 2);                // K and V tile of each warp
+  uint64_t *full_k = bars + 2 * warp, *full_v = full_k + 1;
+  volatile int* abort_flag = (volatile int*)(bars + 8);
+  const int G = n_q / n_kv;
+  const int total = plan[0], nb = plan[1];
+  const int* blk_row = plan + PLAN_HEAD;
+  const int* blk_n = blk_row + PLAN_MAX_ROWS;
+  const int* prefix = blk_n + 2 * PLAN_MAX_ROWS;
+  const int* blk_seq = prefix + PLAN_MAX_ROWS + 1;
+  const int* blk_c0 = blk_seq + PLAN_MAX_ROWS;
+  if ((int)blockIdx.x >= total) return;
+  if (tid == 0) {
+    for (int i = 0; i < 8; ++i) mbar_init(&bars[i], 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  __syncthreads();
+  struct Item { int row, nblk, kvh, chunk, k_begin, k_end, y; };         // y: first row of this warp's page in the tensor maps, -1: no such page
+  int blk = 0;
+  // items come in ascending order: the block that holds the next one is this one's or a little further
+  auto locate = [&](int item) {
+    Item it;
+    while (blk + 1 < nb && prefix[blk + 1] <= item) ++blk;
+    const int local = item - prefix[blk], seq = blk_seq[blk], c0 = blk_c0[blk];
+    it.row = blk_row[blk], it.nblk = blk_n[blk], it.kvh = local % n_kv, it.chunk = c0 + local / n_kv;
+    int ctx_max = 0;
+    for (int i = 0; i < it.nblk; ++i) ctx_max = max(ctx_max, ctx_len[it.row + i]);
+    it.k_begin = it.chunk * DEC_CHUNK;
+    it.k_end = min(ctx_max, it.k_begin + DEC_CHUNK);
+    // a tree row's private table starts at the page index of its block's first chunk
+    const int* bt = seq >= 0 ? block_table + (size_t)seq * max_blocks : vbt + (size_t)(-1 - seq) * VBT_W - c0 * (DEC_CHUNK / PAGE);
+    it.y = it.k_begin + warp * PAGE < it.k_end ? (bt[it.k_begin / PAGE + warp] * n_kv + it.kvh) * PAGE : -1;
+    return it;
+  };
+  auto fetch = [&](uint8_t* dst, const CUtensorMap* map, int y, uint64_t* bar) {
+    mbar_arrive_expect_tx(bar, F8_TILE);
+    tma_load_2d(dst, map, 0, y, bar);
+  };
+  Item it = locate(blockIdx.x);
+  if (lane == 0 && it.y >= 0) {
+    fetch(ktile, &tk, it.y, full_k);
+    fetch(vtile, &tv, it.y, full_v);
+  }
+  uint32_t qa[8][4];
+  int pages = 0, par = 0, q_row = -1, q_kvh = -1, q_nblk = 0;            // pages: consumed so far by this warp; q_*: whose queries qa holds
+  for (int item = blockIdx.x; item < total; item += gridDim.x) {
+    Item next;
+    next.y = -1;
+    if (item + (int)gridDim.x < total) next = locate(item + gridDim.x);
+    const float scale_log2 = scale_log2_in * kv_scale[it.kvh], v_scale = kv_scale[n_kv + it.kvh];     // K was stored as k / k_scale
+    const int ntiles = (it.nblk * G + 15) >> 4, kpos = it.k_begin + warp * PAGE;
+    const bool any = it.y >= 0;                      // uniform for the warp
+    for (int mt = 0; mt < ntiles; ++mt) {
+      const int rows = min(16, it.nblk * G - 16 * mt);
+      int valid[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int t = mt * 16 + g + 8 * r, rb = t / G;
+        valid[r] = rb < it.nblk ? ctx_len[it.row + rb] - kpos : 0;
+      }
+      if (ntiles > 1 || it.row != q_row || it.kvh != q_kvh || it.nblk != q_nblk) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int t = mt * 16 + g + 8 * r, rb = t / G, hh = t % G;
+          const bool live = rb < it.nblk;
+          const uint4* qr = reinterpret_cast<const uint4*>(q + ((size_t)(it.row + (live ? rb : 0)) * n_q + (size_t)it.kvh * G + hh) * HD + 32 * t4);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {             // this lane's 32 values of the head, four to a k step
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (live) v = qr[i];
+            qa[2 * i][r] = bf16x2_to_f16x2(v.x), qa[2 * i][2 + r] = bf16x2_to_f16x2(v.y);
+            qa[2 * i + 1][r] = bf16x2_to_f16x2(v.z), qa[2 * i + 1][2 + r] = bf16x2_to_f16x2(v.w);
+          }
+        }
+        q_row = it.row, q_kvh = it.kvh, q_nblk = it.nblk;
+      }
+      float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[16][4];
+#pragma unroll
+      for (int d = 0; d < 16; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
+      if (any) {
+        float sc[8][4];
+        if (mt == 0) mbar_wait(full_k, pages & 1, abort_flag, status, 50);
+        const uint32_t ks = smem_u32(ktile), vs = smem_u32(vtile);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          uint4 w[2][2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) w[u][h] = lds128(ks + byte_chunk<HD>(8 * (j + u) + g, 2 * t4 + h));
+#pragma unroll
+          for (int u = 0; u < 2; ++u) sc[j + u][0] = sc[j + u][1] = sc[j + u][2] = sc[j + u][3] = 0.f;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const uint4 c = w[u][k >> 2];
+              uint32_t b0, b1;
+              f8x4_to_f16x4((k & 3) == 0 ? c.x : (k & 3) == 1 ? c.y : (k & 3) == 2 ? c.z : c.w, b0, b1);
+              mma_f16(sc[j + u], qa[k], b0, b1);
+            }
+        }
+        if (mt == ntiles - 1) {                      // the K tile has been read: the next item's page may come
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0 && next.y >= 0) fetch(ktile, &tk, next.y, full_k);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int kk = j * 8 + 2 * t4 + (e & 1);
+            const float v = kk < valid[e >> 1] ? sc[j][e] * scale_log2 : -INFINITY;
+            sc[j][e] = v;
+            m[e >> 1] = fmaxf(m[e >> 1], v);
+          }
+        float sub[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], 1));
+          m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], 2));
+          sub[r] = m[r] == -INFINITY ? 0.f : m[r];   // a row that may see none of these keys: all its scores are -inf
+        }
+        if (mt == 0) mbar_wait(full_v, pages & 1, abort_flag, status, 51);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          uint4 vw[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) vw[j] = lds128(vs + byte_chunk<HD>(16 * kk + 8 * (j >> 1) + 2 * t4 + (j & 1), g));
+          uint32_t pa[4];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            float pr[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              pr[e] = exp2f(sc[2 * kk + j][e] - sub[e >> 1]);
+              l[e >> 1] += pr[e];
+            }
+            pa[2 * j] = pack_f16(pr[0], pr[1]);
+            pa[2 * j + 1] = pack_f16(pr[2], pr[3]);
+          }
+          const uint32_t va[4][4] = {{vw[0].x, vw[0].y, vw[0].z, vw[0].w}, {vw[1].x, vw[1].y, vw[1].z, vw[1].w},
+                                     {vw[2].x, vw[2].y, vw[2].z, vw[2].w}, {vw[3].x, vw[3].y, vw[3].z, vw[3].w}};
+#pragma unroll
+          for (int i = 0; i < 4; ++i)                // output column n of MMA 4 i + e = value 16 n + 4 i + e of the head
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t b0[2], b1[2];
+              f8x4_to_f16x4(__byte_perm(va[0][i], va[1][i], h ? 0x7362 : 0x5140), b0[0], b0[1]);
+              f8x4_to_f16x4(__byte_perm(va[2][i], va[3][i], h ? 0x7362 : 0x5140), b1[0], b1[1]);
+              mma_f16(o[4 * i + 2 * h], pa, b0[0], b1[0]);
+              mma_f16(o[4 * i + 2 * h + 1], pa, b0[1], b1[1]);
+            }
+        }
+        if (mt == ntiles - 1) {
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0 && next.y >= 0) fetch(vtile, &tv, next.y, full_v);
+        }
+      } else if (mt == ntiles - 1 && lane == 0 && next.y >= 0) {
+        fetch(ktile, &tk, next.y, full_k);
+        fetch(vtile, &tv, next.y, full_v);
+      }
+      // merge the four pages: every page's partial rescaled to the row's maximum over them, then added in page order
+      float* sm_ml = sm_ml2 + par * 4 * 16 * 2;
+      par ^= 1;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+        l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+        if (t4 == 0) sm_ml[(warp * 16 + g + 8 * r) * 2] = m[r];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        if (g + 8 * r >= rows) continue;
+        float mm = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, sm_ml[(w * 16 + g + 8 * r) * 2]);
+        const float f = m[r] == -INFINITY ? 0.f : exp2f(m[r] - mm);
+        if (t4 == 0) sm_ml[(warp * 16 + g + 8 * r) * 2 + 1] = l[r] * f;
+        float* base = sm_o + (warp * 16 + g + 8 * r) * HDP + 2 * t4;  // [row][MMA d][column n]
+#pragma unroll
+        for (int d = 0; d < 16; ++d) *reinterpret_cast<float2*>(base + d * 8) = make_float2(o[d][2 * r] * f, o[d][2 * r + 1] * f);
+      }
+      __syncthreads();
+      // thread = (row, column n, four MMAs): the four values are taken in an order of their own per thread group, which keeps the banks apart
+      for (int idx = tid; idx < rows * 32; idx += ATT_THREADS) {
+        const int tr = idx >> 5, n = idx & 7, i = (idx >> 3) & 3, t = 16 * mt + tr, rb = t / G, hq = t % G;
+        if (ctx_len[it.row + rb] <= it.k_begin) continue;             // this chunk lies beyond that row's context: nothing of it is ever read
+        const size_t pidx = ((size_t)(it.row + rb) * n_q + (size_t)it.kvh * G + hq) * max_chunks + it.chunk;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int e = (u + i) & 3;
+          const float* src = sm_o + tr * HDP + (4 * i + e) * 8 + n;
+          const float acc = ((src[0] + src[16 * HDP]) + src[32 * HDP]) + src[48 * HDP];
+          part_o[pidx * HD + 16 * n + 4 * i + e] = acc * v_scale;
+        }
+        if ((idx & 31) == 0) {
+          float mm = -INFINITY, lsum = 0.f;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            mm = fmaxf(mm, sm_ml[(w * 16 + tr) * 2]);
+            lsum += sm_ml[(w * 16 + tr) * 2 + 1];
+          }
+          part_ml[pidx * 2] = mm;
+          part_ml[pidx * 2 + 1] = lsum;
+        }
+      }
+    }
+    if (any) ++pages;
+    it = next;
+  }
+}
+
+// Loads in flight per lane of the merge, which is bound by their latency: 6 rows x 126 chunks took 23.6 us with four, 12.3 us with sixteen.
+constexpr int MERGE_LOADS = 16;
 // Merge chunk partials in chunk order -> attention output; then (suh != nullptr) xr = fp16(H(out * suh)) per 128-block
 // (the o_proj input rotation), else plain bf16 output.  One warp per 128 output elements.
 template <int HD>
@@ -689,7 +943,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
     const size_t base = ((size_t)row * n_q + hq) * max_chunks;
     // GL chunks at a time (GL = lanes that share this head): lane c of the group fetches chunk c's (max, sum), the group reduces
     // the max, then every lane walks the chunks in order with the factors broadcast by shuffle and the partial-output loads
-    // issued four at a time
+    // issued MERGE_LOADS at a time
     constexpr int GL = HD / 4 < 32 ? HD / 4 : 32;
     const int gl = lane % GL, gbase = lane - gl;
     float mm = -INFINITY;
@@ -706,13 +960,13 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
       const float l_l = in ? part_ml[(base + c0 + gl) * 2 + 1] : 0.f;
       const float f_l = (m_l == -INFINITY) ? 0.f : exp2f(m_l - mm);
       const int cnt = min(GL, nch - c0);
-      for (int j0 = 0; j0 < cnt; j0 += 4) {
-        float4 p[4];
+      for (int j0 = 0; j0 < cnt; j0 += MERGE_LOADS) {
+        float4 p[MERGE_LOADS];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < MERGE_LOADS; ++j)
           if (j0 + j < cnt) p[j] = *reinterpret_cast<const float4*>(part_o + (base + c0 + j0 + j) * HD + d0);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < MERGE_LOADS; ++j) {
           const int src = gbase + ((j0 + j) % GL);
           const float f = __shfl_sync(0xffffffffu, f_l, src), ll = __shfl_sync(0xffffffffu, l_l, src);
           if (j0 + j < cnt) {
@@ -904,7 +1158,9 @@ RX_API int rx_make_kv_tmap(void* out128, const void* base, long long total_rows,
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-// Tensor map of an FP8 (E4M3) cache [num_pages][n_kv][64][hd] viewed as bytes [num_pages*n_kv*64, hd]; one page of one head is one box.
+// Tensor map of an FP8 (E4M3) cache [num_pages][n_kv][64][hd] viewed as bytes [num_pages*n_kv*64, hd]; one page of one head is one box.  Rows of
+// 128 bytes are swizzled on the way into shared memory (16-byte chunk j of row r lands at j ^ (r % 8)): the decode kernel's fragment loads, four
+// rows at one column, then meet different banks.
 RX_API int rx_make_kv_tmap8(void* out128, const void* base, long long total_rows, int hd) {
   EncodeTiledFn enc = att_encode_tiled();
   if (enc == nullptr) return (int)cudaErrorNotSupported;
@@ -914,7 +1170,8 @@ RX_API int rx_make_kv_tmap8(void* out128, const void* base, long long total_rows
   cuuint32_t box[2] = {(cuuint32_t)hd, PAGE};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc((CUtensorMap*)out128, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, hd == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
@@ -960,6 +1217,22 @@ template <int HD, bool FP8, int MT, int I8>
 static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, const void* q, const int* bt, int max_blocks, const int* row_seq,
                                 const int* ctx_len, float* part_o, float* part_ml, int rows, int n_q, int n_kv, int mc, float scale, int* status,
                                 cudaStream_t st, const float* kv_scale, const int* plan, const float* k_ts, const float* v_ts, const int* vbt) {
+  // persistent: two CTAs per SM at most, never more than the items the window can have
+  const long long bound = (long long)rows * n_kv * mc;
+  const int grid = (int)(bound < 2 * sm_count() ? bound : 2 * sm_count());
+  if constexpr (HD == 128 && FP8 && I8 == 0) {
+    if ((((uintptr_t)q) & 15) == 0) {               // its queries come in 16-byte pieces
+      static bool ready = false;
+      if (!ready) {
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_f8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F8_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        ready = true;
+      }
+      rx::launch(attn_decode_f8_kernel, dim3(grid), dim3(ATT_THREADS), F8_SMEM, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, ctx_len, part_o, part_ml,
+                 n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, vbt);
+      return (int)cudaGetLastError();
+    }
+  }
   constexpr int smem = dec_smem_bytes(HD, FP8, MT);
   static bool configured = false;
   if (!configured) {
@@ -967,9 +1240,6 @@ static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, co
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  // persistent: two CTAs per SM at most, never more than the items the window can have
-  const long long bound = (long long)rows * n_kv * mc;
-  const int grid = (int)(bound < 2 * sm_count() ? bound : 2 * sm_count());
   rx::launch(attn_decode_kernel<HD, FP8, MT, I8>, dim3(grid), dim3(ATT_THREADS), smem, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, row_seq,
              ctx_len, part_o, part_ml, n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, k_ts, v_ts, vbt);
   return (int)cudaGetLastError();
@@ -998,9 +1268,7 @@ static int launch_decode(const CUtensorMap* tk, const CUtensorMap* tv, const voi
 #undef RX_DEC_T
   if (e != 0) return e;
   const int blocks128 = n_q * HD / 128;
-  int gy = (296 + rows - 1) / rows;
-  if (gy > (blocks128 + 3) / 4) gy = (blocks128 + 3) / 4;
-  if (gy < 1) gy = 1;
+  const int gy = (blocks128 + 3) / 4;              // a warp per 128 outputs
   rx::launch(attn_merge_kernel<HD>, dim3(dim3(rows, gy)), dim3(128), 0, st, part_o, part_ml, ctx_len, n_q, mc, (const __half*)suh, (__half*)xr, (uint16_t*)out_bf16);
   return (int)cudaGetLastError();
 }
