@@ -354,6 +354,11 @@ static int launch_gemm(const CUtensorMap& tm, const uint32_t* trellis, float* pa
   return (int)cudaGetLastError();
 }
 
+// the persistent kernel of exl3_gemm_grouped.cu
+bool gemm_persistent_takes(int K, int twice, int splits, int brows);
+int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits,
+                    const int* tile_tab, int max_tiles, int brows, int* status, cudaStream_t st);
+
 }  // namespace rx
 
 using namespace rx;
@@ -411,6 +416,9 @@ RX_API int rx_exl3_gemm_grouped(const void* xs, int pairs_cap, int K, const void
   if (pairs_cap <= 0 || K % 128 != 0 || N % 128 != 0 || splits < 1 || splits > K / KCH || max_tiles < 1 || max_tiles > 65535) return (int)cudaErrorInvalidValue;
   if (tile_rows != rx_exl3_tile_rows(tile_rows) || (expert_elems % 2) != 0) return (int)cudaErrorInvalidValue;
   if ((((uintptr_t)xs) & 15) != 0 || (((uintptr_t)trellis) & 15) != 0) return (int)cudaErrorMisalignedAddress;
+  if (gemm_persistent_takes(K, twice, splits, tile_rows) && expert_elems % 8 == 0)
+    return gemm_persistent(xs, pairs_cap, K, trellis, (size_t)expert_elems / 2, N, twice, codebook, part, splits, (const int*)tile_tab, max_tiles, tile_rows,
+                           status, (cudaStream_t)stream);
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xs, (uint64_t)pairs_cap, (uint64_t)K, (uint32_t)tile_rows);
   if (e != 0) return e;

@@ -1,0 +1,316 @@
+// EXL3 GEMM over a list of (expert, row tile) pairs, 3.0 and 4.0 bpw, decoded weights in TENSOR MEMORY (sm_100a).  Contract of the grouped form in
+// exl3_gemm.cu: part[split][row][n] = partial sums of xs @ W_q[expert], rows sorted by expert, tile_tab[t] = {expert, first row, rows}, live
+// tiles first.  Without a table the tiles are those of a plain GEMM.
+//
+// Bound by the trellis decode (two integer pipes, see exl3_decode.cuh).  Decode as in exl3_gemm_tm.cu: a thread owns one of the strip's 128 columns
+// (one TMEM lane) and emits its k-values as packed fp16 pairs, the MMA reads A from tensor memory and the activations from shared memory.
+// What is different is the schedule: the work items of a routed window are many and short (tile x 128-column strip x K split: 4 chunks of
+// 128 k), so the CTAs are PERSISTENT and every ring runs on across items - the weights of the next item stream in while this one is decoded -
+// and the accumulator is double buffered, its epilogue done by one decode group while the others go on.  One CTA per item in exl3_gemm.cu
+// spent most of its life in its prologue and on shared-memory traffic of the decoded tile: 16 rows x 8 picks of 128 experts (2048 -> 1536 and
+// 768 -> 2048, 3.0 bpw) took XOLD us for both products, XNEW us here.
+//
+// Warp roles: 0 weight producer (one bulk copy per k-tile row), 1 TMEM owner + MMA issuer, 2 activation producer, then NG decode groups of 4 warps.
+// Group e % NG writes out item e, after its first chunk of a later item: the accumulator of item e is needed again by item e + 2 only, whose
+// first MMA waits for it.  No circle of waits: that chunk's A stage was last read by a chunk of item e or before.  Every wait is bounded.
+#include <cuda.h>
+#include "exl3_decode.cuh"
+
+namespace rx {
+
+constexpr int GR_KCH = 128, GR_STRIP = 128, GR_OP_STAGES = 3, GR_RAW_STAGES = 8;
+constexpr int GR_A_COLS = GR_KCH / 2;             // TMEM columns of one A stage (two fp16 per column)
+constexpr int GR_ROLE_WARPS = 3;
+// A decode group waits for "the MMA that last read this stage": sound while no group can run two phases ahead, i.e. with as many stages as groups.
+__host__ __device__ constexpr int gr_a_stages(int ng) { return ng; }
+__host__ __device__ constexpr int gr_acc_cols(int brows) { return brows < 32 ? 32 : brows; }
+__host__ __device__ inline int gr_smem_bytes(int brows, int twice) { return GR_OP_STAGES * brows * 256 + GR_RAW_STAGES * 1024 * twice + 512; }
+
+// One k-tile (16 k) of a thread's column: 8 packed pairs, regs[m] = k (2m, 2m + 1), regs[4 + m] = k (8 + 2m, 9 + 2m).
+// w[0] = the word before the thread's eighth of the tile, w[1..] = the eighth's words; b2: which of its two columns (see exl3_decode.cuh).
+template <int TWICE, int CB>
+__device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1], int b2, uint32_t* regs) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    uint32_t s0, s1, s2, s3;
+    if constexpr (TWICE == 8) {
+      // b2 = 0: the 4 values that straddle the word boundary; b2 = 1: the word's own 4
+      const uint32_t X = __funnelshift_lc(w[m + 1], w[m], b2 ? 32u : 16u);
+      extract4<CB != CB_MUL1>(X, s0, s1, s2, s3);
+    } else {
+      // windows start at bit 19 + 24 m + 12 b2 + 3 i of w: 25 bits from the first one's start hold all four
+      static_assert(TWICE == 6, "widths of this kernel: 3.0 and 4.0 bpw");
+      const int bit0 = 19 + 24 * m, bit1 = 31 + 24 * m;
+      const uint32_t hi = bit0 / 32 == bit1 / 32 ? w[bit0 / 32] : (b2 ? w[bit1 / 32] : w[bit0 / 32]);
+      const uint32_t lo0 = w[bit0 / 32 + 1], lo1 = bit1 / 32 + 1 <= TWICE / 2 ? w[bit1 / 32 + 1 <= TWICE / 2 ? bit1 / 32 + 1 : 0] : 0u;
+      const uint32_t lo = bit0 / 32 == bit1 / 32 ? lo0 : (b2 ? lo1 : lo0);
+      const uint32_t X = __funnelshift_l(lo, hi, b2 ? bit1 % 32 : bit0 % 32);
+      s0 = X >> 16;
+      s1 = (X >> 13) & 0xFFFFu;
+      const uint32_t x2 = X >> 10, x3 = X >> 7;
+      s2 = CB != CB_MUL1 ? low16_mul(x2) : x2 & 0xFFFFu;        // (the multiply pipe has room for two of the masks)
+      s3 = CB != CB_MUL1 ? low16_mul(x3) : x3 & 0xFFFFu;
+    }
+    regs[m] = pair_to_half2<CB>(s0, s1);
+    regs[4 + m] = pair_to_half2<CB>(s2, s3);
+  }
+}
+
+template <int TWICE, int CB, int NG>
+__global__ void __launch_bounds__(GR_ROLE_WARPS * 32 + NG * 128, (NG <= 3 ? 2 : 1))
+exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __restrict__ trellis, size_t expert_words,
+                         float* __restrict__ part, int rows, int K, int N, int splits, int brows, const int* __restrict__ tile_tab, int max_tiles,
+                         int* status) {
+  pdl_launch();
+  constexpr int SA = gr_a_stages(NG), EW = TWICE / 2;            // EW: words of an eighth of a tile
+  constexpr int TILE_WORDS = 4 * TWICE, ROW_BYTES = 8 * TILE_WORDS * 4, RAW_STAGE = 8 * ROW_BYTES;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int b_half = brows * 128, b_stage = 2 * b_half;          // one [brows x 64] swizzled sub-tile
+  uint8_t* b_base = smem;
+  uint8_t* raw_base = smem + GR_OP_STAGES * b_stage;
+  uint64_t* a_full = (uint64_t*)(raw_base + GR_RAW_STAGES * RAW_STAGE);   // [SA] 4 decode warps
+  uint64_t* a_empty = a_full + SA;                   // [SA] tcgen05.commit
+  uint64_t* b_full = a_empty + SA;                   // [OP] activation producer expect_tx
+  uint64_t* b_empty = b_full + GR_OP_STAGES;         // [OP] tcgen05.commit
+  uint64_t* raw_full = b_empty + GR_OP_STAGES;       // [RAW] weight producer expect_tx
+  uint64_t* raw_empty = raw_full + GR_RAW_STAGES;    // [RAW] 4 decode warps
+  uint64_t* acc_full = raw_empty + GR_RAW_STAGES;    // [2] tcgen05.commit
+  uint64_t* acc_empty = acc_full + 2;                // [2] 4 decode warps
+  uint64_t* drained = acc_empty + 2;                 // every MMA of this CTA has completed
+  uint32_t* tmem_slot = (uint32_t*)(drained + 1);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  volatile int* last_flag = abort_flag + 1;          // of the wait before the tensor memory is freed, which an abort does not cut short
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int strips = N / GR_STRIP, per_tile = strips * splits, nch = K / GR_KCH, nt_total = N / 16;
+  const int acc_cols = gr_acc_cols(brows);
+  uint32_t ncols = 32;
+  while ((int)ncols < 2 * acc_cols + SA * GR_A_COLS) ncols <<= 1;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < SA; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
+    for (int i = 0; i < GR_OP_STAGES; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+    for (int i = 0; i < GR_RAW_STAGES; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+    mbar_init(drained, 1);
+    *abort_flag = *last_flag = 0;
+    fence_barrier_init();
+    prefetch_tmap(&tmap_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, ncols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();                                        // the tile table and the rows come from the kernels before
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t a_tmem0 = tmem_base + 2 * acc_cols;
+
+  struct Item { int expert, row0, nrows, strip, split, c0, n; };
+  // item e of this CTA; false past the last one (live tiles come first, and items are taken tile by tile)
+  auto locate = [&](int e, Item& it) {
+    const long long idx = blockIdx.x + (long long)e * gridDim.x;
+    if (idx >= (long long)max_tiles * per_tile) return false;
+    const int tile = (int)(idx / per_tile), rem = (int)(idx - (long long)tile * per_tile);
+    it.split = rem / strips, it.strip = rem - it.split * strips;
+    if (tile_tab != nullptr) {
+      it.expert = tile_tab[3 * tile], it.row0 = tile_tab[3 * tile + 1], it.nrows = tile_tab[3 * tile + 2];
+    } else {
+      it.expert = 0, it.row0 = tile * brows, it.nrows = min(brows, rows - it.row0);
+    }
+    it.c0 = (int)((long long)nch * it.split / splits);
+    it.n = (int)((long long)nch * (it.split + 1) / splits) - it.c0;
+    return it.nrows > 0;
+  };
+  Item it;
+
+  if (warp == 0) {
+    // ---- weight producer: a chunk is 8 k-tile rows of the strip, one copy each
+    bool ok = true;
+    int gc = 0;
+    for (int e = 0; ok && locate(e, it); ++e) {
+      const uint32_t* src = trellis + (size_t)it.expert * expert_words + ((size_t)(it.c0 * 8 + (lane & 7)) * nt_total + (size_t)it.strip * 8) * TILE_WORDS;
+      for (int c = 0; c < it.n && ok; ++c, ++gc) {
+        const int s = gc % GR_RAW_STAGES;
+        if (lane == 0) {
+          if (gc >= GR_RAW_STAGES) ok = mbar_wait(&raw_empty[s], ((gc / GR_RAW_STAGES) - 1) & 1, abort_flag, status, 210, 500);
+          if (ok) mbar_arrive_expect_tx(&raw_full[s], RAW_STAGE);
+        }
+        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        if (ok && lane < 8) bulk_g2s(raw_base + s * RAW_STAGE + lane * ROW_BYTES, src + (size_t)c * 8 * nt_total * TILE_WORDS, ROW_BYTES, &raw_full[s]);
+      }
+    }
+  } else if (warp == 2) {
+    // ---- activation producer: two [brows x 64] swizzled boxes per chunk
+    if (lane == 0) {
+      bool ok = true;
+      int gc = 0;
+      for (int e = 0; ok && locate(e, it); ++e) {
+        for (int c = 0; c < it.n; ++c, ++gc) {
+          const int s = gc % GR_OP_STAGES, x = (it.c0 + c) * GR_KCH;
+          if (gc >= GR_OP_STAGES && !mbar_wait(&b_empty[s], ((gc / GR_OP_STAGES) - 1) & 1, abort_flag, status, 211, 250)) { ok = false; break; }
+          mbar_arrive_expect_tx(&b_full[s], (uint32_t)b_stage);
+          tma_load_2d(b_base + s * b_stage, &tmap_x, x, it.row0, &b_full[s]);
+          tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + 64, it.row0, &b_full[s]);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer: A from tensor memory, B from shared memory; as many rows as the tile has, in sixteens
+    if (lane == 0) {
+      const uint64_t desc0 = umma_desc_k_sw128(smem_u32(b_base));
+      const uint32_t half_units = (uint32_t)b_half >> 4, stage_units = (uint32_t)b_stage >> 4;
+      bool ok = true;
+      int gc = 0;
+      for (int e = 0; ok && locate(e, it); ++e) {
+        if (e >= 2 && !mbar_wait(&acc_empty[e & 1], ((e >> 1) - 1) & 1, abort_flag, status, 222)) break;
+        tc_fence_after();
+        const uint32_t idesc = umma_idesc_f16(GR_STRIP, (it.nrows + 15) & ~15, 0, 0);
+        const uint32_t acc = tmem_base + (e & 1) * acc_cols;
+        for (int c = 0; c < it.n; ++c, ++gc) {
+          const int s = gc % GR_OP_STAGES, sa = gc % SA;
+          if (!mbar_wait(&b_full[s], (gc / GR_OP_STAGES) & 1, abort_flag, status, 220) ||
+              !mbar_wait(&a_full[sa], (gc / SA) & 1, abort_flag, status, 221, 100)) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t bd = desc0 + (uint64_t)(s * stage_units);
+          const uint32_t at = a_tmem0 + sa * GR_A_COLS;
+#pragma unroll
+          for (int k = 0; k < GR_KCH / 16; ++k)
+            tc_mma_f16_ts(acc, at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
+          tc_commit(&a_empty[sa]);
+          tc_commit(&b_empty[s]);
+        }
+        if (ok) tc_commit(&acc_full[e & 1]);
+      }
+      tc_commit(drained);
+    }
+  } else {
+    const int dw = warp - GR_ROLE_WARPS, grp = dw >> 2;
+    const int q = warp & 3;                       // TMEM lane quarter this warp may touch
+    const int n = q * 32 + lane;                  // output column of the strip owned by this thread
+    const int nt = n >> 4, b2 = (n >> 3) & 1, g = n & 7;
+    const int prev_lane = (lane & ~7) | ((lane + 7) & 7);
+    const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+    const uint32_t my_words = (uint32_t)(nt * TILE_WORDS + g * EW) * 4u;     // byte offset of this thread's eighth inside a k-tile row
+    bool ok = true;
+    int next_out = grp;                           // the next item this group writes out
+    auto write_out = [&](int e) {
+      Item o;
+      locate(e, o);
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[e & 1], (e >> 1) & 1, abort_flag, status, 240))) return false;
+      tc_fence_after();
+      float* out = part + ((size_t)o.split * rows + o.row0) * N + o.strip * GR_STRIP + n;
+      for (int cb = 0; cb < o.nrows; cb += 16) {
+        uint32_t r[16];
+        tc_ld_32x32b_x16(tmem_base + (e & 1) * acc_cols + lane_addr + cb, r);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (cb + i < o.nrows) out[(size_t)(cb + i) * N] = __uint_as_float(r[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[e & 1]);
+      return true;
+    };
+    int gc0 = 0, e = 0;                           // chunks of the items before item e
+    for (; ok && locate(e, it); gc0 += it.n, ++e) {
+      for (int gc = gc0 + (grp - gc0 % NG + NG) % NG; gc < gc0 + it.n && ok; gc += NG) {
+        const int rs = gc % GR_RAW_STAGES, os = gc % SA;
+        // (a wait that ran out is the whole warp's: lanes must not part before the next shuffle)
+        ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[rs], (gc / GR_RAW_STAGES) & 1, abort_flag, status, 230, 100));
+        if (!ok) break;
+        const uint32_t raw = smem_u32(raw_base + rs * RAW_STAGE) + my_words;
+#pragma unroll
+        for (int qt = 0; qt < 4; ++qt) {
+          // two k-tiles at a time: the thread's eighth of each and, from the lane before it, the word those follow
+          uint32_t w[2][EW + 1];
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {
+            const uint32_t at = raw + (uint32_t)((qt * 2 + kk) * ROW_BYTES);
+            if constexpr (TWICE == 8) {
+              const uint4 v = lds128(at);
+              w[kk][1] = v.x, w[kk][2] = v.y, w[kk][3] = v.z, w[kk][4] = v.w;
+            } else {
+#pragma unroll
+              for (int i = 0; i < EW; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[kk][1 + i]) : "r"(at + 4u * i));
+            }
+          }
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) w[kk][0] = __shfl_sync(0xffffffffu, w[kk][EW], prev_lane);
+          if (qt == 3) release_read_stage(&raw_empty[rs], lane);   // the stage's last read has landed in registers; proxy fence before the refill
+          uint32_t regs[16];
+          decode_column<TWICE, CB>(w[0], b2, regs);
+          decode_column<TWICE, CB>(w[1], b2, regs + 8);
+          if (qt == 0) {
+            if (gc >= SA) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[os], ((gc / SA) - 1) & 1, abort_flag, status, 231));
+            if (!ok) break;
+            tc_fence_after();
+          }
+          tc_st_32x32b_x16(a_tmem0 + lane_addr + os * GR_A_COLS + qt * 16, regs);
+        }
+        if (!ok) break;
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_full[os]);
+        for (; next_out < e && ok; next_out += NG) ok = write_out(next_out);
+      }
+    }
+    for (; next_out < e && ok; next_out += NG) ok = write_out(next_out);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    if (lane == 0) mbar_wait(drained, 0, last_flag, status, 241);      // nothing may still write the tensor memory that is freed
+    __syncwarp();
+    tmem_dealloc(tmem_base, ncols);
+  }
+}
+
+int make_tmap_f16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+
+template <int TWICE, int CB, int NG>
+static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t expert_words, float* part, int rows, int K, int N, int splits, int brows,
+                          const int* tile_tab, int max_tiles, int* status, cudaStream_t st) {
+  int smem = gr_smem_bytes(brows, TWICE) + 1024;
+  if (NG <= 3 && smem < 80 * 1024) smem = 80 * 1024;   // at most two CTAs per SM: each allocates 256 TMEM columns
+  auto kern = exl3_gemm_grouped_kernel<TWICE, CB, NG>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const long long items = (long long)max_tiles * (N / GR_STRIP) * splits, slots = (NG <= 3 ? 2 : 1) * 148;
+  rx::launch(kern, dim3((unsigned)(items < slots ? items : slots)), dim3(GR_ROLE_WARPS * 32 + NG * 128), smem, st, tm, trellis, expert_words, part, rows, K, N,
+             splits, brows, tile_tab, max_tiles, status);
+  return (int)cudaGetLastError();
+}
+
+// Whether rx_exl3_gemm_persistent takes the product: widths with a column decoder, tiles whose two accumulators fit beside the A stages, splits in
+// whole 128-k chunks.
+bool gemm_persistent_takes(int K, int twice, int splits, int brows) {
+  return (twice == 6 || twice == 8) && brows <= 128 && splits <= K / GR_KCH;
+}
+
+int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits,
+                    const int* tile_tab, int max_tiles, int brows, int* status, cudaStream_t st) {
+  CUtensorMap tm;
+  int e = make_tmap_f16_2d(&tm, xs, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
+  if (e != 0) return e;
+  const uint32_t* tr = (const uint32_t*)trellis;
+#define RX_GR(T, CBV) (brows > 32 ? launch_grouped<T, CBV, 4>(tm, tr, expert_words, (float*)part, rows, K, N, splits, brows, tile_tab, max_tiles, status, st) \
+                                  : launch_grouped<T, CBV, 3>(tm, tr, expert_words, (float*)part, rows, K, N, splits, brows, tile_tab, max_tiles, status, st))
+  switch (codebook) {
+    case CB_3INST: return twice == 6 ? RX_GR(6, CB_3INST) : RX_GR(8, CB_3INST);
+    case CB_MCG: return twice == 6 ? RX_GR(6, CB_MCG) : RX_GR(8, CB_MCG);
+    case CB_MUL1: return twice == 6 ? RX_GR(6, CB_MUL1) : RX_GR(8, CB_MUL1);
+    default: return (int)cudaErrorInvalidValue;
+  }
+#undef RX_GR
+}
+
+}  // namespace rx
