@@ -391,6 +391,10 @@ RX_API int rx_exl3_gemm(const void* xr, int rows, int K, const void* trellis, in
   if ((((uintptr_t)xr) & 15) != 0 || (((uintptr_t)trellis) & 15) != 0) return (int)cudaErrorMisalignedAddress;
   const int brows = rx_exl3_tile_rows(rows);
   const int row_tiles = (rows + brows - 1) / brows;
+  // 65 to 128 rows at 3.0 bpw: one CTA per SM either way, and the persistent kernel's sixteen decode warps beat this one's eight (2048 -> 151,936,
+  // 100 rows: 206 -> 150 us; up to 64 rows the two are level).  Only where both cut K at the same places: a row's bits do not depend on the row count.
+  if (twice == 6 && brows == 128 && (K / 128) % splits == 0 && gemm_persistent_takes(K, twice, splits, brows))
+    return gemm_persistent(xr, rows, K, trellis, 0, N, twice, codebook, part, splits, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xr, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
   if (e != 0) return e;

@@ -8,7 +8,9 @@
 // 128 k), so the CTAs are PERSISTENT and every ring runs on across items - the weights of the next item stream in while this one is decoded -
 // and the accumulator is double buffered, its epilogue done by one decode group while the others go on.  One CTA per item in exl3_gemm.cu
 // spent most of its life in its prologue and on shared-memory traffic of the decoded tile: 16 rows x 8 picks of 128 experts (2048 -> 1536 and
-// 768 -> 2048, 3.0 bpw) took XOLD us for both products, XNEW us here.
+// 768 -> 2048, 3.0 bpw) took 235 us for both products,
+// 146 us here; one row 83 and 26 us.  What is left is the decode's own: the integer pipe is 70 % busy.  (Fetching the next item's table entry
+// ahead costs registers that the decode groups do not have: 5 % slower.)
 //
 // Warp roles: 0 weight producer (one bulk copy per k-tile row), 1 TMEM owner + MMA issuer, 2 activation producer, then NG decode groups of 4 warps.
 // Group e % NG writes out item e, after its first chunk of a later item: the accumulator of item e is needed again by item e + 2 only, whose
@@ -27,27 +29,29 @@ __host__ __device__ constexpr int gr_acc_cols(int brows) { return brows < 32 ? 3
 __host__ __device__ inline int gr_smem_bytes(int brows, int twice) { return GR_OP_STAGES * brows * 256 + GR_RAW_STAGES * 1024 * twice + 512; }
 
 // One k-tile (16 k) of a thread's column: 8 packed pairs, regs[m] = k (2m, 2m + 1), regs[4 + m] = k (8 + 2m, 9 + 2m).
-// w[0] = the word before the thread's eighth of the tile, w[1..] = the eighth's words; b2: which of its two columns (see exl3_decode.cuh).
+// w[0] = the word before the thread's eighth of the tile, w[1..] = the eighth's words (see exl3_decode.cuh); b2: which of its two columns.
+// shift: where the column's first window starts in its word pair (column_shift).
+template <int TWICE>
+__device__ __forceinline__ uint32_t column_shift(int b2) { return TWICE == 8 ? (b2 ? 32u : 16u) : (b2 ? 31u : 19u); }
 template <int TWICE, int CB>
-__device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1], int b2, uint32_t* regs) {
+__device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1], uint32_t shift, uint32_t* regs) {
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     uint32_t s0, s1, s2, s3;
     if constexpr (TWICE == 8) {
       // b2 = 0: the 4 values that straddle the word boundary; b2 = 1: the word's own 4
-      const uint32_t X = __funnelshift_lc(w[m + 1], w[m], b2 ? 32u : 16u);
+      const uint32_t X = __funnelshift_lc(w[m + 1], w[m], shift);
       extract4<CB != CB_MUL1>(X, s0, s1, s2, s3);
     } else {
-      // windows start at bit 19 + 24 m + 12 b2 + 3 i of w: 25 bits from the first one's start hold all four
+      // windows start at bit 19 + 24 m + 12 b2 + 3 i of w: 25 bits from the first one's start hold all four.  The word they start in does not
+      // depend on b2 but for m = 3, and the funnel shift takes its amount modulo 32.
       static_assert(TWICE == 6, "widths of this kernel: 3.0 and 4.0 bpw");
-      const int bit0 = 19 + 24 * m, bit1 = 31 + 24 * m;
-      const uint32_t hi = bit0 / 32 == bit1 / 32 ? w[bit0 / 32] : (b2 ? w[bit1 / 32] : w[bit0 / 32]);
-      const uint32_t lo0 = w[bit0 / 32 + 1], lo1 = bit1 / 32 + 1 <= TWICE / 2 ? w[bit1 / 32 + 1 <= TWICE / 2 ? bit1 / 32 + 1 : 0] : 0u;
-      const uint32_t lo = bit0 / 32 == bit1 / 32 ? lo0 : (b2 ? lo1 : lo0);
-      const uint32_t X = __funnelshift_l(lo, hi, b2 ? bit1 % 32 : bit0 % 32);
+      uint32_t X;
+      if (m < 3) X = __funnelshift_l(w[m + 1], w[m], shift + 24 * m);
+      else X = shift == 31u ? w[3] << 7 : __funnelshift_l(w[3], w[2], 27);
       s0 = X >> 16;
-      s1 = (X >> 13) & 0xFFFFu;
-      const uint32_t x2 = X >> 10, x3 = X >> 7;
+      const uint32_t x1 = X >> 13, x2 = X >> 10, x3 = X >> 7;
+      s1 = x1 & 0xFFFFu;
       s2 = CB != CB_MUL1 ? low16_mul(x2) : x2 & 0xFFFFu;        // (the multiply pipe has room for two of the masks)
       s3 = CB != CB_MUL1 ? low16_mul(x3) : x3 & 0xFFFFu;
     }
@@ -63,6 +67,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
                          int* status) {
   pdl_launch();
   constexpr int SA = gr_a_stages(NG), EW = TWICE / 2;            // EW: words of an eighth of a tile
+  constexpr int QT = NG <= 3 ? 1 : 4;                            // quarters of a chunk unrolled: short items keep to the instruction cache, long ones gain 5 %
   constexpr int TILE_WORDS = 4 * TWICE, ROW_BYTES = 8 * TILE_WORDS * 4, RAW_STAGE = 8 * ROW_BYTES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -75,13 +80,16 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
   uint64_t* b_empty = b_full + GR_OP_STAGES;         // [OP] tcgen05.commit
   uint64_t* raw_full = b_empty + GR_OP_STAGES;       // [RAW] weight producer expect_tx
   uint64_t* raw_empty = raw_full + GR_RAW_STAGES;    // [RAW] 4 decode warps
-  uint64_t* acc_full = raw_empty + GR_RAW_STAGES;    // [2] tcgen05.commit
-  uint64_t* acc_empty = acc_full + 2;                // [2] 4 decode warps
+  // A parity wait tells a phase from the next one only.  A group may ask for item e before item e - 2 is complete, but its own last write-out was
+  // item e - NG, so e - 4 is: four barriers in turn for two accumulators.
+  uint64_t* acc_full = raw_empty + GR_RAW_STAGES;    // [4] tcgen05.commit
+  uint64_t* acc_empty = acc_full + 4;                // [2] 4 decode warps
   uint64_t* drained = acc_empty + 2;                 // every MMA of this CTA has completed
   uint32_t* tmem_slot = (uint32_t*)(drained + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   volatile int* last_flag = abort_flag + 1;          // of the wait before the tensor memory is freed, which an abort does not cut short
 
+  int* split_c0 = (int*)(last_flag + 1);              // [splits + 1] first chunk of each split
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strips = N / GR_STRIP, per_tile = strips * splits, nch = K / GR_KCH, nt_total = N / 16;
   const int acc_cols = gr_acc_cols(brows);
@@ -91,12 +99,14 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     for (int i = 0; i < SA; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
     for (int i = 0; i < GR_OP_STAGES; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
     for (int i = 0; i < GR_RAW_STAGES; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+    for (int i = 0; i < 4; ++i) mbar_init(&acc_full[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], 4);
     mbar_init(drained, 1);
     *abort_flag = *last_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
   }
+  if (warp == 2 && lane <= splits) split_c0[lane] = (int)((unsigned)(nch * lane) / (unsigned)splits);
   if (warp == 1) {
     tmem_alloc(tmem_slot, ncols);
     tmem_relinquish();
@@ -108,31 +118,43 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t a_tmem0 = tmem_base + 2 * acc_cols;
 
-  struct Item { int expert, row0, nrows, strip, split, c0, n; };
-  // item e of this CTA; false past the last one (live tiles come first, and items are taken tile by tile)
-  auto locate = [&](int e, Item& it) {
-    const long long idx = blockIdx.x + (long long)e * gridDim.x;
-    if (idx >= (long long)max_tiles * per_tile) return false;
-    const int tile = (int)(idx / per_tile), rem = (int)(idx - (long long)tile * per_tile);
-    it.split = rem / strips, it.strip = rem - it.split * strips;
+  // Items are taken tile by tile: a tile's splits, a split's strips.  A walker steps from item to item of this CTA by additions with carries.
+  struct Walk { int tile, split, strip; };
+  auto walk_of = [&](unsigned idx) {
+    Walk w;
+    w.tile = (int)(idx / (unsigned)per_tile);
+    const unsigned rem = idx - (unsigned)w.tile * (unsigned)per_tile;
+    w.split = (int)(rem / (unsigned)strips);
+    w.strip = (int)(rem - (unsigned)w.split * (unsigned)strips);
+    return w;
+  };
+  auto step = [&](Walk& w, const Walk& d) {
+    w.strip += d.strip, w.split += d.split, w.tile += d.tile;
+    if (w.strip >= strips) w.strip -= strips, ++w.split;
+    if (w.split >= splits) w.split -= splits, ++w.tile;
+  };
+  struct Item { int expert, row0, nrows; };
+  auto tile_of = [&](const Walk& w, Item& it) {        // false past the last item (live tiles come first)
+    if (w.tile >= max_tiles) return false;
     if (tile_tab != nullptr) {
-      it.expert = tile_tab[3 * tile], it.row0 = tile_tab[3 * tile + 1], it.nrows = tile_tab[3 * tile + 2];
+      it.expert = tile_tab[3 * w.tile], it.row0 = tile_tab[3 * w.tile + 1], it.nrows = tile_tab[3 * w.tile + 2];
     } else {
-      it.expert = 0, it.row0 = tile * brows, it.nrows = min(brows, rows - it.row0);
+      it.expert = 0, it.row0 = w.tile * brows, it.nrows = min(brows, rows - it.row0);
     }
-    it.c0 = (int)((long long)nch * it.split / splits);
-    it.n = (int)((long long)nch * (it.split + 1) / splits) - it.c0;
     return it.nrows > 0;
   };
   Item it;
+  Walk at = walk_of(blockIdx.x);
+  const Walk stride = walk_of(gridDim.x);
 
   if (warp == 0) {
     // ---- weight producer: a chunk is 8 k-tile rows of the strip, one copy each
     bool ok = true;
     int gc = 0;
-    for (int e = 0; ok && locate(e, it); ++e) {
-      const uint32_t* src = trellis + (size_t)it.expert * expert_words + ((size_t)(it.c0 * 8 + (lane & 7)) * nt_total + (size_t)it.strip * 8) * TILE_WORDS;
-      for (int c = 0; c < it.n && ok; ++c, ++gc) {
+    for (; ok && tile_of(at, it); step(at, stride)) {
+      const int c0 = split_c0[at.split], n = split_c0[at.split + 1] - c0;
+      const uint32_t* src = trellis + (size_t)it.expert * expert_words + ((size_t)(c0 * 8 + (lane & 7)) * nt_total + (size_t)at.strip * 8) * TILE_WORDS;
+      for (int c = 0; c < n && ok; ++c, ++gc) {
         const int s = gc % GR_RAW_STAGES;
         if (lane == 0) {
           if (gc >= GR_RAW_STAGES) ok = mbar_wait(&raw_empty[s], ((gc / GR_RAW_STAGES) - 1) & 1, abort_flag, status, 210, 500);
@@ -147,9 +169,10 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     if (lane == 0) {
       bool ok = true;
       int gc = 0;
-      for (int e = 0; ok && locate(e, it); ++e) {
-        for (int c = 0; c < it.n; ++c, ++gc) {
-          const int s = gc % GR_OP_STAGES, x = (it.c0 + c) * GR_KCH;
+      for (; ok && tile_of(at, it); step(at, stride)) {
+        const int c0 = split_c0[at.split], n = split_c0[at.split + 1] - c0;
+        for (int c = 0; c < n; ++c, ++gc) {
+          const int s = gc % GR_OP_STAGES, x = (c0 + c) * GR_KCH;
           if (gc >= GR_OP_STAGES && !mbar_wait(&b_empty[s], ((gc / GR_OP_STAGES) - 1) & 1, abort_flag, status, 211, 250)) { ok = false; break; }
           mbar_arrive_expect_tx(&b_full[s], (uint32_t)b_stage);
           tma_load_2d(b_base + s * b_stage, &tmap_x, x, it.row0, &b_full[s]);
@@ -164,25 +187,26 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
       const uint32_t half_units = (uint32_t)b_half >> 4, stage_units = (uint32_t)b_stage >> 4;
       bool ok = true;
       int gc = 0;
-      for (int e = 0; ok && locate(e, it); ++e) {
+      for (int e = 0; ok && tile_of(at, it); ++e, step(at, stride)) {
+        const int n = split_c0[at.split + 1] - split_c0[at.split];
         if (e >= 2 && !mbar_wait(&acc_empty[e & 1], ((e >> 1) - 1) & 1, abort_flag, status, 222)) break;
         tc_fence_after();
         const uint32_t idesc = umma_idesc_f16(GR_STRIP, (it.nrows + 15) & ~15, 0, 0);
         const uint32_t acc = tmem_base + (e & 1) * acc_cols;
-        for (int c = 0; c < it.n; ++c, ++gc) {
+        for (int c = 0; c < n; ++c, ++gc) {
           const int s = gc % GR_OP_STAGES, sa = gc % SA;
           if (!mbar_wait(&b_full[s], (gc / GR_OP_STAGES) & 1, abort_flag, status, 220) ||
               !mbar_wait(&a_full[sa], (gc / SA) & 1, abort_flag, status, 221, 100)) { ok = false; break; }
           tc_fence_after();
           const uint64_t bd = desc0 + (uint64_t)(s * stage_units);
-          const uint32_t at = a_tmem0 + sa * GR_A_COLS;
+          const uint32_t a_at = a_tmem0 + sa * GR_A_COLS;
 #pragma unroll
           for (int k = 0; k < GR_KCH / 16; ++k)
-            tc_mma_f16_ts(acc, at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
+            tc_mma_f16_ts(acc, a_at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
           tc_commit(&a_empty[sa]);
           tc_commit(&b_empty[s]);
         }
-        if (ok) tc_commit(&acc_full[e & 1]);
+        if (ok) tc_commit(&acc_full[e & 3]);
       }
       tc_commit(drained);
     }
@@ -190,18 +214,21 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     const int dw = warp - GR_ROLE_WARPS, grp = dw >> 2;
     const int q = warp & 3;                       // TMEM lane quarter this warp may touch
     const int n = q * 32 + lane;                  // output column of the strip owned by this thread
-    const int nt = n >> 4, b2 = (n >> 3) & 1, g = n & 7;
+    const int nt = n >> 4, g = n & 7;
+    const uint32_t shift = column_shift<TWICE>((n >> 3) & 1);
     const int prev_lane = (lane & ~7) | ((lane + 7) & 7);
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t my_words = (uint32_t)(nt * TILE_WORDS + g * EW) * 4u;     // byte offset of this thread's eighth inside a k-tile row
     bool ok = true;
-    int next_out = grp;                           // the next item this group writes out
+    int next_out = grp;                           // the next item this group writes out, and where it stands
+    Walk out_at = walk_of(blockIdx.x + (unsigned)grp * gridDim.x);
+    const Walk out_stride = walk_of((unsigned)NG * gridDim.x);
     auto write_out = [&](int e) {
       Item o;
-      locate(e, o);
-      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[e & 1], (e >> 1) & 1, abort_flag, status, 240))) return false;
+      tile_of(out_at, o);
+      if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[e & 3], (e >> 2) & 1, abort_flag, status, 240))) return false;
       tc_fence_after();
-      float* out = part + ((size_t)o.split * rows + o.row0) * N + o.strip * GR_STRIP + n;
+      float* out = part + ((size_t)out_at.split * rows + o.row0) * N + out_at.strip * GR_STRIP + n;
       for (int cb = 0; cb < o.nrows; cb += 16) {
         uint32_t r[16];
         tc_ld_32x32b_x16(tmem_base + (e & 1) * acc_cols + lane_addr + cb, r);
@@ -213,37 +240,39 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[e & 1]);
+      step(out_at, out_stride);
       return true;
     };
-    int gc0 = 0, e = 0;                           // chunks of the items before item e
-    for (; ok && locate(e, it); gc0 += it.n, ++e) {
-      for (int gc = gc0 + (grp - gc0 % NG + NG) % NG; gc < gc0 + it.n && ok; gc += NG) {
+    int gc0 = 0, e = 0;                           // chunks up to the end of item e
+    for (int gc = grp; ok && tile_of(at, it); ++e, step(at, stride)) {
+      gc0 += split_c0[at.split + 1] - split_c0[at.split];
+      for (; gc < gc0 && ok; gc += NG) {
         const int rs = gc % GR_RAW_STAGES, os = gc % SA;
         // (a wait that ran out is the whole warp's: lanes must not part before the next shuffle)
         ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[rs], (gc / GR_RAW_STAGES) & 1, abort_flag, status, 230, 100));
         if (!ok) break;
         const uint32_t raw = smem_u32(raw_base + rs * RAW_STAGE) + my_words;
-#pragma unroll
+#pragma unroll QT
         for (int qt = 0; qt < 4; ++qt) {
           // two k-tiles at a time: the thread's eighth of each and, from the lane before it, the word those follow
           uint32_t w[2][EW + 1];
 #pragma unroll
           for (int kk = 0; kk < 2; ++kk) {
-            const uint32_t at = raw + (uint32_t)((qt * 2 + kk) * ROW_BYTES);
+            const uint32_t src = raw + (uint32_t)((qt * 2 + kk) * ROW_BYTES);
             if constexpr (TWICE == 8) {
-              const uint4 v = lds128(at);
+              const uint4 v = lds128(src);
               w[kk][1] = v.x, w[kk][2] = v.y, w[kk][3] = v.z, w[kk][4] = v.w;
             } else {
 #pragma unroll
-              for (int i = 0; i < EW; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[kk][1 + i]) : "r"(at + 4u * i));
+              for (int i = 0; i < EW; ++i) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[kk][1 + i]) : "r"(src + 4u * i));
             }
           }
 #pragma unroll
           for (int kk = 0; kk < 2; ++kk) w[kk][0] = __shfl_sync(0xffffffffu, w[kk][EW], prev_lane);
           if (qt == 3) release_read_stage(&raw_empty[rs], lane);   // the stage's last read has landed in registers; proxy fence before the refill
           uint32_t regs[16];
-          decode_column<TWICE, CB>(w[0], b2, regs);
-          decode_column<TWICE, CB>(w[1], b2, regs + 8);
+          decode_column<TWICE, CB>(w[0], shift, regs);
+          decode_column<TWICE, CB>(w[1], shift, regs + 8);
           if (qt == 0) {
             if (gc >= SA) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[os], ((gc / SA) - 1) & 1, abort_flag, status, 231));
             if (!ok) break;
@@ -284,16 +313,18 @@ static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  const long long items = (long long)max_tiles * (N / GR_STRIP) * splits, slots = (NG <= 3 ? 2 : 1) * 148;
+  const long long items = (long long)max_tiles * (N / GR_STRIP) * splits;
+  if (items >= (1ll << 30)) return (int)cudaErrorInvalidValue;          // (item numbers are 32-bit)
+  const long long slots = (NG <= 3 ? 2 : 1) * 148;
   rx::launch(kern, dim3((unsigned)(items < slots ? items : slots)), dim3(GR_ROLE_WARPS * 32 + NG * 128), smem, st, tm, trellis, expert_words, part, rows, K, N,
              splits, brows, tile_tab, max_tiles, status);
   return (int)cudaGetLastError();
 }
 
 // Whether rx_exl3_gemm_persistent takes the product: widths with a column decoder, tiles whose two accumulators fit beside the A stages, splits in
-// whole 128-k chunks.
+// whole 128-k chunks and no more of them than its table of their bounds holds.
 bool gemm_persistent_takes(int K, int twice, int splits, int brows) {
-  return (twice == 6 || twice == 8) && brows <= 128 && splits <= K / GR_KCH;
+  return (twice == 6 || twice == 8) && brows <= 128 && splits <= K / GR_KCH && splits < 32;
 }
 
 int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits,
