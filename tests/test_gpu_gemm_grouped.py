@@ -58,12 +58,13 @@ def test_grouped_gemm(bits, cb, counts, K, N, splits):
 
 
 @pytest.mark.parametrize("rows", [65, 100, 128])
-def test_plain_gemm_of_65_to_128_rows_at_3_bits(rows):
+@pytest.mark.parametrize("bits,splits", [(3, 4), (4, 4), (4, 3)])
+def test_plain_gemm_of_65_to_128_rows(rows, bits, splits):
     """These windows take the persistent kernel; smaller ones the general one: the same bits for a row either way."""
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
-    K, N, splits = 1024, 384, 4
-    KK, xs, tr, dense = _problem(1, K, N, 3, "3inst", [rows], 1)
+    K, N = 1024, 384
+    KK, xs, tr, dense = _problem(1, K, N, bits, "3inst", [rows], 1)
     w = KK.Exl3Weight(tr[0].contiguous(), torch.ones(K, dtype=torch.float16, device="cuda"), torch.ones(N, dtype=torch.float16, device="cuda"), None, "3inst")
     st, part, few = KK.new_status(), torch.zeros(splits, rows, N, device="cuda"), torch.zeros(splits, 33, N, device="cuda")
     KK.exl3_gemm(xs, w, part, splits, st)
