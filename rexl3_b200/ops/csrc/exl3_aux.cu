@@ -129,8 +129,7 @@ __global__ void __launch_bounds__(1024) norm_rot_in_kernel(const uint16_t* __res
 // ONE: a single plane, known at compile time.  The loop over planes keeps eight loads in registers; a kernel that carries it for nothing holds a
 // third as many warps per SM (100 registers against 32-48), which for the many rows of a prompt is what bounded these kernels.
 template <bool ONE = false>
-__device__ __forceinline__ void finish_block(const float* __restrict__ part, int S, size_t split_stride, size_t off, const __half* svh,
-                                             const float* bias, int n0, float (&y)[4]) {
+__device__ __forceinline__ void sum_planes(const float* __restrict__ part, int S, size_t split_stride, size_t off, float (&y)[4]) {
   // loads are issued eight at a time (independent, so their latencies overlap) and added in split order
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (ONE || S == 1) acc = __ldg(reinterpret_cast<const float4*>(part + off));
@@ -148,6 +147,11 @@ __device__ __forceinline__ void finish_block(const float* __restrict__ part, int
       }
   }
   y[0] = acc.x; y[1] = acc.y; y[2] = acc.z; y[3] = acc.w;
+}
+template <bool ONE = false>
+__device__ __forceinline__ void finish_block(const float* __restrict__ part, int S, size_t split_stride, size_t off, const __half* svh,
+                                             const float* bias, int n0, float (&y)[4]) {
+  sum_planes<ONE>(part, S, split_stride, off, y);
   fwht128_warp(y);
   float sv[4];
   load4_f16(svh + n0, sv);
@@ -229,6 +233,70 @@ __global__ void __launch_bounds__(1024) finish_add_norm_rot_kernel(const float* 
     fwht128_warp(v);
     store4_f16(xr + (size_t)row * N + n0, v);
   }
+}
+
+// The same for the rows of a decode window, bound by latency: one SM is slow to fetch the planes of a row (7 x 5120 floats), and 32 warps need two passes
+// over its 40 blocks.  So a cluster of four CTAs takes a row, a warp one 128-block of it, kept in registers; the blocks' sums of squares reach every
+// CTA through the cluster's shared memory and are added there in block order.  The weights are loaded before the wait for the predecessor.
+// One row of 5120 in 7 planes 3.2 us, 5.8 by one CTA; 64 rows 4.0 and 6.0 (launch included); clusters of eight 3.0 and 4.7.
+constexpr int FEW_CTAS = 4, FEW_WARPS = 16;
+__global__ void __cluster_dims__(FEW_CTAS, 1, 1) __launch_bounds__(FEW_WARPS * 32) finish_add_norm_rot_few_kernel(
+    const float* __restrict__ part, int S, int M, int N, const __half* __restrict__ svh, const float* __restrict__ bias, uint16_t* __restrict__ h,
+    const uint16_t* __restrict__ norm_w, float eps, const __half* __restrict__ suh_next, __half* __restrict__ xr, uint16_t* __restrict__ xn_out) {
+  pdl_launch();
+  __shared__ float blk_ss[FEW_CTAS * FEW_WARPS];
+  const int row = blockIdx.x / FEW_CTAS, rank = blockIdx.x % FEW_CTAS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = N / 128;
+  const int b = rank * (blockDim.x >> 5) + warp, n0 = b * 128 + lane * 4;
+  const bool live = b < nb, out = suh_next != nullptr || xn_out != nullptr, sums = out && norm_w != nullptr;
+  if (sums) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // every CTA of the cluster has begun: its shared memory may be written
+  alignas(16) float bi[4] = {};
+  float sv[4] = {}, w[4] = {}, s[4] = {};
+  if (live) {
+    load4_f16(svh + n0, sv);
+    if (bias != nullptr) *reinterpret_cast<float4*>(bi) = *reinterpret_cast<const float4*>(bias + n0);
+    if (sums) load4_bf16(norm_w + n0, w);
+    if (suh_next != nullptr) load4_f16(suh_next + n0, s);
+  }
+  pdl_wait();
+  float r[4] = {};
+  if (live) {
+    float y[4];
+    load4_bf16(h + (size_t)row * N + n0, r);
+    sum_planes(part, S, (size_t)M * N, (size_t)row * N + n0, y);
+    fwht128_warp(y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      y[i] = __fmul_rn(y[i], sv[i]);
+      if (bias != nullptr) y[i] += bi[i];
+      r[i] = bf16_to_f(f_to_bf16(r[i] + y[i]));
+    }
+    store4_bf16(h + (size_t)row * N + n0, r);
+  }
+  if (!out) return;
+  float rinv = 1.f;
+  if (sums) {
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = __fmaf_rn(r[i], r[i], ss);
+    ss = warp_sum(ss);
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (live && lane < FEW_CTAS)
+      asm volatile("{.reg .b32 a; mapa.shared::cluster.u32 a, %0, %1; st.shared::cluster.f32 [a], %2;}" ::"r"(smem_u32(&blk_ss[b])), "r"(lane), "f"(ss) : "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    float tot = 0.f;
+    for (int i = 0; i < nb; ++i) tot += blk_ss[i];
+    rinv = rsqrtf(tot / (float)N + eps);
+  }
+  if (!live) return;
+  float v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = sums ? __fmul_rn(bf16_to_f(f_to_bf16(r[i] * rinv)), w[i]) : r[i];
+  if (xn_out != nullptr) store4_bf16(xn_out + (size_t)row * N + n0, v);
+  if (suh_next == nullptr) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __fmul_rn(v[i], s[i]);
+  fwht128_warp(v);
+  store4_f16(xr + (size_t)row * N + n0, v);
 }
 
 // The same for the many rows of a prompt slice (one plane, rows of up to ROWS_NB * 1024 elements), bound by memory: a CTA of eight warps per row, a warp's
@@ -389,6 +457,14 @@ RX_API int rx_finish_add_norm_rot(const void* part, int S, int M, int N, const v
   if (S == 1 && M >= 512 && N <= ROWS_NB * 1024) {
     rx::launch(finish_add_norm_rot_rows_kernel, dim3(M), dim3(256), 0, (cudaStream_t)stream, (const float*)part, N, (const __half*)svh, (const float*)bias,
                (uint16_t*)h_bf16, (const uint16_t*)norm_w, eps, (const __half*)suh_next, (__half*)xr, (uint16_t*)xn_out);
+    return (int)cudaGetLastError();
+  }
+  // Up to 64 rows (256 CTAs) the clusters are the faster form of rows of 4096 and more, up to 16 rows also of shorter ones, which one CTA has in one
+  // pass: 37 rows of 2048 in 18 planes take 4.65 us by clusters, 4.40 otherwise; 37 rows of 4096 in 9 planes 4.75 and 5.10; 74 of 5120 6.5 and 6.1.
+  if ((N >= 4096 ? M <= 64 : M <= 16) && N <= FEW_CTAS * FEW_WARPS * 128) {
+    const int warps = (N / 128 + FEW_CTAS - 1) / FEW_CTAS;
+    rx::launch(finish_add_norm_rot_few_kernel, dim3(M * FEW_CTAS), dim3(warps * 32), 0, (cudaStream_t)stream, (const float*)part, S, M, N, (const __half*)svh,
+               (const float*)bias, (uint16_t*)h_bf16, (const uint16_t*)norm_w, eps, (const __half*)suh_next, (__half*)xr, (uint16_t*)xn_out);
     return (int)cudaGetLastError();
   }
   static bool configured = false;

@@ -34,6 +34,28 @@ def test_add_norm_rot_rows_do_not_depend_on_their_number(N, norm):
     assert (whole[0].double() - y).abs().max() <= 2.0 ** -8 * y.abs().max() + 1e-5      # one rounding to bf16
 
 
+@pytest.mark.parametrize("N", [128, 640, 3968, 4096, 5120, 8192, 8320])     # clusters: up to 16 rows below 4096, up to 64 from there to 8192
+@pytest.mark.parametrize("S", [1, 7, 18])
+@pytest.mark.parametrize("norm,rot,xn", [(True, True, True), (False, True, False), (True, False, True), (True, False, False)])
+def test_add_norm_rot_of_few_rows(N, S, norm, rot, xn):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(N + S)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    M, w = 146, _weight(N, g)
+    part, h0, nw, suh = r(S, M, N), r(M, N).bfloat16(), (1 + 0.1 * r(N)).bfloat16() if norm else None, r(N).half() if rot else None
+
+    def run(*cuts):
+        out = [h0.clone(), torch.zeros(M, N, dtype=torch.float16, device="cuda"), torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")]
+        for a, b in zip(cuts, cuts[1:]):
+            o = [t[a:b] for t in out]
+            K.finish_add_norm_rot(part[:, a:b].contiguous(), S, b - a, w, o[0], nw, 1e-6, suh, o[1], o[2] if xn else None)
+        return out
+    for x, y in zip(run(0, M), run(0, 1, 17, 81, M)):
+        assert torch.isfinite(x.float()).all() and torch.equal(x, y)
+
+
 @pytest.mark.parametrize("hd,n_q,n_kv", [(128, 40, 8), (128, 3, 1), (64, 4, 2)])
 def test_qkv_rope_rows_do_not_depend_on_their_number(hd, n_q, n_kv):
     if not torch.cuda.is_available():
