@@ -418,8 +418,9 @@ struct CombineDst {
 // grid = (M, gy).  part: f32 [S][pairs_cap][d] (down GEMM).  y[row] = sum_slot w[row][slot] * finish(part[pos(row, slot)]) in slot order,
 // skipping pairs this rank does not own; + shared[row] (f32 [M, d] or nullptr; only one rank passes it).  The row goes to slot `rank`
 // of every rank's all-reduce buffer, then the last CTA publishes the flags.
-// ONE: a single plane; eight slots' blocks are then loaded before the first is used (2100 rows x 8 picks of 2048: 113 -> 58 us).
-template <bool ONE>
+// PLANES: 1 and 4 for windows of one plane and of up to four; eight (four) slots' blocks are then loaded before the first is used, where one slot after the
+// other was a chain of as many memory latencies (2100 rows x 8 picks of 2048: 113 -> 58 us; 16 rows in three planes: 12.2 -> 8.4 us).  0: any number of planes.
+template <int PLANES>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ part, int S, int pairs_cap, int M, int d, int topk, const int* __restrict__ ids,
                                    const float* __restrict__ w, const int* __restrict__ pos_of_pair, const __half* __restrict__ svh_down,
                                    const float* __restrict__ shared, const __grid_constant__ CombineDst tp) {
@@ -430,21 +431,27 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
   for (int b = blockIdx.y * nw + warp; b < d / 128; b += gridDim.y * nw) {
     const int n0 = b * 128 + lane * 4;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (ONE) {
-      for (int j0 = 0; j0 < topk; j0 += 8) {
-        int pos[8];
-        float4 p[8];
+    if (PLANES > 0) {
+      constexpr int SLOTS = PLANES == 1 ? 8 : 4, PL = PLANES > 0 ? PLANES : 1;
+      for (int j0 = 0; j0 < topk; j0 += SLOTS) {
+        int pos[SLOTS];
+        float4 p[SLOTS][PL];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) pos[j] = j0 + j < topk ? pos_of_pair[row * topk + j0 + j] : -1;
+        for (int j = 0; j < SLOTS; ++j) pos[j] = j0 + j < topk ? pos_of_pair[row * topk + j0 + j] : -1;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (pos[j] >= 0) p[j] = __ldg(reinterpret_cast<const float4*>(part + (size_t)pos[j] * d + n0));
+        for (int j = 0; j < SLOTS; ++j)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+          for (int s = 0; s < PL; ++s)
+            if (pos[j] >= 0 && s < S) p[j][s] = __ldg(reinterpret_cast<const float4*>(part + (size_t)s * plane + (size_t)pos[j] * d + n0));
+#pragma unroll
+        for (int j = 0; j < SLOTS; ++j) {
           if (pos[j] < 0) continue;     // warp-uniform
           const int pair = row * topk + j0 + j;
           float y[4];
-          moe_rotate_scale(p[j], svh_down == nullptr ? nullptr : svh_down + (size_t)ids[pair] * d + n0, y);
+#pragma unroll
+          for (int s = 1; s < PL; ++s)
+            if (s < S) { p[j][0].x += p[j][s].x; p[j][0].y += p[j][s].y; p[j][0].z += p[j][s].z; p[j][0].w += p[j][s].w; }
+          moe_rotate_scale(p[j][0], svh_down == nullptr ? nullptr : svh_down + (size_t)ids[pair] * d + n0, y);
           const float wj = w[pair];
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[i] = fmaf(wj, y[i], acc[i]);
@@ -736,7 +743,7 @@ RX_API int rx_moe_combine(const void* part, int S, int pairs_cap, int M, int d, 
   if (gy < 1) gy = 1;
   int warps = (blocks + gy - 1) / gy;
   if (warps > 8) warps = 8;
-  return (int)rx::launch(S == 1 ? moe_combine_kernel<true> : moe_combine_kernel<false>, dim3(M, gy), dim3(32 * warps), 0, (cudaStream_t)stream, (const float*)part, S, pairs_cap, M, d, topk,
+  return (int)rx::launch(S == 1 ? moe_combine_kernel<1> : S <= 4 ? moe_combine_kernel<4> : moe_combine_kernel<0>, dim3(M, gy), dim3(32 * warps), 0, (cudaStream_t)stream, (const float*)part, S, pairs_cap, M, d, topk,
                          (const int*)ids, (const float*)w, (const int*)pos_of_pair, (const __half*)svh_down, (const float*)shared, tp);
 }
 

@@ -38,8 +38,8 @@ def test_plan_is_a_stable_sort(pairs, E, lo, hi):
 
 
 @pytest.mark.parametrize("M,topk", [(3, 1), (70, 8), (70, 10), (5, 17)])
-def test_one_plane_forms_equal_the_general_ones(M, topk):
-    """A second plane of zeros selects the general form and changes no bit of a sum."""
+def test_forms_of_few_planes_equal_the_general_ones(M, topk):
+    """Further planes of zeros select the other forms (one plane, up to four, any number) and change no bit of a sum."""
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
     from rexl3_b200.models.moe import CombineDst
@@ -53,7 +53,7 @@ def test_one_plane_forms_equal_the_general_ones(M, topk):
     w, svh, gu, dn = r(pairs).abs(), r(E, d).half(), r(pairs, 2 * F), r(pairs, d)
     svh_gu, suh, exp, tot = r(E, 2 * F).half(), r(E, F).half(), ids.clone(), torch.tensor([pairs], dtype=torch.int32, device="cuda")
     got = []
-    for S in (1, 2):
+    for S in (1, 2, 4, 5):
         planes = lambda t: torch.stack([t] + [torch.zeros_like(t)] * (S - 1))  # noqa: E731,B023
         slot, act = torch.zeros(M, d, device="cuda"), torch.zeros(pairs, F, dtype=torch.float16, device="cuda")
         dst = CombineDst()
@@ -64,6 +64,7 @@ def test_one_plane_forms_equal_the_general_ones(M, topk):
         lib.check(L.rx_moe_swiglu_rot(b.data_ptr(), S, pairs, F, exp.data_ptr(), tot.data_ptr(), svh_gu.data_ptr(), suh.data_ptr(), act.data_ptr(),
                                       lib.stream_ptr()), "rx_moe_swiglu_rot")
         got.append((slot, act))
-    for x, y in zip(*got):
-        assert torch.isfinite(x.float()).all() and x.abs().max() > 0 and torch.equal(x, y)
+    for other in got[1:]:
+        for x, y in zip(got[0], other):
+            assert torch.isfinite(x.float()).all() and x.abs().max() > 0 and torch.equal(x, y)
 
