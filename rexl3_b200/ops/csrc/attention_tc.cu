@@ -5,14 +5,19 @@
 // row's arithmetic does not depend on how the prompt was cut into chunks (chunked == whole, as the reference's prefill requires,
 // crates/cuda/csrc/attention.cu:768, nemotron_attn_prefill.cu:1-8; tiles, schedule and data path are new).
 //
-// Tensor memory (512 columns, 256 per tile): Q as the MMA's A operand (64 columns: 128 rows x 128 bf16), the scores S (64 fp32
-// columns; the bf16 probabilities P overwrite its first 32 columns and are the A operand of the PV MMA) and the output accumulator O
-// (128 fp32 columns).  Both MMAs therefore read only their B operand (a K or V page) from shared memory, and every page brought by
-// TMA serves both tiles.
+// Tensor memory (512 columns, 256 per tile): the scores S, two buffers in turn (64 fp32 columns each; the bf16 probabilities P overwrite a buffer's first
+// 32 columns and are the A operand of the PV MMA), and the output accumulator O (128 fp32 columns).  Q, the A operand of the QK MMA, stays in shared
+// memory.  Every page brought by TMA serves both tiles.
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer and TMEM owner, 2..5 / 6..9 = softmax of tile 0 / 1 (thread = query row = TMEM lane).  The
-// issuer alternates between the tiles (PV_t(j), QK_t(j+1) for t = 0, 1), so one tile's softmax runs while the tensor core works for the
-// other, and two softmax warps per scheduler hide each other's latencies.  The running maximum of a row moves only when it grows by more than 2^8 (the probabilities then stay below 2^8, harmless in fp32
+// Warps: 0 = TMA producer, 1 and 10 = MMA issuers of tile 0 and 1 (1 also owns the tensor memory), 2..5 / 6..9 = softmax of tile 0 / 1 (thread = query
+// row = TMEM lane).  An issuer runs QK two pages ahead of PV, so a tile's next scores are there when its softmax has finished a page, and two softmax warps
+// per scheduler hide each other's latencies.
+// What bounds it is the issue of the MMAs: an MMA of 128 x 64 x 16 keeps its thread for 66 cycles, one of 128 x 128 x 16 for 78 (32 and 64 of the tensor
+// core), a wait that is already over for 80.  8192 rows, 40 heads: 776 us (0.89 PFLOP/s); 1089 with one issuer for both tiles, 1173 with its
+// waits for pages between P and the MMAs, 1242 with one S buffer beside Q in tensor memory.  Whole-warp issue by a predicate (1248) and the
+// two tiles' QK and PV issued in turn (1372) were slower.
+//
+// The running maximum of a row moves only when it grows by more than 2^8 (the probabilities then stay below 2^8, harmless in fp32
 // sums and bf16 products); O is rescaled only in those steps.  Every such decision is per row, so a row's bits never depend on its
 // neighbours in the tile.  All waits are bounded (status words), no cluster multicast.
 #include <cuda.h>
@@ -26,9 +31,11 @@ constexpr int TC_ROWS = 128;                       // query rows per tile (TMEM 
 constexpr int TC_TILES = 2;                        // tiles per CTA: two softmax warpgroups take turns on the tensor core
 constexpr int TC_STAGES = 4;
 constexpr int TC_TILE = TC_PAGE * TC_HD * 2;       // bytes of one K (or V) page of one head: 16 KB
-constexpr int TC_THREADS = 64 + TC_TILES * 128;
-// tensor-memory columns of tile t: base 256 t; Q (A operand, 64) | S (64 fp32, P bf16 overwrites its first 32) | O (128 fp32)
-constexpr int TC_Q = 0, TC_S = 64, TC_O = 128, TC_TCOLS = 256, TC_COLS = 512;
+constexpr int TC_ISSUER_1 = 2 + TC_TILES * 4;      // the warp that issues the second tile's MMAs (the first's: warp 1)
+constexpr int TC_THREADS = 32 * (TC_ISSUER_1 + 1);
+constexpr int TC_QBOX = TC_ROWS * 128;             // bytes of one 64-wide half of a Q tile (K-major, 128B swizzle)
+// tensor-memory columns of tile t: base 256 t; two S buffers (64 fp32 each, P bf16 overwrites the first 32) | O (128 fp32)
+constexpr int TC_S = 64, TC_O = 128, TC_TCOLS = 256, TC_COLS = 512;
 
 __device__ __forceinline__ void tc_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -86,17 +93,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* k_sm = smem;                                  // [stage][box (64 d)][64 keys][128 B]
   uint8_t* v_sm = smem + TC_STAGES * TC_TILE;
-  uint64_t* bars = (uint64_t*)(smem + 2 * TC_STAGES * TC_TILE);
+  uint8_t* q_sm = smem + 2 * TC_STAGES * TC_TILE;         // [tile][half][128 rows][128 B]
+  uint64_t* bars = (uint64_t*)(q_sm + TC_TILES * 2 * TC_QBOX);
   uint64_t* k_full = bars;                         // [STAGES] TMA
   uint64_t* v_full = k_full + TC_STAGES;           // [STAGES] TMA
-  uint64_t* k_empty = v_full + TC_STAGES;          // [STAGES] commit after the page's last QK
-  uint64_t* v_empty = k_empty + TC_STAGES;         // [STAGES] commit after the page's last PV
-  uint64_t* s_full = v_empty + TC_STAGES;          // [TILES] commit after QK
-  uint64_t* p_ready = s_full + TC_TILES;           // [TILES] the tile's 4 softmax warps
-  uint64_t* pv_done = p_ready + TC_TILES;          // [TILES] commit after PV
+  uint64_t* k_empty = v_full + TC_STAGES;          // [STAGES] both tiles' commits after QK
+  uint64_t* v_empty = k_empty + TC_STAGES;         // [STAGES] both tiles' commits after PV
+  uint64_t* s_full = v_empty + TC_STAGES;          // [TILES][2] commit after QK
+  uint64_t* p_ready = s_full + 2 * TC_TILES;       // [TILES][2] the tile's 4 softmax warps
+  uint64_t* pv_done = p_ready + 2 * TC_TILES;      // [TILES] commit after PV
   uint64_t* q_ready = pv_done + TC_TILES;          // [1] all 8 softmax warps
-  uint64_t* drained = q_ready + 1;                 // [1] commit after the last MMA
-  uint32_t* tmem_slot = (uint32_t*)(drained + 1);
+  uint64_t* drained = q_ready + 1;                 // [TILES] commit after the last MMA
+  uint32_t* tmem_slot = (uint32_t*)(drained + TC_TILES);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int s_idx = blockIdx.z, hq = blockIdx.y;
@@ -119,10 +127,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
   const int npages = max(nst[0], nst[1]);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < TC_STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1); }
-    for (int i = 0; i < TC_TILES; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); mbar_init(&pv_done[i], 1); }
+    for (int i = 0; i < TC_STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], TC_TILES); mbar_init(&v_empty[i], TC_TILES); }
+    for (int i = 0; i < 2 * TC_TILES; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); }
+    for (int i = 0; i < TC_TILES; ++i) mbar_init(&pv_done[i], 1);
     mbar_init(q_ready, 4 * TC_TILES);
-    mbar_init(drained, 1);
+    for (int i = 0; i < TC_TILES; ++i) mbar_init(&drained[i], 1);
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tk);
@@ -154,49 +163,59 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
         tma_load_2d(v_sm + st * TC_TILE + 8192, &tv, 64, y, &v_full[st]);
       }
     }
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
+  } else if (warp == 1 || warp == TC_ISSUER_1) {
+    // ---------------------------------------------------------------- MMA issuer of one tile
     if (lane == 0) {
+      const int t = warp == 1 ? 0 : 1, mine = nst[t];
       const uint32_t idesc_qk = umma_idesc_f16(TC_ROWS, TC_PAGE, 1, 1);                 // bf16 x bf16, both K-major
       const uint32_t idesc_pv = umma_idesc_f16(TC_ROWS, TC_HD, 1, 1) | (1u << 16);      // B (V) is MN-major
+      const uint64_t qd = umma_desc_k_sw128(smem_u32(q_sm + t * 2 * TC_QBOX));
+      const uint32_t tb = tmem_base + t * TC_TCOLS;
       bool ok = mbar_wait(q_ready, 0, abort_flag, a.status, 72);
-      tc_fence_after();
-      // S_t = Q_t K(j)^T; the page's last user (the second tile while it still has steps, else the first) frees the K stage
-      auto issue_qk = [&](int t, int j) -> bool {
+      // S = Q K(j)^T into buffer j & 1, once the page is there.  Every page of the CTA is handed back by both tiles, also one that this tile does not need.
+      auto k_page = [&](int j) { return j >= npages || mbar_wait(&k_full[j % TC_STAGES], (j / TC_STAGES) & 1, abort_flag, a.status, 73); };
+      auto qk = [&](int j) {
         const int st = j % TC_STAGES;
-        if (!mbar_wait(&k_full[st], (j / TC_STAGES) & 1, abort_flag, a.status, 73)) return false;
-        tc_fence_after();
+        if (j >= npages) return;
+        if (j >= mine) {
+          mbar_arrive(&k_empty[st]);
+          return;
+        }
         const uint64_t kd = umma_desc_k_sw128(smem_u32(k_sm + st * TC_TILE));
-        const uint32_t tb = tmem_base + t * TC_TCOLS;
+        const uint32_t s_col = tb + (j & 1) * TC_S;
 #pragma unroll
         for (int kk = 0; kk < TC_HD / 16; ++kk)
-          tc_mma_f16_ts(tb + TC_S, tb + TC_Q + kk * 8, kd + (uint64_t)((kk >> 2) * (8192 >> 4) + (kk & 3) * 2), idesc_qk, kk != 0);
-        if (t == 1 || j >= nst[1]) tc_commit(&k_empty[st]);
-        tc_commit(&s_full[t]);
-        return true;
+          tc_mma_f16(s_col, qd + (uint64_t)((kk >> 2) * (TC_QBOX >> 4) + (kk & 3) * 2), kd + (uint64_t)((kk >> 2) * (8192 >> 4) + (kk & 3) * 2), idesc_qk, kk != 0);
+        tc_commit(&s_full[2 * t + (j & 1)]);
+        tc_commit(&k_empty[st]);
       };
-      for (int t = 0; t < TC_TILES && ok; ++t)
-        if (nst[t] > 0) ok = issue_qk(t, 0);
+      for (int j = 0; j < 2 && ok; ++j) {
+        ok = k_page(j);
+        tc_fence_after();
+        if (ok) qk(j);
+      }
       for (int j = 0; j < npages && ok; ++j) {
+        // the pages first (a wait costs 80 cycles even when it is over): once P is there, nothing stands between it and its MMAs
         const int st = j % TC_STAGES;
-        for (int t = 0; t < TC_TILES && ok; ++t) {
-          if (j >= nst[t]) continue;
-          if (!mbar_wait(&p_ready[t], j & 1, abort_flag, a.status, 74)) { ok = false; break; }
-          if (!mbar_wait(&v_full[st], (j / TC_STAGES) & 1, abort_flag, a.status, 75)) { ok = false; break; }
-          tc_fence_after();
+        ok = mbar_wait(&v_full[st], (j / TC_STAGES) & 1, abort_flag, a.status, 75) && k_page(j + 2);
+        if (ok && j < mine) ok = mbar_wait(&p_ready[2 * t + (j & 1)], (j >> 1) & 1, abort_flag, a.status, 74);
+        if (!ok) break;
+        tc_fence_after();
+        if (j < mine) {
           const uint32_t vbase = smem_u32(v_sm + st * TC_TILE);
-          const uint32_t tb = tmem_base + t * TC_TCOLS;
 #pragma unroll
           for (int kk = 0; kk < TC_PAGE / 16; ++kk)
-            tc_mma_f16_ts(tb + TC_O, tb + TC_S + kk * 8, umma_desc_mn_sw128(vbase + kk * 2048, 8192u, 1024u), idesc_pv, (j | kk) != 0);
-          if (t == 1 || j >= nst[1]) tc_commit(&v_empty[st]);
+            tc_mma_f16_ts(tb + TC_O, tb + (j & 1) * TC_S + kk * 8, umma_desc_mn_sw128(vbase + kk * 2048, 8192u, 1024u), idesc_pv, (j | kk) != 0);
           tc_commit(&pv_done[t]);
-          if (j + 1 < nst[t]) ok = issue_qk(t, j + 1);      // overwrites S_t / P_t after PV_t(j) has read it (MMAs run in issue order)
+          tc_commit(&v_empty[st]);
+        } else {
+          mbar_arrive(&v_empty[st]);
         }
+        qk(j + 2);                                            // overwrites P(j) after PV(j) has read it (a thread's MMAs run in issue order)
       }
       // every MMA issued so far has completed when this commit arrives: the columns may then be returned
-      tc_commit(drained);
-      for (int i = 0; i < (1 << 22) && !mbar_try_wait(drained, 0); ++i) {}   // bounded, and not cut short by the abort word
+      tc_commit(&drained[t]);
+      for (int i = 0; i < (1 << 22) && !mbar_try_wait(&drained[t], 0); ++i) {}   // bounded, and not cut short by the abort word
     }
   } else {
     // ---------------------------------------------------------------- softmax warps: thread = query row = TMEM lane of its tile
@@ -208,29 +227,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
     const int kmax = p0 + lrow;                           // last key this row may see
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + t * TC_TCOLS;
     const int nsteps = nst[t];
-    // Q row -> tensor memory (A operand layout: column c = elements 2c, 2c + 1)
+    // Q row -> shared memory: 128-byte rows, 16-byte chunk c of a half at c ^ (row & 7)
     {
       const uint4* src = reinterpret_cast<const uint4*>(a.q + ((size_t)(r_base + (live ? lrow : 0)) * a.n_q + hq) * TC_HD);
+      uint8_t* dst = q_sm + t * 2 * TC_QBOX + row * 128;
 #pragma unroll
-      for (int part = 0; part < 2; ++part) {
-        uint32_t r[32];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          uint4 v = live ? __ldg(src + part * 8 + i) : make_uint4(0u, 0u, 0u, 0u);
-          r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
-        }
-        tc_st_32x32b_x32(lane_addr + TC_Q + part * 32, r);
-      }
-      tc_wait_st();
-      tc_fence_before();
+      for (int i = 0; i < 16; ++i)
+        *reinterpret_cast<uint4*>(dst + (i >> 3) * TC_QBOX + (((i & 7) ^ (row & 7)) << 4)) = live ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+      fence_proxy_async();                                // (the MMA reads it through the async proxy)
       __syncwarp();
       if (lane == 0) mbar_arrive(q_ready);
     }
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < nsteps && ok; ++j) {
-      const uint32_t s_addr = lane_addr + TC_S;
-      ok = mbar_wait(&s_full[t], j & 1, abort_flag, a.status, 76);
+      const uint32_t s_addr = lane_addr + (j & 1) * TC_S;
+      ok = mbar_wait(&s_full[2 * t + (j & 1)], (j >> 1) & 1, abort_flag, a.status, 76);
       if (!ok) break;
       tc_fence_after();
       const int key0 = j * TC_PAGE;
@@ -293,7 +305,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_ready[t]);
+      if (lane == 0) mbar_arrive(&p_ready[2 * t + (j & 1)]);
     }
     // epilogue: O / l -> bf16 -> out
     if (ok && nsteps > 0) ok = mbar_wait(&pv_done[t], (nsteps - 1) & 1, abort_flag, a.status, 78);
@@ -334,7 +346,7 @@ RX_API int rx_attn_prefill_tc(const void* tmap_k, const void* tmap_v, const void
                               const void* q_start, const void* q_len, const void* pos0, void* out, int nseq, int max_qlen, int n_q, int n_kv, int hd,
                               float scale, int* status, void* stream, int v_desc_variant) {
   if (hd != TC_HD || n_q % n_kv != 0 || nseq <= 0 || max_qlen <= 0) return (int)cudaErrorInvalidValue;
-  const int smem = 2 * TC_STAGES * TC_TILE + 256 + 1024;
+  const int smem = 2 * TC_STAGES * TC_TILE + TC_TILES * 2 * TC_QBOX + 256 + 1024;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
