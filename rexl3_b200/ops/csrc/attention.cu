@@ -490,7 +490,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
                    const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_seq, const int* __restrict__ ctx_len,
                    float* __restrict__ part_o, float* __restrict__ part_ml, int n_q, int n_kv, int max_chunks, float scale_log2_in, int* status,
                    const float* __restrict__ kv_scale, const int* __restrict__ plan, const float* __restrict__ k_ts, const float* __restrict__ v_ts,
-                   const int* __restrict__ vbt) {
+                   const int* __restrict__ vbt, int chunk_end) {
   static_assert(!I8 || FP8, "the int8 cache uses the byte-page path");
   pdl_launch();
   pdl_wait();
@@ -505,7 +505,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kw = warp;                               // this warp's 16-key slice of every page
   const int G = n_q / n_kv;
-  const int total = plan[0], nb = plan[1];
+  constexpr bool HEAD_ONLY = HD == 128 && FP8 && I8 == 0;       // may be asked for the chunks below chunk_end alone (0: all of them)
+  const int nb = plan[1], total = HEAD_ONLY && chunk_end > 0 ? nb * chunk_end * n_kv : plan[0];
   const int* blk_row = plan + PLAN_HEAD;
   const int* blk_n = blk_row + PLAN_MAX_ROWS;
   const int* prefix = blk_n + 2 * PLAN_MAX_ROWS;
@@ -520,12 +521,18 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
   __syncthreads();
   int gp = 0;                                        // pages this CTA has consumed so far: stage and barrier phase follow it
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
-    int lo = 0, hi = nb - 1;                         // the block whose item range holds `item`
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (prefix[mid] <= item) lo = mid; else hi = mid - 1;
+    int lo = 0, local;
+    if (HEAD_ONLY && chunk_end > 0) {                // chunk_end chunks of every block, those that it has not are passed over
+      lo = item / (chunk_end * n_kv), local = item - lo * chunk_end * n_kv;
+      if (local / n_kv >= blk_n[PLAN_MAX_ROWS + lo] || blk_c0[lo] + local / n_kv >= chunk_end) continue;
+    } else {                                         // the block whose item range holds `item`
+      int hi = nb - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (prefix[mid] <= item) lo = mid; else hi = mid - 1;
+      }
+      local = item - prefix[lo];
     }
-    const int local = item - prefix[lo];
     const int row = blk_row[lo], nblk = blk_n[lo], kvh = local % n_kv, chunk = blk_c0[lo] + local / n_kv;
     const int seq = blk_seq[lo];
     const float scale_log2 = (FP8 && !I8) ? scale_log2_in * kv_scale[kvh] : scale_log2_in;     // K was stored as k / k_scale
@@ -700,13 +707,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 
 // E4M3 cache with 128-wide heads.  Same work items and masks as attn_decode_kernel, bound by HBM instead of by the expansion (that kernel turns every page
 // into fp16 tiles in shared memory, between two block barriers per page: 182 us for 6 sequences x 32,100 keys, 394 MB, where this one takes
-// 87 us).  A warp takes one whole page of the item's four: it is its own producer (two tiles, K and V; the next item's page is fetched into a
+// 86 us, and the other one 12 us for the first 1024 keys, which stay with it: see the launch).  A warp takes one whole page of the item's four: it is its own producer (two tiles, K and V; the next item's page is fetched into a
 // tile as soon as the warp has read it), needs no block barrier before the merge and no running maximum, and its MMAs run in eight
 // and more independent chains (one 16-key slice of every page per warp left it waiting for MMA latencies: 143 us).  The bytes go straight
 // into the fragments: the order of the head's 128 values along the MMAs' k (scores) and n (outputs) is free, so a lane takes 32 neighbouring bytes of
 // a K row and 16 of a V row, and a conversion of two bytes is a fragment register (V: after a byte permute that pairs two keys).  A block of
 // more than 16 (row, head) pairs goes over the page once per m16 tile, with the same instructions for every tile: a row's bits depend on
 // neither its tile nor its block mates.  A failed wait does not leave the loop (warps meet at barriers): every later wait then returns at once.
+constexpr int F8_FIRST_CHUNK = 4;           // it takes the chunks from this one on
 constexpr int F8_TILE = PAGE * 128, F8_HDP = 128 + 8;
 constexpr int F8_SMEM = 8 * F8_TILE + 4 * 16 * F8_HDP * 4 + 2 * 4 * 16 * 2 * 4 + 8 * 8 + 16 + 1024;
 // four bytes -> two fp16 pairs
@@ -717,7 +725,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2)
 attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const uint16_t* __restrict__ q,
                       const int* __restrict__ block_table, int max_blocks, const int* __restrict__ ctx_len, float* __restrict__ part_o,
                       float* __restrict__ part_ml, int n_q, int n_kv, int max_chunks, float scale_log2_in, int* status,
-                      const float* __restrict__ kv_scale, const int* __restrict__ plan, const int* __restrict__ vbt) {
+                      const float* __restrict__ kv_scale, const int* __restrict__ plan, const int* __restrict__ vbt, int chunk_begin) {
   constexpr int HD = 128, HDP = F8_HDP;
   pdl_launch();
   pdl_wait();
@@ -746,11 +754,11 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
   __syncthreads();
   struct Item { int row, nblk, kvh, chunk, k_begin, k_end, y; };         // y: first row of this warp's page in the tensor maps, -1: no such page
   int blk = 0;
-  // items come in ascending order: the block that holds the next one is this one's or a little further
-  auto locate = [&](int item) {
-    Item it;
+  // items come in ascending order: the block that holds the next one is this one's or a little further.  false: a chunk below chunk_begin
+  auto locate = [&](int item, Item& it) {
     while (blk + 1 < nb && prefix[blk + 1] <= item) ++blk;
     const int local = item - prefix[blk], seq = blk_seq[blk], c0 = blk_c0[blk];
+    if (c0 + local / n_kv < chunk_begin) return false;
     it.row = blk_row[blk], it.nblk = blk_n[blk], it.kvh = local % n_kv, it.chunk = c0 + local / n_kv;
     int ctx_max = 0;
     for (int i = 0; i < it.nblk; ++i) ctx_max = max(ctx_max, ctx_len[it.row + i]);
@@ -759,23 +767,27 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
     // a tree row's private table starts at the page index of its block's first chunk
     const int* bt = seq >= 0 ? block_table + (size_t)seq * max_blocks : vbt + (size_t)(-1 - seq) * VBT_W - c0 * (DEC_CHUNK / PAGE);
     it.y = it.k_begin + warp * PAGE < it.k_end ? (bt[it.k_begin / PAGE + warp] * n_kv + it.kvh) * PAGE : -1;
-    return it;
+    return true;
   };
   auto fetch = [&](uint8_t* dst, const CUtensorMap* map, int y, uint64_t* bar) {
     mbar_arrive_expect_tx(bar, F8_TILE);
     tma_load_2d(dst, map, 0, y, bar);
   };
-  Item it = locate(blockIdx.x);
+  Item it;
+  int item = blockIdx.x;
+  while (item < total && !locate(item, it)) item += gridDim.x;
+  if (item >= total) return;                           // (the same for the whole block)
   if (lane == 0 && it.y >= 0) {
     fetch(ktile, &tk, it.y, full_k);
     fetch(vtile, &tv, it.y, full_v);
   }
   uint32_t qa[8][4];
   int pages = 0, par = 0, q_row = -1, q_kvh = -1, q_nblk = 0;            // pages: consumed so far by this warp; q_*: whose queries qa holds
-  for (int item = blockIdx.x; item < total; item += gridDim.x) {
+  while (item < total) {
     Item next;
     next.y = -1;
-    if (item + (int)gridDim.x < total) next = locate(item + gridDim.x);
+    item += gridDim.x;                                 // the next one of this block's
+    while (item < total && !locate(item, next)) item += gridDim.x;
     const float scale_log2 = scale_log2_in * kv_scale[it.kvh], v_scale = kv_scale[n_kv + it.kvh];     // K was stored as k / k_scale
     const int ntiles = (it.nblk * G + 15) >> 4, kpos = it.k_begin + warp * PAGE;
     const bool any = it.y >= 0;                      // uniform for the warp
@@ -1237,8 +1249,12 @@ static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, co
   // persistent: two CTAs per SM at most, never more than the items the window can have
   const long long bound = (long long)rows * n_kv * mc;
   const int grid = (int)(bound < 2 * sm_count() ? bound : 2 * sm_count());
+  int chunk_end = 0, head_grid = grid;
   if constexpr (HD == 128 && FP8 && I8 == 0) {
-    if ((((uintptr_t)q) & 15) == 0) {               // its queries come in 16-byte pieces
+    // attn_decode_f8_kernel from key 1024 on (its queries come in 16-byte pieces), a matter of the key's position alone, so a row's bits do not depend on
+    // the window.  Below, the kernel of the other byte caches: it costs little there, and a short sequence, whose new row is a large part of the cache's
+    // bytes, keeps them to the bit.
+    if (mc > F8_FIRST_CHUNK && (((uintptr_t)q) & 15) == 0) {
       static bool ready = false;
       if (!ready) {
         cudaError_t e = cudaFuncSetAttribute(attn_decode_f8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F8_SMEM);
@@ -1246,8 +1262,12 @@ static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, co
         ready = true;
       }
       rx::launch(attn_decode_f8_kernel, dim3(grid), dim3(ATT_THREADS), F8_SMEM, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, ctx_len, part_o, part_ml,
-                 n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, vbt);
-      return (int)cudaGetLastError();
+                 n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, vbt, F8_FIRST_CHUNK);
+      cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return (int)e;
+      chunk_end = F8_FIRST_CHUNK;
+      const long long head = (long long)rows * n_kv * F8_FIRST_CHUNK;
+      head_grid = (int)(head < 2 * sm_count() ? head : 2 * sm_count());
     }
   }
   constexpr int smem = dec_smem_bytes(HD, FP8, MT);
@@ -1257,8 +1277,8 @@ static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, co
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  rx::launch(attn_decode_kernel<HD, FP8, MT, I8>, dim3(grid), dim3(ATT_THREADS), smem, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, row_seq,
-             ctx_len, part_o, part_ml, n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, k_ts, v_ts, vbt);
+  rx::launch(attn_decode_kernel<HD, FP8, MT, I8>, dim3(head_grid), dim3(ATT_THREADS), smem, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, row_seq,
+             ctx_len, part_o, part_ml, n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, k_ts, v_ts, vbt, chunk_end);
   return (int)cudaGetLastError();
 }
 

@@ -40,7 +40,7 @@ def _run(K, maps, q, scale, seq, ctx, bt, n_q, n_kv, msr):
 def test_decode_over_e4m3_pages(n_q, n_kv, rows):
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
-    ctxs = [0, 1, 62, 63, 64, 254, 255, 256, 511, 700, 1023, 3000]
+    ctxs = [0, 1, 62, 63, 64, 254, 255, 256, 511, 700, 1023, 1024, 1279, 1280, 3000]
     K, kc, vc, q, scale, seq, ctx, bt, maps = _case(ctxs, rows, n_q, n_kv, n_q + rows)
     out = _run(K, maps, q, scale, seq, ctx, bt, n_q, n_kv, rows)
     for r in range(len(seq)):
