@@ -181,6 +181,8 @@ __global__ void __launch_bounds__(256) finish_store_kernel(const float* __restri
 
 // h[row] += y (bf16 residual stream, updated in place); then xr = fp16(H(rmsnorm(h) * w * suh_next)).
 // norm_w == nullptr skips the norm, suh_next == nullptr skips the rotation output entirely (residual update only).
+// The products with suh_next stay plain: they are fused into the rotation's first additions, here and in norm_rot_in_kernel alike (a norm weight times
+// a scale that is not +-1 has more bits than fp32 holds).
 __global__ void __launch_bounds__(1024) finish_add_norm_rot_kernel(const float* __restrict__ part, int S, int M, int N, const __half* __restrict__ svh,
                                            const float* __restrict__ bias, uint16_t* __restrict__ h, const uint16_t* __restrict__ norm_w,
                                            float eps, const __half* __restrict__ suh_next, __half* __restrict__ xr,
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(1024) finish_add_norm_rot_kernel(const float* 
     if (xn_out != nullptr) store4_bf16(xn_out + (size_t)row * N + n0, v);   // the normalised row itself (router input, per-expert rotations)
     if (suh_next == nullptr) continue;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __fmul_rn(v[i], s[i]);
+    for (int i = 0; i < 4; ++i) v[i] *= s[i];
     fwht128_warp(v);
     store4_f16(xr + (size_t)row * N + n0, v);
   }
@@ -294,7 +296,7 @@ __global__ void __cluster_dims__(FEW_CTAS, 1, 1) __launch_bounds__(FEW_WARPS * 3
   if (xn_out != nullptr) store4_bf16(xn_out + (size_t)row * N + n0, v);
   if (suh_next == nullptr) return;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = __fmul_rn(v[i], s[i]);
+  for (int i = 0; i < 4; ++i) v[i] *= s[i];
   fwht128_warp(v);
   store4_f16(xr + (size_t)row * N + n0, v);
 }
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(256) finish_add_norm_rot_rows_kernel(const flo
     float s[4];
     load4_f16(suh_next + n0, s);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[i][e] = __fmul_rn(v[i][e], s[e]);
+    for (int e = 0; e < 4; ++e) v[i][e] *= s[e];
     fwht128_warp(v[i]);
     store4_f16(xr + base + b * 128, v[i]);
   }

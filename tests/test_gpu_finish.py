@@ -56,6 +56,25 @@ def test_add_norm_rot_of_few_rows(N, S, norm, rot, xn):
         assert torch.isfinite(x.float()).all() and torch.equal(x, y)
 
 
+@pytest.mark.parametrize("M", [1, 16, 37, 64, 65, 523])               # clusters, one CTA a row, the row form
+@pytest.mark.parametrize("N", [640, 2048, 5120])
+def test_add_norm_rot_rounds_as_norm_rot_in(M, N):
+    """Residual rows of powers of two have the same sum of squares in any order; the rotated rows are then those of norm_rot_in, bit for bit, also
+    for input scales that are not +-1."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = _weight(N, g)
+    w.bias = None
+    h = torch.exp2(torch.randint(-2, 3, (M, N), device="cuda", generator=g).float()).bfloat16()
+    nw, suh = (1 + 0.1 * torch.randn(N, device="cuda", generator=g)).bfloat16(), torch.randn(N, device="cuda", generator=g).half()
+    xr, want = (torch.zeros(M, N, dtype=torch.float16, device="cuda") for _ in range(2))
+    K.norm_rot_in(h, nw, 1e-6, suh, want)
+    K.finish_add_norm_rot(torch.zeros(2, M, N, device="cuda"), 2 if M < 512 else 1, M, w, h.clone(), nw, 1e-6, suh, xr)
+    assert torch.isfinite(xr).all() and xr.abs().max() > 0 and torch.equal(xr, want)
+
+
 @pytest.mark.parametrize("hd,n_q,n_kv", [(128, 40, 8), (128, 3, 1), (64, 4, 2)])
 def test_qkv_rope_rows_do_not_depend_on_their_number(hd, n_q, n_kv):
     if not torch.cuda.is_available():
