@@ -27,27 +27,6 @@ namespace rx {
 constexpr int SSM_P = 64, SSM_N = 128, SSM_HIST = 3;
 constexpr int SCAN_OUT = 1, SCAN_STATE = 2;
 
-// two fp32 operations in one instruction (each half rounds as its scalar form): halves the issue slots of the recurrences
-__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float f2_sum(uint64_t v) {
-  float lo, hi;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-  return lo + hi;
-}
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // asynchronous copies into shared memory: the inputs of the next tokens arrive while the current ones are computed
 __device__ __forceinline__ void cp16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -428,49 +407,41 @@ __global__ void __launch_bounds__(256) ssm_gate_norm_kernel(const float* __restr
 // output gate is a sigmoid instead of SiLU.  Everything else is the same code.
 constexpr int GDN_D = 128;
 
+// the write of a token: beta (v - S.k / |k|), with the key's 1 / |k| once more (k enters the update normalised as well)
+__device__ __forceinline__ float gdn_delta(float v, float kv, float beta, float kinv) { return __fmaf_rn(-kv, kinv, v) * beta * kinv; }
 // One token of the delta rule for the 64 state values of a thread (value column j, one half of the keys): decay, S.k (both halves meet in one
-// shuffle), the rank-one write, S.q.  A dot product is taken over eighths of the keys (16 each, four partial sums), then as a tree
-// over the eighths: the order of gdn_scan_split_kernel, whose threads hold one eighth of two columns, so that both leave the same bits.
+// shuffle), the rank-one write, S.q.  Four partial sums per dot product, key i in sum i % 4, keep the dependent chains at 16 instead of 64; a thread of
+// gdn_scan_split_kernel holds one such chain, so that both kernels leave the same bits.
 // sk / sq / sd: this half's 64 keys, queries and (KDA) decays in shared memory, 16-byte aligned.  o is returned before the 1 / |q| factor.
 template <bool KDA>
 __device__ __forceinline__ void gdn_token_update(float (&st)[64], const float* sk, const float* sq, const float* sd, float decay, float v, float beta,
-                                                 float kinv, float& kv_out, float& o_out) {
-  float part[4];
+                                                 float kinv, float& o_out) {
+  float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    float k0 = 0.f, k1 = 0.f, k2 = 0.f, k3 = 0.f;
-#pragma unroll
-    for (int i = 16 * u; i < 16 * u + 16; i += 4) {
-      const float4 kk = *reinterpret_cast<const float4*>(sk + i);
-      if (KDA) {
-        const float4 dd = *reinterpret_cast<const float4*>(sd + i);
-        st[i] *= dd.x; st[i + 1] *= dd.y; st[i + 2] *= dd.z; st[i + 3] *= dd.w;
-      } else {
-        st[i] *= decay; st[i + 1] *= decay; st[i + 2] *= decay; st[i + 3] *= decay;
-      }
-      k0 = __fmaf_rn(st[i], kk.x, k0); k1 = __fmaf_rn(st[i + 1], kk.y, k1); k2 = __fmaf_rn(st[i + 2], kk.z, k2); k3 = __fmaf_rn(st[i + 3], kk.w, k3);
+  for (int i = 0; i < 64; i += 4) {
+    const float4 kk = *reinterpret_cast<const float4*>(sk + i);
+    if (KDA) {
+      const float4 dd = *reinterpret_cast<const float4*>(sd + i);
+      st[i] *= dd.x; st[i + 1] *= dd.y; st[i + 2] *= dd.z; st[i + 3] *= dd.w;
+    } else {
+      st[i] *= decay; st[i + 1] *= decay; st[i + 2] *= decay; st[i + 3] *= decay;
     }
-    part[u] = (k0 + k1) + (k2 + k3);
+    k0 = __fmaf_rn(st[i], kk.x, k0); k1 = __fmaf_rn(st[i + 1], kk.y, k1); k2 = __fmaf_rn(st[i + 2], kk.z, k2); k3 = __fmaf_rn(st[i + 3], kk.w, k3);
   }
-  float kv = (part[0] + part[1]) + (part[2] + part[3]);
-  kv = (kv + __shfl_xor_sync(0xffffffffu, kv, 1)) * kinv;
-  const float delta = __fsub_rn(v, kv) * beta * kinv;          // k enters the update normalised as well
+  float kv = (k0 + k1) + (k2 + k3);
+  kv = kv + __shfl_xor_sync(0xffffffffu, kv, 1);
+  const float delta = gdn_delta(v, kv, beta, kinv);
+  float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
-#pragma unroll
-    for (int i = 16 * u; i < 16 * u + 16; i += 4) {
-      const float4 kk = *reinterpret_cast<const float4*>(sk + i);
-      const float4 qq = *reinterpret_cast<const float4*>(sq + i);
-      st[i] = __fmaf_rn(kk.x, delta, st[i]); st[i + 1] = __fmaf_rn(kk.y, delta, st[i + 1]);
-      st[i + 2] = __fmaf_rn(kk.z, delta, st[i + 2]); st[i + 3] = __fmaf_rn(kk.w, delta, st[i + 3]);
-      o0 = __fmaf_rn(st[i], qq.x, o0); o1 = __fmaf_rn(st[i + 1], qq.y, o1); o2 = __fmaf_rn(st[i + 2], qq.z, o2); o3 = __fmaf_rn(st[i + 3], qq.w, o3);
-    }
-    part[u] = (o0 + o1) + (o2 + o3);
+  for (int i = 0; i < 64; i += 4) {
+    const float4 kk = *reinterpret_cast<const float4*>(sk + i);
+    const float4 qq = *reinterpret_cast<const float4*>(sq + i);
+    st[i] = __fmaf_rn(kk.x, delta, st[i]); st[i + 1] = __fmaf_rn(kk.y, delta, st[i + 1]);
+    st[i + 2] = __fmaf_rn(kk.z, delta, st[i + 2]); st[i + 3] = __fmaf_rn(kk.w, delta, st[i + 3]);
+    o0 = __fmaf_rn(st[i], qq.x, o0); o1 = __fmaf_rn(st[i + 1], qq.y, o1); o2 = __fmaf_rn(st[i + 2], qq.z, o2); o3 = __fmaf_rn(st[i + 3], qq.w, o3);
   }
-  float o = (part[0] + part[1]) + (part[2] + part[3]);
+  float o = (o0 + o1) + (o2 + o3);
   o = o + __shfl_xor_sync(0xffffffffu, o, 1);
-  kv_out = kv;
   o_out = o;
 }
 
@@ -539,8 +510,8 @@ __global__ void __launch_bounds__(256, 2) gdn_scan_kernel(const float* __restric
       decay = __expf(A * a);
     }
     const float beta = 1.f / (1.f + __expf(-proj[(size_t)r * ldp + goff + h]));
-    float kv, o;
-    gdn_token_update<KDA>(st, sk, sq, sdec + (KDA ? half * 64 : 0), decay, v, beta, kinv, kv, o);
+    float o;
+    gdn_token_update<KDA>(st, sk, sq, sdec + (KDA ? half * 64 : 0), decay, v, beta, kinv, o);
     o *= qinv;
     const float ss2 = warp_sum(half == 0 ? __fmul_rn(o, o) : 0.f);
     if (lane == 0) red2[warp] = ss2;
@@ -562,9 +533,9 @@ __global__ void __launch_bounds__(256, 2) gdn_scan_kernel(const float* __restric
 }
 
 // ---- prefill / commit form of the delta-rule scan.  A head's 128 value columns evolve independently (S_j only meets q and k): they are split over
-// GDN_JS CTAs of four warps.  A thread holds 2 columns x 16 keys: what bounds the kernel is the way of k and q out of shared memory (a vector
-// load costs four cycles of the SM however many lanes read the same word), and two columns share what is loaded; one column x 32 keys ran at
-// 70 % of that limit and took 811 us where this form takes 549 us (900 + 1148 tokens, 48 heads).  Products are packed pairs; a token's critical path is
+// GDN_JS CTAs of four warps.  A thread holds two columns x one of the partial sums of gdn_token_update, 16 keys (4 i + sub of a half): what bounds the
+// kernel is the way of k and q out of shared memory (a vector load costs four cycles of the SM however many lanes read the same word), and two columns
+// share what is loaded; k, q and the decays are laid out by thread, so that its 16 keys are four vectors.  A token's critical path is
 // a 16-key dot product, three shuffles and the rank-one write; the output sums of four tokens go over the lanes together, off that path.  What a
 // token needs besides (1 / |q|, 1 / |k|, decay, write strength) is computed for GDN_TC tokens at a time by the CTA from the inputs that cp.async
 // brought into two buffers (norm sums per token and warp: 40 shuffles, 0.96 us per token, 1105 us).  Every rounding and every order of a sum
@@ -575,7 +546,7 @@ template <bool KDA> struct GdnChunk {
   static constexpr int TC = KDA ? 8 : 16;
   float q[TC][GDN_PAD], k[TC][GDN_PAD], d[KDA ? TC : 1][GDN_PAD], v[TC][GDN_D / GDN_JS], a[TC], b[TC];
 };
-__device__ __forceinline__ int gdn_pad(int i) { return i + ((i >> 4) << 2); }
+__device__ __forceinline__ int gdn_place(int i) { return (((i >> 4) & 4) + (i & 3)) * 20 + ((i >> 2) & 15); }     // key i: thread group, place in its 16
 template <bool KDA>
 __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
                                                             int goff, int M, int Hk, int Hv, const int* __restrict__ row_seq,
@@ -590,28 +561,26 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
   const int r0 = seg_start[blockIdx.x], len = seg_len[blockIdx.x];
   if (len <= 0) return;
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int sub = lane & 3, half = (lane >> 2) & 1, jl = warp * 8 + (lane >> 3) + 4 * (lane & 1), j = blockIdx.z * JC + jl;
-  const int dj = (lane & 1) ? -4 : 4;     // slot 0 is column j, slot 1 column j + dj: of a pair, a lane passes slot 1 on in a sum's tree
+  const int sub = lane & 3, half = (lane >> 2) & 1, jl = warp * 8 + (lane >> 3), j = blockIdx.z * JC + jl;     // columns j and j + 4
+  const bool odd = (lane & 1) != 0;       // an odd lane holds them the other way round: of a pair, a lane passes its slot 1 on in a sum's tree
   const int seq = row_seq[r0], hk = h / (Hv / Hk), DI = Hv * GDN_D;
-  uint64_t st[2][8];                                                   // keys 64 half + 16 sub + (0 .. 15) of the two columns
-  float* sp = s_pool + ((size_t)seq * Hv + h) * (GDN_D * GDN_D) + (size_t)((j >> 4) * 16 + sub * 4) * 128 + (2 * (j & 15) + half) * 4;
+  float st[2][16];                                                     // keys 64 half + 4 (0 .. 15) + sub of the two columns
+  float* sp = s_pool + ((size_t)seq * Hv + h) * (GDN_D * GDN_D) + (size_t)(j >> 4) * (16 * 128) + (2 * (j & 15) + half) * 4 + sub;
   const bool fresh = positions[r0] == 0;
 #pragma unroll
-  for (int c = 0; c < 2; ++c)
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      ulonglong2 v = make_ulonglong2(0ull, 0ull);
-      if (!fresh) v = *reinterpret_cast<const ulonglong2*>(sp + u * 128 + c * 8 * dj);
-      st[c][2 * u] = v.x, st[c][2 * u + 1] = v.y;
-    }
+  for (int m = 0; m < 16; ++m) {
+    const float a = fresh ? 0.f : sp[m * 128], b = fresh ? 0.f : sp[m * 128 + 32];
+    st[0][m] = odd ? b : a, st[1][m] = odd ? a : b;
+  }
   const float A = a_neg[h], dtb = KDA ? dt_bias[h * GDN_D + tid] : dt_bias[h];
+  const int place = gdn_place(tid);
   auto issue = [&](int c) {                                            // past the end the last row again (never used)
     GdnChunk<KDA>& d = buf[c & 1];
-    const int k = tid & 31;
-    for (int t = warp; t < TC; t += 4) {
-      const float* xr = xbc + (size_t)(r0 + min(c * TC + t, len - 1)) * C;
-      cp16(&d.q[t][gdn_pad(4 * k)], xr + hk * GDN_D + 4 * k);
-      cp16(&d.k[t][gdn_pad(4 * k)], xr + (Hk + hk) * GDN_D + 4 * k);
+#pragma unroll
+    for (int t = 0; t < TC; ++t) {
+      const float* xr = xbc + (size_t)(r0 + min(c * TC + t, len - 1)) * C + hk * GDN_D + tid;
+      cp4(&d.q[t][place], xr);
+      cp4(&d.k[t][place], xr + Hk * GDN_D);
     }
     if (tid < TC * 8) {
       const int t = tid >> 3, kv = tid & 7;
@@ -620,7 +589,7 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
     if (KDA) {
 #pragma unroll
       for (int t = 0; t < TC; ++t)
-        cp4(&d.d[t][gdn_pad(tid)], proj + (size_t)(r0 + min(c * TC + t, len - 1)) * ldp + goff + Hv + h * GDN_D + tid);
+        cp4(&d.d[t][place], proj + (size_t)(r0 + min(c * TC + t, len - 1)) * ldp + goff + Hv + h * GDN_D + tid);
     }
     if (tid < TC) {
       const float* pr = proj + (size_t)(r0 + min(c * TC + tid, len - 1)) * ldp + goff;
@@ -629,7 +598,7 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
     }
     cp_commit();
   };
-  const int kb = (4 * half + sub) * 20;
+  const int kb = (4 * half + sub) * 20, j0 = jl + (odd ? 4 : 0);       // j0: the column of slot 0
   // NT tokens (4, or 1 at the end): the states in turn, then the NT x 2 output sums over the eight lanes of a column pair together
   auto tokens = [&](const GdnChunk<KDA>& d, auto n, int t0, int r) {
     constexpr int NT = decltype(n)::value;
@@ -638,51 +607,47 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
     for (int i = 0; i < NT; ++i) {
       const int t = t0 + i;
       const float4 gt = gate[t];
-      const float val = d.v[t][jl];
-      uint64_t kk[8], a[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
+      float kk[16], a[2] = {0.f, 0.f};
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&d.k[t][kb + 4 * u]);
-        kk[2 * u] = v.x, kk[2 * u + 1] = v.y;
-        ulonglong2 dd;
-        if (KDA) dd = *reinterpret_cast<const ulonglong2*>(&d.d[t][kb + 4 * u]);
-        else dd.x = dd.y = f2_pack(gt.x, gt.x);
+        const float4 v = *reinterpret_cast<const float4*>(&d.k[t][kb + 4 * u]);
+        kk[4 * u] = v.x, kk[4 * u + 1] = v.y, kk[4 * u + 2] = v.z, kk[4 * u + 3] = v.w;
+        float4 dd = make_float4(gt.x, gt.x, gt.x, gt.x);
+        if (KDA) dd = *reinterpret_cast<const float4*>(&d.d[t][kb + 4 * u]);
+        const float de[4] = {dd.x, dd.y, dd.z, dd.w};
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          st[c][2 * u] = f2_mul(st[c][2 * u], dd.x);
-          st[c][2 * u + 1] = f2_mul(st[c][2 * u + 1], dd.y);
-          a[c][0] = f2_fma(st[c][2 * u], v.x, a[c][0]);
-          a[c][1] = f2_fma(st[c][2 * u + 1], v.y, a[c][1]);
-        }
+        for (int m = 4 * u; m < 4 * u + 4; ++m)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            st[c][m] *= de[m & 3];
+            a[c] = __fmaf_rn(st[c][m], kk[m], a[c]);
+          }
       }
-      float kv = f2_sum(a[0][0]) + f2_sum(a[0][1]);
-      const float kv1 = f2_sum(a[1][0]) + f2_sum(a[1][1]);
-      kv += __shfl_xor_sync(0xffffffffu, kv1, 1);
+      float kv = a[0] + __shfl_xor_sync(0xffffffffu, a[1], 1);         // the four partial sums of a half, then the halves
       kv += __shfl_xor_sync(0xffffffffu, kv, 2);
-      kv = (kv + __shfl_xor_sync(0xffffffffu, kv, 4)) * gt.z;
-      const float delta = __fsub_rn(val, kv) * gt.y * gt.z, delta1 = __shfl_xor_sync(0xffffffffu, delta, 1);
-      const uint64_t dl[2] = {f2_pack(delta, delta), f2_pack(delta1, delta1)};
-      a[0][0] = a[0][1] = a[1][0] = a[1][1] = 0ull;
+      kv += __shfl_xor_sync(0xffffffffu, kv, 4);
+      const float delta = gdn_delta(d.v[t][j0], kv, gt.y, gt.z), dl[2] = {delta, __shfl_xor_sync(0xffffffffu, delta, 1)};
+      a[0] = a[1] = 0.f;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(&d.q[t][kb + 4 * u]);
+        const float4 v = *reinterpret_cast<const float4*>(&d.q[t][kb + 4 * u]);
+        const float qq[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          st[c][2 * u] = f2_fma(kk[2 * u], dl[c], st[c][2 * u]);
-          st[c][2 * u + 1] = f2_fma(kk[2 * u + 1], dl[c], st[c][2 * u + 1]);
-          a[c][0] = f2_fma(st[c][2 * u], qq.x, a[c][0]);
-          a[c][1] = f2_fma(st[c][2 * u + 1], qq.y, a[c][1]);
-        }
+        for (int m = 4 * u; m < 4 * u + 4; ++m)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            st[c][m] = __fmaf_rn(kk[m], dl[c], st[c][m]);
+            a[c] = __fmaf_rn(st[c][m], qq[m & 3], a[c]);
+          }
       }
-#pragma unroll
-      for (int c = 0; c < 2; ++c) o[i][c] = f2_sum(a[c][0]) + f2_sum(a[c][1]);
+      o[i][0] = a[0], o[i][1] = a[1];
     }
     if (!(mode & SCAN_OUT)) return;
     const bool b1 = (lane & 2) != 0, b2 = (lane & 4) != 0;
     float m[NT];
 #pragma unroll
     for (int i = 0; i < NT; ++i) m[i] = o[i][0] + __shfl_xor_sync(0xffffffffu, o[i][1], 1);
-    float* yp = y32 + (size_t)r * DI + h * GDN_D + j;
+    float* yp = y32 + (size_t)r * DI + h * GDN_D + blockIdx.z * JC + j0;
     if constexpr (NT == 4) {                                           // bits 1 and 2 pick the token
       const float n0 = (b1 ? m[2] : m[0]) + __shfl_xor_sync(0xffffffffu, b1 ? m[0] : m[2], 2);
       const float n1 = (b1 ? m[3] : m[1]) + __shfl_xor_sync(0xffffffffu, b1 ? m[1] : m[3], 2);
@@ -708,8 +673,9 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
     for (int i = 0; i < TC / 4; ++i)
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
-        const float* x = (w ? d.k[warp + 4 * i] : d.q[warp + 4 * i]) + (lane >> 3) * 40 + (lane & 7);
-        rs[i][w] = (__fmul_rn(x[0], x[0]) + __fmul_rn(x[20], x[20])) + (__fmul_rn(x[8], x[8]) + __fmul_rn(x[28], x[28]));
+        // values n, n + 8, n + 16 and n + 24 of a 32 stand two places apart each
+        const float* x = (w ? d.k[warp + 4 * i] : d.q[warp + 4 * i]) + gdn_place(32 * (lane >> 3) + (lane & 7));
+        rs[i][w] = (__fmul_rn(x[0], x[0]) + __fmul_rn(x[4], x[4])) + (__fmul_rn(x[2], x[2]) + __fmul_rn(x[6], x[6]));
       }
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1)
@@ -740,9 +706,9 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
     if (KDA) {
 #pragma unroll
       for (int t = 0; t < TC; ++t) {
-        float ai = d.d[t][gdn_pad(tid)] + dtb;
+        float ai = d.d[t][place] + dtb;
         ai = ai > 20.f ? ai : log1pf(__expf(ai));
-        d.d[t][gdn_pad(tid)] = __expf(A * ai);
+        d.d[t][place] = __expf(A * ai);
       }
     }
     __syncthreads();
@@ -754,9 +720,7 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
   pdl_launch();
   if (!(mode & SCAN_STATE)) return;
 #pragma unroll
-  for (int c = 0; c < 2; ++c)
-#pragma unroll
-    for (int u = 0; u < 4; ++u) *reinterpret_cast<ulonglong2*>(sp + u * 128 + c * 8 * dj) = make_ulonglong2(st[c][2 * u], st[c][2 * u + 1]);
+  for (int m = 0; m < 16; ++m) sp[m * 128] = odd ? st[1][m] : st[0][m], sp[m * 128 + 32] = odd ? st[0][m] : st[1][m];
   ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h * GDN_JS + blockIdx.z, (int)(gridDim.y * GDN_JS));
 }
 

@@ -39,6 +39,54 @@ def test_delta_prefill_equals_row_form(lens, pad, kda):
         assert torch.isfinite(a.float()).all() and torch.equal(a, b)
 
 
+def _fma(a, b, c):
+    return (a.double() * b.double() + c.double()).float()        # (one rounding but for cases of 2^-29: products of fp32 are exact in fp64)
+
+
+def _norm_inv(x):
+    s = (x * x).view(4, 32)
+    for o in (16, 8, 4, 2, 1):
+        s = s[:, :o] + s[:, o:]
+    return torch.rsqrt(s[0, 0] + s[1, 0] + s[2, 0] + s[3, 0] + 1e-6)
+
+
+def _dot(st, x):
+    """S.x of every column (st [columns, 128]): per half of the keys four sums over every fourth key, then (0 + 1) + (2 + 3), then the halves."""
+    acc = torch.zeros(st.shape[0], 2, 4, device="cuda")
+    for i in range(16):
+        acc = _fma(st.view(-1, 2, 16, 4)[:, :, i], x.view(2, 16, 4)[:, i], acc)
+    s = (acc[..., 0] + acc[..., 1]) + (acc[..., 2] + acc[..., 3])
+    return s[:, 0] + s[:, 1]
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("T", [1, 6, 21])
+def test_delta_rule_adds_in_its_order(split, T):
+    """States and outputs bit for bit as the delta rule in fp32 gives them in the documented order of its sums (no decay, write strength 1)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import kernels as K
+    D, C = 128, 3 * 128
+    r, proj, seq, pos, st, ln, conv = _inputs(D + C + 2, C, T, D + C + 2, [T], T)
+    proj[:, D + C] = 60.0                                             # sigmoid -> 1
+    pool, xbc, y32 = r(1, D * D), torch.empty(T * C, device="cuda"), torch.zeros(T, D, device="cuda")
+    pos += 3                                                          # goes on from the pool
+    S = pool.view(8, 16, 16, 2, 4).permute(0, 2, 3, 1, 4).reshape(D, D)   # [column / 16][step][column % 16][half][e] -> [column][key]
+    one, zero = torch.ones(1, device="cuda"), torch.zeros(1, device="cuda")
+    K.gdn_mixer(proj, T, 1, 1, D, seq, pos, *((st, ln, 1) if split else (None, None, 0)), 0.5 * r(C, 4).bfloat16(), r(C).bfloat16(), one, zero,
+                torch.ones(D, dtype=torch.bfloat16, device="cuda"), 1e-6, conv, pool, xbc, torch.zeros(T, D, dtype=torch.bfloat16, device="cuda"),
+                y32=y32 if split else None)
+    want = []
+    for q, k, v in xbc.view(T, 3, D):
+        kinv = _norm_inv(k)
+        delta = _fma(-_dot(S, k), kinv, v) * kinv
+        S = _fma(delta[:, None], k, S)
+        want.append(_dot(S, q) * (_norm_inv(q) * 0.08838834764831845))
+    assert torch.isfinite(S).all() and torch.equal(pool.view(8, 16, 16, 2, 4).permute(0, 2, 3, 1, 4).reshape(D, D), S)
+    if split:
+        assert torch.equal(y32, torch.stack(want))
+
+
 @pytest.mark.parametrize("lens", [[1], [3, 1], [16, 4, 5], [33, 2, 17, 1], [64, 7]])
 @pytest.mark.parametrize("H,G,pad", [(8, 2, 0), (8, 2, 1), (6, 2, 2), (48, 1, 0)])      # groups of 256, 192 and 3072 channels
 def test_mamba_prefill_equals_row_form(lens, H, G, pad):
