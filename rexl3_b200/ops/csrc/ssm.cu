@@ -225,15 +225,21 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const float* __restrict__
 // output is one of the sixteen chains that ssm_scan_kernel adds up.  Every rounding and every order of a sum is that kernel's: states and outputs
 // are the same bits.  (Packed pairs along n took 436 us, 463 us this way: what they save in issue slots is small, two of the three operations
 // read three registers, which the packed form issues every third cycle; a 4 x 4 tile on twice the warps is bound by the loads again: 506 us.)
-// The inputs of SSM_TC tokens at a time come by cp.async into two buffers, x dt and the decays are made from them by the CTA: two block barriers per
-// SSM_TC tokens, no global load on the per-token path.  The dependents are released only when the recurrence is done: released at the start, their
+// The inputs of TC tokens at a time come by cp.async into two buffers, x dt and the decays are made from them by the CTA: two block barriers per
+// TC tokens, no global load on the per-token path.  The dependents are released only when the recurrence is done: released at the start, their
 // waiting CTAs (thousands) took the SMs' slots and slowed it by half.
 // One sequence of 2047 tokens, 128 heads: 463 us; 2159 us before (1 x 32 tiles, one warp per CTA, register ring; 3220 us with early release).
-// grid (segments, H, SSM_PS), 128 threads.
-constexpr int SSM_PS = 2, SSM_CP = SSM_P / SSM_PS, SSM_TC = 16;
-struct SsmChunk { float B[SSM_TC][SSM_N], C[SSM_TC][SSM_N], x[SSM_TC][SSM_CP], dt[SSM_TC]; };
+// The states come and go through shared memory, whole rows in 16-byte pieces: a thread's own values, every fourth of a row, are half sectors, and a commit
+// is little else than its states (8 x 1 rows 57.5 us with them, 32 us in the one-warp form, 20 us now).
+// grid (segments, H, SSM_PS), 128 threads; TC tokens to a chunk.
+constexpr int SSM_PS = 2, SSM_CP = SSM_P / SSM_PS;
+template <int TC> struct SsmChunk { float B[TC][SSM_N], C[TC][SSM_N], x[TC][SSM_CP], dt[TC]; };
 // where n stands in a token's B and C: the eight values of a thread (nq, k) as two vectors, sixteen threads' vectors side by side
 __device__ __forceinline__ int ssm_place(int n) { return ((n >> 4) & 1) * 64 + ((n >> 5) * 4 + (n & 3)) * 4 + ((n >> 2) & 3); }
+// where value n of a state row stands on its way through shared memory: the lanes of a warp, at any m, then meet different banks
+constexpr int SSM_SROW = SSM_N + 4;
+__device__ __forceinline__ int ssm_stage(int n) { return n ^ ((n >> 5) << 2); }
+template <int TC>
 __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
                                                             int dtoff, int M, int H, int G, const int* __restrict__ row_seq,
                                                             const int* __restrict__ positions, const int* __restrict__ seg_start,
@@ -241,8 +247,12 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
                                                             const float* __restrict__ a_neg, const float* __restrict__ d_skip,
                                                             float* __restrict__ ssm_pool, float* conv_pool, float* __restrict__ y, int mode) {
   pdl_wait();
-  __shared__ __align__(16) SsmChunk buf[2];
-  __shared__ float xdt[SSM_TC][SSM_CP], dec[SSM_TC];                         // x dt and the decay of the current chunk
+  // two chunks; the states' way in and out takes the second one's place
+  constexpr int STAGE = SSM_CP * SSM_SROW * 4, CHUNK = (int)sizeof(SsmChunk<TC>);
+  __shared__ __align__(16) uint8_t raw[CHUNK + (CHUNK > STAGE ? CHUNK : STAGE)];
+  SsmChunk<TC>* buf = reinterpret_cast<SsmChunk<TC>*>(raw);
+  float* stage = reinterpret_cast<float*>(raw + CHUNK);
+  __shared__ float xdt[TC][SSM_CP], dec[TC];                         // x dt and the decay of the current chunk
   const int r0 = seg_start[blockIdx.x], len = seg_len[blockIdx.x];
   if (len <= 0) return;
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ln = lane & 15, lp = lane >> 4;
@@ -251,25 +261,24 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
   // upper slots, without selects.
   const int pl = warp * 8 + lp * 4, sel = (ln & 1 ? 2 : 0) | (ln & 2 ? 1 : 0);
   float st[4][8];
-  float* sp = ssm_pool + (((size_t)seq * H + h) * SSM_P + p0 + pl) * SSM_N + (ln >> 2) * 32 + (ln & 3);
+  float* sp = ssm_pool + (((size_t)seq * H + h) * SSM_P + p0) * SSM_N;
   const bool fresh = positions[r0] == 0;
+  if (!fresh)
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int m = 0; m < 8; ++m) st[p][m] = fresh ? 0.f : sp[(p ^ sel) * SSM_N + 4 * m];
+    for (int i = 0; i < SSM_CP / 4; ++i) cp16(&stage[(4 * i + warp) * SSM_SROW + ssm_stage(4 * lane)], sp + (4 * i + warp) * SSM_N + 4 * lane);
   const int place = ssm_place(tid);
-  auto issue = [&](int c) {                         // tokens c * SSM_TC ..; past the end the last row again (never used)
-    SsmChunk& d = buf[c & 1];
+  auto issue = [&](int c) {                         // tokens c * TC ..; past the end the last row again (never used)
+    SsmChunk<TC>& d = buf[c & 1];
     const float* src = xbc + DI + g * SSM_N + tid;
 #pragma unroll
-    for (int t = 0; t < SSM_TC; ++t) {
-      const float* xr = src + (size_t)(r0 + min(c * SSM_TC + t, len - 1)) * C;
+    for (int t = 0; t < TC; ++t) {
+      const float* xr = src + (size_t)(r0 + min(c * TC + t, len - 1)) * C;
       cp4(&d.B[t][place], xr);
       cp4(&d.C[t][place], xr + G * SSM_N);
     }
     const int t = tid >> 3;
-    cp16(&d.x[t][4 * (tid & 7)], xbc + (size_t)(r0 + min(c * SSM_TC + t, len - 1)) * C + h * SSM_P + p0 + 4 * (tid & 7));
-    if (tid < SSM_TC) cp4(&d.dt[tid], proj + (size_t)(r0 + min(c * SSM_TC + tid, len - 1)) * ldp + dtoff + h);
+    if (t < TC) cp16(&d.x[t][4 * (tid & 7)], xbc + (size_t)(r0 + min(c * TC + t, len - 1)) * C + h * SSM_P + p0 + 4 * (tid & 7));
+    if (tid < TC) cp4(&d.dt[tid], proj + (size_t)(r0 + min(c * TC + tid, len - 1)) * ldp + dtoff + h);
     cp_commit();
   };
   const float A = a_neg[h], Dh = d_skip[h], dtb = dt_bias[h];
@@ -277,7 +286,7 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
   float* yp = y + h * SSM_P + p0 + pl + sel;        // slot 0's row: the one whose sums end in this lane
   // NT tokens (4, or 1 at the end): the states in turn, then all NT x 4 output sums over the 16 lanes together, each step halving what a lane
   // carries on.  A sum's tree over the lanes (distances 1, 2, 4, 8) does not depend on NT.
-  auto tokens = [&](const SsmChunk& d, auto n, int t0, int r) {
+  auto tokens = [&](const SsmChunk<TC>& d, auto n, int t0, int r) {
     constexpr int NT = decltype(n)::value;
     float k[NT];
 #pragma unroll
@@ -315,13 +324,20 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
     }
   };
   issue(0);
-  const int nc = (len + SSM_TC - 1) / SSM_TC;
+  const int own = (ln >> 2) * 32 + (ln & 3);
+  cp_wait_all();
+  __syncthreads();
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int m = 0; m < 8; ++m) st[p][m] = fresh ? 0.f : stage[(pl + (p ^ sel)) * SSM_SROW + ssm_stage(own + 4 * m)];
+  const int nc = (len + TC - 1) / TC;
   for (int c = 0; c < nc; ++c) {
     cp_wait_all();
     __syncthreads();                                // chunk c has landed, everybody is done with chunk c - 1
     if (c + 1 < nc) issue(c + 1);
-    const SsmChunk& d = buf[c & 1];
-    {
+    const SsmChunk<TC>& d = buf[c & 1];
+    if (TC == 16 || tid < 8 * TC) {
       const int t = tid >> 3, p = 4 * (tid & 7);    // eight threads per token
       float dt = d.dt[t] + dtb;
       dt = dt > 20.f ? dt : log1pf(__expf(dt));     // softplus
@@ -330,17 +346,22 @@ __global__ void __launch_bounds__(128) ssm_scan_split_kernel(const float* __rest
       if (p == 0) dec[t] = __expf(dt * A);
     }
     __syncthreads();
-    const int nt = min(SSM_TC, len - c * SSM_TC);
+    const int nt = min(TC, len - c * TC);
     int t = 0;
-    for (; t + 4 <= nt; t += 4) tokens(d, std::integral_constant<int, 4>(), t, r0 + c * SSM_TC + t);
-    for (; t < nt; ++t) tokens(d, std::integral_constant<int, 1>(), t, r0 + c * SSM_TC + t);
+    for (; t + 4 <= nt; t += 4) tokens(d, std::integral_constant<int, 4>(), t, r0 + c * TC + t);
+    for (; t < nt; ++t) tokens(d, std::integral_constant<int, 1>(), t, r0 + c * TC + t);
   }
   pdl_launch();
   if (!(mode & SCAN_STATE)) return;
+  __syncthreads();                                  // (the last tokens have been read)
 #pragma unroll
   for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int m = 0; m < 8; ++m) sp[(p ^ sel) * SSM_N + 4 * m] = st[p][m];
+    for (int m = 0; m < 8; ++m) stage[(pl + (p ^ sel)) * SSM_SROW + ssm_stage(own + 4 * m)] = st[p][m];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < SSM_CP / 4; ++i)
+    *reinterpret_cast<float4*>(sp + (4 * i + warp) * SSM_N + 4 * lane) = *reinterpret_cast<const float4*>(&stage[(4 * i + warp) * SSM_SROW + ssm_stage(4 * lane)]);
   ssm_conv_commit(proj, ldp, xoff, conv_pool, C, row_seq, positions, r0 + len - 1, seq, h * SSM_PS + blockIdx.z, (int)(gridDim.y * SSM_PS));
 }
 
@@ -537,26 +558,25 @@ __global__ void __launch_bounds__(256, 2) gdn_scan_kernel(const float* __restric
 // kernel is the way of k and q out of shared memory (a vector load costs four cycles of the SM however many lanes read the same word), and two columns
 // share what is loaded; k, q and the decays are laid out by thread, so that its 16 keys are four vectors.  A token's critical path is
 // a 16-key dot product, three shuffles and the rank-one write; the output sums of four tokens go over the lanes together, off that path.  What a
-// token needs besides (1 / |q|, 1 / |k|, decay, write strength) is computed for GDN_TC tokens at a time by the CTA from the inputs that cp.async
+// token needs besides (1 / |q|, 1 / |k|, decay, write strength) is computed for TC tokens at a time by the CTA from the inputs that cp.async
 // brought into two buffers (norm sums per token and warp: 40 shuffles, 0.96 us per token, 1105 us).  Every rounding and every order of a sum
 // is gdn_scan_kernel's, so states and outputs are the same bits; the per-head gated norm, which needs all 128 outputs, runs afterwards in
 // gdn_norm_kernel.  The dependents are released at the end (see ssm_scan_split_kernel).  grid (segments, Hv, GDN_JS), 128 threads.
 constexpr int GDN_JS = 4, GDN_PAD = GDN_D + 32;                       // 16 keys every 20 floats: eight lanes' vectors in different banks
-template <bool KDA> struct GdnChunk {
-  static constexpr int TC = KDA ? 8 : 16;
+template <bool KDA, int TC> struct GdnChunk {
   float q[TC][GDN_PAD], k[TC][GDN_PAD], d[KDA ? TC : 1][GDN_PAD], v[TC][GDN_D / GDN_JS], a[TC], b[TC];
 };
 __device__ __forceinline__ int gdn_place(int i) { return (((i >> 4) & 4) + (i & 3)) * 20 + ((i >> 2) & 15); }     // key i: thread group, place in its 16
-template <bool KDA>
+template <bool KDA, int TC>
 __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __restrict__ xbc, int C, const float* __restrict__ proj, int ldp, int xoff,
                                                             int goff, int M, int Hk, int Hv, const int* __restrict__ row_seq,
                                                             const int* __restrict__ positions, const int* __restrict__ seg_start,
                                                             const int* __restrict__ seg_len, const float* __restrict__ dt_bias,
                                                             const float* __restrict__ a_neg, float* __restrict__ s_pool, float* conv_pool,
                                                             float* __restrict__ y32, int mode) {
-  constexpr int TC = GdnChunk<KDA>::TC, JC = GDN_D / GDN_JS;
+  constexpr int JC = GDN_D / GDN_JS;
   pdl_wait();
-  __shared__ __align__(16) GdnChunk<KDA> buf[2];
+  __shared__ __align__(16) GdnChunk<KDA, TC> buf[2];
   __shared__ __align__(16) float4 gate[TC];                            // decay, beta, 1 / |k|, 1 / |q| of a token
   const int r0 = seg_start[blockIdx.x], len = seg_len[blockIdx.x];
   if (len <= 0) return;
@@ -575,7 +595,7 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
   const float A = a_neg[h], dtb = KDA ? dt_bias[h * GDN_D + tid] : dt_bias[h];
   const int place = gdn_place(tid);
   auto issue = [&](int c) {                                            // past the end the last row again (never used)
-    GdnChunk<KDA>& d = buf[c & 1];
+    GdnChunk<KDA, TC>& d = buf[c & 1];
 #pragma unroll
     for (int t = 0; t < TC; ++t) {
       const float* xr = xbc + (size_t)(r0 + min(c * TC + t, len - 1)) * C + hk * GDN_D + tid;
@@ -600,7 +620,7 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
   };
   const int kb = (4 * half + sub) * 20, j0 = jl + (odd ? 4 : 0);       // j0: the column of slot 0
   // NT tokens (4, or 1 at the end): the states in turn, then the NT x 2 output sums over the eight lanes of a column pair together
-  auto tokens = [&](const GdnChunk<KDA>& d, auto n, int t0, int r) {
+  auto tokens = [&](const GdnChunk<KDA, TC>& d, auto n, int t0, int r) {
     constexpr int NT = decltype(n)::value;
     float o[NT][2];
 #pragma unroll
@@ -666,7 +686,7 @@ __global__ void __launch_bounds__(128) gdn_scan_split_kernel(const float* __rest
     cp_wait_all();
     __syncthreads();                                                   // chunk c has landed, everybody is done with chunk c - 1
     if (c + 1 < nc) issue(c + 1);
-    GdnChunk<KDA>& d = buf[c & 1];
+    GdnChunk<KDA, TC>& d = buf[c & 1];
     // norms: gdn_scan_kernel's warp sums over 32 values (tree over lane distances 16, 8, 4, 2, 1), eight lanes with four values each
     float rs[TC / 4][2];
 #pragma unroll
@@ -791,11 +811,15 @@ RX_API int rx_ssm_mixer(const void* proj, int ldp, int M, int H, int P, int G, i
   if (P != SSM_P || N != SSM_N || G <= 0 || H % G || M <= 0) return (int)cudaErrorInvalidValue;
   const int DI = H * P, C = DI + 2 * G * N, xoff = DI, dtoff = DI + C;
   if (ldp < dtoff + H) return (int)cudaErrorInvalidValue;
+  if ((((uintptr_t)ssm_pool) & 15) != 0) return (int)cudaErrorMisalignedAddress;       // every form moves the states in 16-byte pieces
   cudaStream_t st = (cudaStream_t)stream;
   if (mode & SCAN_OUT)
     launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
+  // Commits begin early (the layers' follow one another: one row 7.4 us alone, 5.7 so for the delta net), and short ones take chunks of four tokens: a quarter
+  // of the shared memory and of the gates' work (8 x 1 rows of the delta net 21.3 -> 15.8 us, of Mamba2 57.5 -> 20.1 together with the states' way).
+  const bool short_commit = mode == SCAN_STATE && M <= 4 * nseg;
   if (seg_start != nullptr && (((uintptr_t)xbc) & 15) == 0)     // segments known on the host (prefill, commit); its copies take 16 bytes
-    launch_alone(ssm_scan_split_kernel, dim3(nseg, H, SSM_PS), dim3(128), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
+    launch_pdl(mode == SCAN_STATE, short_commit ? ssm_scan_split_kernel<4> : ssm_scan_split_kernel<16>, dim3(nseg, H, SSM_PS), dim3(128), 0, st, (const float*)xbc, C, (const float*)proj, ldp, xoff, dtoff, M, H, G,
            (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len, (const float*)dt_bias, (const float*)a_neg,
            (const float*)d_skip, (float*)ssm_pool, (float*)conv_pool, (float*)y, mode);
   else
@@ -824,8 +848,12 @@ RX_API int rx_gdn_mixer(const void* proj, int ldp, int M, int Hk, int Hv, int D,
   if (mode & SCAN_OUT)
     launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
   if (seg_start != nullptr && y32 != nullptr && ((((uintptr_t)xbc) | ((uintptr_t)y32)) & 15) == 0) {
-    // segments known on the host (prefill, commit): the column-split scan with prefetched inputs, then the norm (same bits as the fused kernel)
-    launch_alone(kda ? gdn_scan_split_kernel<true> : gdn_scan_split_kernel<false>, dim3(nseg, Hv, GDN_JS), dim3(128), 0, st, (const float*)xbc, C,
+    // segments known on the host (prefill, commit): the column-split scan with prefetched inputs, then the norm (same bits as the fused kernel).  Commits
+    // begin early and short ones take chunks of four tokens (see rx_ssm_mixer).
+    const bool short_commit = mode == SCAN_STATE && M <= 4 * nseg;
+    auto gdn_scan = kda ? gdn_scan_split_kernel<true, 8> : gdn_scan_split_kernel<false, 16>;
+    if (short_commit) gdn_scan = kda ? gdn_scan_split_kernel<true, 4> : gdn_scan_split_kernel<false, 4>;
+    launch_pdl(mode == SCAN_STATE, gdn_scan, dim3(nseg, Hv, GDN_JS), dim3(128), 0, st, (const float*)xbc, C,
            (const float*)proj, ldp, xoff, goff, M, Hk, Hv, (const int*)row_seq, (const int*)positions, (const int*)seg_start, (const int*)seg_len,
            (const float*)dt_bias, (const float*)a_neg, (float*)s_pool, (float*)conv_pool, (float*)y32, mode);
     if (mode & SCAN_OUT)

@@ -108,6 +108,46 @@ def test_mamba_prefill_equals_row_form(lens, H, G, pad):
         assert torch.isfinite(a).all() and torch.equal(a, b)
 
 
+@pytest.mark.parametrize("kept", [[1], [4], [1, 4, 2, 0, 3], [9, 1, 1, 0], [5, 3, 5], [17, 16]])       # up to four rows a segment: short chunks
+@pytest.mark.parametrize("kind", ["mamba", "delta", "kda"])
+def test_commit_equals_row_form(kind, kept):
+    """The pools after a commit over the first `kept` rows of a window's segments against those after a direct run of these rows alone."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import kernels as K
+    lens = [max(1, k) if len(kept) == 4 else k + (i % 2) for i, k in enumerate(kept)]     # some segments lose rows, some lose all
+    M, kda = sum(lens), kind == "kda"
+    if kind == "mamba":
+        H, G = 8, 2
+        C, width = H * 64 + 2 * G * 128, 2 * H * 64 + 2 * G * 128 + H
+    else:
+        H, D = 6, 128
+        C, width = (4 + H) * D, (4 + 2 * H) * D + H + (H * D if kda else H)
+    r, proj, seq, pos, st, ln, conv0 = _inputs(width, C, M, width, lens, 7)
+    if kind == "mamba":
+        args = (0.5 * r(C, 4).bfloat16(), 0.1 * r(C).bfloat16(), r(H) - 2, -r(H).abs(), r(H), (1 + 0.1 * r(H * 64)).bfloat16())
+        s0 = 0.3 * r(len(lens), H, 64, 128)
+    else:
+        args = (r(C, 4).bfloat16(), r(C).bfloat16(), r(H * D if kda else H), -r(H).abs(), (1 + 0.1 * r(D)).bfloat16())
+        s0 = 0.3 * r(len(lens), H, D, D)
+
+    def run(proj, seq, pos, seg, conv, pool, xbc, mode):
+        n, y = proj.shape[0], torch.empty(proj.shape[0] * H * 128, device="cuda")
+        out = torch.zeros(n, H * (64 if kind == "mamba" else 128), dtype=torch.bfloat16, device="cuda")
+        if kind == "mamba":
+            K.ssm_mixer(proj, n, H, 64, G, 128, seq, pos, *seg, *args, 1e-6, conv, pool, xbc, y, out, mode=mode)
+        else:
+            K.gdn_mixer(proj, n, 2, H, D, seq, pos, *seg, *args, 1e-6, conv, pool, xbc, out, kda=kda, mode=mode, y32=y if seg[0] is not None else None)
+    conv, pool, xbc = conv0.clone(), s0.clone(), torch.empty(M * C, device="cuda")
+    run(proj, seq, pos, (None, None, 0), conv, pool, xbc, K.SCAN_RECORD)
+    assert torch.equal(conv, conv0) and torch.equal(pool, s0)
+    run(proj, seq, pos, (st, torch.tensor(kept, dtype=torch.int32, device="cuda"), len(kept)), conv, pool, xbc, K.SCAN_COMMIT)
+    rows = torch.tensor([sum(lens[:i]) + t for i, k in enumerate(kept) for t in range(k)], device="cuda")
+    conv1, pool1 = conv0.clone(), s0.clone()
+    run(proj[rows].contiguous(), seq[rows].contiguous(), pos[rows].contiguous(), (None, None, 0), conv1, pool1, torch.empty(len(rows) * C, device="cuda"), K.SCAN_FINAL)
+    assert not torch.equal(pool, s0) and torch.equal(pool, pool1) and torch.equal(conv, conv1)
+
+
 def test_conv_walking_rows_equals_one_row_per_thread():
     """The walking form of the convolution (rows in eighths, taken from 148 blocks on) against the one-row form, which an odd row stride selects:
     bit for bit, over segments that begin inside an eighth, and with the last eighth not full."""
