@@ -95,14 +95,13 @@ __global__ void __launch_bounds__(256) ssm_conv_rows_kernel(const float* __restr
   pdl_wait();
   const int rb = blockIdx.x * CONV_RB, c = (blockIdx.y * 256 + threadIdx.x) * 2;
   if (c >= C) return;
-  float x[CONV_RB + 3][2];                          // rows rb - 3 .. rb + CONV_RB - 1
-  int seq[CONV_RB];
+  float2 x[CONV_RB + 3];                            // rows rb - 3 .. rb + CONV_RB - 1
+  int seq[CONV_RB + 3];
 #pragma unroll
-  for (int i = 0; i < CONV_RB; ++i) {
-    const int r = min(rb + i, M - 1);
-    seq[i] = row_seq[r];
-    const float2 v = *reinterpret_cast<const float2*>(proj + (size_t)r * ldp + xoff + c);
-    x[i + 3][0] = v.x, x[i + 3][1] = v.y;
+  for (int i = 0; i < CONV_RB + 3; ++i) {
+    const int r = max(0, min(rb + i - 3, M - 1));
+    seq[i] = rb + i < 3 ? -1 : row_seq[r];
+    x[i] = *reinterpret_cast<const float2*>(proj + (size_t)r * ldp + xoff + c);
   }
   float w[2][4], bias[2];
 #pragma unroll
@@ -111,34 +110,46 @@ __global__ void __launch_bounds__(256) ssm_conv_rows_kernel(const float* __restr
 #pragma unroll
     for (int j = 0; j < 4; ++j) w[e][j] = ssm_bf(conv_w[(c + e) * 4 + j]);
   }
-#pragma unroll
-  for (int j = 0; j < 3; ++j)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) x[j][e] = ssm_conv_in(proj, ldp, xoff, pool, C, row_seq, positions, rb, 3 - j, c + e);
-#pragma unroll
-  for (int i = 0; i < CONV_RB; ++i) {
-    const int r = rb + i;
-    if (r >= M) break;
-    float in[4][2];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) in[j][0] = x[i + j][0], in[j][1] = x[i + j][1];
-    const bool near = i >= 3 ? seq[i] != seq[i - 3] : i > 0 && seq[i] != seq[0];
-    if (near) {                                     // another sequence's rows are among the three before: take them where they are kept
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) in[j][e] = ssm_conv_in(proj, ldp, xoff, pool, C, row_seq, positions, r, 3 - j, c + e);
-    }
+  auto put = [&](int i, float2 a, float2 b, float2 d) {
+    const float in[2][4] = {{a.x, b.x, d.x, x[i + 3].x}, {a.y, b.y, d.y, x[i + 3].y}};
     float o[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       float acc = bias[e];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc += w[e][j] * in[j][e];
+      for (int j = 0; j < 4; ++j) acc += w[e][j] * in[e][j];
       o[e] = ssm_silu(acc);
     }
-    *reinterpret_cast<float2*>(xbc + (size_t)r * C + c) = make_float2(o[0], o[1]);
+    if (rb + i < M) *reinterpret_cast<float2*>(xbc + (size_t)(rb + i) * C + c) = make_float2(o[0], o[1]);
+  };
+  bool whole = true;                                // every row's three predecessors are its sequence's
+#pragma unroll
+  for (int i = 0; i < CONV_RB; ++i) whole = whole && seq[i] == seq[i + 3];
+  if (whole) {
+#pragma unroll
+    for (int i = 0; i < CONV_RB; ++i) put(i, x[i], x[i + 1], x[i + 2]);
+    return;
   }
+  // Short segments: what a row's own segment does not have in this launch comes from the pool (positions first - 3 .. first - 1 of the segment) or
+  // is zero.  All rows' values are on their way before the first is used (layer of the delta net, 16 x 5 rows 62.5 us row after row, 56.3 so).
+  float2 p[CONV_RB][3];
+  int own = 0;
+#pragma unroll
+  for (int i = 0; i < CONV_RB; ++i) {
+    if (i == 0) own = seq[2] != seq[3] ? 0 : seq[1] != seq[3] ? 1 : seq[0] != seq[3] ? 2 : 3;
+    else own = seq[i + 3] == seq[i + 2] ? min(own + 1, 3) : 0;
+    const int pos = own < 3 ? positions[min(rb + i, M - 1)] : 0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {                   // 3 - j positions back
+      p[i][j] = x[i + j];
+      if (3 - j > own) {
+        p[i][j] = make_float2(0.f, 0.f);
+        if (pos >= 3 - j) p[i][j] = *reinterpret_cast<const float2*>(pool + ((size_t)seq[i + 3] * SSM_HIST + j + own) * C + c);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < CONV_RB; ++i) put(i, p[i][0], p[i][1], p[i][2]);
 }
 
 // Recurrence.  grid (segments or rows, H).  With a segment table (seg_start != nullptr) block x is segment x; without one block x is
@@ -782,13 +793,14 @@ __global__ void __launch_bounds__(256) gdn_norm_kernel(const float* __restrict__
   else op[0] = b[0], op[1] = b[1], op[2] = b[2], op[3] = b[3];
 }
 
-// The walking form needs pairs of channels (even widths, 8-byte alignment) and enough rows to fill the chip with eighths of them: from about 30
-// rows of 10240 channels on it is the faster one.
+// The walking form needs pairs of channels (even widths, 8-byte alignment), enough rows to fill the chip with eighths of them (64 of 10240 channels), and
+// rows that follow one another: prompt slices and verify windows.  A plain decode window has one row of each sequence and keeps the other form
+// (layer of the delta net, 64 x 1 rows 104.6 us and 108.1, 256 x 1 388 and 397; 16 x 5 rows 59.2 and 56.3, 32 x 8 167 and 158).
 static void launch_conv(const void* proj, int ldp, int xoff, int C, const void* row_seq, const void* positions, const void* conv_w, const void* conv_b,
-                        const void* conv_pool, void* xbc, int M, cudaStream_t st) {
-  const bool pairs = C % 2 == 0 && ldp % 2 == 0 && xoff % 2 == 0 && ((((uintptr_t)proj) | ((uintptr_t)xbc)) & 7) == 0;
+                        const void* conv_pool, void* xbc, int M, bool follow, cudaStream_t st) {
+  const bool pairs = C % 2 == 0 && ldp % 2 == 0 && xoff % 2 == 0 && ((((uintptr_t)proj) | ((uintptr_t)xbc) | ((uintptr_t)conv_pool)) & 7) == 0;
   const int cg = (C + 511) / 512;
-  if (pairs && (long long)(M / CONV_RB) * cg >= 148)
+  if (follow && pairs && (long long)(M / CONV_RB) * cg >= 148)
     launch(ssm_conv_rows_kernel, dim3((M + CONV_RB - 1) / CONV_RB, cg), dim3(256), 0, st, (const float*)proj, ldp, xoff, C, (const int*)row_seq,
            (const int*)positions, (const uint16_t*)conv_w, (const uint16_t*)conv_b, (const float*)conv_pool, (float*)xbc, M);
   else
@@ -814,7 +826,7 @@ RX_API int rx_ssm_mixer(const void* proj, int ldp, int M, int H, int P, int G, i
   if ((((uintptr_t)ssm_pool) & 15) != 0) return (int)cudaErrorMisalignedAddress;       // every form moves the states in 16-byte pieces
   cudaStream_t st = (cudaStream_t)stream;
   if (mode & SCAN_OUT)
-    launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
+    launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, seg_start != nullptr || mode == SCAN_OUT, st);
   // Commits begin early (the layers' follow one another: one row 7.4 us alone, 5.7 so for the delta net), and short ones take chunks of four tokens: a quarter
   // of the shared memory and of the gates' work (8 x 1 rows of the delta net 21.3 -> 15.8 us, of Mamba2 57.5 -> 20.1 together with the states' way).
   const bool short_commit = mode == SCAN_STATE && M <= 4 * nseg;
@@ -846,7 +858,7 @@ RX_API int rx_gdn_mixer(const void* proj, int ldp, int M, int Hk, int Hv, int D,
   if (ldp < goff + Hv + (kda ? Hv * D : Hv)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   if (mode & SCAN_OUT)
-    launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, st);
+    launch_conv(proj, ldp, xoff, C, row_seq, positions, conv_w, conv_b, conv_pool, xbc, M, seg_start != nullptr || mode == SCAN_OUT, st);
   if (seg_start != nullptr && y32 != nullptr && ((((uintptr_t)xbc) | ((uintptr_t)y32)) & 15) == 0) {
     // segments known on the host (prefill, commit): the column-split scan with prefetched inputs, then the norm (same bits as the fused kernel).  Commits
     // begin early and short ones take chunks of four tokens (see rx_ssm_mixer).
