@@ -13,6 +13,7 @@
 // each take 16 keys of every page and are merged in warp order.
 // Prefill (this file: FP8 caches and 64-wide heads): one CTA per (64 query rows, q head, sequence); warps own 16 query rows each and
 // walk the pages causally.  bf16 caches with 128-wide heads run the tcgen05 / tensor-memory kernel of attention_tc.cu instead.
+#include <type_traits>
 #include <cuda.h>
 #include <cuda_fp8.h>
 #include <cuda_fp4.h>
@@ -490,7 +491,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
                    const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_seq, const int* __restrict__ ctx_len,
                    float* __restrict__ part_o, float* __restrict__ part_ml, int n_q, int n_kv, int max_chunks, float scale_log2_in, int* status,
                    const float* __restrict__ kv_scale, const int* __restrict__ plan, const float* __restrict__ k_ts, const float* __restrict__ v_ts,
-                   const int* __restrict__ vbt, int chunk_end) {
+                   const int* __restrict__ vbt) {
   static_assert(!I8 || FP8, "the int8 cache uses the byte-page path");
   pdl_launch();
   pdl_wait();
@@ -505,8 +506,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kw = warp;                               // this warp's 16-key slice of every page
   const int G = n_q / n_kv;
-  constexpr bool HEAD_ONLY = HD == 128 && FP8 && I8 == 0;       // may be asked for the chunks below chunk_end alone (0: all of them)
-  const int nb = plan[1], total = HEAD_ONLY && chunk_end > 0 ? nb * chunk_end * n_kv : plan[0];
+  const int total = plan[0], nb = plan[1];
   const int* blk_row = plan + PLAN_HEAD;
   const int* blk_n = blk_row + PLAN_MAX_ROWS;
   const int* prefix = blk_n + 2 * PLAN_MAX_ROWS;
@@ -521,18 +521,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
   __syncthreads();
   int gp = 0;                                        // pages this CTA has consumed so far: stage and barrier phase follow it
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
-    int lo = 0, local;
-    if (HEAD_ONLY && chunk_end > 0) {                // chunk_end chunks of every block, those that it has not are passed over
-      lo = item / (chunk_end * n_kv), local = item - lo * chunk_end * n_kv;
-      if (local / n_kv >= blk_n[PLAN_MAX_ROWS + lo] || blk_c0[lo] + local / n_kv >= chunk_end) continue;
-    } else {                                         // the block whose item range holds `item`
-      int hi = nb - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (prefix[mid] <= item) lo = mid; else hi = mid - 1;
-      }
-      local = item - prefix[lo];
+    int lo = 0, hi = nb - 1;                         // the block whose item range holds `item`
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (prefix[mid] <= item) lo = mid; else hi = mid - 1;
     }
+    const int local = item - prefix[lo];
     const int row = blk_row[lo], nblk = blk_n[lo], kvh = local % n_kv, chunk = blk_c0[lo] + local / n_kv;
     const int seq = blk_seq[lo];
     const float scale_log2 = (FP8 && !I8) ? scale_log2_in * kv_scale[kvh] : scale_log2_in;     // K was stored as k / k_scale
@@ -705,18 +699,20 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
   }
 }
 
-// E4M3 cache with 128-wide heads.  Same work items and masks as attn_decode_kernel, bound by HBM instead of by the expansion (that kernel turns every page
-// into fp16 tiles in shared memory, between two block barriers per page: 182 us for 6 sequences x 32,100 keys, 394 MB, where this one takes
-// 86 us, and the other one 12 us for the first 1024 keys, which stay with it: see the launch).  A warp takes one whole page of the item's four: it is its own producer (two tiles, K and V; the next item's page is fetched into a
-// tile as soon as the warp has read it), needs no block barrier before the merge and no running maximum, and its MMAs run in eight
-// and more independent chains (one 16-key slice of every page per warp left it waiting for MMA latencies: 143 us).  The bytes go straight
-// into the fragments: the order of the head's 128 values along the MMAs' k (scores) and n (outputs) is free, so a lane takes 32 neighbouring bytes of
-// a K row and 16 of a V row, and a conversion of two bytes is a fragment register (V: after a byte permute that pairs two keys).  A block of
-// more than 16 (row, head) pairs goes over the page once per m16 tile, with the same instructions for every tile: a row's bits depend on
-// neither its tile nor its block mates.  A failed wait does not leave the loop (warps meet at barriers): every later wait then returns at once.
-constexpr int F8_FIRST_CHUNK = 4;           // it takes the chunks from this one on
+// E4M3 cache with 128-wide heads: the work items, masks and sums of attn_decode_kernel, whose expansion of every page into fp16 tiles, between two block
+// barriers, bound it.  All four pages of a chunk are in shared memory at once, so a warp takes its 16-key slices of the four together: their scores
+// are eight independent MMA chains (one page's two left it waiting for MMA latencies), their probabilities and values straight-line code, and there
+// is no block barrier before the merge of the warps.  With the merge of the chunks, 6 rows x 32,100 keys (394 MB) take 123 us, 214 by the other kernel;
+// 64 x 4000 keys 155 and 269, 64 x 900 50 and 73, 16 x 300 10.6 and 13.4.  What is left is the latency of one warp's chain of steps at two CTAs per SM, which the
+// accumulators' registers and the tiles allow.  The bytes go straight into the fragments: which of its 16 values
+// an MMA step takes at which place along k does not matter to its sum, and neither does the order of the columns of the output, so a lane takes
+// four neighbouring bytes of a K row per step and 16 of a V row, and a conversion of two bytes is a fragment register (V: after a byte permute that pairs
+// two keys).  The next item's K is brought by the warp that is the last to have read
+// this one's, its V at the merge.  Every step and its order is attn_decode_kernel's, so both leave the same bits, whichever of them alignment selects.
+// A block of more than 16 (row, head) pairs goes over the pages once per m16 tile, with the same instructions for every tile: a row's bits depend on
+// neither its tile nor its block mates.  A warp whose wait failed stays with the loop (warps meet at barriers) but reads and fetches nothing more.
 constexpr int F8_TILE = PAGE * 128, F8_HDP = 128 + 8;
-constexpr int F8_SMEM = 8 * F8_TILE + 4 * 16 * F8_HDP * 4 + 2 * 4 * 16 * 2 * 4 + 8 * 8 + 16 + 1024;
+constexpr int F8_SMEM = 8 * F8_TILE + 4 * 16 * F8_HDP * 4 + 2 * 4 * 16 * 2 * 4 + 32 + 1024;
 // four bytes -> two fp16 pairs
 __device__ __forceinline__ void f8x4_to_f16x4(uint32_t b, uint32_t& lo, uint32_t& hi) {
   asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}" : "=r"(lo), "=r"(hi) : "r"(b));
@@ -725,19 +721,19 @@ __global__ void __launch_bounds__(ATT_THREADS, 2)
 attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const uint16_t* __restrict__ q,
                       const int* __restrict__ block_table, int max_blocks, const int* __restrict__ ctx_len, float* __restrict__ part_o,
                       float* __restrict__ part_ml, int n_q, int n_kv, int max_chunks, float scale_log2_in, int* status,
-                      const float* __restrict__ kv_scale, const int* __restrict__ plan, const int* __restrict__ vbt, int chunk_begin) {
-  constexpr int HD = 128, HDP = F8_HDP;
+                      const float* __restrict__ kv_scale, const int* __restrict__ plan, const int* __restrict__ vbt) {
+  constexpr int HD = 128, HDP = F8_HDP, NP = DEC_CHUNK / PAGE;
   pdl_launch();
   pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-  uint8_t *ktile = smem + warp * 2 * F8_TILE, *vtile = ktile + F8_TILE;
-  float* sm_o = (float*)(smem + 8 * F8_TILE);                           // [page][16][HDP]: one tile's partial outputs
-  float* sm_ml2 = sm_o + 4 * 16 * HDP;                                  // two of [page][16][2], tiles in turn
-  uint64_t* bars = (uint64_t*)(sm_ml2 + 2 * 4 * 16 * 2);                // K and V tile of each warp
-  uint64_t *full_k = bars + 2 * warp, *full_v = full_k + 1;
-  volatile int* abort_flag = (volatile int*)(bars + 8);
+  uint8_t *ktile = smem, *vtile = smem + NP * F8_TILE;                  // [page]
+  float* sm_o = (float*)(smem + 2 * NP * F8_TILE);                      // [slice][16][HDP]: one tile's partial outputs
+  float* sm_ml2 = sm_o + 4 * 16 * HDP;                                  // two of [slice][16][2], tiles in turn
+  uint64_t *full_k = (uint64_t*)(sm_ml2 + 2 * 4 * 16 * 2), *full_v = full_k + 1;      // a chunk's pages share a barrier
+  int* n_read = (int*)(full_v + 1);                                     // warps that have read the K tiles, over all items
+  volatile int* abort_flag = (volatile int*)(n_read + 1);
   const int G = n_q / n_kv;
   const int total = plan[0], nb = plan[1];
   const int* blk_row = plan + PLAN_HEAD;
@@ -747,53 +743,51 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
   const int* blk_c0 = blk_seq + PLAN_MAX_ROWS;
   if ((int)blockIdx.x >= total) return;
   if (tid == 0) {
-    for (int i = 0; i < 8; ++i) mbar_init(&bars[i], 1);
-    *abort_flag = 0;
+    mbar_init(full_k, 1), mbar_init(full_v, 1);
+    *abort_flag = *n_read = 0;
     fence_barrier_init();
   }
   __syncthreads();
-  struct Item { int row, nblk, kvh, chunk, k_begin, k_end, y; };         // y: first row of this warp's page in the tensor maps, -1: no such page
+  struct Item { int row, nblk, kvh, chunk, k_begin, k_end, y; };         // y: first row of page `lane` of the chunk in the tensor maps, -1: no such page
   int blk = 0;
-  // items come in ascending order: the block that holds the next one is this one's or a little further.  false: a chunk below chunk_begin
+  // items come in ascending order: the block that holds the next one is this one's or a little further
   auto locate = [&](int item, Item& it) {
     while (blk + 1 < nb && prefix[blk + 1] <= item) ++blk;
     const int local = item - prefix[blk], seq = blk_seq[blk], c0 = blk_c0[blk];
-    if (c0 + local / n_kv < chunk_begin) return false;
     it.row = blk_row[blk], it.nblk = blk_n[blk], it.kvh = local % n_kv, it.chunk = c0 + local / n_kv;
     int ctx_max = 0;
     for (int i = 0; i < it.nblk; ++i) ctx_max = max(ctx_max, ctx_len[it.row + i]);
     it.k_begin = it.chunk * DEC_CHUNK;
     it.k_end = min(ctx_max, it.k_begin + DEC_CHUNK);
     // a tree row's private table starts at the page index of its block's first chunk
-    const int* bt = seq >= 0 ? block_table + (size_t)seq * max_blocks : vbt + (size_t)(-1 - seq) * VBT_W - c0 * (DEC_CHUNK / PAGE);
-    it.y = it.k_begin + warp * PAGE < it.k_end ? (bt[it.k_begin / PAGE + warp] * n_kv + it.kvh) * PAGE : -1;
-    return true;
+    const int* bt = seq >= 0 ? block_table + (size_t)seq * max_blocks : vbt + (size_t)(-1 - seq) * VBT_W - c0 * NP;
+    it.y = lane < NP && it.k_begin + lane * PAGE < it.k_end ? (bt[it.k_begin / PAGE + lane] * n_kv + it.kvh) * PAGE : -1;
   };
-  auto fetch = [&](uint8_t* dst, const CUtensorMap* map, int y, uint64_t* bar) {
-    mbar_arrive_expect_tx(bar, F8_TILE);
-    tma_load_2d(dst, map, 0, y, bar);
+  auto fetch = [&](uint8_t* tiles, const CUtensorMap* map, int y, uint64_t* bar) {      // by a whole warp: lane p brings page p
+    const uint32_t pages = __popc(__ballot_sync(0xffffffffu, y >= 0));
+    if (lane == 0 && pages != 0) mbar_arrive_expect_tx(bar, pages * F8_TILE);
+    __syncwarp();
+    if (y >= 0) tma_load_2d(tiles + lane * F8_TILE, map, 0, y, bar);
   };
   Item it;
   int item = blockIdx.x;
-  while (item < total && !locate(item, it)) item += gridDim.x;
-  if (item >= total) return;                           // (the same for the whole block)
-  if (lane == 0 && it.y >= 0) {
-    fetch(ktile, &tk, it.y, full_k);
-    fetch(vtile, &tv, it.y, full_v);
-  }
+  locate(item, it);
+  if (warp == 0) fetch(ktile, &tk, it.y, full_k);
+  if (warp == 1) fetch(vtile, &tv, it.y, full_v);
   uint32_t qa[8][4];
-  int pages = 0, par = 0, q_row = -1, q_kvh = -1, q_nblk = 0;            // pages: consumed so far by this warp; q_*: whose queries qa holds
+  int par = 0, done = 0, q_row = -1, q_kvh = -1, q_nblk = 0;     // done: items so far; q_*: whose queries qa holds
+  bool ok = true;                                      // the same for the whole warp
   while (item < total) {
     Item next;
     next.y = -1;
     item += gridDim.x;                                 // the next one of this block's
-    while (item < total && !locate(item, next)) item += gridDim.x;
+    if (item < total) locate(item, next);
     const float scale_log2 = scale_log2_in * kv_scale[it.kvh], v_scale = kv_scale[n_kv + it.kvh];     // K was stored as k / k_scale
-    const int ntiles = (it.nblk * G + 15) >> 4, kpos = it.k_begin + warp * PAGE;
-    const bool any = it.y >= 0;                      // uniform for the warp
+    const int ntiles = (it.nblk * G + 15) >> 4, kpos = it.k_begin + warp * 16;
     for (int mt = 0; mt < ntiles; ++mt) {
       const int rows = min(16, it.nblk * G - 16 * mt);
-      int valid[2];
+      const bool last = mt == ntiles - 1;
+      int valid[2];                                    // keys from kpos on that the lane's two rows may see
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int t = mt * 16 + g + 8 * r, rb = t / G;
@@ -804,105 +798,156 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
         for (int r = 0; r < 2; ++r) {
           const int t = mt * 16 + g + 8 * r, rb = t / G, hh = t % G;
           const bool live = rb < it.nblk;
-          const uint4* qr = reinterpret_cast<const uint4*>(q + ((size_t)(it.row + (live ? rb : 0)) * n_q + (size_t)it.kvh * G + hh) * HD + 32 * t4);
+          const uint2* qr = reinterpret_cast<const uint2*>(q + ((size_t)(it.row + (live ? rb : 0)) * n_q + (size_t)it.kvh * G + hh) * HD) + t4;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {             // this lane's 32 values of the head, four to a k step
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (live) v = qr[i];
-            qa[2 * i][r] = bf16x2_to_f16x2(v.x), qa[2 * i][2 + r] = bf16x2_to_f16x2(v.y);
-            qa[2 * i + 1][r] = bf16x2_to_f16x2(v.z), qa[2 * i + 1][2 + r] = bf16x2_to_f16x2(v.w);
+          for (int k = 0; k < 8; ++k) {               // values 16 k + 4 t4 .. + 3: the lane's four of this k step
+            uint2 v = make_uint2(0u, 0u);
+            if (live) v = qr[4 * k];
+            qa[k][r] = bf16x2_to_f16x2(v.x), qa[k][2 + r] = bf16x2_to_f16x2(v.y);
           }
         }
         q_row = it.row, q_kvh = it.kvh, q_nblk = it.nblk;
       }
-      float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[16][4];
+      // scores of the four slices, 16 keys each, as eight MMA chains (a page that is not there gives what the mask takes out)
+      float s[NP][2][4];
 #pragma unroll
-      for (int d = 0; d < 16; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
-      if (any) {
-        float sc[8][4];
-        if (mt == 0) mbar_wait(full_k, pages & 1, abort_flag, status, 50);
-        const uint32_t ks = smem_u32(ktile), vs = smem_u32(vtile);
+      for (int p = 0; p < NP; ++p)
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          uint4 w[2][2];
+        for (int u = 0; u < 2; ++u) s[p][u][0] = s[p][u][1] = s[p][u][2] = s[p][u][3] = 0.f;
+      if (mt == 0) ok = ok && __all_sync(0xffffffffu, mbar_wait(full_k, done & 1, abort_flag, status, 50));
+      if (ok) {
+        const uint32_t ks = smem_u32(ktile);
 #pragma unroll
-          for (int u = 0; u < 2; ++u)
+        for (int h = 0; h < 2; ++h) {
+          uint32_t w[NP][2][4];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) w[u][h] = lds128(ks + byte_chunk<HD>(8 * (j + u) + g, 2 * t4 + h));
+          for (int p = 0; p < NP; ++p)
 #pragma unroll
-          for (int u = 0; u < 2; ++u) sc[j + u][0] = sc[j + u][1] = sc[j + u][2] = sc[j + u][3] = 0.f;
+            for (int u = 0; u < 2; ++u)
+              ldsm_x4(ks + p * F8_TILE + byte_chunk<HD>(16 * warp + 8 * u + (lane & 7), 4 * h + (lane >> 3)), w[p][u][0], w[p][u][1], w[p][u][2], w[p][u][3]);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
+          for (int k = 0; k < 4; ++k)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const uint4 c = w[u][k >> 2];
-              uint32_t b0, b1;
-              f8x4_to_f16x4((k & 3) == 0 ? c.x : (k & 3) == 1 ? c.y : (k & 3) == 2 ? c.z : c.w, b0, b1);
-              mma_f16(sc[j + u], qa[k], b0, b1);
-            }
+            for (int p = 0; p < NP; ++p)
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                uint32_t b0, b1;
+                f8x4_to_f16x4(w[p][u][k], b0, b1);
+                mma_f16(s[p][u], qa[4 * h + k], b0, b1);
+              }
         }
-        if (mt == ntiles - 1) {                      // the K tile has been read: the next item's page may come
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0 && next.y >= 0) fetch(ktile, &tk, next.y, full_k);
-        }
+      }
+      int readers = 0;
+      if (last) {                                      // the warp that is the last to have read the K tiles brings the next item's
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) asm volatile("atom.acq_rel.cta.shared.add.u32 %0, [%1], 1;" : "=r"(readers) : "r"(smem_u32(n_read)) : "memory");
+      }
+      // attn_softmax16's rule: a row's maximum is its first slice's and moves where a later one exceeds it by more than 2^8, which is rare
+      float m[2] = {-INFINITY, -INFINITY}, rest[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+      for (int p = 0; p < NP; ++p)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int kk = j * 8 + 2 * t4 + (e & 1);
-            const float v = kk < valid[e >> 1] ? sc[j][e] * scale_log2 : -INFINITY;
-            sc[j][e] = v;
-            m[e >> 1] = fmaxf(m[e >> 1], v);
+            const int kk = p * PAGE + j * 8 + 2 * t4 + (e & 1);
+            const float v = kk < valid[e >> 1] ? s[p][j][e] * scale_log2 : -INFINITY;
+            s[p][j][e] = v;
+            if (p == 0) m[e >> 1] = fmaxf(m[e >> 1], v);
+            else rest[e >> 1] = fmaxf(rest[e >> 1], v);
           }
-        float sub[2];
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], 1));
-          m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], 2));
-          sub[r] = m[r] == -INFINITY ? 0.f : m[r];   // a row that may see none of these keys: all its scores are -inf
+          m[r] = fmaxf(m[r], __shfl_xor_sync(0xffffffffu, m[r], o));
+          rest[r] = fmaxf(rest[r], __shfl_xor_sync(0xffffffffu, rest[r], o));
         }
-        if (mt == 0) mbar_wait(full_v, pages & 1, abort_flag, status, 51);
+      // (a row with keys but no maximum has NaN scores only: they count for nothing, and it takes the general way)
+      const bool moves = __any_sync(0xffffffffu, rest[0] > m[0] + 8.f || rest[1] > m[1] + 8.f || (m[0] == -INFINITY && valid[0] > 0) || (m[1] == -INFINITY && valid[1] > 0));
+      if (last && (__shfl_sync(0xffffffffu, readers, 0) & 3) == 3 && ok) fetch(ktile, &tk, next.y, full_k);
+      float corr[NP][2];
+      uint32_t pa[NP][4];
+      auto probabilities = [&](int p, auto general) {
+        float sub[2], rs[2] = {0.f, 0.f};
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          uint4 vw[4];
+        for (int r = 0; r < 2; ++r) sub[r] = m[r] == -INFINITY ? 0.f : m[r];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) vw[j] = lds128(vs + byte_chunk<HD>(16 * kk + 8 * (j >> 1) + 2 * t4 + (j & 1), g));
-          uint32_t pa[4];
+        for (int j = 0; j < 2; ++j) {
+          float pr[4];
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            float pr[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              pr[e] = exp2f(sc[2 * kk + j][e] - sub[e >> 1]);
-              l[e >> 1] += pr[e];
-            }
-            pa[2 * j] = pack_f16(pr[0], pr[1]);
-            pa[2 * j + 1] = pack_f16(pr[2], pr[3]);
+          for (int e = 0; e < 4; ++e) {
+            pr[e] = exp2f(s[p][j][e] - sub[e >> 1]);
+            if (general.value && m[e >> 1] == -INFINITY) pr[e] = 0.f;
+            rs[e >> 1] += pr[e];
           }
-          const uint32_t va[4][4] = {{vw[0].x, vw[0].y, vw[0].z, vw[0].w}, {vw[1].x, vw[1].y, vw[1].z, vw[1].w},
-                                     {vw[2].x, vw[2].y, vw[2].z, vw[2].w}, {vw[3].x, vw[3].y, vw[3].z, vw[3].w}};
+          pa[p][2 * j] = pack_f16(pr[0], pr[1]);
+          pa[p][2 * j + 1] = pack_f16(pr[2], pr[3]);
+        }
 #pragma unroll
-          for (int i = 0; i < 4; ++i)                // output column n of MMA 4 i + e = value 16 n + 4 i + e of the head
+        for (int r = 0; r < 2; ++r) l[r] = __fadd_rn(l[r], rs[r]);
+      };
+      if (!moves) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t b0[2], b1[2];
-              f8x4_to_f16x4(__byte_perm(va[0][i], va[1][i], h ? 0x7362 : 0x5140), b0[0], b0[1]);
-              f8x4_to_f16x4(__byte_perm(va[2][i], va[3][i], h ? 0x7362 : 0x5140), b1[0], b1[1]);
-              mma_f16(o[4 * i + 2 * h], pa, b0[0], b1[0]);
-              mma_f16(o[4 * i + 2 * h + 1], pa, b0[1], b1[1]);
+        for (int p = 0; p < NP; ++p) probabilities(p, std::false_type());
+      } else {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            corr[p][r] = 1.f;
+            if (p == 0) continue;
+            float mx = fmaxf(fmaxf(s[p][0][2 * r], s[p][0][2 * r + 1]), fmaxf(s[p][1][2 * r], s[p][1][2 * r + 1]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            if (mx > m[r] + 8.f) {
+              corr[p][r] = m[r] == -INFINITY ? 1.f : exp2f(m[r] - mx);
+              m[r] = mx;
             }
+            l[r] = __fmul_rn(l[r], corr[p][r]);
+          }
+          probabilities(p, std::true_type());
         }
-        if (mt == ntiles - 1) {
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0 && next.y >= 0) fetch(vtile, &tv, next.y, full_v);
-        }
-      } else if (mt == ntiles - 1 && lane == 0 && next.y >= 0) {
-        fetch(ktile, &tk, next.y, full_k);
-        fetch(vtile, &tv, next.y, full_v);
       }
-      // merge the four pages: every page's partial rescaled to the row's maximum over them, then added in page order
+      float o[16][4];
+#pragma unroll
+      for (int d = 0; d < 16; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
+      if (mt == 0) ok = ok && __all_sync(0xffffffffu, mbar_wait(full_v, done & 1, abort_flag, status, 51));
+      auto values = [&](int p) {
+        const uint32_t vs = smem_u32(vtile) + p * F8_TILE;
+        uint4 vw[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) vw[j] = lds128(vs + byte_chunk<HD>(16 * warp + 8 * (j >> 1) + 2 * t4 + (j & 1), g));
+        const uint32_t va[4][4] = {{vw[0].x, vw[0].y, vw[0].z, vw[0].w}, {vw[1].x, vw[1].y, vw[1].z, vw[1].w},
+                                   {vw[2].x, vw[2].y, vw[2].z, vw[2].w}, {vw[3].x, vw[3].y, vw[3].z, vw[3].w}};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)                  // output column n of MMA 4 i + e = value 16 n + 4 i + e of the head
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t b0[2], b1[2];
+            f8x4_to_f16x4(__byte_perm(va[0][i], va[1][i], h ? 0x7362 : 0x5140), b0[0], b0[1]);
+            f8x4_to_f16x4(__byte_perm(va[2][i], va[3][i], h ? 0x7362 : 0x5140), b1[0], b1[1]);
+            mma_f16(o[4 * i + 2 * h], pa[p], b0[0], b1[0]);
+            mma_f16(o[4 * i + 2 * h + 1], pa[p], b0[1], b1[1]);
+          }
+      };
+      if (ok && !moves && kpos + (NP - 1) * PAGE < it.k_end) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) values(p);
+      } else if (ok) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          if (kpos + p * PAGE >= it.k_end) break;      // no row of the block sees any of the slice's keys: its V bytes are not touched
+          if (moves && __any_sync(0xffffffffu, corr[p][0] != 1.f || corr[p][1] != 1.f)) {
+#pragma unroll
+            for (int d = 0; d < 16; ++d) o[d][0] *= corr[p][0], o[d][1] *= corr[p][0], o[d][2] *= corr[p][1], o[d][3] *= corr[p][1];
+          }
+          values(p);
+        }
+      }
+      if (last) fence_proxy_async();                   // (the V tiles are refilled after the next barrier)
+      // merge the four slices: every warp's partial rescaled to the row's maximum over them, then added in slice order
       float* sm_ml = sm_ml2 + par * 4 * 16 * 2;
       par ^= 1;
 #pragma unroll
@@ -912,6 +957,7 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
         if (t4 == 0) sm_ml[(warp * 16 + g + 8 * r) * 2] = m[r];
       }
       __syncthreads();
+      if (last && warp == 0 && ok) fetch(vtile, &tv, next.y, full_v);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         if (g + 8 * r >= rows) continue;
@@ -949,7 +995,7 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
         }
       }
     }
-    if (any) ++pages;
+    ++done;
     it = next;
   }
 }
@@ -1249,12 +1295,8 @@ static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, co
   // persistent: two CTAs per SM at most, never more than the items the window can have
   const long long bound = (long long)rows * n_kv * mc;
   const int grid = (int)(bound < 2 * sm_count() ? bound : 2 * sm_count());
-  int chunk_end = 0, head_grid = grid;
   if constexpr (HD == 128 && FP8 && I8 == 0) {
-    // attn_decode_f8_kernel from key 1024 on (its queries come in 16-byte pieces), a matter of the key's position alone, so a row's bits do not depend on
-    // the window.  Below, the kernel of the other byte caches: it costs little there, and a short sequence, whose new row is a large part of the cache's
-    // bytes, keeps them to the bit.
-    if (mc > F8_FIRST_CHUNK && (((uintptr_t)q) & 15) == 0) {
+    if ((((uintptr_t)q) & 7) == 0) {                 // its queries come in 8-byte pieces; the other kernel leaves the same bits
       static bool ready = false;
       if (!ready) {
         cudaError_t e = cudaFuncSetAttribute(attn_decode_f8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F8_SMEM);
@@ -1262,12 +1304,8 @@ static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, co
         ready = true;
       }
       rx::launch(attn_decode_f8_kernel, dim3(grid), dim3(ATT_THREADS), F8_SMEM, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, ctx_len, part_o, part_ml,
-                 n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, vbt, F8_FIRST_CHUNK);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return (int)e;
-      chunk_end = F8_FIRST_CHUNK;
-      const long long head = (long long)rows * n_kv * F8_FIRST_CHUNK;
-      head_grid = (int)(head < 2 * sm_count() ? head : 2 * sm_count());
+                 n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, vbt);
+      return (int)cudaGetLastError();
     }
   }
   constexpr int smem = dec_smem_bytes(HD, FP8, MT);
@@ -1277,8 +1315,8 @@ static int launch_decode_kernel(const CUtensorMap* tk, const CUtensorMap* tv, co
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  rx::launch(attn_decode_kernel<HD, FP8, MT, I8>, dim3(head_grid), dim3(ATT_THREADS), smem, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, row_seq,
-             ctx_len, part_o, part_ml, n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, k_ts, v_ts, vbt, chunk_end);
+  rx::launch(attn_decode_kernel<HD, FP8, MT, I8>, dim3(grid), dim3(ATT_THREADS), smem, st, *tk, *tv, (const uint16_t*)q, bt, max_blocks, row_seq,
+             ctx_len, part_o, part_ml, n_q, n_kv, mc, scale * 1.4426950408889634f, status, kv_scale, plan, k_ts, v_ts, vbt);
   return (int)cudaGetLastError();
 }
 

@@ -376,8 +376,7 @@ def attn_decode(tk: KvTensorMap, tv: KvTensorMap, q, block_table, row_seq, ctx_l
     _lib.check(L.rx_attn_decode(tk.ptr, tv.ptr, q.data_ptr(), block_table.data_ptr(), block_table.shape[1], row_seq.data_ptr(), ctx_len.data_ptr(),
                                 scratch.data_ptr(), rows, n_q, n_kv, hd, max_ctx, scale, _lib.ptr(suh), _lib.ptr(xr), _lib.ptr(out),
                                 status.data_ptr(), _lib.stream_ptr(), _lib.ptr(kv_scale), int(max_seq_rows), _lib.ptr(plan), _lib.ptr(kts), _lib.ptr(vts), _lib.ptr(vbt)), "rx_attn_decode")
-    split = kv_scale is not None and hd == 128 and max_ctx > 1024 and q.data_ptr() % 16 == 0      # two kernels: keys below 1024, and from there on
-    _lib.count((2 if plan is not None else 3) + split)
+    _lib.count(2 if plan is not None else 3)
 
 
 def kv_move_rows(tensor_ptrs, row_bytes: int, n_kv: int, moves, n_moves: int) -> None:

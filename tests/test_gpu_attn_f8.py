@@ -55,3 +55,20 @@ def test_decode_over_e4m3_pages(n_q, n_kv, rows):
     # the same rows one by one: the same bits, whatever tile and block they had
     one = torch.cat([_run(K, maps, q[r:r + 1].contiguous(), scale, seq[r:r + 1], ctx[r:r + 1], bt, n_q, n_kv, 1) for r in range(len(seq))])
     assert torch.equal(out, one)
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(40, 8), (3, 3), (16, 1)])
+@pytest.mark.parametrize("rows", [1, 3, 7])
+@pytest.mark.parametrize("spread", [1.0, 40.0])           # 40: the running maxima move
+def test_sums_do_not_depend_on_the_kernel(n_q, n_kv, rows, spread):
+    """Queries that are not 8-byte aligned go through the kernel that expands the pages: the same bits, in short contexts and long ones."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    ctxs = [0, 1, 15, 16, 63, 64, 81, 255, 256, 300, 700, 1023, 1024, 1025, 1279, 1280, 1999, 3000]
+    K, kc, vc, q, scale, seq, ctx, bt, maps = _case(ctxs, rows, n_q, n_kv, n_q + rows)
+    q = (q.float() * spread).bfloat16()
+    off = torch.empty(q.numel() + 2, dtype=q.dtype, device="cuda")[2:].view(q.shape)
+    off.copy_(q)
+    assert q.data_ptr() % 8 == 0 and off.data_ptr() % 8 == 4
+    a, b = (_run(K, maps, x, scale, seq, ctx, bt, n_q, n_kv, rows) for x in (q, off))
+    assert torch.isfinite(a.float()).all() and a.abs().max() > 0 and torch.equal(a, b)
