@@ -333,6 +333,9 @@ __device__ __forceinline__ void attn_softmax16(float (&s)[2][4], int valid_lo, i
   for (int r = 0; r < 2; ++r) l[r] += rs[r];
 }
 
+// The plan's readers begin before its writer has finished and wait for it.  Their pointer to it is not marked __restrict__: loads through a pointer to
+// data that is constant by declaration may be moved up, also past the wait.
+
 // The decode kernel's step: like attn_step for MT tiles at once over the same 16 keys.  Each K / V fragment is fetched from shared memory once
 // and feeds every tile's MMA.  `ntiles` (uniform) = tiles that hold a live row.
 template <int HD, int MT, bool F16>
@@ -490,7 +493,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const uint16_t* __restrict__ q,
                    const int* __restrict__ block_table, int max_blocks, const int* __restrict__ row_seq, const int* __restrict__ ctx_len,
                    float* __restrict__ part_o, float* __restrict__ part_ml, int n_q, int n_kv, int max_chunks, float scale_log2_in, int* status,
-                   const float* __restrict__ kv_scale, const int* __restrict__ plan, const float* __restrict__ k_ts, const float* __restrict__ v_ts,
+                   const float* __restrict__ kv_scale, const int* plan, const float* __restrict__ k_ts, const float* __restrict__ v_ts,
                    const int* __restrict__ vbt) {
   static_assert(!I8 || FP8, "the int8 cache uses the byte-page path");
   pdl_launch();
@@ -721,7 +724,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 2)
 attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv, const uint16_t* __restrict__ q,
                       const int* __restrict__ block_table, int max_blocks, const int* __restrict__ ctx_len, float* __restrict__ part_o,
                       float* __restrict__ part_ml, int n_q, int n_kv, int max_chunks, float scale_log2_in, int* status,
-                      const float* __restrict__ kv_scale, const int* __restrict__ plan, const int* __restrict__ vbt) {
+                      const float* __restrict__ kv_scale, const int* plan, const int* __restrict__ vbt) {
   constexpr int HD = 128, HDP = F8_HDP, NP = DEC_CHUNK / PAGE;
   pdl_launch();
   pdl_wait();

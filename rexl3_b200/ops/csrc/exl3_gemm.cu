@@ -52,7 +52,7 @@ __host__ __device__ inline GemmSmemLayout gemm_layout(int twice, int brows) {
 template <int TWICE, int CB>
 __global__ void __launch_bounds__(GEMM_THREADS, 2)
 exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __restrict__ trellis, float* __restrict__ part,
-                 int rows, int K, int N, int splits, int brows, int row_tiles, int* status, const int* __restrict__ tile_tab,
+                 int rows, int K, int N, int splits, int brows, int row_tiles, int* status, const int* tile_tab,
                  size_t expert_words) {
   pdl_launch();
   // Row window of this CTA.  Plain GEMM: tile z of the row dimension.  Grouped (mixture-of-experts) form: tile_tab[z] =

@@ -63,7 +63,7 @@ __device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1]
 template <int TWICE, int CB, int NG>
 __global__ void __launch_bounds__(GR_ROLE_WARPS * 32 + NG * 128, (NG <= 3 ? 2 : 1))
 exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __restrict__ trellis, size_t expert_words,
-                         float* __restrict__ part, int rows, int K, int N, int splits, int brows, const int* __restrict__ tile_tab, int max_tiles,
+                         float* __restrict__ part, int rows, int K, int N, int splits, int brows, const int* tile_tab, int max_tiles,
                          int* status) {
   pdl_launch();
   constexpr int SA = gr_a_stages(NG), EW = TWICE / 2;            // EW: words of an eighth of a tile

@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t e8m0_to_half2(uint32_t b) {
 
 __global__ void __launch_bounds__(MX_THREADS, 2)
 mxfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const uint8_t* __restrict__ scales,
-                  float* __restrict__ part, int rows, int K, int N, int splits, int brows, int* status, const int* __restrict__ tile_tab) {
+                  float* __restrict__ part, int rows, int K, int N, int splits, int brows, int* status, const int* tile_tab) {
   pdl_launch();
   pdl_wait();                       // the tile table comes from the planning kernel just before
   const int e = tile_tab[3 * blockIdx.z];
