@@ -713,7 +713,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
 // two keys).  The next item's K is brought by the warp that is the last to have read
 // this one's, its V at the merge.  Every step and its order is attn_decode_kernel's, so both leave the same bits, whichever of them alignment selects.
 // A block of more than 16 (row, head) pairs goes over the pages once per m16 tile, with the same instructions for every tile: a row's bits depend on
-// neither its tile nor its block mates.  A warp whose wait failed stays with the loop (warps meet at barriers) but reads and fetches nothing more.
+// neither its tile nor its block mates.  A warp whose wait failed stays with the loop (warps meet at barriers) but reads and fetches nothing more;
+// what is on its way is waited for at the end.
 constexpr int F8_TILE = PAGE * 128, F8_HDP = 128 + 8;
 constexpr int F8_SMEM = 8 * F8_TILE + 4 * 16 * F8_HDP * 4 + 2 * 4 * 16 * 2 * 4 + 32 + 1024;
 // four bytes -> two fp16 pairs
@@ -737,6 +738,7 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
   uint64_t *full_k = (uint64_t*)(sm_ml2 + 2 * 4 * 16 * 2), *full_v = full_k + 1;      // a chunk's pages share a barrier
   int* n_read = (int*)(full_v + 1);                                     // warps that have read the K tiles, over all items
   volatile int* abort_flag = (volatile int*)(n_read + 1);
+  volatile int* n_sent = abort_flag + 1;                                // chunks fetched so far, K and V
   const int G = n_q / n_kv;
   const int total = plan[0], nb = plan[1];
   const int* blk_row = plan + PLAN_HEAD;
@@ -747,7 +749,7 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
   if ((int)blockIdx.x >= total) return;
   if (tid == 0) {
     mbar_init(full_k, 1), mbar_init(full_v, 1);
-    *abort_flag = *n_read = 0;
+    *abort_flag = *n_read = n_sent[0] = n_sent[1] = 0;
     fence_barrier_init();
   }
   __syncthreads();
@@ -768,7 +770,10 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
   };
   auto fetch = [&](uint8_t* tiles, const CUtensorMap* map, int y, uint64_t* bar) {      // by a whole warp: lane p brings page p
     const uint32_t pages = __popc(__ballot_sync(0xffffffffu, y >= 0));
-    if (lane == 0 && pages != 0) mbar_arrive_expect_tx(bar, pages * F8_TILE);
+    if (lane == 0 && pages != 0) {
+      mbar_arrive_expect_tx(bar, pages * F8_TILE);
+      n_sent[bar == full_v] += 1;
+    }
     __syncwarp();
     if (y >= 0) tma_load_2d(tiles + lane * F8_TILE, map, 0, y, bar);
   };
@@ -1001,6 +1006,10 @@ attn_decode_f8_kernel(const __grid_constant__ CUtensorMap tk, const __grid_const
     ++done;
     it = next;
   }
+  // A wait that gave up leaves copies on their way into this CTA's memory: they are waited for, bounded, and not cut short by the abort word.
+  __syncthreads();
+  if (*abort_flag != 0 && tid < 2 && n_sent[tid] > 0)
+    for (int i = 0; i < (1 << 22) && !mbar_try_wait(full_k + tid, (n_sent[tid] - 1) & 1); ++i) {}
 }
 
 // Loads in flight per lane of the merge, which is bound by their latency: 6 rows x 126 chunks took 23.6 us with four, 12.3 us with sixteen.

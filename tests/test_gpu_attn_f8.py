@@ -72,3 +72,22 @@ def test_sums_do_not_depend_on_the_kernel(n_q, n_kv, rows, spread):
     assert q.data_ptr() % 8 == 0 and off.data_ptr() % 8 == 4
     a, b = (_run(K, maps, x, scale, seq, ctx, bt, n_q, n_kv, rows) for x in (q, off))
     assert torch.isfinite(a.float()).all() and a.abs().max() > 0 and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("how", ["abort", "limit"])
+def test_waits_that_give_up_leave_the_device_usable(how):
+    """The abort word, or a wait limit of a microsecond: the call returns, says so if a wait gave up, and the next call is right."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    n_q, n_kv = 40, 8
+    K, kc, vc, q, scale, seq, ctx, bt, maps = _case([5000, 9, 700, 3000], 7, n_q, n_kv, 5)
+    want = _run(K, maps, q, scale, seq, ctx, bt, n_q, n_kv, 7)
+    for _ in range(3):
+        st, mx, out = K.new_status(), int(ctx.max()), torch.zeros_like(q)
+        K.set_abort(st) if how == "abort" else K.set_wait_limit(st, 1)
+        K.attn_decode(*maps, q, bt, seq, ctx, K.attn_decode_scratch(q.shape[0], n_q, 128, mx), n_q, n_kv, 128, mx, 1 / math.sqrt(128), None, None, out, st,
+                      kv_scale=scale, max_seq_rows=7)
+        code = st.tolist()[0]
+        assert code in (0, K.ST_ABORTED if how == "abort" else K.ST_TIMEOUT)
+        assert code != 0 or torch.equal(out, want)
+        assert torch.equal(_run(K, maps, q, scale, seq, ctx, bt, n_q, n_kv, 7), want)
