@@ -1054,12 +1054,11 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
           if (j0 + j < cnt) p[j] = *reinterpret_cast<const float4*>(part_o + (base + c0 + j0 + j) * HD + d0);
 #pragma unroll
         for (int j = 0; j < MERGE_LOADS; ++j) {
+          if (j0 + j >= cnt) break;                  // (the same for the whole row)
           const int src = gbase + ((j0 + j) % GL);
           const float f = __shfl_sync(0xffffffffu, f_l, src), ll = __shfl_sync(0xffffffffu, l_l, src);
-          if (j0 + j < cnt) {
-            acc[0] += f * p[j].x; acc[1] += f * p[j].y; acc[2] += f * p[j].z; acc[3] += f * p[j].w;
-            lsum += f * ll;
-          }
+          acc[0] += f * p[j].x; acc[1] += f * p[j].y; acc[2] += f * p[j].z; acc[3] += f * p[j].w;
+          lsum += f * ll;
         }
       }
     }
