@@ -108,18 +108,18 @@ __device__ __forceinline__ void load_kv_page_i8(uint8_t* kdst, uint8_t* vdst, fl
   bulk_g2s(sc + PAGE, v_ts + (size_t)y, PAGE * 4, bar);
 }
 
-// Where the 16 bytes of chunk j of a key stand in a byte page: rows of 128 bytes are loaded with the 128-byte swizzle (rx_make_kv_tmap8).
+// Where the 16 bytes of chunk j of a key stand in a byte page loaded with the 128-byte swizzle (rx_make_kv_tmap_f8).
 template <int HD>
 __device__ __forceinline__ int byte_chunk(int key, int j) { return key * HD + ((HD == 128 ? j ^ (key & 7) : j) << 4); }
 
-// sc != nullptr: the bytes are int8 and sc[key] is the key's scale (else: E4M3 bytes)
-template <int HD>
+// sc != nullptr: the bytes are int8 and sc[key] is the key's scale (else: E4M3 bytes).  SWIZZLED: see byte_chunk; else row by row.
+template <int HD, bool SWIZZLED>
 __device__ __forceinline__ void expand_page8(const uint8_t* src, uint8_t* dst, const float* sc = nullptr) {
   constexpr int CHUNKS = PAGE * HD / 16;          // 16 values each
   const uint32_t dbase = smem_u32(dst);
   for (int c = threadIdx.x; c < CHUNKS; c += blockDim.x) {
     const int key = c / (HD / 16), j = c % (HD / 16);
-    const uint4 r = *reinterpret_cast<const uint4*>(src + byte_chunk<HD>(key, j));
+    const uint4 r = *reinterpret_cast<const uint4*>(src + (SWIZZLED ? byte_chunk<HD>(key, j) : c * 16));
     const uint32_t w[4] = {r.x, r.y, r.z, r.w};
     uint32_t h[8];
     if (sc != nullptr) {
@@ -607,8 +607,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant
           expand_page4<HD>(smem + s * TILE, conv, (const uint8_t*)(tsc + s * 2 * PAGE));
           expand_page4<HD>(smem + (KV_STAGES + s) * TILE, conv + T16, (const uint8_t*)(tsc + s * 2 * PAGE + PAGE));
         } else {
-          expand_page8<HD>(smem + s * TILE, conv, I8 ? tsc + s * 2 * PAGE : nullptr);
-          expand_page8<HD>(smem + (KV_STAGES + s) * TILE, conv + T16, I8 ? tsc + s * 2 * PAGE + PAGE : nullptr);
+          expand_page8<HD, I8 == 0>(smem + s * TILE, conv, I8 ? tsc + s * 2 * PAGE : nullptr);
+          expand_page8<HD, I8 == 0>(smem + (KV_STAGES + s) * TILE, conv + T16, I8 ? tsc + s * 2 * PAGE + PAGE : nullptr);
         }
         __syncthreads();
       }
@@ -1180,8 +1180,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constan
         expand_page4<HD>(smem + s * TILE, conv, (const uint8_t*)(tsc + s * 2 * PAGE));
         expand_page4<HD>(smem + (KV_STAGES + s) * TILE, conv + T16, (const uint8_t*)(tsc + s * 2 * PAGE + PAGE));
       } else {
-        expand_page8<HD>(smem + s * TILE, conv, I8 ? tsc + s * 2 * PAGE : nullptr);
-        expand_page8<HD>(smem + (KV_STAGES + s) * TILE, conv + T16, I8 ? tsc + s * 2 * PAGE + PAGE : nullptr);
+        expand_page8<HD, false>(smem + s * TILE, conv, I8 ? tsc + s * 2 * PAGE : nullptr);
+        expand_page8<HD, false>(smem + (KV_STAGES + s) * TILE, conv + T16, I8 ? tsc + s * 2 * PAGE + PAGE : nullptr);
       }
       __syncthreads();
       if (mine) attn_step<HD, 64, true>(qa, smem_u32(conv), smem_u32(conv + T16), 0, v0, v1, scale_log2, m, l, o);
@@ -1244,10 +1244,9 @@ RX_API int rx_make_kv_tmap(void* out128, const void* base, long long total_rows,
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
-// Tensor map of an FP8 (E4M3) cache [num_pages][n_kv][64][hd] viewed as bytes [num_pages*n_kv*64, hd]; one page of one head is one box.  Rows of
-// 128 bytes are swizzled on the way into shared memory (16-byte chunk j of row r lands at j ^ (r % 8)): the decode kernel's fragment loads, four
-// rows at one column, then meet different banks.
-RX_API int rx_make_kv_tmap8(void* out128, const void* base, long long total_rows, int hd) {
+// Tensor map of a byte cache [num_pages][n_kv][64][hd] viewed as [num_pages*n_kv*64, hd]; one page of one head is one box, row by row: what the kernels that
+// expand the pages take (prefill attention over E4M3, all of int8 and q4).
+static int byte_tmap(void* out128, const void* base, long long total_rows, int hd, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn enc = att_encode_tiled();
   if (enc == nullptr) return (int)cudaErrorNotSupported;
   if (hd % 64 != 0 || hd > 256 || (((uintptr_t)base) & 127) != 0) return (int)cudaErrorInvalidValue;
@@ -1256,9 +1255,18 @@ RX_API int rx_make_kv_tmap8(void* out128, const void* base, long long total_rows
   cuuint32_t box[2] = {(cuuint32_t)hd, PAGE};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc((CUtensorMap*)out128, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, hd == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+RX_API int rx_make_kv_tmap8(void* out128, const void* base, long long total_rows, int hd) {
+  return byte_tmap(out128, base, total_rows, hd, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+// The same for decode attention over an E4M3 cache.  Rows of 128 bytes are swizzled on the way into shared memory (16-byte chunk j of row r lands at
+// j ^ (r % 8)): the fragment loads of attn_decode_f8_kernel, four to eight rows at one column, then meet different banks.  Expanding swizzled pages costs
+// 2 to 4 % (prompt of 2000 rows over E4M3 257 -> 262 us, 16 x 300 int8 keys 13.9 -> 14.5 us), so nothing else takes them.
+RX_API int rx_make_kv_tmap_f8(void* out128, const void* base, long long total_rows, int hd) {
+  return byte_tmap(out128, base, total_rows, hd, hd == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 RX_API int rx_attn_decode_chunk() { return DEC_CHUNK; }

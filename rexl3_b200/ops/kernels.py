@@ -328,24 +328,32 @@ def topk(logits: torch.Tensor, count: int, scratch, ids: torch.Tensor, vals: tor
 
 
 class KvTensorMap:
-    """Host-side TMA descriptor of one layer's K or V cache (bf16 [pages, n_kv, 64, hd])."""
+    """Host-side TMA descriptors of one layer's K or V cache (bf16 or bytes [pages, n_kv, 64, hd]): `ptr` for decode attention, `rows_ptr` for prefill
+    (they differ for E4M3 bytes, whose decode kernel takes its pages swizzled)."""
 
     def __init__(self, cache: torch.Tensor):
         pages, n_kv, page, hd = cache.shape
         assert page == 64 and cache.dtype in (torch.bfloat16, torch.uint8, torch.int8) and cache.is_contiguous()
-        self.buf = np.zeros(128, dtype=np.uint8)
+        self.buf = self.buf_rows = np.zeros(128, dtype=np.uint8)
         self._keep = cache
         self.fp8 = cache.dtype == torch.uint8          # E4M3 bytes
         self.i8 = cache.dtype == torch.int8            # int8 with one scale per (token, KV head), kept beside the cache
         L = _lib.load()
         if self.fp8 or self.i8:
             _lib.check(L.rx_make_kv_tmap8(self.buf.ctypes.data, cache.data_ptr(), pages * n_kv * page, hd), "rx_make_kv_tmap8")
+            if self.fp8:
+                self.buf = np.zeros(128, dtype=np.uint8)
+                _lib.check(L.rx_make_kv_tmap_f8(self.buf.ctypes.data, cache.data_ptr(), pages * n_kv * page, hd), "rx_make_kv_tmap_f8")
         else:
             _lib.check(L.rx_make_kv_tmap(self.buf.ctypes.data, cache.data_ptr(), pages * n_kv * page, hd), "rx_make_kv_tmap")
 
     @property
     def ptr(self) -> int:
         return self.buf.ctypes.data
+
+    @property
+    def rows_ptr(self) -> int:
+        return self.buf_rows.ctypes.data
 
 
 def attn_decode_scratch(rows: int, n_q: int, hd: int, max_ctx: int, device="cuda") -> torch.Tensor:
@@ -418,14 +426,14 @@ def attn_prefill(tk: KvTensorMap, tv: KvTensorMap, q, block_table, seq_ids, q_st
     L = _lib.load()
     if q4:
         assert hd == 128 and kts is not None and kts.dtype == torch.uint8
-        _lib.check(L.rx_attn_prefill_q4(tk.ptr, tv.ptr, q.data_ptr(), block_table.data_ptr(), block_table.shape[1], seq_ids.data_ptr(), q_start.data_ptr(),
+        _lib.check(L.rx_attn_prefill_q4(tk.rows_ptr, tv.rows_ptr, q.data_ptr(), block_table.data_ptr(), block_table.shape[1], seq_ids.data_ptr(), q_start.data_ptr(),
                                         q_len.data_ptr(), pos0.data_ptr(), out.data_ptr(), nseq, max_qlen, n_q, n_kv, hd, scale, status.data_ptr(),
                                         _lib.stream_ptr(), kts.data_ptr(), vts.data_ptr()), "rx_attn_prefill_q4")
         _lib.count()
         return
     assert tk.fp8 == (kv_scale is not None), "an FP8 cache needs its per-head scales (and only an FP8 cache takes them)"
     assert tk.i8 == (kv_tscale is not None), "an int8 cache needs its per-token scales (and only an int8 cache takes them)"
-    _lib.check(L.rx_attn_prefill(tk.ptr, tv.ptr, q.data_ptr(), block_table.data_ptr(), block_table.shape[1], seq_ids.data_ptr(), q_start.data_ptr(),
+    _lib.check(L.rx_attn_prefill(tk.rows_ptr, tv.rows_ptr, q.data_ptr(), block_table.data_ptr(), block_table.shape[1], seq_ids.data_ptr(), q_start.data_ptr(),
                                  q_len.data_ptr(), pos0.data_ptr(), out.data_ptr(), nseq, max_qlen, n_q, n_kv, hd, scale, status.data_ptr(),
                                  _lib.stream_ptr(), _lib.ptr(kv_scale), _lib.ptr(kts), _lib.ptr(vts)), "rx_attn_prefill")
     _lib.count()
@@ -436,7 +444,7 @@ def attn_prefill_tc(tk: KvTensorMap, tv: KvTensorMap, q, block_table, seq_ids, q
     """The tcgen05 / TMEM prefill attention (bf16 caches, head_dim 128)."""
     assert not tk.fp8 and hd == 128
     L = _lib.load()
-    _lib.check(L.rx_attn_prefill_tc(tk.ptr, tv.ptr, q.data_ptr(), block_table.data_ptr(), block_table.shape[1], seq_ids.data_ptr(), q_start.data_ptr(),
+    _lib.check(L.rx_attn_prefill_tc(tk.rows_ptr, tv.rows_ptr, q.data_ptr(), block_table.data_ptr(), block_table.shape[1], seq_ids.data_ptr(), q_start.data_ptr(),
                                     q_len.data_ptr(), pos0.data_ptr(), out.data_ptr(), nseq, max_qlen, n_q, n_kv, hd, scale, status.data_ptr(),
                                     _lib.stream_ptr(), v_desc_variant), "rx_attn_prefill_tc")
     _lib.count()

@@ -121,6 +121,7 @@ def _declare(lib):
         "rx_topk": (c_int, [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void]),
         "rx_make_kv_tmap": (c_int, [c_void, c_void, c_ll, c_int]),
         "rx_make_kv_tmap8": (c_int, [c_void, c_void, c_ll, c_int]),
+        "rx_make_kv_tmap_f8": (c_int, [c_void, c_void, c_ll, c_int]),
         "rx_attn_decode_chunk": (c_int, []),
         "rx_attn_decode_scratch_floats": (c_ll, [c_int, c_int, c_int, c_int]),
         "rx_attn_decode": (c_int, [c_void, c_void, c_void, c_void, c_int, c_void, c_void, c_void, c_int, c_int, c_int, c_int, c_int, c_f,
