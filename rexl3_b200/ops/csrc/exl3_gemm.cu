@@ -414,7 +414,7 @@ RX_API int rx_exl3_gemm(const void* xr, int rows, int K, const void* trellis, in
 
 // Grouped (mixture-of-experts) form.  xs: fp16 [pairs_cap, K], rows sorted by expert (each row already rotated with its expert's
 // suh).  trellis: int16 [E][K/16, N/16, 16*bits].  tile_tab: device int32 [max_tiles][3] = {expert, first row, rows} (rows == 0: idle
-// tile).  part: fp32 [splits, pairs_cap, N].  `tile_rows` is the MMA N of every tile (16..256, fixed for the launch).
+// tile, anywhere in the table).  part: fp32 [splits, pairs_cap, N].  `tile_rows` is the MMA N of every tile (16..256, fixed for the launch).
 RX_API int rx_exl3_gemm_grouped(const void* xs, int pairs_cap, int K, const void* trellis, long long expert_elems, int N, int twice, int codebook,
                                 void* part, int splits, const void* tile_tab, int max_tiles, int tile_rows, int* status, void* stream) {
   if (pairs_cap <= 0 || K % 128 != 0 || N % 128 != 0 || splits < 1 || splits > K / KCH || max_tiles < 1 || max_tiles > 65535) return (int)cudaErrorInvalidValue;

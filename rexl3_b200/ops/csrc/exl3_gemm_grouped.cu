@@ -1,6 +1,6 @@
 // EXL3 GEMM over a list of (expert, row tile) pairs, 3.0 and 4.0 bpw, decoded weights in TENSOR MEMORY (sm_100a).  Contract of the grouped form in
-// exl3_gemm.cu: part[split][row][n] = partial sums of xs @ W_q[expert], rows sorted by expert, tile_tab[t] = {expert, first row, rows}, live
-// tiles first.  Without a table the tiles are those of a plain GEMM.
+// exl3_gemm.cu: part[split][row][n] = partial sums of xs @ W_q[expert], rows sorted by expert, tile_tab[t] = {expert, first row, rows}; tiles of no
+// rows, which the planner puts last, may stand anywhere.  Without a table the tiles are those of a plain GEMM.
 //
 // Bound by the trellis decode (two integer pipes, see exl3_decode.cuh).  Decode as in exl3_gemm_tm.cu: a thread owns one of the strip's 128 columns
 // (one TMEM lane) and emits its k-values as packed fp16 pairs, the MMA reads A from tensor memory and the activations from shared memory.
@@ -89,7 +89,8 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   volatile int* last_flag = abort_flag + 1;          // of the wait before the tensor memory is freed, which an abort does not cut short
 
-  int* split_c0 = (int*)(last_flag + 1);              // [splits + 1] first chunk of each split
+  volatile int* tile_end = last_flag + 1;             // the last live tile + 1, -1: not known yet
+  int* split_c0 = (int*)(tile_end + 1);               // [splits + 1] first chunk of each split
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strips = N / GR_STRIP, per_tile = strips * splits, nch = K / GR_KCH, nt_total = N / 16;
   const int acc_cols = gr_acc_cols(brows);
@@ -103,6 +104,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     for (int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], 4);
     mbar_init(drained, 1);
     *abort_flag = *last_flag = 0;
+    *tile_end = -1;
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
   }
@@ -134,14 +136,19 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     if (w.split >= splits) w.split -= splits, ++w.tile;
   };
   struct Item { int expert, row0, nrows; };
-  auto tile_of = [&](const Walk& w, Item& it) {        // false past the last item (live tiles come first)
+  auto tile_of = [&](const Walk& w, Item& it) {        // false past the last item
     if (w.tile >= max_tiles) return false;
     if (tile_tab != nullptr) {
       it.expert = tile_tab[3 * w.tile], it.row0 = tile_tab[3 * w.tile + 1], it.nrows = tile_tab[3 * w.tile + 2];
     } else {
       it.expert = 0, it.row0 = w.tile * brows, it.nrows = min(brows, rows - it.row0);
     }
-    return it.nrows > 0;
+    if (it.nrows > 0) return true;
+    // an idle tile: the end, or, before live ones, an item like the others whose rows are written nowhere
+    it.expert = it.row0 = it.nrows = 0;
+    int end = -1;
+    for (int i = 0; i < (1 << 20) && (end = *tile_end) < 0; ++i) {}
+    return w.tile < end;
   };
   Item it;
   Walk at = walk_of(blockIdx.x);
@@ -182,6 +189,15 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     }
   } else if (warp == 1) {
     // ---- MMA issuer: A from tensor memory, B from shared memory; as many rows as the tile has, in sixteens
+    {
+      int last = -1;
+      if (tile_tab != nullptr)
+#pragma unroll 4
+        for (int t = lane; t < max_tiles; t += 32)
+          if (tile_tab[3 * t + 2] > 0) last = t;
+      last = __reduce_max_sync(0xffffffffu, last);
+      if (lane == 0) *tile_end = last + 1;
+    }
     if (lane == 0) {
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(b_base));
       const uint32_t half_units = (uint32_t)b_half >> 4, stage_units = (uint32_t)b_stage >> 4;
@@ -191,7 +207,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
         const int n = split_c0[at.split + 1] - split_c0[at.split];
         if (e >= 2 && !mbar_wait(&acc_empty[e & 1], ((e >> 1) - 1) & 1, abort_flag, status, 222)) break;
         tc_fence_after();
-        const uint32_t idesc = umma_idesc_f16(GR_STRIP, (it.nrows + 15) & ~15, 0, 0);
+        const uint32_t idesc = umma_idesc_f16(GR_STRIP, max(16, (it.nrows + 15) & ~15), 0, 0);
         const uint32_t acc = tmem_base + (e & 1) * acc_cols;
         for (int c = 0; c < n; ++c, ++gc) {
           const int s = gc % GR_OP_STAGES, sa = gc % SA;

@@ -57,6 +57,27 @@ def test_grouped_gemm(bits, cb, counts, K, N, splits):
         assert torch.equal(got[t], got[16])
 
 
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("tile_rows", [16, 128])
+@pytest.mark.parametrize("counts,K,N,splits", [([3, 1, 17, 32], 384, 256, 3), ([5] * 40, 512, 640, 2)])
+def test_idle_tiles_may_stand_anywhere(bits, tile_rows, counts, K, N, splits):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import lib
+    L, rows = lib.load(), sum(counts)
+    KK, xs, tr, _ = _problem(len(counts), K, N, bits, "3inst", counts, bits + K)
+    tiles = _tiles(counts, tile_rows, 0)
+    got = []
+    for tab in (tiles, [(0, 0, 0)] * 3 + [t for u in tiles for t in (u, (0, 0, 0))] + [(0, 0, 0)] * 40, tiles[::-1]):
+        tab = torch.tensor(tab, dtype=torch.int32, device="cuda")
+        part, st = torch.full((splits, rows, N), float("nan"), device="cuda"), KK.new_status()
+        lib.check(L.rx_exl3_gemm_grouped(xs.data_ptr(), rows, K, tr.data_ptr(), tr[0].numel(), N, 2 * bits, KK.CB_ID["3inst"], part.data_ptr(), splits,
+                                         tab.data_ptr(), tab.shape[0], tile_rows, st.data_ptr(), lib.stream_ptr()), "rx_exl3_gemm_grouped")
+        KK.check_status(st)
+        got.append(part)
+    assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 @pytest.mark.parametrize("rows", [65, 100, 128])
 @pytest.mark.parametrize("bits,splits", [(3, 4), (4, 4), (4, 3)])
 def test_plain_gemm_of_65_to_128_rows(rows, bits, splits):
