@@ -20,6 +20,7 @@
 // No cluster multicast anywhere; every wait is bounded and unwinds through the abort flag.
 #include <cuda.h>
 #include "exl3_decode.cuh"
+#include "exl3_gemm.cuh"
 
 namespace rx {
 
@@ -354,11 +355,6 @@ static int launch_gemm(const CUtensorMap& tm, const uint32_t* trellis, float* pa
   return (int)cudaGetLastError();
 }
 
-// the persistent kernel of exl3_gemm_grouped.cu
-bool gemm_persistent_takes(int K, int twice, int splits, int brows);
-int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits,
-                    const int* tile_tab, int max_tiles, int brows, int* status, cudaStream_t st);
-
 }  // namespace rx
 
 using namespace rx;
@@ -394,7 +390,7 @@ RX_API int rx_exl3_gemm(const void* xr, int rows, int K, const void* trellis, in
   // 65 to 128 rows at 3.0 bpw: one CTA per SM either way, and the persistent kernel's sixteen decode warps beat this one's eight (2048 -> 151,936,
   // 100 rows: 206 -> 150 us; up to 64 rows the two are level).  Only where both cut K at the same places: a row's bits do not depend on the row count.
   if (twice == 6 && brows == 128 && (K / 128) % splits == 0 && gemm_persistent_takes(K, twice, splits, brows))
-    return gemm_persistent(xr, rows, K, trellis, 0, N, twice, codebook, part, splits, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
+    return gemm_persistent(xr, rows, K, trellis, 0, N, twice, codebook, part, splits, 128, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xr, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
   if (e != 0) return e;
@@ -421,7 +417,7 @@ RX_API int rx_exl3_gemm_grouped(const void* xs, int pairs_cap, int K, const void
   if (tile_rows != rx_exl3_tile_rows(tile_rows) || (expert_elems % 2) != 0) return (int)cudaErrorInvalidValue;
   if ((((uintptr_t)xs) & 15) != 0 || (((uintptr_t)trellis) & 15) != 0) return (int)cudaErrorMisalignedAddress;
   if (gemm_persistent_takes(K, twice, splits, tile_rows) && expert_elems % 8 == 0)
-    return gemm_persistent(xs, pairs_cap, K, trellis, (size_t)expert_elems / 2, N, twice, codebook, part, splits, (const int*)tile_tab, max_tiles, tile_rows,
+    return gemm_persistent(xs, pairs_cap, K, trellis, (size_t)expert_elems / 2, N, twice, codebook, part, splits, KCH, (const int*)tile_tab, max_tiles, tile_rows,
                            status, (cudaStream_t)stream);
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xs, (uint64_t)pairs_cap, (uint64_t)K, (uint32_t)tile_rows);

@@ -17,10 +17,11 @@
 // first MMA waits for it.  No circle of waits: that chunk's A stage was last read by a chunk of item e or before.  Every wait is bounded.
 #include <cuda.h>
 #include "exl3_decode.cuh"
+#include "exl3_gemm.cuh"
 
 namespace rx {
 
-constexpr int GR_KCH = 128, GR_STRIP = 128, GR_OP_STAGES = 3, GR_RAW_STAGES = 8;
+constexpr int GR_KCH = 128, GR_HALF = 64, GR_STRIP = 128, GR_OP_STAGES = 3, GR_RAW_STAGES = 8;
 constexpr int GR_A_COLS = GR_KCH / 2;             // TMEM columns of one A stage (two fp16 per column)
 constexpr int GR_ROLE_WARPS = 3;
 // A decode group waits for "the MMA that last read this stage": sound while no group can run two phases ahead, i.e. with as many stages as groups.
@@ -63,7 +64,7 @@ __device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1]
 template <int TWICE, int CB, int NG>
 __global__ void __launch_bounds__(GR_ROLE_WARPS * 32 + NG * 128, (NG <= 3 ? 2 : 1))
 exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __restrict__ trellis, size_t expert_words,
-                         float* __restrict__ part, int rows, int K, int N, int splits, int brows, const int* tile_tab, int max_tiles,
+                         float* __restrict__ part, int rows, int K, int N, int splits, int cut, int brows, const int* tile_tab, int max_tiles,
                          int* status) {
   pdl_launch();
   constexpr int SA = gr_a_stages(NG), EW = TWICE / 2;            // EW: words of an eighth of a tile
@@ -90,9 +91,9 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
   volatile int* last_flag = abort_flag + 1;          // of the wait before the tensor memory is freed, which an abort does not cut short
 
   volatile int* tile_end = last_flag + 1;             // the last live tile + 1, -1: not known yet
-  int* split_c0 = (int*)(tile_end + 1);               // [splits + 1] first chunk of each split
+  int* split_c0 = (int*)(tile_end + 1);               // [splits + 1] where each split begins, in halves of a chunk
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int strips = N / GR_STRIP, per_tile = strips * splits, nch = K / GR_KCH, nt_total = N / 16;
+  const int strips = N / GR_STRIP, per_tile = strips * splits, nt_total = N / 16;
   const int acc_cols = gr_acc_cols(brows);
   uint32_t ncols = 32;
   while ((int)ncols < 2 * acc_cols + SA * GR_A_COLS) ncols <<= 1;
@@ -108,7 +109,8 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
   }
-  if (warp == 2 && lane <= splits) split_c0[lane] = (int)((unsigned)(nch * lane) / (unsigned)splits);
+  // splits are cut at multiples of `cut` k (64 or 128), where the other kernels of the same form cut them: the last chunk of a split may be half a chunk
+  if (warp == 2 && lane <= splits) split_c0[lane] = (int)((unsigned)(K / cut * lane) / (unsigned)splits) * (cut / GR_HALF);
   if (warp == 1) {
     tmem_alloc(tmem_slot, ncols);
     tmem_relinquish();
@@ -159,16 +161,16 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     bool ok = true;
     int gc = 0;
     for (; ok && tile_of(at, it); step(at, stride)) {
-      const int c0 = split_c0[at.split], n = split_c0[at.split + 1] - c0;
-      const uint32_t* src = trellis + (size_t)it.expert * expert_words + ((size_t)(c0 * 8 + (lane & 7)) * nt_total + (size_t)at.strip * 8) * TILE_WORDS;
+      const int c0 = split_c0[at.split], halves = split_c0[at.split + 1] - c0, n = (halves + 1) >> 1;
+      const uint32_t* src = trellis + (size_t)it.expert * expert_words + ((size_t)(c0 * 4 + (lane & 7)) * nt_total + (size_t)at.strip * 8) * TILE_WORDS;
       for (int c = 0; c < n && ok; ++c, ++gc) {
         const int s = gc % GR_RAW_STAGES;
         if (lane == 0) {
           if (gc >= GR_RAW_STAGES) ok = mbar_wait(&raw_empty[s], ((gc / GR_RAW_STAGES) - 1) & 1, abort_flag, status, 210, 500);
-          if (ok) mbar_arrive_expect_tx(&raw_full[s], RAW_STAGE);
+          if (ok) mbar_arrive_expect_tx(&raw_full[s], 2 * c + 2 > halves ? RAW_STAGE / 2 : RAW_STAGE);
         }
         ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-        if (ok && lane < 8) bulk_g2s(raw_base + s * RAW_STAGE + lane * ROW_BYTES, src + (size_t)c * 8 * nt_total * TILE_WORDS, ROW_BYTES, &raw_full[s]);
+        if (ok && lane < min(8, 4 * (halves - 2 * c))) bulk_g2s(raw_base + s * RAW_STAGE + lane * ROW_BYTES, src + (size_t)c * 8 * nt_total * TILE_WORDS, ROW_BYTES, &raw_full[s]);
       }
     }
   } else if (warp == 2) {
@@ -177,13 +179,14 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
       bool ok = true;
       int gc = 0;
       for (; ok && tile_of(at, it); step(at, stride)) {
-        const int c0 = split_c0[at.split], n = split_c0[at.split + 1] - c0;
+        const int c0 = split_c0[at.split], halves = split_c0[at.split + 1] - c0, n = (halves + 1) >> 1;
         for (int c = 0; c < n; ++c, ++gc) {
-          const int s = gc % GR_OP_STAGES, x = (c0 + c) * GR_KCH;
+          const int s = gc % GR_OP_STAGES, x = c0 * GR_HALF + c * GR_KCH;
+          const bool half = 2 * c + 2 > halves;
           if (gc >= GR_OP_STAGES && !mbar_wait(&b_empty[s], ((gc / GR_OP_STAGES) - 1) & 1, abort_flag, status, 211, 250)) { ok = false; break; }
-          mbar_arrive_expect_tx(&b_full[s], (uint32_t)b_stage);
+          mbar_arrive_expect_tx(&b_full[s], (uint32_t)(half ? b_half : b_stage));
           tma_load_2d(b_base + s * b_stage, &tmap_x, x, it.row0, &b_full[s]);
-          tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + 64, it.row0, &b_full[s]);
+          if (!half) tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + GR_HALF, it.row0, &b_full[s]);
         }
       }
     }
@@ -204,7 +207,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
       bool ok = true;
       int gc = 0;
       for (int e = 0; ok && tile_of(at, it); ++e, step(at, stride)) {
-        const int n = split_c0[at.split + 1] - split_c0[at.split];
+        const int halves = split_c0[at.split + 1] - split_c0[at.split], n = (halves + 1) >> 1;
         if (e >= 2 && !mbar_wait(&acc_empty[e & 1], ((e >> 1) - 1) & 1, abort_flag, status, 222)) break;
         tc_fence_after();
         const uint32_t idesc = umma_idesc_f16(GR_STRIP, max(16, (it.nrows + 15) & ~15), 0, 0);
@@ -218,7 +221,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
           const uint32_t a_at = a_tmem0 + sa * GR_A_COLS;
 #pragma unroll
           for (int k = 0; k < GR_KCH / 16; ++k)
-            tc_mma_f16_ts(acc, a_at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
+            if (k < GR_HALF / 16 || 2 * c + 2 <= halves) tc_mma_f16_ts(acc, a_at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
           tc_commit(&a_empty[sa]);
           tc_commit(&b_empty[s]);
         }
@@ -261,7 +264,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     };
     int gc0 = 0, e = 0;                           // chunks up to the end of item e
     for (int gc = grp; ok && tile_of(at, it); ++e, step(at, stride)) {
-      gc0 += split_c0[at.split + 1] - split_c0[at.split];
+      gc0 += (split_c0[at.split + 1] - split_c0[at.split] + 1) >> 1;
       for (; gc < gc0 && ok; gc += NG) {
         const int rs = gc % GR_RAW_STAGES, os = gc % SA;
         // (a wait that ran out is the whole warp's: lanes must not part before the next shuffle)
@@ -318,7 +321,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
 int make_tmap_f16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 template <int TWICE, int CB, int NG>
-static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t expert_words, float* part, int rows, int K, int N, int splits, int brows,
+static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t expert_words, float* part, int rows, int K, int N, int splits, int cut, int brows,
                           const int* tile_tab, int max_tiles, int* status, cudaStream_t st) {
   int smem = gr_smem_bytes(brows, TWICE) + 1024;
   if (NG <= 3 && smem < 80 * 1024) smem = 80 * 1024;   // at most two CTAs per SM: each allocates 256 TMEM columns
@@ -333,24 +336,24 @@ static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t
   if (items >= (1ll << 30)) return (int)cudaErrorInvalidValue;          // (item numbers are 32-bit)
   const long long slots = (NG <= 3 ? 2 : 1) * 148;
   rx::launch(kern, dim3((unsigned)(items < slots ? items : slots)), dim3(GR_ROLE_WARPS * 32 + NG * 128), smem, st, tm, trellis, expert_words, part, rows, K, N,
-             splits, brows, tile_tab, max_tiles, status);
+             splits, cut, brows, tile_tab, max_tiles, status);
   return (int)cudaGetLastError();
 }
 
-// Whether rx_exl3_gemm_persistent takes the product: widths with a column decoder, tiles whose two accumulators fit beside the A stages, splits in
-// whole 128-k chunks and no more of them than its table of their bounds holds.
+// Whether gemm_persistent takes the product: widths with a column decoder, tiles whose two accumulators fit beside the A stages, splits of a chunk
+// and more and no more of them than its table of their bounds holds.
 bool gemm_persistent_takes(int K, int twice, int splits, int brows) {
   return (twice == 6 || twice == 8) && brows <= 128 && splits <= K / GR_KCH && splits < 32;
 }
 
-int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits,
+int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits, int cut,
                     const int* tile_tab, int max_tiles, int brows, int* status, cudaStream_t st) {
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xs, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
   if (e != 0) return e;
   const uint32_t* tr = (const uint32_t*)trellis;
-#define RX_GR(T, CBV) (brows > 32 ? launch_grouped<T, CBV, 4>(tm, tr, expert_words, (float*)part, rows, K, N, splits, brows, tile_tab, max_tiles, status, st) \
-                                  : launch_grouped<T, CBV, 3>(tm, tr, expert_words, (float*)part, rows, K, N, splits, brows, tile_tab, max_tiles, status, st))
+#define RX_GR(T, CBV) (brows > 32 ? launch_grouped<T, CBV, 4>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st) \
+                                  : launch_grouped<T, CBV, 3>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st))
   switch (codebook) {
     case CB_3INST: return twice == 6 ? RX_GR(6, CB_3INST) : RX_GR(8, CB_3INST);
     case CB_MCG: return twice == 6 ? RX_GR(6, CB_MCG) : RX_GR(8, CB_MCG);

@@ -17,6 +17,7 @@
 // the first group also runs the epilogue.  Bounded waits everywhere; no cluster multicast.
 #include <cuda.h>
 #include "exl3_decode.cuh"
+#include "exl3_gemm.cuh"
 #include "tp.cuh"
 
 namespace rx {
@@ -260,11 +261,6 @@ int make_tmap_f16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t
 
 int make_tmap_trellis(CUtensorMap* out, const void* base, uint64_t kt_rows, uint64_t row_words, uint32_t box_words, uint32_t box_rows);
 
-// the persistent kernel of exl3_gemm_grouped.cu
-bool gemm_persistent_takes(int K, int twice, int splits, int brows);
-int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits,
-                    const int* tile_tab, int max_tiles, int brows, int* status, cudaStream_t st);
-
 template <int CB, int NG>
 static int launch_tm(const CUtensorMap& tm, const CUtensorMap& tw, float* part, int rows, int K, int N, int splits, int brows, int row_tiles,
                      int* status, cudaStream_t st, const GemmTp& tp) {
@@ -298,7 +294,7 @@ static int gemm_b4(const void* xr, int rows, int K, const void* trellis, int N, 
   // 65 to 128 rows on one rank: one CTA per SM either way, and a CTA that walks several items spares each its prologue and tail (verify window of 80
   // rows on eight layers 2165 -> 2120 us; up to 64 rows two CTAs per SM hide the prologue and this form is the better one: step of 64 rows 2130, 2290 us).
   if (brows == 128 && tp.strips_per_rank == 0 && tp.in_flag == nullptr && gemm_persistent_takes(K, 8, splits, brows))
-    return gemm_persistent(xr, rows, K, trellis, 0, N, 8, codebook, part, splits, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
+    return gemm_persistent(xr, rows, K, trellis, 0, N, 8, codebook, part, splits, 128, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xr, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
   if (e != 0) return e;

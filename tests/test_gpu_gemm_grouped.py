@@ -58,6 +58,29 @@ def test_grouped_gemm(bits, cb, counts, K, N, splits):
 
 
 @pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("K,splits", [(384, 2), (640, 2), (640, 3), (1408, 5), (512, 4)])       # all but the last: splits that end in half a chunk
+def test_splits_are_cut_at_64(bits, K, splits):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import lib
+    counts, N = [3, 40, 1, 100], 256
+    L, rows = lib.load(), sum(counts)
+    KK, xs, tr, dense = _problem(len(counts), K, N, bits, "3inst", counts, bits + K)
+    off = np.concatenate([[0], np.cumsum(counts)])
+    for tile_rows in (16, 128):
+        tab = torch.tensor(_tiles(counts, tile_rows, 3), dtype=torch.int32, device="cuda")
+        part, st = torch.full((splits, rows, N), float("nan"), device="cuda"), KK.new_status()
+        lib.check(L.rx_exl3_gemm_grouped(xs.data_ptr(), rows, K, tr.data_ptr(), tr[0].numel(), N, 2 * bits, KK.CB_ID["3inst"], part.data_ptr(), splits,
+                                         tab.data_ptr(), tab.shape[0], tile_rows, st.data_ptr(), lib.stream_ptr()), "rx_exl3_gemm_grouped")
+        KK.check_status(st)
+        for s in range(splits):
+            k0, k1 = K // 64 * s // splits * 64, K // 64 * (s + 1) // splits * 64
+            for e in range(len(counts)):
+                x, w = xs[off[e]:off[e + 1], k0:k1].double(), dense[e][k0:k1]
+                assert ((part[s, off[e]:off[e + 1]].double() - x @ w).abs() <= K * 2.0 ** -24 * (x.abs() @ w.abs()) + 1e-30).all()
+
+
+@pytest.mark.parametrize("bits", [3, 4])
 @pytest.mark.parametrize("tile_rows", [16, 128])
 @pytest.mark.parametrize("counts,K,N,splits", [([3, 1, 17, 32], 384, 256, 3), ([5] * 40, 512, 640, 2)])
 def test_idle_tiles_may_stand_anywhere(bits, tile_rows, counts, K, N, splits):
