@@ -150,6 +150,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer: one page of K and of V per step
     if (lane == 0) {
+      int n_k = 0, n_v = 0;                               // pages issued
       for (int j = 0; j < npages; ++j) {
         const int st = j % TC_STAGES;
         const int y = (bt[j] * a.n_kv + kvh) * TC_PAGE;
@@ -157,11 +158,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
         mbar_arrive_expect_tx(&k_full[st], TC_TILE);
         tma_load_2d(k_sm + st * TC_TILE, &tk, 0, y, &k_full[st]);
         tma_load_2d(k_sm + st * TC_TILE + 8192, &tk, 64, y, &k_full[st]);
+        ++n_k;
         if (j >= TC_STAGES && !mbar_wait(&v_empty[st], ((j / TC_STAGES) - 1) & 1, abort_flag, a.status, 71, 100)) break;
         mbar_arrive_expect_tx(&v_full[st], TC_TILE);
         tma_load_2d(v_sm + st * TC_TILE, &tv, 0, y, &v_full[st]);
         tma_load_2d(v_sm + st * TC_TILE + 8192, &tv, 64, y, &v_full[st]);
+        ++n_v;
       }
+      ring_landed(k_full, TC_STAGES, n_k);
+      ring_landed(v_full, TC_STAGES, n_v);
     }
   } else if (warp == 1 || warp == TC_ISSUER_1) {
     // ---------------------------------------------------------------- MMA issuer of one tile

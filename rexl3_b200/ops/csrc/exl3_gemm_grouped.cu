@@ -173,6 +173,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
         if (ok && lane < min(8, 4 * (halves - 2 * c))) bulk_g2s(raw_base + s * RAW_STAGE + lane * ROW_BYTES, src + (size_t)c * 8 * nt_total * TILE_WORDS, ROW_BYTES, &raw_full[s]);
       }
     }
+    if (lane == 0) ring_landed(raw_full, GR_RAW_STAGES, ok ? gc : gc - 1);      // (the chunk whose wait gave up was counted)
   } else if (warp == 2) {
     // ---- activation producer: two [brows x 64] swizzled boxes per chunk
     if (lane == 0) {
@@ -189,6 +190,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
           if (!half) tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + GR_HALF, it.row0, &b_full[s]);
         }
       }
+      ring_landed(b_full, GR_OP_STAGES, gc);
     }
   } else if (warp == 1) {
     // ---- MMA issuer: A from tensor memory, B from shared memory; as many rows as the tile has, in sixteens

@@ -117,3 +117,31 @@ def test_plain_gemm_of_65_to_128_rows(rows, bits, splits):
     assert torch.equal(part[:, :33], few)
     x = xs.double()
     assert ((part.double().sum(0) - x @ dense[0]).abs() <= K * 2.0 ** -23 * (x.abs() @ dense[0].abs())).all()
+
+
+@pytest.mark.parametrize("how", ["abort", "limit"])
+def test_waits_that_give_up_leave_the_device_usable(how):
+    """The abort word, or a wait limit of a microsecond: the call returns, says so if a wait gave up, and the next call is right."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import lib
+    counts, K, N = [70] * 24, 2048, 1536
+    L, rows = lib.load(), sum(counts)
+    KK, xs, tr, _ = _problem(len(counts), K, N, 3, "3inst", counts, 9)
+    tab = torch.tensor(_tiles(counts, 128, 9), dtype=torch.int32, device="cuda")
+
+    def run(st):
+        part = torch.zeros(2, rows, N, device="cuda")
+        lib.check(L.rx_exl3_gemm_grouped(xs.data_ptr(), rows, K, tr.data_ptr(), tr[0].numel(), N, 6, 0, part.data_ptr(), 2, tab.data_ptr(), tab.shape[0], 128,
+                                         st.data_ptr(), lib.stream_ptr()), "rx_exl3_gemm_grouped")
+        return part, st.tolist()[0]
+    want, code = run(KK.new_status())
+    assert code == 0
+    for _ in range(3):
+        st = KK.new_status()
+        KK.set_abort(st) if how == "abort" else KK.set_wait_limit(st, 1)
+        part, code = run(st)
+        assert code in (0, KK.ST_ABORTED if how == "abort" else KK.ST_TIMEOUT)
+        assert code != 0 or torch.equal(part, want)
+        part, code = run(KK.new_status())
+        assert code == 0 and torch.equal(part, want)
