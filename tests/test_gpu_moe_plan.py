@@ -68,3 +68,39 @@ def test_forms_of_few_planes_equal_the_general_ones(M, topk):
         for x, y in zip(got[0], other):
             assert torch.isfinite(x.float()).all() and x.abs().max() > 0 and torch.equal(x, y)
 
+
+
+@pytest.mark.parametrize("S", [2, 3, 4, 5, 9])
+@pytest.mark.parametrize("M,topk", [(3, 1), (70, 8), (5, 17)])
+def test_planes_are_added_in_order(S, M, topk):
+    """Random planes against one plane that holds their sums, added in plane order in fp32: every plane counts once, in its place, in every form."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.models.moe import CombineDst
+    from rexl3_b200.ops import lib
+    L, E, d, F, pairs = lib.load(), 24, 384, 256, M * topk
+    g = torch.Generator(device="cuda").manual_seed(M * topk + S)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    ids = torch.randint(0, E, (pairs,), device="cuda", generator=g).int()
+    pos = torch.randperm(pairs, device="cuda", generator=g).int()
+    pos[::7] = -1
+    w, svh, gu, dn = r(pairs).abs(), r(E, d).half(), r(S, pairs, 2 * F), r(S, pairs, d)
+    svh_gu, suh, tot = r(E, 2 * F).half(), r(E, F).half(), torch.tensor([pairs], dtype=torch.int32, device="cuda")
+
+    def added(t):
+        acc = t[0]
+        for p in t[1:]:
+            acc = acc + p
+        return acc[None].contiguous()
+    got = []
+    for a, b in ((dn, gu), (added(dn), added(gu))):
+        slot, act = torch.zeros(M, d, device="cuda"), torch.zeros(pairs, F, dtype=torch.float16, device="cuda")
+        dst = CombineDst()
+        dst.ranks, dst.rank, dst.rows_cap, dst.dst[0] = 1, 0, M, slot.data_ptr()
+        lib.check(L.rx_moe_combine(a.data_ptr(), a.shape[0], pairs, M, d, topk, ids.data_ptr(), w.data_ptr(), pos.data_ptr(), svh.data_ptr(), None,
+                                   ctypes.byref(dst), lib.stream_ptr()), "rx_moe_combine")
+        lib.check(L.rx_moe_swiglu_rot(b.data_ptr(), b.shape[0], pairs, F, ids.data_ptr(), tot.data_ptr(), svh_gu.data_ptr(), suh.data_ptr(), act.data_ptr(),
+                                      lib.stream_ptr()), "rx_moe_swiglu_rot")
+        got.append((slot, act))
+    for x, y in zip(*got):
+        assert torch.isfinite(x.float()).all() and x.abs().max() > 0 and torch.equal(x, y)

@@ -161,3 +161,14 @@ def test_tree_window_over_quantized_caches(qmodel, ctx_len):
     assert np.array_equal(ref.ids, nxt.ids) and np.array_equal(ref.values, nxt.values)
     be.release(1)
     assert be.pool.free_blocks() == be.pool.total_blocks()
+
+
+@pytest.mark.parametrize("ctx_len", [1020, 1025, 1300])
+def test_tree_window_over_a_long_e4m3_context(ctx_len):
+    """The same with several chunks below the tree: it begins inside a chunk, at a chunk's first key, and runs over the end of one."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.models import dense
+    m = dense.DenseGPU(dense.random_weights(dense.CONFIGS["test-hd128"], seed=3), num_pages=160, max_rows=64, max_seqs=8, max_blocks_per_seq=24, max_prefill_rows=1536,
+                       kv_dtype="fp8")
+    test_tree_window_over_quantized_caches(m, ctx_len)
