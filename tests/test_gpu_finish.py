@@ -34,6 +34,26 @@ def test_add_norm_rot_rows_do_not_depend_on_their_number(N, norm):
     assert (whole[0].double() - y).abs().max() <= 2.0 ** -8 * y.abs().max() + 1e-5      # one rounding to bf16
 
 
+@pytest.mark.parametrize("M,N", [(592, 5120), (593, 3072), (593, 5120), (601, 4224), (593, 5248), (4096, 2048), (4097, 1152), (4097, 2048), (4097, 1024)])
+def test_add_norm_rot_at_the_edges_of_the_row_form(M, N):
+    """Both sides of every bound of the row form: the same bits as in calls of few rows."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    w, part, h0, nw, suh = _weight(N, g), r(M, N), r(M, N).bfloat16(), (1 + 0.1 * r(N)).bfloat16(), r(N).half()
+    got = []
+    for step in (M, 300):
+        out = [h0.clone(), torch.zeros(M, N, dtype=torch.float16, device="cuda"), torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")]
+        for a in range(0, M, step):
+            b = min(M, a + step)
+            K.finish_add_norm_rot(part[a:b], 1, b - a, w, out[0][a:b], nw, 1e-6, suh, out[1][a:b], out[2][a:b])
+        got.append(out)
+    for x, y in zip(*got):
+        assert torch.isfinite(x.float()).all() and torch.equal(x, y)
+
+
 @pytest.mark.parametrize("N", [128, 640, 3968, 4096, 5120, 8192, 8320])     # clusters: up to 16 rows below 4096, up to 64 from there to 8192
 @pytest.mark.parametrize("S", [1, 7, 18])
 @pytest.mark.parametrize("norm,rot,xn", [(True, True, True), (False, True, False), (True, False, True), (True, False, False)])
