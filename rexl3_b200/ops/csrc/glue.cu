@@ -188,49 +188,53 @@ struct TopkShared { uint64_t group[TOPK_GROUPS], list[TOPK_LIST], least; int n; 
 // second stage).  The count-th largest of the maxima of 64 thread groups is no larger than the count-th largest key, so only keys from there on
 // can be among the results - hardly more than `count` of them -, and each finds its own place by counting the larger
 // ones: 4.0 and 3.7 us; 80 rows 34 -> 7.6 and 9.1 -> 3.8 us.
-// Only where one group is far below the others do more keys pass than the list holds; then the rounds are run.
+// Only where one group is far below the others do more keys pass than the list holds; then the rounds are run.  One or two results are found faster by
+// rounds (one of 152k, one row 3.4 and 5.4 us, 80 rows 16 and 24 us; two 4.4 and 5.7, 25 and 24 us; three 5.2 and 5.5, 34 and 24 us).
+constexpr int TOPK_ROUNDS = 2;
 __device__ __forceinline__ void block_select(uint64_t (&k)[TOPK_PER_THREAD], int count, uint64_t* out, TopkShared& sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint64_t m[TOPK_PER_THREAD / 2];
+  if (count > TOPK_ROUNDS) {
+    uint64_t m[TOPK_PER_THREAD / 2];
 #pragma unroll
-  for (int i = 0; i < TOPK_PER_THREAD / 2; ++i) m[i] = u64_max(k[i], k[i + TOPK_PER_THREAD / 2]);
+    for (int i = 0; i < TOPK_PER_THREAD / 2; ++i) m[i] = u64_max(k[i], k[i + TOPK_PER_THREAD / 2]);
 #pragma unroll
-  for (int h = TOPK_PER_THREAD / 4; h > 0; h >>= 1)
+    for (int h = TOPK_PER_THREAD / 4; h > 0; h >>= 1)
 #pragma unroll
-    for (int i = 0; i < h; ++i) m[i] = u64_max(m[i], m[i + h]);
+      for (int i = 0; i < h; ++i) m[i] = u64_max(m[i], m[i + h]);
 #pragma unroll
-  for (int o = 1; o < TOPK_THREADS / TOPK_GROUPS; o <<= 1) m[0] = u64_max(m[0], __shfl_xor_sync(0xffffffffu, m[0], o));
-  if (tid % (TOPK_THREADS / TOPK_GROUPS) == 0) sm.group[tid / (TOPK_THREADS / TOPK_GROUPS)] = m[0];
-  if (tid == 0) sm.n = 0;
-  __syncthreads();
-  if (tid < TOPK_GROUPS) {
-    const uint64_t mine = sm.group[tid];
-    int place = 0;
-#pragma unroll 16
-    for (int j = 0; j < TOPK_GROUPS; ++j) place += sm.group[j] > mine || (sm.group[j] == mine && j < tid);
-    if (place == count - 1) sm.least = mine;
-  }
-  __syncthreads();
-  const uint64_t least = sm.least;
-#pragma unroll
-  for (int i = 0; i < TOPK_PER_THREAD; ++i)
-    if (k[i] != 0 && k[i] >= least) {
-      const int at = atomicAdd(&sm.n, 1);
-      if (at < TOPK_LIST) sm.list[at] = k[i];
-    }
-  __syncthreads();
-  const int n = sm.n;
-  if (n <= TOPK_LIST) {
-    for (int i = tid; i < n; i += TOPK_THREADS) {
-      const uint64_t mine = sm.list[i];
-      int place = 0;
-#pragma unroll 4
-      for (int j = 0; j < n; ++j) place += sm.list[j] > mine;
-      if (place < count) out[place] = mine;
-    }
-    for (int r = n + tid; r < count; r += TOPK_THREADS) out[r] = 0;
+    for (int o = 1; o < TOPK_THREADS / TOPK_GROUPS; o <<= 1) m[0] = u64_max(m[0], __shfl_xor_sync(0xffffffffu, m[0], o));
+    if (tid % (TOPK_THREADS / TOPK_GROUPS) == 0) sm.group[tid / (TOPK_THREADS / TOPK_GROUPS)] = m[0];
+    if (tid == 0) sm.n = 0;
     __syncthreads();
-    return;
+    if (tid < TOPK_GROUPS) {
+      const uint64_t mine = sm.group[tid];
+      int place = 0;
+#pragma unroll 16
+      for (int j = 0; j < TOPK_GROUPS; ++j) place += sm.group[j] > mine || (sm.group[j] == mine && j < tid);
+      if (place == count - 1) sm.least = mine;
+    }
+    __syncthreads();
+    const uint64_t least = sm.least;
+#pragma unroll
+    for (int i = 0; i < TOPK_PER_THREAD; ++i)
+      if (k[i] != 0 && k[i] >= least) {
+        const int at = atomicAdd(&sm.n, 1);
+        if (at < TOPK_LIST) sm.list[at] = k[i];
+      }
+    __syncthreads();
+    const int n = sm.n;
+    if (n <= TOPK_LIST) {
+      for (int i = tid; i < n; i += TOPK_THREADS) {
+        const uint64_t mine = sm.list[i];
+        int place = 0;
+#pragma unroll 4
+        for (int j = 0; j < n; ++j) place += sm.list[j] > mine;
+        if (place < count) out[place] = mine;
+      }
+      for (int r = n + tid; r < count; r += TOPK_THREADS) out[r] = 0;
+      __syncthreads();
+      return;
+    }
   }
   for (int r = 0; r < count; ++r) {
     uint64_t best = 0;

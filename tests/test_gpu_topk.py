@@ -30,3 +30,16 @@ def test_topk_is_the_head_of_a_full_sort(vocab, kind, count):
     K.topk(x, count, K.topk_scratch(5, vocab, count), got_i, got_v)
     v, i = x.sort(dim=-1, descending=True, stable=True)
     assert torch.equal(got_i.long(), i[:, :count]) and torch.equal(got_v, v[:, :count])
+
+
+@pytest.mark.parametrize("count", [2, 3])                   # the last count that is found by rounds, the first by the threshold
+@pytest.mark.parametrize("vocab", [3, 300, 151936])
+def test_topk_on_both_sides_of_the_forms(vocab, count):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import kernels as K
+    x = (torch.randn(7, vocab, device="cuda", generator=torch.Generator(device="cuda").manual_seed(vocab)) * 3).round() + 0.0
+    got_i, got_v = torch.zeros(7, count, dtype=torch.int32, device="cuda"), torch.zeros(7, count, device="cuda")
+    K.topk(x, count, K.topk_scratch(7, vocab, count), got_i, got_v)
+    v, i = x.sort(dim=-1, descending=True, stable=True)
+    assert torch.equal(got_i.long(), i[:, :count]) and torch.equal(got_v, v[:, :count])
