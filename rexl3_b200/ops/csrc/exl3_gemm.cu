@@ -388,8 +388,9 @@ RX_API int rx_exl3_gemm(const void* xr, int rows, int K, const void* trellis, in
   const int brows = rx_exl3_tile_rows(rows);
   const int row_tiles = (rows + brows - 1) / brows;
   // 65 to 128 rows at 3.0 bpw: one CTA per SM either way, and the persistent kernel's sixteen decode warps beat this one's eight (2048 -> 151,936,
-  // 100 rows: 206 -> 150 us; up to 64 rows the two are level).  Only where both cut K at the same places: a row's bits do not depend on the row count.
-  if (twice == 6 && brows == 128 && (K / 128) % splits == 0 && gemm_persistent_takes(K, twice, splits, brows))
+  // 100 rows: 206 -> 150 us; up to 64 rows the two are level), where its CTAs have more than one item (2048 -> 1536, 96 items: 6.8 and 7.3 us).
+  // Only where both cut K at the same places: a row's bits do not depend on the row count.
+  if (twice == 6 && brows == 128 && (long long)(N / STRIP) * splits > 148 && (K / 128) % splits == 0 && gemm_persistent_takes(K, twice, splits, brows))
     return gemm_persistent(xr, rows, K, trellis, 0, N, twice, codebook, part, splits, 128, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xr, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);

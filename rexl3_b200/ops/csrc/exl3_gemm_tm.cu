@@ -293,7 +293,8 @@ static int gemm_b4(const void* xr, int rows, int K, const void* trellis, int N, 
   const int row_tiles = (rows + brows - 1) / brows;
   // 65 to 128 rows on one rank: one CTA per SM either way, and a CTA that walks several items spares each its prologue and tail (verify window of 80
   // rows on eight layers 2165 -> 2120 us; up to 64 rows two CTAs per SM hide the prologue and this form is the better one: step of 64 rows 2130, 2290 us).
-  if (brows == 128 && tp.strips_per_rank == 0 && tp.in_flag == nullptr && gemm_persistent_takes(K, 8, splits, brows))
+  // With one item for a CTA there is nothing to spare (2048 -> 1536, 80 rows, 96 items: 5.8 us by this form, 7.0 by the persistent one).
+  if (brows == 128 && (long long)(N / 128) * splits > 148 && tp.strips_per_rank == 0 && tp.in_flag == nullptr && gemm_persistent_takes(K, 8, splits, brows))
     return gemm_persistent(xr, rows, K, trellis, 0, N, 8, codebook, part, splits, 128, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xr, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);

@@ -119,6 +119,24 @@ def test_plain_gemm_of_65_to_128_rows(rows, bits, splits):
     assert ((part.double().sum(0) - x @ dense[0]).abs() <= K * 2.0 ** -23 * (x.abs() @ dense[0].abs())).all()
 
 
+@pytest.mark.parametrize("rows", [65, 128])
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("N", [4736, 4864])                # 148 and 152 items: one for a CTA, and more
+def test_plain_gemm_of_many_items(rows, bits, N):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    K, splits = 1024, 4
+    KK, xs, tr, dense = _problem(1, K, N, bits, "3inst", [rows], 1)
+    w = KK.Exl3Weight(tr[0].contiguous(), None, None, None, "3inst")
+    st, part, few = KK.new_status(), torch.zeros(splits, rows, N, device="cuda"), torch.zeros(splits, 33, N, device="cuda")
+    KK.exl3_gemm(xs, w, part, splits, st)
+    KK.exl3_gemm(xs[:33].contiguous(), w, few, splits, st)
+    KK.check_status(st)
+    assert torch.equal(part[:, :33], few)
+    x = xs.double()
+    assert ((part.double().sum(0) - x @ dense[0]).abs() <= K * 2.0 ** -23 * (x.abs() @ dense[0].abs())).all()
+
+
 @pytest.mark.parametrize("how", ["abort", "limit"])
 def test_waits_that_give_up_leave_the_device_usable(how):
     """The abort word, or a wait limit of a microsecond: the call returns, says so if a wait gave up, and the next call is right."""
