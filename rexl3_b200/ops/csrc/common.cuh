@@ -113,8 +113,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
-// The copies of the last `issued` phases of a ring of `stages` barriers have landed.  A producer waits for them before it returns (bounded, and not cut short by
-// an abort): a consumer whose wait gave up does not, and a copy must not arrive in memory that this CTA has left.
+// Waits (bounded, and not cut short by an abort) until the copies of the last of `issued` phases of a ring of `stages` barriers have landed: a consumer whose
+// wait gave up does not, and a copy must not arrive in memory that its CTA has left.
 __device__ __forceinline__ void ring_landed(uint64_t* bars, int stages, int issued) {
   for (int c = issued > stages ? issued - stages : 0; c < issued; ++c)
     for (int i = 0; i < (1 << 20) && !mbar_try_wait(&bars[c % stages], (uint32_t)(c / stages) & 1); ++i) __nanosleep(100);

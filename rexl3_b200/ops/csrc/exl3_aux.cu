@@ -456,9 +456,9 @@ RX_API int rx_finish_add_norm_rot(const void* part, int S, int M, int N, const v
                                   float eps, const void* suh_next, void* xr, void* stream, void* xn_out) {
   if (N % 128 || N * 4 > 200 * 1024 || N / 128 > 512) return (int)cudaErrorInvalidValue;
   // Up to 592 rows the form below is two waves of two 32-warp CTAs per SM at most and the faster one (592 rows of 5120: 10.8 us, 13.9 by the row form; 593
-  // rows 14.4 and 13.9, 1500 rows 25.4 and 23.4); for shorter rows, of which an SM holds more, much longer (1184 rows of 2048 9.3 and 10.1, 8192 rows
-  // 66.5 and 61.9; rows of 1024 always).
-  if (S == 1 && N > 1024 && N <= ROWS_NB * 1024 && M > (N >= 3072 ? 592 : 4096)) {
+  // rows 14.4 and 13.9, 1500 rows 25.4 and 23.4); for shorter rows, of which an SM holds more, longer (1184 rows of 2048 9.3 and 10.1, 2100
+  // level, 8192 66.5 and 61.9; rows of 1024 always).
+  if (S == 1 && N > 1024 && N <= ROWS_NB * 1024 && M > (N >= 3072 ? 592 : 2048)) {
     rx::launch(finish_add_norm_rot_rows_kernel, dim3(M), dim3(256), 0, (cudaStream_t)stream, (const float*)part, N, (const __half*)svh, (const float*)bias,
                (uint16_t*)h_bf16, (const uint16_t*)norm_w, eps, (const __half*)suh_next, (__half*)xr, (uint16_t*)xn_out);
     return (int)cudaGetLastError();

@@ -91,7 +91,8 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
   volatile int* last_flag = abort_flag + 1;          // of the wait before the tensor memory is freed, which an abort does not cut short
 
   volatile int* tile_end = last_flag + 1;             // the last live tile + 1, -1: not known yet
-  int* split_c0 = (int*)(tile_end + 1);               // [splits + 1] where each split begins, in halves of a chunk
+  volatile int* n_sent = tile_end + 1;                // [2] chunks that the producers have issued: weights, activations
+  int* split_c0 = (int*)(n_sent + 2);                 // [splits + 1] where each split begins, in halves of a chunk
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strips = N / GR_STRIP, per_tile = strips * splits, nt_total = N / 16;
   const int acc_cols = gr_acc_cols(brows);
@@ -173,7 +174,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
         if (ok && lane < min(8, 4 * (halves - 2 * c))) bulk_g2s(raw_base + s * RAW_STAGE + lane * ROW_BYTES, src + (size_t)c * 8 * nt_total * TILE_WORDS, ROW_BYTES, &raw_full[s]);
       }
     }
-    if (lane == 0) ring_landed(raw_full, GR_RAW_STAGES, ok ? gc : gc - 1);      // (the chunk whose wait gave up was counted)
+    if (lane == 0) n_sent[0] = ok ? gc : gc - 1;       // (the chunk whose wait gave up was counted)
   } else if (warp == 2) {
     // ---- activation producer: two [brows x 64] swizzled boxes per chunk
     if (lane == 0) {
@@ -190,7 +191,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
           if (!half) tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + GR_HALF, it.row0, &b_full[s]);
         }
       }
-      ring_landed(b_full, GR_OP_STAGES, gc);
+      n_sent[1] = gc;
     }
   } else if (warp == 1) {
     // ---- MMA issuer: A from tensor memory, B from shared memory; as many rows as the tile has, in sixteens
@@ -313,6 +314,10 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
   }
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0 && lane == 0) {                // consumers that gave up have not seen the last copies arrive
+    if (warp == 0) ring_landed(raw_full, GR_RAW_STAGES, n_sent[0]);
+    if (warp == 2) ring_landed(b_full, GR_OP_STAGES, n_sent[1]);
+  }
   if (warp == 1) {
     if (lane == 0) mbar_wait(drained, 0, last_flag, status, 241);      // nothing may still write the tensor memory that is freed
     __syncwarp();

@@ -70,10 +70,13 @@ __global__ void __launch_bounds__(256) moe_router_logits_kernel(const uint16_t* 
 #pragma unroll
   for (int i = 0; i < R; ++i)
 #pragma unroll
-    for (int j = 0; j < C; ++j) {
-      const float v = warp_sum(acc[i][j]);
-      if (lane == 0 && r0 + i < M && e0 + j < E) logits[(size_t)(r0 + i) * E + e0 + j] = v;
-    }
+    for (int j = 0; j < C; ++j) acc[i][j] = warp_sum(acc[i][j]);      // (side by side: with a store after each they are a chain)
+  if (lane != 0) return;
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < C; ++j)
+      if (r0 + i < M && e0 + j < E) logits[(size_t)(r0 + i) * E + e0 + j] = acc[i][j];
 }
 // 4 x 4 from the size on that fills the chip with two CTAs per SM
 static cudaError_t router_logits(const void* x, const void* gate, int M, int d, int E, void* logits, void* stream) {
@@ -207,9 +210,11 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const uint16_t* __restr
 // A stable counting sort: each of the 32 warps owns a run of pairs and counts it 32 pairs at a time (lanes that chose the same expert find
 // each other with one match), the counts are summed over the warps and the experts, and each warp places its run in a second pass.  Bound by
 // the latency of a few hundred dependent steps: two passes of pairs / 1024 steps, where a ballot per owned expert took experts / 32 times as many
-// (128 experts: 356 -> 43 us for 16,800 pairs, 14 -> 5 us for 128).  Dynamic shared memory: 32 x E counters.
+// (128 experts: 356 -> 43 us for 16,800 pairs, 14 -> 5 us for 128).  A CTA has a thread per expert and a warp per 32 pairs, up to 1024: with all 32 warps
+// a small window paid for empty ones (8 pairs, 16 experts 5.2 us).  Dynamic shared memory: (warps) x E counters.
 constexpr int PLAN_WARPS = 32;
-__device__ __forceinline__ int plan_scan(int v, int* tmp, int& all) {      // exclusive sum over the CTA's 1024 threads, in thread order
+template <int W>
+__device__ __forceinline__ int plan_scan(int v, int* tmp, int& all) {      // exclusive sum over the CTA's threads, in thread order
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int s = v;
 #pragma unroll
@@ -220,7 +225,7 @@ __device__ __forceinline__ int plan_scan(int v, int* tmp, int& all) {      // ex
   if (lane == 31) tmp[warp] = s;
   __syncthreads();
   int before = 0, run = 0;
-  for (int w = 0; w < PLAN_WARPS; ++w) {
+  for (int w = 0; w < (W > 0 ? W : (int)blockDim.x / 32); ++w) {
     if (w == warp) before = run;
     run += tmp[w];
   }
@@ -228,18 +233,19 @@ __device__ __forceinline__ int plan_scan(int v, int* tmp, int& all) {      // ex
   all = run;
   return before + s - v;
 }
+template <int W>                              // warps, 0: as many as the CTA has
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* ids, int pairs, int E, int e_lo, int e_hi, int tile_rows, int max_tiles,
                                                         int* __restrict__ offs, int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos,
                                                         int* __restrict__ expert_of_pos, int* __restrict__ tile_tab, int* __restrict__ total) {
   pdl_launch();
   pdl_wait();
-  extern __shared__ int plan_cnt[];           // [PLAN_WARPS][E]: counts, then the position of a warp's next pair of an expert
+  extern __shared__ int plan_cnt[];           // [warps][E]: counts, then the position of a warp's next pair of an expert
   __shared__ int tmp[PLAN_WARPS];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (int i = t; i < PLAN_WARPS * E; i += 1024) plan_cnt[i] = 0;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = W > 0 ? W : blockDim.x / 32, threads = 32 * warps;
+  for (int i = t; i < warps * E; i += threads) plan_cnt[i] = 0;
   __syncthreads();
   int* mine = plan_cnt + warp * E;
-  const int run = (pairs + 1023) / 1024 * 32, p_begin = warp * run, p_end = min(pairs, p_begin + run);
+  const int run = (pairs + threads - 1) / threads * 32, p_begin = warp * run, p_end = min(pairs, p_begin + run);
   for (int p0 = p_begin; p0 < p_end; p0 += 32) {
     const int p = p0 + lane;
     const int e = p < p_end ? ids[p] : -1;
@@ -251,17 +257,17 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* ids, int pair
   __syncthreads();
   int cnt = 0, all, tiles;
   if (t < E)
-    for (int w = 0; w < PLAN_WARPS; ++w) {
+    for (int w = 0; w < warps; ++w) {
       const int c = plan_cnt[w * E + t];
       plan_cnt[w * E + t] = cnt;
       cnt += c;
     }
-  const int start = plan_scan(cnt, tmp, all);
+  const int start = plan_scan<W>(cnt, tmp, all);
   const int ntile = (cnt + tile_rows - 1) / tile_rows;
-  const int tile0 = plan_scan(ntile, tmp, tiles);
+  const int tile0 = plan_scan<W>(ntile, tmp, tiles);
   if (t < E) {
     offs[t] = start;
-    for (int w = 0; w < PLAN_WARPS; ++w) plan_cnt[w * E + t] += start;
+    for (int w = 0; w < warps; ++w) plan_cnt[w * E + t] += start;
     for (int i = 0; i < ntile && tile0 + i < max_tiles; ++i) {
       int* tab = tile_tab + 3 * (tile0 + i);
       tab[0] = t;
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* ids, int pair
     offs[E] = all;
     *total = all;
   }
-  for (int i = 3 * min(tiles, max_tiles) + t; i < 3 * max_tiles; i += 1024) tile_tab[i] = 0;
+  for (int i = 3 * min(tiles, max_tiles) + t; i < 3 * max_tiles; i += threads) tile_tab[i] = 0;
   __syncthreads();
   for (int p0 = p_begin; p0 < p_end; p0 += 32) {
     const int p = p0 + lane;
@@ -438,7 +444,7 @@ struct CombineDst {
 // PLANES: 1 and 4 for windows of one plane and of up to four; eight (four) slots' blocks are then loaded before the first is used, where one slot after the
 // other was a chain of as many memory latencies (2100 rows x 8 picks of 2048: 113 -> 58 us; 16 rows in three planes: 12.2 -> 8.4 us).  0: any number of planes.
 template <int PLANES>
-__global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ part, int S, int pairs_cap, int M, int d, int topk, const int* __restrict__ ids,
+__global__ void __launch_bounds__(PLANES > 0 ? 256 : 1024) moe_combine_kernel(const float* __restrict__ part, int S, int pairs_cap, int M, int d, int topk, const int* __restrict__ ids,
                                    const float* __restrict__ w, const int* __restrict__ pos_of_pair, const __half* __restrict__ svh_down,
                                    const float* __restrict__ shared, const __grid_constant__ CombineDst tp) {
   pdl_launch();
@@ -702,14 +708,16 @@ RX_API int rx_moe_router_grouped(const void* x, const void* gate, const void* bi
 RX_API int rx_moe_plan(const void* ids, int pairs, int E, int e_lo, int e_hi, int tile_rows, int max_tiles, void* offs, void* pos_of_pair,
                        void* pair_of_pos, void* expert_of_pos, void* tile_tab, void* total, void* stream) {
   if (pairs < 1 || E < 1 || E > 512 || e_lo < 0 || e_hi > E || e_lo >= e_hi || tile_rows < 16 || max_tiles < 1) return (int)cudaErrorInvalidValue;
-  const size_t smem = (size_t)PLAN_WARPS * E * sizeof(int);
+  const int need = (pairs > E ? pairs : E), warps = need < 32 * PLAN_WARPS ? (need + 31) / 32 : PLAN_WARPS;
+  const size_t smem = (size_t)warps * E * sizeof(int);
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_WARPS * 512 * (int)sizeof(int));
+    cudaError_t e = cudaFuncSetAttribute(moe_plan_kernel<PLAN_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_WARPS * 512 * (int)sizeof(int));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_plan_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_WARPS * 512 * (int)sizeof(int));
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return (int)rx::launch(moe_plan_kernel, dim3(1), dim3(1024), smem, (cudaStream_t)stream, (const int*)ids, pairs, E, e_lo, e_hi, tile_rows, max_tiles,
+  return (int)rx::launch(warps == PLAN_WARPS ? moe_plan_kernel<PLAN_WARPS> : moe_plan_kernel<0>, dim3(1), dim3(32 * warps), smem, (cudaStream_t)stream, (const int*)ids, pairs, E, e_lo, e_hi, tile_rows, max_tiles,
                          (int*)offs, (int*)pos_of_pair, (int*)pair_of_pos, (int*)expert_of_pos, (int*)tile_tab, (int*)total);
 }
 
