@@ -61,7 +61,8 @@ __device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1]
   }
 }
 
-template <int TWICE, int CB, int NG>
+// HALVES: the last chunk of a split may be half a chunk (its checks cost the MMA issuer and the producers 1 % of a window of 80 rows).
+template <int TWICE, int CB, int NG, bool HALVES>
 __global__ void __launch_bounds__(GR_ROLE_WARPS * 32 + NG * 128, (NG <= 3 ? 2 : 1))
 exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __restrict__ trellis, size_t expert_words,
                          float* __restrict__ part, int rows, int K, int N, int splits, int cut, int brows, const int* tile_tab, int max_tiles,
@@ -110,7 +111,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
   }
-  // splits are cut at multiples of `cut` k (64 or 128), where the other kernels of the same form cut them: the last chunk of a split may be half a chunk
+  // splits are cut at multiples of `cut` k (64 or 128), where the other kernels of the same form cut them
   if (warp == 2 && lane <= splits) split_c0[lane] = (int)((unsigned)(K / cut * lane) / (unsigned)splits) * (cut / GR_HALF);
   if (warp == 1) {
     tmem_alloc(tmem_slot, ncols);
@@ -168,10 +169,10 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
         const int s = gc % GR_RAW_STAGES;
         if (lane == 0) {
           if (gc >= GR_RAW_STAGES) ok = mbar_wait(&raw_empty[s], ((gc / GR_RAW_STAGES) - 1) & 1, abort_flag, status, 210, 500);
-          if (ok) mbar_arrive_expect_tx(&raw_full[s], 2 * c + 2 > halves ? RAW_STAGE / 2 : RAW_STAGE);
+          if (ok) mbar_arrive_expect_tx(&raw_full[s], HALVES && 2 * c + 2 > halves ? RAW_STAGE / 2 : RAW_STAGE);
         }
         ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-        if (ok && lane < min(8, 4 * (halves - 2 * c))) bulk_g2s(raw_base + s * RAW_STAGE + lane * ROW_BYTES, src + (size_t)c * 8 * nt_total * TILE_WORDS, ROW_BYTES, &raw_full[s]);
+        if (ok && lane < (HALVES ? min(8, 4 * (halves - 2 * c)) : 8)) bulk_g2s(raw_base + s * RAW_STAGE + lane * ROW_BYTES, src + (size_t)c * 8 * nt_total * TILE_WORDS, ROW_BYTES, &raw_full[s]);
       }
     }
     if (lane == 0) n_sent[0] = ok ? gc : gc - 1;       // (the chunk whose wait gave up was counted)
@@ -184,7 +185,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
         const int c0 = split_c0[at.split], halves = split_c0[at.split + 1] - c0, n = (halves + 1) >> 1;
         for (int c = 0; c < n; ++c, ++gc) {
           const int s = gc % GR_OP_STAGES, x = c0 * GR_HALF + c * GR_KCH;
-          const bool half = 2 * c + 2 > halves;
+          const bool half = HALVES && 2 * c + 2 > halves;
           if (gc >= GR_OP_STAGES && !mbar_wait(&b_empty[s], ((gc / GR_OP_STAGES) - 1) & 1, abort_flag, status, 211, 250)) { ok = false; break; }
           mbar_arrive_expect_tx(&b_full[s], (uint32_t)(half ? b_half : b_stage));
           tma_load_2d(b_base + s * b_stage, &tmap_x, x, it.row0, &b_full[s]);
@@ -224,7 +225,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
           const uint32_t a_at = a_tmem0 + sa * GR_A_COLS;
 #pragma unroll
           for (int k = 0; k < GR_KCH / 16; ++k)
-            if (k < GR_HALF / 16 || 2 * c + 2 <= halves) tc_mma_f16_ts(acc, a_at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
+            if (!HALVES || k < GR_HALF / 16 || 2 * c + 2 <= halves) tc_mma_f16_ts(acc, a_at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
           tc_commit(&a_empty[sa]);
           tc_commit(&b_empty[s]);
         }
@@ -327,12 +328,12 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
 
 int make_tmap_f16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
-template <int TWICE, int CB, int NG>
+template <int TWICE, int CB, int NG, bool HALVES>
 static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t expert_words, float* part, int rows, int K, int N, int splits, int cut, int brows,
                           const int* tile_tab, int max_tiles, int* status, cudaStream_t st) {
   int smem = gr_smem_bytes(brows, TWICE) + 1024;
   if (NG <= 3 && smem < 80 * 1024) smem = 80 * 1024;   // at most two CTAs per SM: each allocates 256 TMEM columns
-  auto kern = exl3_gemm_grouped_kernel<TWICE, CB, NG>;
+  auto kern = exl3_gemm_grouped_kernel<TWICE, CB, NG, HALVES>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
@@ -359,8 +360,10 @@ int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t
   int e = make_tmap_f16_2d(&tm, xs, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
   if (e != 0) return e;
   const uint32_t* tr = (const uint32_t*)trellis;
-#define RX_GR(T, CBV) (brows > 32 ? launch_grouped<T, CBV, 4>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st) \
-                                  : launch_grouped<T, CBV, 3>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st))
+  const bool halves = cut == GR_HALF && (K / GR_KCH) % splits != 0;
+#define RX_GR_H(T, CBV, H) (brows > 32 ? launch_grouped<T, CBV, 4, H>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st) \
+                                       : launch_grouped<T, CBV, 3, H>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st))
+#define RX_GR(T, CBV) (halves ? RX_GR_H(T, CBV, true) : RX_GR_H(T, CBV, false))
   switch (codebook) {
     case CB_3INST: return twice == 6 ? RX_GR(6, CB_3INST) : RX_GR(8, CB_3INST);
     case CB_MCG: return twice == 6 ? RX_GR(6, CB_MCG) : RX_GR(8, CB_MCG);
@@ -368,6 +371,7 @@ int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t
     default: return (int)cudaErrorInvalidValue;
   }
 #undef RX_GR
+#undef RX_GR_H
 }
 
 }  // namespace rx
