@@ -246,7 +246,7 @@ inline int& pdl_enabled() { static int on = 1; return on; }
 // Grids of more than PDL_MAX_CTAS CTAs (two per SM) are launched plainly: their CTAs, waiting, hold the slots of a predecessor with several waves or
 // a long tail, which costs more than the launch latency that is saved.  Measured with the limit at 296 / without one: MoE prompt slice of 2100 rows
 // 3.41 / 3.90 ms (the gather's 16,800 CTAs beside the one-CTA plan), verify window of 80 rows 2.20 / 2.27 ms, step of 64 rows 2.14 / 2.18 ms; limits
-// between 600 and 20,000 only helped the first.
+// between 600 and 20,000 only helped the first.  A vocabulary's head (1187 strips), whose weights then wait with it, loses 1.4 of 234 us.
 constexpr long long PDL_MAX_CTAS = 296;
 
 template <typename... P, typename... A>

@@ -570,7 +570,8 @@ __global__ void __launch_bounds__(256, 2) gdn_scan_kernel(const float* __restric
 // share what is loaded; k, q and the decays are laid out by thread, so that its 16 keys are four vectors.  A token's critical path is
 // a 16-key dot product, three shuffles and the rank-one write; the output sums of four tokens go over the lanes together, off that path.  What a
 // token needs besides (1 / |q|, 1 / |k|, decay, write strength) is computed for TC tokens at a time by the CTA from the inputs that cp.async
-// brought into two buffers (norm sums per token and warp: 40 shuffles, 0.96 us per token, 1105 us).  Every rounding and every order of a sum
+// brought into two buffers (norm sums per token and warp: 40 shuffles, 0.96 us per token).  With convolution and norm, 1024
+// tokens of one sequence, 48 heads, take 462 us (1090 with one warp per 16 columns; 422 with dot products in eighths of the keys, which are other sums).  Every rounding and every order of a sum
 // is gdn_scan_kernel's, so states and outputs are the same bits; the per-head gated norm, which needs all 128 outputs, runs afterwards in
 // gdn_norm_kernel.  The dependents are released at the end (see ssm_scan_split_kernel).  grid (segments, Hv, GDN_JS), 128 threads.
 constexpr int GDN_JS = 4, GDN_PAD = GDN_D + 32;                       // 16 keys every 20 floats: eight lanes' vectors in different banks
