@@ -148,11 +148,32 @@ def test_commit_equals_row_form(kind, kept):
     assert not torch.equal(pool, s0) and torch.equal(pool, pool1) and torch.equal(conv, conv1)
 
 
-@pytest.mark.parametrize("lens", [[1, 2, 3, 11, 8, 60, 1, 1], [1] * 70, [5] * 16, [2, 1, 4, 3] * 8, [64], [63, 1]])
+def test_conv_walking_rows_equals_one_row_per_thread():
+    """The walking form of the convolution (rows in eighths, taken from 148 blocks on) against the one-row form, which an odd row stride selects:
+    bit for bit, over segments that begin inside an eighth, and with the last eighth not full."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import kernels as K
+    Hk, Hv, D = 16, 48, 128
+    lens = [1, 2, 3, 11, 8, 60, 1, 1]
+    M, C = sum(lens), (2 * Hk + Hv) * D
+    width = (2 * Hk + 2 * Hv) * D + 2 * Hv
+    got = []
+    for pad in (0, 1):
+        r, proj, seq, pos, st, ln, conv0 = _inputs(width, C, M, width + pad, lens, 11)
+        args = (r(C, 4).bfloat16(), r(C).bfloat16(), r(Hv), -r(Hv).abs(), (1 + 0.1 * r(D)).bfloat16())
+        xbc, out = torch.empty(M * C, device="cuda"), torch.zeros(M, Hv * D, dtype=torch.bfloat16, device="cuda")
+        K.gdn_mixer(proj, M, Hk, Hv, D, seq, pos, st, ln, len(lens), *args, 1e-6, conv0, r(len(lens), Hv, D, D), xbc, out,
+                    y32=torch.empty(M * Hv * D, device="cuda"))
+        got.append((xbc, out, conv0))
+    for a, b in zip(*got):
+        assert torch.isfinite(a.float()).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("lens", [[1] * 70, [5] * 16, [2, 1, 4, 3] * 8, [64], [63, 1]])
 @pytest.mark.parametrize("record", [False, True])
-def test_conv_walking_rows_equals_one_row_per_thread(lens, record):
-    """The walking form of the convolution (rows in eighths, taken from 148 blocks on by prompt slices and recorded windows) against the one-row form,
-    which an odd row stride selects: bit for bit, over segments that begin inside an eighth, and with the last eighth not full."""
+def test_conv_walking_rows_over_short_segments(lens, record):
+    """The same over segments shorter than the convolution, in prompt slices and recorded windows, with sequences that go on from position 1."""
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
     from rexl3_b200.ops import kernels as K
