@@ -508,11 +508,15 @@ class DenseGPU:
                 r = rows if name != "lm_head" else min(rows, 256)
                 part_elems = max(part_elems, s * r * n)
         from ..utils import canary
-        g = lambda name, shape, dt: canary.guarded(f"{type(self).__name__}.{name}", shape, dt, dev)  # noqa: E731  (guard bands with REXL3_CANARY=1)
+        g = lambda name, shape, dt, zero=False: canary.guarded(f"{type(self).__name__}.{name}", shape, dt, dev, zero)  # noqa: E731  (guard bands with REXL3_CANARY=1)
         self.part = g("part", part_elems, torch.float32)
         # split projections (per-linear input rotations) run one GEMM per part into this second buffer before the partials are placed
         split = any(isinstance(v, SplitWeight) for L in self.layers for v in L.values())
         self._part_split = torch.empty(part_elems, dtype=torch.float32, device=dev) if split else None
+        # prompt slices of many rows: the decoded fp16 tiles of the largest matrix that goes that way
+        wide = [w for L in self.layers for n, w in L.items() if n in ("qkv", "o", "gate_up", "down") and self.splits.get(("prefill", n), 1) == 1 and
+                (K.wide_takes(w, R) or K.wide_takes(w, R, n == "gate_up"))]
+        self.wide = g("wide", max(K.wide_bytes(w.K, w.N) for w in wide), torch.uint8, zero=True) if wide else None
         kmax = max(k for k, _ in shapes.values())
         self.xr = g("xr", R * kmax, torch.float16)
         self.xr2 = g("xr2", R * cfg.ffn_padded, torch.float16)
@@ -595,7 +599,7 @@ class DenseGPU:
                 dst[:, :, off:off + p.N].copy_(self._part_split[:s * rows * p.N].view(s, rows, p.N))
                 off += p.N
             return s
-        self.K.exl3_gemm(xr, w, self.part, s, self.status)
+        self.K.exl3_gemm(xr, w, self.part, s, self.status, work=self.wide if cls == "prefill" else None)
         return s
 
     def _mixer(self, li, L, M, cls, xr_d, xr_a, q, positions, slots, row_seq, ctx_len, block_table, prefill, max_ctx, scale):
@@ -636,8 +640,12 @@ class DenseGPU:
         """Everything between the o_proj GEMM (its partials are in self.part, `s_o` splits) and the next layer's rotated input."""
         cfg, K = self.cfg, self.K
         K.finish_add_norm_rot(self.part, s_o, M, L["o"], h, L["ffn_norm"], cfg.eps, L["gate_up"].suh, xr_d)
-        s = self._linear(xr_d, L["gate_up"], M, cls, "gate_up")
-        K.finish_swiglu_rot(self.part, s, M, L["gate_up"], L["down"].suh, xr_f)
+        work = self.wide if cls == "prefill" and self.splits[(cls, "gate_up")] == 1 and K.wide_takes(L["gate_up"], M, True) else None
+        if work is not None and work.numel() >= K.wide_bytes(L["gate_up"].K, L["gate_up"].N):
+            K.exl3_gemm_swiglu_rot(xr_d, L["gate_up"], L["down"].suh, xr_f, work, self.status)
+        else:
+            s = self._linear(xr_d, L["gate_up"], M, cls, "gate_up")
+            K.finish_swiglu_rot(self.part, s, M, L["gate_up"], L["down"].suh, xr_f)
         s = self._linear(xr_f, L["down"], M, cls, "down")
         ov = self.interventions.get(li) if self.interventions else None
         if ov is None:

@@ -80,13 +80,40 @@ def tile_rows(rows: int) -> int:
     return _lib.load().rx_exl3_tile_rows(rows)
 
 
-def exl3_gemm(xr: torch.Tensor, w: Exl3Weight, part: torch.Tensor, splits: int, status: torch.Tensor, force_generic: bool = False) -> None:
-    """part[s, row, n] = partial sums of xr @ W_q over split s.  xr: fp16 [rows, K] contiguous; part: fp32 >= splits*rows*N."""
+def wide_takes(w, rows: int, swiglu: bool = False) -> bool:
+    """Whether `rows` rows through `w` in one split (and, with `swiglu`, what `finish_swiglu_rot` does) are faster by the kernel that decodes the matrix
+    once into a workspace.  The bits are the same."""
+    return isinstance(w, Exl3Weight) and w.twice == 8 and bool(_lib.load().rx_exl3_wide_takes(rows, w.K, w.N, int(swiglu)))
+
+
+def wide_bytes(K: int, N: int) -> int:
+    """Bytes of workspace that kernel needs (zeroed when allocated; calls that may overlap need one each)."""
+    return _lib.load().rx_exl3_wide_bytes(K, N)
+
+
+def exl3_gemm_swiglu_rot(xr: torch.Tensor, w: Exl3Weight, suh_down: torch.Tensor, act: torch.Tensor, work: torch.Tensor, status: torch.Tensor) -> None:
+    """`exl3_gemm` and `finish_swiglu_rot` in one kernel for the rows of a prompt slice (where `wide_takes`): act fp16 [rows, N / 2]."""
+    rows, K = xr.shape
+    assert xr.dtype == torch.float16 and xr.is_contiguous() and K == w.K and w.twice == 8
+    assert act.dtype == torch.float16 and act.is_contiguous() and act.numel() >= rows * w.N // 2
+    _lib.check(_lib.load().rx_exl3_gemm_wide_swiglu(xr.data_ptr(), rows, K, w.trellis.data_ptr(), w.N // 2, CB_ID[w.codebook], w.svh.data_ptr(), _lib.ptr(w.bias),
+                                                    suh_down.data_ptr(), act.data_ptr(), work.data_ptr(), work.numel(), status.data_ptr(), _lib.stream_ptr()),
+               "rx_exl3_gemm_wide_swiglu")
+    _lib.count()
+
+
+def exl3_gemm(xr: torch.Tensor, w: Exl3Weight, part: torch.Tensor, splits: int, status: torch.Tensor, force_generic: bool = False,
+              work: "torch.Tensor | None" = None) -> None:
+    """part[s, row, n] = partial sums of xr @ W_q over split s.  xr: fp16 [rows, K] contiguous; part: fp32 >= splits*rows*N.  `work` (uint8, see
+    `wide_bytes`): prompt slices may go through the kernel that decodes the matrix once; the bits are the same."""
     rows, K = xr.shape
     assert xr.dtype == torch.float16 and xr.is_contiguous() and K == w.K
     assert part.dtype == torch.float32 and part.numel() >= splits * rows * w.N
     L = _lib.load()
-    if w.twice == 8 and not force_generic:
+    if work is not None and splits == 1 and not force_generic and wide_takes(w, rows) and work.numel() >= wide_bytes(K, w.N):
+        _lib.check(L.rx_exl3_gemm_wide(xr.data_ptr(), rows, K, w.trellis.data_ptr(), w.N, CB_ID[w.codebook], part.data_ptr(), work.data_ptr(), work.numel(),
+                                       status.data_ptr(), _lib.stream_ptr()), "rx_exl3_gemm_wide")
+    elif w.twice == 8 and not force_generic:
         # 4.0 bpw: decoded weights go straight to tensor memory
         _lib.check(L.rx_exl3_gemm_b4(xr.data_ptr(), rows, K, w.trellis.data_ptr(), w.N, CB_ID[w.codebook], part.data_ptr(), splits,
                                      status.data_ptr(), _lib.stream_ptr()), "rx_exl3_gemm_b4")
