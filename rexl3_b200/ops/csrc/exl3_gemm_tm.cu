@@ -95,7 +95,8 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();   // the weights were not written by the previous kernel, everything else may have been
+  // The weights were not written by the previous kernel, everything else may have been: the decode warps begin while it still runs, up to the depth of the A ring.
+  if (warp < TM_ROLE_WARPS) pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t a_tmem0 = tmem_base + acc_cols;
 
@@ -213,6 +214,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       if (lane == 0) mbar_arrive(&a_full[os]);
     }
     if (dw < 4) {
+      pdl_wait();
       const bool done = mbar_wait(acc_full, 0, abort_flag, status, 140, 100);
       tc_fence_after();
       if (done && *abort_flag == 0) {
