@@ -149,7 +149,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer: one page of K and of V per step
-    if (lane == 0) {
+    if (elect_one()) {
       int n_k = 0, n_v = 0;                               // pages issued
       for (int j = 0; j < npages; ++j) {
         const int st = j % TC_STAGES;
@@ -170,7 +170,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_cons
     }
   } else if (warp == 1 || warp == TC_ISSUER_1) {
     // ---------------------------------------------------------------- MMA issuer of one tile
-    if (lane == 0) {
+    if (elect_one()) {
       const int t = warp == 1 ? 0 : 1, mine = nst[t];
       const uint32_t idesc_qk = umma_idesc_f16(TC_ROWS, TC_PAGE, 1, 1);                 // bf16 x bf16, both K-major
       const uint32_t idesc_pv = umma_idesc_f16(TC_ROWS, TC_HD, 1, 1) | (1u << 16);      // B (V) is MN-major

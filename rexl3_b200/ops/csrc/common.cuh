@@ -153,6 +153,15 @@ __device__ __forceinline__ void prefetch_tmap(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
+// One lane of a converged warp.  A role that issues tensor-core or copy instructions is entered by `if (elect_one())`: the compiler then knows that one lane
+// runs and keeps descriptors and addresses in uniform registers.  Behind `if (lane == 0)` it moves every operand there before each instruction: 48 cycles
+// from one MMA to the next instead of 12, with an idle scheduler, and the issuer was what bounded the decode GEMMs (1400 of 1900 cycles a chunk of 128 k).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- tcgen05 / TMEM
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");

@@ -119,7 +119,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
 
   if (warp == 0) {
     // ------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       // Step i issues the compressed weights of chunk i and the activation tile of chunk i - AHEAD: the weight
       // stream (HBM) runs ahead of the activation tiles (L2 hits).  Neither wait can block the other ring for good:
       // decode warps release a raw stage before they wait for an operand stage.
@@ -149,7 +149,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_f16(STRIP, brows, 0, 0);
       bool ok = true;
       for (int c = 0; c < nchunks && ok; ++c) {

@@ -178,7 +178,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     if (lane == 0) n_sent[0] = ok ? gc : gc - 1;       // (the chunk whose wait gave up was counted)
   } else if (warp == 2) {
     // ---- activation producer: two [brows x 64] swizzled boxes per chunk
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int gc = 0;
       for (; ok && tile_of(at, it); step(at, stride)) {
@@ -205,7 +205,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
       last = __reduce_max_sync(0xffffffffu, last);
       if (lane == 0) *tile_end = last + 1;
     }
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(b_base));
       const uint32_t half_units = (uint32_t)b_half >> 4, stage_units = (uint32_t)b_stage >> 4;
       bool ok = true;

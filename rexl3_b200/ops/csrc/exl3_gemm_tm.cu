@@ -102,7 +102,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
 
   if (warp == 0) {
     // ---- weight producer: ONE 2-D tiled copy per chunk (8 k-tile rows x 1 KB of this strip)
-    if (lane == 0) {
+    if (elect_one()) {
       int y = (c_begin + TM_RAW_STAGES) * 8;
       const int x = strip * 256;
       for (int c = TM_RAW_STAGES; c < nchunks; ++c, y += 8) {   // the first ring's worth was issued in the prologue
@@ -114,7 +114,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     }
   } else if (warp == 2) {
     // ---- activation producer: two [brows x 64] swizzled boxes per chunk
-    if (lane == 0) {
+    if (elect_one()) {
       int x = c_begin * TM_KCH;
       const int y = row_tile * brows;
       int waited_src = -1;
@@ -137,7 +137,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     }
   } else if (warp == 1) {
     // ---- MMA issuer: A from tensor memory, B from shared memory
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_f16(TM_STRIP, brows, 0, 0);
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(b_base));
       const uint32_t half_units = (uint32_t)b_half >> 4, stage_units = (uint32_t)b_stage >> 4;

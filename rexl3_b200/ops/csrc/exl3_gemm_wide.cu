@@ -291,7 +291,7 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
 
   if (warp == 0) {
     // ---- copies: this CTA's 128 rows of xr and its half of the tile's columns
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true;
       for (int i = 0; i < plan.n && ok; ++i) {
@@ -321,7 +321,7 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     }
   } else if (warp == 1) {
     // ---- MMA issuer of the pair
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       int it = 0;
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(smem));
       bool ok = true;

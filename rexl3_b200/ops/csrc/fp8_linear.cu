@@ -96,7 +96,7 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const int w_row0 = strip * F8_STRIP;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int AHEAD = AHEAD_B;
       bool ok = true;
       bool waited = false;
@@ -119,7 +119,7 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_f16(F8_STRIP, brows, 1, 1);
       bool ok = true;
       for (int c = 0; c < nchunks && ok; ++c) {

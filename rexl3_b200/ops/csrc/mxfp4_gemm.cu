@@ -120,7 +120,7 @@ mxfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr int AHEAD = 4;
       bool ok = true;
       for (int i = 0; i < nchunks + AHEAD && ok; ++i) {
@@ -141,7 +141,7 @@ mxfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc_f16(MX_STRIP, brows, 0, 0);
       bool ok = true;
       for (int c = 0; c < nchunks && ok; ++c) {
