@@ -513,6 +513,7 @@ class DenseGPU:
         # split projections (per-linear input rotations) run one GEMM per part into this second buffer before the partials are placed
         split = any(isinstance(v, SplitWeight) for L in self.layers for v in L.values())
         self._part_split = torch.empty(part_elems, dtype=torch.float32, device=dev) if split else None
+        self.step_flags = torch.zeros(K.step_flags(), dtype=torch.int32, device=dev)
         # prompt slices of many rows: the decoded fp16 tiles of the largest matrix that goes that way
         wide = [w for L in self.layers for n, w in L.items() if n in ("qkv", "o", "gate_up", "down") and self.splits.get(("prefill", n), 1) == 1 and
                 (K.wide_takes(w, R) or K.wide_takes(w, R, n == "gate_up"))]
@@ -599,7 +600,7 @@ class DenseGPU:
                 dst[:, :, off:off + p.N].copy_(self._part_split[:s * rows * p.N].view(s, rows, p.N))
                 off += p.N
             return s
-        self.K.exl3_gemm(xr, w, self.part, s, self.status, work=self.wide if cls == "prefill" else None)
+        self.K.exl3_gemm(xr, w, self.part, s, self.status, work=self.wide if cls == "prefill" else None, flags=self.step_flags if cls == "decode" else None)
         return s
 
     def _mixer(self, li, L, M, cls, xr_d, xr_a, q, positions, slots, row_seq, ctx_len, block_table, prefill, max_ctx, scale):

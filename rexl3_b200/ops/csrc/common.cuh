@@ -113,6 +113,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// bounded wait for a counter that other CTAs raise
+__device__ __forceinline__ bool wait_count(const int* count, int want, volatile int* abort_flag, int* status, int site) {
+  if (ld_acquire_gpu(count) < want) {
+    const uint64_t t0 = globaltimer_ns(), limit = wait_limit_ns(status);
+    while (ld_acquire_gpu(count) < want) {
+      const bool stop = host_abort(status);
+      if (stop || globaltimer_ns() - t0 > limit) {
+        set_status(status, stop ? ST_ABORTED : ST_TIMEOUT, site, want);
+        *abort_flag = 1;
+      }
+      if (*abort_flag != 0) return false;
+      __nanosleep(50);
+    }
+  }
+  return true;
+}
+
 // Waits (bounded, and not cut short by an abort) until the copies of the last of `issued` phases of a ring of `stages` barriers have landed: a consumer whose
 // wait gave up does not, and a copy must not arrive in memory that its CTA has left.
 __device__ __forceinline__ void ring_landed(uint64_t* bars, int stages, int issued) {

@@ -113,12 +113,6 @@ __device__ __forceinline__ void stg256(void* p, const uint32_t* r) {
                "r"(r[7])
                : "memory");
 }
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 // Half of a 128-point transform that one thread holds: the additions of fwht128_warp but the last, in its order
 __device__ __forceinline__ void fwht64_thread(uint32_t (&r)[64]) {
 #pragma unroll
@@ -221,23 +215,6 @@ struct WidePlan {
   }
 };
 
-// bounded wait for a counter that other CTAs raise
-__device__ __forceinline__ bool wide_wait_count(const int* count, int want, volatile int* abort_flag, int* status, int site) {
-  if (ld_acquire_gpu(count) < want) {
-    const uint64_t t0 = globaltimer_ns(), limit = wait_limit_ns(status);
-    while (ld_acquire_gpu(count) < want) {
-      const bool stop = host_abort(status);
-      if (stop || globaltimer_ns() - t0 > limit) {
-        set_status(status, stop ? ST_ABORTED : ST_TIMEOUT, site, want);
-        *abort_flag = 1;
-      }
-      if (*abort_flag != 0) return false;
-      __nanosleep(50);
-    }
-  }
-  return true;
-}
-
 template <int CB, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WD_THREADS, 1)
 exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w64,
@@ -305,7 +282,7 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
           const int s = it % WD_STAGES;
           if (kb == item.kb0 || kb % (WD_SEG * WD_PIECE_K / 64) == 0) {
             const int seg = kb / (WD_SEG * WD_PIECE_K / 64);
-            ok = wide_wait_count(ready + w.ct * segs + seg, 8 * min(WD_SEG, kpieces - seg * WD_SEG), abort_flag, a.status, 160);
+            ok = wait_count(ready + w.ct * segs + seg, 8 * min(WD_SEG, kpieces - seg * WD_SEG), abort_flag, a.status, 160);
             if (!ok) break;
             asm volatile("fence.proxy.async;" ::: "memory");   // written by ordinary stores, read by the copy engine
           }
@@ -357,7 +334,7 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     // the accumulator of item n, before its products: handed on by the pair before
     auto take = [&](int n) {
       const int from = plan.slot - 1;
-      if (!__all_sync(0xffffffffu, wide_wait_count(handed + from * 8 + rank * 4 + q, 1, abort_flag, a.status, 165))) return;
+      if (!__all_sync(0xffffffffu, wait_count(handed + from * 8 + rank * 4 + q, 1, abort_flag, a.status, 165))) return;
       const float* src = a.hand + from * WD_HAND + mine;
       for (int c = 0; c < 256; c += 16) {
         uint32_t r[16];

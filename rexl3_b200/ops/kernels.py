@@ -86,6 +86,11 @@ def wide_takes(w, rows: int, swiglu: bool = False) -> bool:
     return isinstance(w, Exl3Weight) and w.twice == 8 and bool(_lib.load().rx_exl3_wide_takes(rows, w.K, w.N, int(swiglu)))
 
 
+def step_flags() -> int:
+    """Words of the flags buffer that `exl3_gemm` takes for decode windows (int32, zeroed when allocated; calls that may overlap need one each)."""
+    return _lib.load().rx_exl3_step_flags()
+
+
 def wide_bytes(K: int, N: int) -> int:
     """Bytes of workspace that kernel needs (zeroed when allocated; calls that may overlap need one each)."""
     return _lib.load().rx_exl3_wide_bytes(K, N)
@@ -103,7 +108,7 @@ def exl3_gemm_swiglu_rot(xr: torch.Tensor, w: Exl3Weight, suh_down: torch.Tensor
 
 
 def exl3_gemm(xr: torch.Tensor, w: Exl3Weight, part: torch.Tensor, splits: int, status: torch.Tensor, force_generic: bool = False,
-              work: "torch.Tensor | None" = None) -> None:
+              work: "torch.Tensor | None" = None, flags: "torch.Tensor | None" = None) -> None:
     """part[s, row, n] = partial sums of xr @ W_q over split s.  xr: fp16 [rows, K] contiguous; part: fp32 >= splits*rows*N.  `work` (uint8, see
     `wide_bytes`): prompt slices may go through the kernel that decodes the matrix once; the bits are the same."""
     rows, K = xr.shape
@@ -113,6 +118,9 @@ def exl3_gemm(xr: torch.Tensor, w: Exl3Weight, part: torch.Tensor, splits: int, 
     if work is not None and splits == 1 and not force_generic and wide_takes(w, rows) and work.numel() >= wide_bytes(K, w.N):
         _lib.check(L.rx_exl3_gemm_wide(xr.data_ptr(), rows, K, w.trellis.data_ptr(), w.N, CB_ID[w.codebook], part.data_ptr(), work.data_ptr(), work.numel(),
                                        status.data_ptr(), _lib.stream_ptr()), "rx_exl3_gemm_wide")
+    elif flags is not None and w.twice == 8 and not force_generic and L.rx_exl3_step_takes(rows, K, w.N, splits):
+        _lib.check(L.rx_exl3_gemm_step(xr.data_ptr(), rows, K, w.trellis.data_ptr(), w.N, CB_ID[w.codebook], part.data_ptr(), splits, flags.data_ptr(),
+                                       status.data_ptr(), _lib.stream_ptr()), "rx_exl3_gemm_step")
     elif w.twice == 8 and not force_generic:
         # 4.0 bpw: decoded weights go straight to tensor memory
         _lib.check(L.rx_exl3_gemm_b4(xr.data_ptr(), rows, K, w.trellis.data_ptr(), w.N, CB_ID[w.codebook], part.data_ptr(), splits,

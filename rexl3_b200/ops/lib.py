@@ -44,6 +44,9 @@ def _declare(lib):
         "rx_exl3_gemm": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_int, c_void, c_int, c_void, c_void]),
         "rx_exl3_gemm_b4": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_void, c_int, c_void, c_void]),
         "rx_exl3_gemm_b4_tp": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_void, c_int, c_void, c_void, c_void]),
+        "rx_exl3_step_flags": (c_int, []),
+        "rx_exl3_step_takes": (c_int, [c_int, c_int, c_int, c_int]),
+        "rx_exl3_gemm_step": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_void, c_int, c_void, c_void, c_void]),
         "rx_exl3_wide_takes": (c_int, [c_int, c_int, c_int, c_int]),
         "rx_exl3_wide_bytes": (c_ll, [c_int, c_int]),
         "rx_exl3_gemm_wide": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_void, c_void, c_ll, c_void, c_void]),
