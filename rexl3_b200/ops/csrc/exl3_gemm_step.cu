@@ -240,8 +240,8 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         mbar_arrive(&acc_empty[f & 1]);
       }
     };
-    // The accumulator of the last piece f, as the CTA before left it.  The group that has written out piece f - 2, whose place it takes, brings it in: a wait of
-    // another group could miss two phases of that buffer's barrier.
+    // The accumulator of the last piece f, as the CTA before left it.  The group that writes out piece f - 2, whose place it takes, brings it in: a wait of another
+    // group could miss two phases of that buffer's barrier.
     auto take_in = [&](const StepPiece& o, int f) {
       kernel_before();
       if (!__all_sync(0xffffffffu, wait_count(flag_out - 4, 1, abort_flag, a.status, 178))) return false;
@@ -268,14 +268,17 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       for (; ok && next_out < end; next_out += ST_NG) {
         ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[next_out % ST_OUT], (next_out / ST_OUT) & 1, abort_flag, a.status, 176));
         if (ok) write_out(piece(next_out), next_out);
-        if (ok && next_out == pieces - 3 && piece(pieces - 1).take) ok = take_in(piece(pieces - 1), pieces - 1);
       }
     };
     int gc0 = 0;                                  // chunks up to the end of piece f
     for (int gc = grp; ok && f < pieces; ++f) {
       const StepPiece p = piece(f);
       gc0 += p.n;
-      if (p.take && f < 2 && grp == f) ok = take_in(p, f);
+      // (not before: the CTA before may still be at it)
+      if (p.take && grp == (f < 2 ? f : (f - 2) % ST_NG)) {
+        write_before(f - 1);
+        if (ok) ok = take_in(p, f);
+      }
       for (; gc < gc0 && ok; gc += ST_NG) {
         const int rs = gc % ST_RAW, os = gc % ST_STAGES;
         ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[rs], (gc / ST_RAW) & 1, abort_flag, a.status, 179, 100));
