@@ -1087,6 +1087,79 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
   }
 }
 
+// The same for a few rows of many chunks, bound by the latency of each warp's walk along them: a CTA takes 128 outputs, a lane one of them, with
+// twice the chunks in flight, and there are four times the warps; the rotation follows in the CTA's first warp.  A sum meets the chunks in the same order.
+constexpr int MERGE_FEW_LOADS = 32;
+template <int HD>
+__global__ void __launch_bounds__(128) attn_merge_few_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const int* __restrict__ ctx_len,
+                                                             int n_q, int max_chunks, const __half* __restrict__ suh, __half* __restrict__ xr,
+                                                             uint16_t* __restrict__ out_bf16) {
+  pdl_launch();
+  __shared__ alignas(16) float vals[128];
+  const int row = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31, width = n_q * HD;
+  pdl_wait();
+  const int nch = (ctx_len[row] + DEC_CHUNK - 1) / DEC_CHUNK;
+  const int e = b * 128 + threadIdx.x, hq = e / HD, d = e % HD;
+  const size_t base = ((size_t)row * n_q + hq) * max_chunks;
+  float mm = -INFINITY;
+  for (int c0 = 0; c0 < nch; c0 += 128) {
+    float m[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = c0 + 32 * i + lane < nch ? part_ml[(base + c0 + 32 * i + lane) * 2] : -INFINITY;
+    mm = fmaxf(mm, fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])));
+  }
+  mm = warp_max(mm);
+  float acc = 0.f, lsum = 0.f;
+  for (int c0 = 0; c0 < nch; c0 += MERGE_FEW_LOADS) {
+    const int cnt = min(MERGE_FEW_LOADS, nch - c0);
+    float p[MERGE_FEW_LOADS];
+#pragma unroll
+    for (int j = 0; j < MERGE_FEW_LOADS; ++j)
+      if (j < cnt) p[j] = part_o[(base + c0 + j) * HD + d];
+    const float m_l = lane < cnt ? part_ml[(base + c0 + lane) * 2] : -INFINITY;
+    const float l_l = lane < cnt ? part_ml[(base + c0 + lane) * 2 + 1] : 0.f;
+    const float f_l = (m_l == -INFINITY) ? 0.f : exp2f(m_l - mm);
+#pragma unroll
+    for (int j = 0; j < MERGE_FEW_LOADS; ++j) {
+      if (j >= cnt) break;                           // (the same for the whole row)
+      const float f = __shfl_sync(0xffffffffu, f_l, j), ll = __shfl_sync(0xffffffffu, l_l, j);
+      acc += f * p[j];
+      lsum += f * ll;
+    }
+  }
+  const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
+  vals[threadIdx.x] = __bfloat162float(__float2bfloat16_rn(acc * inv));
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int e0 = b * 128 + lane * 4;
+  const float4 t = *reinterpret_cast<const float4*>(vals + lane * 4);
+  float v[4] = {t.x, t.y, t.z, t.w};
+  if (out_bf16 != nullptr) *reinterpret_cast<uint2*>(out_bf16 + (size_t)row * width + e0) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+  if (suh != nullptr) {
+    const uint2 su = *reinterpret_cast<const uint2*>(suh + e0);
+    const float2 s01 = __half22float2(*reinterpret_cast<const __half2*>(&su.x)), s23 = __half22float2(*reinterpret_cast<const __half2*>(&su.y));
+    v[0] *= s01.x; v[1] *= s01.y; v[2] *= s23.x; v[3] *= s23.y;
+    fwht128_warp(v);
+    const __half2 a = __floats2half2_rn(v[0], v[1]), c2 = __floats2half2_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(xr + (size_t)row * width + e0) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c2));
+  }
+}
+
+template <int HD>
+static void launch_merge(const float* part_o, const float* part_ml, const int* ctx_len, int rows, int n_q, int mc, const void* suh, void* xr, void* out_bf16,
+                         cudaStream_t st) {
+  const int blocks128 = n_q * HD / 128;
+  // Up to two CTAs per SM, which may also begin early: 6 rows of 40 heads in 126 chunks 9.8 -> 6.4 us alone, 21 -> 16 us behind 32K keys; 16 rows (640 CTAs) in 16
+  // chunks 4.8 and 5.7.  One row in 8 chunks is level, but more SMs hold a waiting CTA then, where the next product could begin: step 918 -> 933 us.
+  if ((long long)rows * blocks128 <= PDL_MAX_CTAS && mc > 32) {
+    rx::launch(attn_merge_few_kernel<HD>, dim3(rows, blocks128), dim3(128), 0, st, part_o, part_ml, ctx_len, n_q, mc, (const __half*)suh, (__half*)xr,
+               (uint16_t*)out_bf16);
+    return;
+  }
+  const int gy = (blocks128 + 3) / 4;              // a warp per 128 outputs
+  rx::launch(attn_merge_kernel<HD>, dim3(rows, gy), dim3(128), 0, st, part_o, part_ml, ctx_len, n_q, mc, (const __half*)suh, (__half*)xr, (uint16_t*)out_bf16);
+}
+
 // ------------------------------------------------------------------------------------------------ prefill (causal flash)
 // Queries: rows [q_start[s], q_start[s] + q_len[s]) of `q` belong to sequence s at positions pos0[s].. ; keys are the
 // sequence's cached tokens [0, pos0 + local row] (the chunk's own K/V are already in the cache).  out: bf16 [rows][n_q*HD].
@@ -1361,9 +1434,7 @@ static int launch_decode(const CUtensorMap* tk, const CUtensorMap* tv, const voi
   else e = RX_DEC_T(2);
 #undef RX_DEC_T
   if (e != 0) return e;
-  const int blocks128 = n_q * HD / 128;
-  const int gy = (blocks128 + 3) / 4;              // a warp per 128 outputs
-  rx::launch(attn_merge_kernel<HD>, dim3(dim3(rows, gy)), dim3(128), 0, st, part_o, part_ml, ctx_len, n_q, mc, (const __half*)suh, (__half*)xr, (uint16_t*)out_bf16);
+  launch_merge<HD>(part_o, part_ml, ctx_len, rows, n_q, mc, suh, xr, out_bf16, st);
   return (int)cudaGetLastError();
 }
 
