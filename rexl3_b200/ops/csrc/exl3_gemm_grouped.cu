@@ -34,8 +34,14 @@ __host__ __device__ inline int gr_smem_bytes(int brows, int twice) { return GR_O
 // shift: where the column's first window starts in its word pair (column_shift).
 template <int TWICE>
 __device__ __forceinline__ uint32_t column_shift(int b2) { return TWICE == 8 ? (b2 ? 32u : 16u) : (b2 ? 31u : 19u); }
-template <int TWICE, int CB>
+template <int TWICE, int CB, bool ALIGN>
 __device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1], uint32_t shift, uint32_t* regs) {
+  uint32_t y[4] = {};
+  if constexpr (TWICE == 6 && ALIGN) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) y[i] = __funnelshift_l(w[i + 1], w[i], shift);
+    y[3] = w[3] << shift;
+  }
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     uint32_t s0, s1, s2, s3;
@@ -48,11 +54,18 @@ __device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1]
       // depend on b2 but for m = 3, and the funnel shift takes its amount modulo 32.
       static_assert(TWICE == 6, "widths of this kernel: 3.0 and 4.0 bpw");
       uint32_t X;
-      if (m < 3) X = __funnelshift_l(w[m + 1], w[m], shift + 24 * m);
-      else X = shift == 31u ? w[3] << 7 : __funnelshift_l(w[3], w[2], 27);
-      s0 = X >> 16;
-      const uint32_t x1 = X >> 13, x2 = X >> 10, x3 = X >> 7;
-      s1 = x1 & 0xFFFFu;
+      if constexpr (ALIGN) {
+        // the words once brought to the first window's start: no shift by a register behind it (2 % of a decode window; prompt tiles lose 1 %)
+        X = m == 0 ? y[0] : m == 3 ? __funnelshift_l(y[3], y[2], 8) : __funnelshift_l(y[m], y[m - 1], m == 1 ? 24 : 16);
+        s0 = __byte_perm(X, 0, 0x4432);
+        s1 = __byte_perm(X << 3, 0, 0x4432);
+      } else {
+        if (m < 3) X = __funnelshift_l(w[m + 1], w[m], shift + 24 * m);
+        else X = shift == 31u ? w[3] << 7 : __funnelshift_l(w[3], w[2], 27);
+        s0 = X >> 16;
+        s1 = (X >> 13) & 0xFFFFu;
+      }
+      const uint32_t x2 = X >> 10, x3 = X >> 7;
       s2 = CB != CB_MUL1 ? low16_mul(x2) : x2 & 0xFFFFu;        // (the multiply pipe has room for two of the masks)
       s3 = CB != CB_MUL1 ? low16_mul(x3) : x3 & 0xFFFFu;
     }
@@ -69,7 +82,9 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
                          int* status) {
   pdl_launch();
   constexpr int SA = gr_a_stages(NG), EW = TWICE / 2;            // EW: words of an eighth of a tile
-  constexpr int QT = NG <= 3 ? 1 : 4;                            // quarters of a chunk unrolled: short items keep to the instruction cache, long ones gain 5 %
+  // Quarters of a chunk unrolled: short items keep to the instruction cache, long ones gain 5 % (86 experts 2048 -> 1536 in 4 splits 96.7 us with one, 93.2 with
+  // two or four; 79 experts 768 -> 2048 in 3 splits 52.0, 52.0, 54.8).
+  constexpr int QT = NG <= 3 ? 2 : 4;
   constexpr int TILE_WORDS = 4 * TWICE, ROW_BYTES = 8 * TILE_WORDS * 4, RAW_STAGE = 8 * ROW_BYTES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -294,8 +309,8 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
           for (int kk = 0; kk < 2; ++kk) w[kk][0] = __shfl_sync(0xffffffffu, w[kk][EW], prev_lane);
           if (qt == 3) release_read_stage(&raw_empty[rs], lane);   // the stage's last read has landed in registers; proxy fence before the refill
           uint32_t regs[16];
-          decode_column<TWICE, CB>(w[0], shift, regs);
-          decode_column<TWICE, CB>(w[1], shift, regs + 8);
+          decode_column<TWICE, CB, NG <= 3>(w[0], shift, regs);
+          decode_column<TWICE, CB, NG <= 3>(w[1], shift, regs + 8);
           if (qt == 0) {
             if (gc >= SA) ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[os], ((gc / SA) - 1) & 1, abort_flag, status, 231));
             if (!ok) break;
