@@ -114,7 +114,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();   // the weights were not written by the previous kernel, everything else may have been
+  // The weights were not written by the previous kernel, everything else may have been: the first weights come and are decoded while it still runs.
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -138,6 +138,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
             bulk_g2s(smem + L.raw_off + s * RAW_STAGE + r * ROW_BYTES, src, ROW_BYTES, &raw_full[s]);
           }
         }
+        if (i == AHEAD) pdl_wait();
         if (i >= AHEAD) {
           const int c = i - AHEAD, s = c % OP_STAGES;
           if (c >= OP_STAGES) ok = mbar_wait(&op_empty[s], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 11);
@@ -262,6 +263,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     }
     // ------------------------------------------------ epilogue (warps 2..5 cover TMEM lane quarters 2,3,0,1)
     if (dw < 4) {
+      pdl_wait();
       const bool done = mbar_wait(acc_full, 0, abort_flag, status, 40);
       tc_fence_after();
       if (done && *abort_flag == 0) {
