@@ -302,6 +302,21 @@ inline cudaError_t launch_alone(void (*kern)(P...), dim3 grid, dim3 block, size_
   return launch_pdl(false, kern, grid, block, smem, st, args...);
 }
 
+// ---------------------------------------------------------------- thread-block clusters
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int ld_cluster(const int* own, uint32_t rank) {     // the same shared-memory word of another CTA of the cluster
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(mapa_u32(smem_u32(own), rank)) : "memory");
+  return v;
+}
+
 // ---------------------------------------------------------------- small math helpers
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -204,15 +204,25 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const uint16_t* __restr
   if (lane < topk) out_w[(size_t)row * topk + lane] = out_w[(size_t)row * topk + lane] / picked_sum * scale;
 }
 
-// Single CTA.  ids: int32 [pairs].  Outputs: offs int32 [E + 1] (positions of expert e are offs[e] .. offs[e+1]; experts outside
+// One CTA or one cluster.  ids: int32 [pairs].  Outputs: offs int32 [E + 1] (positions of expert e are offs[e] .. offs[e+1]; experts outside
 // [e_lo, e_hi) get empty ranges), pos_of_pair int32 [pairs] (-1: not owned), pair_of_pos / expert_of_pos int32 [pairs],
 // tile_tab int32 [max_tiles][3], total int32 [1].
-// A stable counting sort: each of the 32 warps owns a run of pairs and counts it 32 pairs at a time (lanes that chose the same expert find
-// each other with one match), the counts are summed over the warps and the experts, and each warp places its run in a second pass.  Bound by
-// the latency of a few hundred dependent steps: two passes of pairs / 1024 steps, where a ballot per owned expert took experts / 32 times as many
-// (128 experts: 356 -> 43 us for 16,800 pairs, 14 -> 5 us for 128).  A CTA has a thread per expert and a warp per 32 pairs, up to 1024: with all 32 warps
+// A stable counting sort: each warp owns a run of pairs and counts it 32 pairs at a time (lanes that chose the same expert find each other with a ballot
+// per bit of its number), the counts are summed over the warps and the experts, and each warp places its run in a second pass.  A single CTA is bound by one
+// SM's stores, which are scattered by expert: 32 wavefronts each.  So from 2048 pairs on a cluster of eight CTAs shares the runs and reads each other's
+// counts through distributed shared memory (128 experts, with the launch: 16,800 pairs 49 -> 16 us, 4800 pairs 16.4 -> 12.3 us; 2048 pairs 12.3 us either
+// way, 1024 pairs 10.2 us in one CTA and 12.3 in eight).  A CTA has a thread per expert and a warp per 32 pairs, up to 1024: with all 32 warps
 // a small window paid for empty ones (8 pairs, 16 experts 5.2 us).  Dynamic shared memory: (warps) x E counters.
-constexpr int PLAN_WARPS = 32;
+constexpr int PLAN_WARPS = 32, PLAN_AHEAD = 8, PLAN_CLUSTER = 8, PLAN_CLUSTER_PAIRS = 2048;
+// The lanes that chose the same expert: a ballot per bit of its number (E <= 512: at most nine, independent of one another).
+__device__ __forceinline__ unsigned plan_same(int e, bool own, int E) {
+  unsigned same = __ballot_sync(0xffffffffu, own);
+  for (int b = 0; (1 << b) < E; ++b) {
+    const unsigned set = __ballot_sync(0xffffffffu, (e >> b) & 1);
+    same &= (e >> b) & 1 ? set : ~set;
+  }
+  return same;
+}
 template <int W>
 __device__ __forceinline__ int plan_scan(int v, int* tmp, int& all) {      // exclusive sum over the CTA's threads, in thread order
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -233,70 +243,130 @@ __device__ __forceinline__ int plan_scan(int v, int* tmp, int& all) {      // ex
   all = run;
   return before + s - v;
 }
-template <int W>                              // warps, 0: as many as the CTA has
-__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* ids, int pairs, int E, int e_lo, int e_hi, int tile_rows, int max_tiles,
-                                                        int* __restrict__ offs, int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos,
-                                                        int* __restrict__ expert_of_pos, int* __restrict__ tile_tab, int* __restrict__ total) {
+template <int W, int CL>                      // warps, 0: as many as the CTA has; CTAs (of one cluster)
+__device__ __forceinline__ void moe_plan(const int* ids, int pairs, int E, int e_lo, int e_hi, int tile_rows, int max_tiles,
+                                         int* __restrict__ offs, int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos,
+                                         int* __restrict__ expert_of_pos, int* __restrict__ tile_tab, int* __restrict__ total) {
   pdl_launch();
   pdl_wait();
   extern __shared__ int plan_cnt[];           // [warps][E]: counts, then the position of a warp's next pair of an expert
   __shared__ int tmp[PLAN_WARPS];
+  __shared__ int own_cnt[CL > 1 ? 512 : 1];   // this CTA's pairs of every expert, read by the cluster's other CTAs
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = W > 0 ? W : blockDim.x / 32, threads = 32 * warps;
+  const int rank = CL > 1 ? (int)blockIdx.x : 0;
   for (int i = t; i < warps * E; i += threads) plan_cnt[i] = 0;
   __syncthreads();
   int* mine = plan_cnt + warp * E;
-  const int run = (pairs + threads - 1) / threads * 32, p_begin = warp * run, p_end = min(pairs, p_begin + run);
-  for (int p0 = p_begin; p0 < p_end; p0 += 32) {
-    const int p = p0 + lane;
-    const int e = p < p_end ? ids[p] : -1;
-    const bool own = e >= e_lo && e < e_hi;
-    const unsigned same = __match_any_sync(0xffffffffu, own ? e : -1);
-    if (own && lane == __ffs(same) - 1) mine[e] += __popc(same);
-    __syncwarp();
+  const int run = (pairs + CL * threads - 1) / (CL * threads) * 32, p_begin = (rank * warps + warp) * run, p_end = min(pairs, p_begin + run);
+  for (int p0 = p_begin; p0 < p_end; p0 += 32 * PLAN_AHEAD) {
+    int ev[PLAN_AHEAD];
+#pragma unroll
+    for (int u = 0; u < PLAN_AHEAD; ++u) ev[u] = p0 + 32 * u + lane < p_end ? ids[p0 + 32 * u + lane] : -1;
+#pragma unroll
+    for (int u = 0; u < PLAN_AHEAD; ++u) {
+      if (p0 + 32 * u >= p_end) break;
+      const int e = ev[u];
+      const bool own = e >= e_lo && e < e_hi;
+      const unsigned same = plan_same(e, own, E);
+      if (own && lane == __ffs(same) - 1) mine[e] += __popc(same);
+      __syncwarp();
+    }
   }
   __syncthreads();
   int cnt = 0, all, tiles;
-  if (t < E)
-    for (int w = 0; w < warps; ++w) {
-      const int c = plan_cnt[w * E + t];
-      plan_cnt[w * E + t] = cnt;
-      cnt += c;
+  int held[W > 0 ? W : 1];                    // (in registers: through shared memory each step of the sum waits for the one before)
+  if (t < E) {
+    if (W > 0) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) held[w] = plan_cnt[w * E + t];
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        const int c = held[w];
+        held[w] = cnt;
+        cnt += c;
+      }
+    } else
+      for (int w = 0; w < warps; ++w) {
+        const int c = plan_cnt[w * E + t];
+        plan_cnt[w * E + t] = cnt;
+        cnt += c;
+      }
+  }
+  int before = 0;                             // pairs of this expert in the CTAs before this one
+  if (CL > 1) {
+    if (t < E) own_cnt[t] = cnt;
+    cluster_sync();
+    if (t < E) {
+      int c[CL];
+#pragma unroll
+      for (int r = 0; r < CL; ++r) c[r] = ld_cluster(own_cnt + t, r);
+      cnt = 0;
+#pragma unroll
+      for (int r = 0; r < CL; ++r) {
+        if (r == rank) before = cnt;
+        cnt += c[r];
+      }
     }
+    cluster_sync();                           // no CTA ends while another reads its counts
+  }
   const int start = plan_scan<W>(cnt, tmp, all);
   const int ntile = (cnt + tile_rows - 1) / tile_rows;
   const int tile0 = plan_scan<W>(ntile, tmp, tiles);
   if (t < E) {
-    offs[t] = start;
-    for (int w = 0; w < warps; ++w) plan_cnt[w * E + t] += start;
-    for (int i = 0; i < ntile && tile0 + i < max_tiles; ++i) {
+    if (rank == 0) offs[t] = start;
+    if (W > 0) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) plan_cnt[w * E + t] = held[w] + start + before;
+    } else
+      for (int w = 0; w < warps; ++w) plan_cnt[w * E + t] += start;
+    for (int i = rank; i < ntile && tile0 + i < max_tiles; i += CL) {
       int* tab = tile_tab + 3 * (tile0 + i);
       tab[0] = t;
       tab[1] = start + i * tile_rows;
       tab[2] = min(tile_rows, cnt - i * tile_rows);
     }
   }
-  if (t == 0) {
+  if (t == 0 && rank == 0) {
     offs[E] = all;
     *total = all;
   }
-  for (int i = 3 * min(tiles, max_tiles) + t; i < 3 * max_tiles; i += threads) tile_tab[i] = 0;
+  for (int i = 3 * min(tiles, max_tiles) + rank * threads + t; i < 3 * max_tiles; i += CL * threads) tile_tab[i] = 0;
   __syncthreads();
-  for (int p0 = p_begin; p0 < p_end; p0 += 32) {
-    const int p = p0 + lane;
-    const int e = p < p_end ? ids[p] : -1;
-    const bool own = e >= e_lo && e < e_hi;
-    const unsigned same = __match_any_sync(0xffffffffu, own ? e : -1);
-    int pos = -1;
-    if (own) pos = mine[e] + __popc(same & ((1u << lane) - 1u));
-    __syncwarp();
-    if (own && lane == __ffs(same) - 1) mine[e] += __popc(same);
-    __syncwarp();
-    if (p < p_end) pos_of_pair[p] = pos;
-    if (own) {
-      pair_of_pos[pos] = p;
-      expert_of_pos[pos] = e;
+  for (int p0 = p_begin; p0 < p_end; p0 += 32 * PLAN_AHEAD) {
+    int ev[PLAN_AHEAD];
+#pragma unroll
+    for (int u = 0; u < PLAN_AHEAD; ++u) ev[u] = p0 + 32 * u + lane < p_end ? ids[p0 + 32 * u + lane] : -1;
+#pragma unroll
+    for (int u = 0; u < PLAN_AHEAD; ++u) {
+      if (p0 + 32 * u >= p_end) break;
+      const int p = p0 + 32 * u + lane, e = ev[u];
+      const bool own = e >= e_lo && e < e_hi;
+      const unsigned same = plan_same(e, own, E);
+      int pos = -1;
+      if (own) pos = mine[e] + __popc(same & ((1u << lane) - 1u));
+      __syncwarp();
+      if (own && lane == __ffs(same) - 1) mine[e] += __popc(same);
+      __syncwarp();
+      if (p < p_end) pos_of_pair[p] = pos;
+      if (own) {
+        pair_of_pos[pos] = p;
+        expert_of_pos[pos] = e;
+      }
     }
   }
+}
+
+template <int W>
+__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* ids, int pairs, int E, int e_lo, int e_hi, int tile_rows, int max_tiles,
+                                                        int* __restrict__ offs, int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos,
+                                                        int* __restrict__ expert_of_pos, int* __restrict__ tile_tab, int* __restrict__ total) {
+  moe_plan<W, 1>(ids, pairs, E, e_lo, e_hi, tile_rows, max_tiles, offs, pos_of_pair, pair_of_pos, expert_of_pos, tile_tab, total);
+}
+__global__ void __launch_bounds__(1024) __cluster_dims__(PLAN_CLUSTER, 1, 1)
+    moe_plan_cluster_kernel(const int* ids, int pairs, int E, int e_lo, int e_hi, int tile_rows, int max_tiles, int* __restrict__ offs,
+                            int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos, int* __restrict__ expert_of_pos, int* __restrict__ tile_tab,
+                            int* __restrict__ total) {
+  moe_plan<PLAN_WARPS, PLAN_CLUSTER>(ids, pairs, E, e_lo, e_hi, tile_rows, max_tiles, offs, pos_of_pair, pair_of_pos, expert_of_pos, tile_tab, total);
 }
 
 // grid = pairs.  x: bf16 [M, d]; suh: f16 [E, d]; xs: f16 [pairs_cap, d].
@@ -323,6 +393,91 @@ __global__ void moe_gather_rot_kernel(const uint16_t* __restrict__ x, const int*
     uint2 o;
     o.x = *reinterpret_cast<const uint32_t*>(&a); o.y = *reinterpret_cast<const uint32_t*>(&bb);
     *reinterpret_cast<uint2*>(xs + (size_t)pos * d + n0) = o;
+  }
+}
+
+// The 128-point transform of fwht128_warp by eight lanes: element j * 32 + (lane & 7) * 4 + i of the block is v[j][i].  The strides come in the same order
+// (1, 2 in the lane, 4, 8, 16 across lanes, 32, 64 in the lane), so the sums are the same to the bit; a block costs 12 shuffles of a warp, not 20, and a lane
+// has four times the loads in flight.
+__device__ __forceinline__ void fwht128_oct(float (&v)[4][4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float a0 = v[j][0] + v[j][1], a1 = v[j][0] - v[j][1], a2 = v[j][2] + v[j][3], a3 = v[j][2] - v[j][3];
+    v[j][0] = a0 + a2; v[j][1] = a1 + a3; v[j][2] = a0 - a2; v[j][3] = a1 - a3;
+  }
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const float sgn = (lane & o) ? -1.f : 1.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float other = __shfl_xor_sync(0xffffffffu, v[j][i], o);
+        v[j][i] = fmaf(sgn, v[j][i], other);
+      }
+  }
+  const float s = 0.08838834764831845f;  // 1/sqrt(128)
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a0 = v[0][i] + v[1][i], a1 = v[0][i] - v[1][i], a2 = v[2][i] + v[3][i], a3 = v[2][i] - v[3][i];
+    v[0][i] = (a0 + a2) * s; v[1][i] = (a1 + a3) * s; v[2][i] = (a0 - a2) * s; v[3][i] = (a1 - a3) * s;
+  }
+}
+__device__ __forceinline__ void moe_half4(const uint2 u, float (&f)[4]) {
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+__device__ __forceinline__ uint2 moe_to_half4(const float (&f)[4]) {
+  const __half2 a = __floats2half2_rn(f[0], f[1]), b = __floats2half2_rn(f[2], f[3]);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// The same rows for a prompt slice: eight lanes take one 128-block of a row and write it for all the experts that the row picked, so that the row is read once
+// and four experts' rotations are in flight.
+__global__ void __launch_bounds__(256) moe_gather_rot_rows_kernel(const uint16_t* __restrict__ x, const int* __restrict__ ids, const int* __restrict__ pos_of_pair,
+                                                                  int pairs, int topk, int d, const __half* __restrict__ suh, __half* __restrict__ xs) {
+  pdl_launch();
+  pdl_wait();
+  constexpr int SLOTS = 4;
+  const int blocks = d / 128, item = (int)((blockIdx.x * 256u + threadIdx.x) >> 3);
+  const int row = item / blocks, n0 = (item - row * blocks) * 128 + (threadIdx.x & 7) * 4;
+  const int first = row * topk;                  // (past the last row: no pair, and the lanes only keep the shuffles company)
+  float xv[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint2 u = first < pairs ? *reinterpret_cast<const uint2*>(x + (size_t)row * d + n0 + 32 * j) : make_uint2(0u, 0u);
+    xv[j][0] = __uint_as_float(u.x << 16); xv[j][1] = __uint_as_float(u.x & 0xFFFF0000u);
+    xv[j][2] = __uint_as_float(u.y << 16); xv[j][3] = __uint_as_float(u.y & 0xFFFF0000u);
+  }
+  for (int s0 = 0; s0 < topk; s0 += SLOTS) {
+    int pos[SLOTS];
+    uint2 su[SLOTS][4];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      const bool have = s0 + s < topk && first + s0 + s < pairs;
+      pos[s] = have ? pos_of_pair[first + s0 + s] : -1;
+      const int e = have && suh != nullptr ? ids[first + s0 + s] : 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        su[s][j] = suh != nullptr && pos[s] >= 0 ? *reinterpret_cast<const uint2*>(suh + (size_t)e * d + n0 + 32 * j) : make_uint2(0u, 0u);
+    }
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s) {
+      if (!__any_sync(0xffffffffu, pos[s] >= 0)) continue;
+      float v[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float f[4] = {1.f, 1.f, 1.f, 1.f};
+        if (suh != nullptr) moe_half4(su[s][j], f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[j][i] = xv[j][i] * f[i];
+      }
+      if (suh != nullptr) fwht128_oct(v);
+      if (pos[s] < 0) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<uint2*>(xs + (size_t)pos[s] * d + n0 + 32 * j) = moe_to_half4(v[j]);
+    }
   }
 }
 
@@ -391,6 +546,59 @@ __global__ void __launch_bounds__(256) moe_swiglu_rot_kernel(const float* __rest
     o.x = *reinterpret_cast<const uint32_t*>(&a); o.y = *reinterpret_cast<const uint32_t*>(&bb);
     *reinterpret_cast<uint2*>(xs2 + (size_t)pos * F + n0) = o;
   }
+}
+
+// The same finish of a single plane for a prompt slice: eight lanes take one 128-block of a pair.
+__global__ void __launch_bounds__(256) moe_swiglu_rot_rows_kernel(const float* __restrict__ part, int F, const int* __restrict__ expert_of_pos,
+                                                                  const int* __restrict__ total, const __half* __restrict__ svh_gu,
+                                                                  const __half* __restrict__ suh_down, __half* __restrict__ xs2) {
+  pdl_launch();
+  pdl_wait();
+  const int blocks = F / 128, item = (int)((blockIdx.x * 256u + threadIdx.x) >> 3);
+  const int pos = item / blocks, n0 = (item - pos * blocks) * 128 + (threadIdx.x & 7) * 4, N = 2 * F;
+  const bool live = pos < *total;
+  if (!__any_sync(0xffffffffu, live)) return;
+  float g[4][4] = {}, u[4][4] = {}, s[4][4] = {};
+  uint2 vg[4] = {}, vu[4] = {}, sd[4] = {};
+  if (live) {
+    const float* row = part + (size_t)pos * N + n0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(row + 32 * j)), b = __ldg(reinterpret_cast<const float4*>(row + F + 32 * j));
+      g[j][0] = a.x; g[j][1] = a.y; g[j][2] = a.z; g[j][3] = a.w;
+      u[j][0] = b.x; u[j][1] = b.y; u[j][2] = b.z; u[j][3] = b.w;
+    }
+    const int e = expert_of_pos[pos];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (svh_gu != nullptr) {
+        vg[j] = *reinterpret_cast<const uint2*>(svh_gu + (size_t)e * N + n0 + 32 * j);
+        vu[j] = *reinterpret_cast<const uint2*>(svh_gu + (size_t)e * N + F + n0 + 32 * j);
+      }
+      if (suh_down != nullptr) sd[j] = *reinterpret_cast<const uint2*>(suh_down + (size_t)e * F + n0 + 32 * j);
+    }
+  }
+  if (svh_gu != nullptr) {
+    fwht128_oct(g);
+    fwht128_oct(u);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float fg[4] = {1.f, 1.f, 1.f, 1.f}, fu[4] = {1.f, 1.f, 1.f, 1.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[j][i] = 1.f;
+    if (svh_gu != nullptr) { moe_half4(vg[j], fg); moe_half4(vu[j], fu); }
+    if (suh_down != nullptr) moe_half4(sd[j], s[j]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float a = g[j][i] * fg[i], b = u[j][i] * fu[i];
+      g[j][i] = m_bf16_to_f(m_f_to_bf16(a / (1.f + __expf(-a)) * b)) * s[j][i];
+    }
+  }
+  if (suh_down != nullptr) fwht128_oct(g);
+  if (!live) return;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) *reinterpret_cast<uint2*>(xs2 + (size_t)pos * F + n0 + 32 * j) = moe_to_half4(g[j]);
 }
 
 // The same finish for experts WITHOUT a gate (the latent-MoE feed-forward of the Mamba2 hybrids: down(relu(up(x))^2), reference
@@ -516,6 +724,63 @@ __global__ void __launch_bounds__(PLANES > 0 ? 256 : 1024) moe_combine_kernel(co
   __syncthreads();
   if (threadIdx.x == 0)
     tp_publish_last(tp.local_count, gridDim.x * gridDim.y, tp.dst_flag, tp.ranks, tp.rank, tp_ticket(tp.epoch, tp.use_index));
+}
+
+// The same sum of a single plane on one rank for a prompt slice: eight lanes take one 128-block of a row through its slots, four slots' loads at a time.
+__global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* __restrict__ part, int M, int d, int topk, const int* __restrict__ ids,
+                                                               const float* __restrict__ w, const int* __restrict__ pos_of_pair,
+                                                               const __half* __restrict__ svh_down, const float* __restrict__ shared, float* __restrict__ dst) {
+  pdl_launch();
+  pdl_wait();
+  constexpr int SLOTS = 4;
+  const int blocks = d / 128, item = (int)((blockIdx.x * 256u + threadIdx.x) >> 3);
+  const int row = item / blocks, n0 = (item - row * blocks) * 128 + (threadIdx.x & 7) * 4;
+  const bool live = row < M;
+  float acc[4][4] = {};
+  for (int j0 = 0; j0 < topk; j0 += SLOTS) {
+    int pos[SLOTS];
+    float4 p[SLOTS][4];
+#pragma unroll
+    for (int t = 0; t < SLOTS; ++t) {
+      pos[t] = live && j0 + t < topk ? pos_of_pair[row * topk + j0 + t] : -1;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        p[t][j] = pos[t] >= 0 ? __ldg(reinterpret_cast<const float4*>(part + (size_t)pos[t] * d + n0 + 32 * j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int t = 0; t < SLOTS; ++t) {
+      if (!__any_sync(0xffffffffu, pos[t] >= 0)) continue;
+      const int pair = row * topk + j0 + t;
+      const float wj = pos[t] >= 0 ? w[pair] : 0.f;
+      const int e = pos[t] >= 0 && svh_down != nullptr ? ids[pair] : 0;
+      float y[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { y[j][0] = p[t][j].x; y[j][1] = p[t][j].y; y[j][2] = p[t][j].z; y[j][3] = p[t][j].w; }
+      uint2 sv[4] = {};
+      if (svh_down != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sv[j] = *reinterpret_cast<const uint2*>(svh_down + (size_t)e * d + n0 + 32 * j);
+        fwht128_oct(y);
+      }
+      if (pos[t] < 0) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float f[4] = {1.f, 1.f, 1.f, 1.f};
+        if (svh_down != nullptr) moe_half4(sv[j], f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[j][i] = fmaf(wj, svh_down != nullptr ? y[j][i] * f[i] : y[j][i], acc[j][i]);
+      }
+    }
+  }
+  if (!live) return;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (shared != nullptr) {
+      const float4 sh = *reinterpret_cast<const float4*>(shared + (size_t)row * d + n0 + 32 * j);
+      acc[j][0] += sh.x; acc[j][1] += sh.y; acc[j][2] += sh.z; acc[j][3] += sh.w;
+    }
+    *reinterpret_cast<float4*>(dst + (size_t)row * d + n0 + 32 * j) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ token all-to-all (data-parallel rows)
@@ -712,17 +977,33 @@ RX_API int rx_moe_plan(const void* ids, int pairs, int E, int e_lo, int e_hi, in
   const size_t smem = (size_t)warps * E * sizeof(int);
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(moe_plan_kernel<PLAN_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_WARPS * 512 * (int)sizeof(int));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_plan_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_WARPS * 512 * (int)sizeof(int));
+    const int most = PLAN_WARPS * 512 * (int)sizeof(int);
+    cudaError_t e = cudaFuncSetAttribute(moe_plan_kernel<PLAN_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_plan_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_plan_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return (int)rx::launch(warps == PLAN_WARPS ? moe_plan_kernel<PLAN_WARPS> : moe_plan_kernel<0>, dim3(1), dim3(32 * warps), smem, (cudaStream_t)stream, (const int*)ids, pairs, E, e_lo, e_hi, tile_rows, max_tiles,
+  const bool cluster = pairs >= PLAN_CLUSTER_PAIRS;
+  return (int)rx::launch(cluster ? moe_plan_cluster_kernel : warps == PLAN_WARPS ? moe_plan_kernel<PLAN_WARPS> : moe_plan_kernel<0>,
+                         dim3(cluster ? PLAN_CLUSTER : 1), dim3(32 * warps), smem, (cudaStream_t)stream, (const int*)ids, pairs, E, e_lo, e_hi, tile_rows, max_tiles,
                          (int*)offs, (int*)pos_of_pair, (int*)pair_of_pos, (int*)expert_of_pos, (int*)tile_tab, (int*)total);
 }
 
+// The forms of eight lanes a block take 32 blocks a CTA: bound by the shuffles and the issue of the transform (L1 85 % busy, its data pipe carries both), where
+// a warp a block spent two thirds more shuffles and waited for one block's loads at a time.  2100 rows x 8 picks, 2048 wide, experts of 768, with the
+// launch: gather 45 -> 33 us, SwiGLU 55 -> 48, combine 76 -> 49; 8192 rows: 154 -> 95, 176 -> 150, 242 -> 138.  A window leaves their fewer warps idle, so each
+// begins where it is the faster one, in 128-blocks of its input: gather 4096 blocks 11.1 -> 10.2 us, 2048 blocks 9.0 -> 10.2; SwiGLU 12,288 blocks
+// 14.3 -> 14.2, 6144 blocks 10.2 -> 12.2; combine 640 blocks 16.4 -> 12.2, 528 blocks 12.3 -> 13.1.
+constexpr long long GATHER_ROWS_MIN = 2560, SWIGLU_ROWS_MIN = 12288, COMBINE_ROWS_MIN = 640;
+static int moe_rows_grid(int rows, int blocks) { return (int)(((long long)rows * blocks + 31) / 32); }
+static bool moe_rows_form(int rows, int blocks, long long least) { return (long long)rows * blocks >= least && (long long)rows * blocks < (1ll << 28); }
+
 RX_API int rx_moe_gather_rot(const void* x, const void* ids, const void* pos_of_pair, int pairs, int topk, int d, const void* suh, void* xs, void* stream) {
   if (pairs < 1 || d % 128 != 0) return (int)cudaErrorInvalidValue;
+  if (topk > 0 && moe_rows_form((pairs + topk - 1) / topk, d / 128, GATHER_ROWS_MIN))
+    return (int)rx::launch(moe_gather_rot_rows_kernel, dim3(moe_rows_grid((pairs + topk - 1) / topk, d / 128)), dim3(256), 0, (cudaStream_t)stream,
+                           (const uint16_t*)x, (const int*)ids, (const int*)pos_of_pair, pairs, topk, d, (const __half*)suh, (__half*)xs);
   int warps = d / 128;
   if (warps > 8) warps = 8;
   return (int)rx::launch(moe_gather_rot_kernel, dim3(pairs), dim3(32 * warps), 0, (cudaStream_t)stream, (const uint16_t*)x, (const int*)ids,
@@ -732,6 +1013,9 @@ RX_API int rx_moe_gather_rot(const void* x, const void* ids, const void* pos_of_
 RX_API int rx_moe_swiglu_rot(const void* part, int S, int pairs_cap, int F, const void* expert_of_pos, const void* total, const void* svh_gu,
                              const void* suh_down, void* xs2, void* stream) {
   if (pairs_cap < 1 || F % 128 != 0 || S < 1) return (int)cudaErrorInvalidValue;
+  if (S == 1 && moe_rows_form(pairs_cap, F / 128, SWIGLU_ROWS_MIN))
+    return (int)rx::launch(moe_swiglu_rot_rows_kernel, dim3(moe_rows_grid(pairs_cap, F / 128)), dim3(256), 0, (cudaStream_t)stream, (const float*)part, F,
+                           (const int*)expert_of_pos, (const int*)total, (const __half*)svh_gu, (const __half*)suh_down, (__half*)xs2);
   int warps = F / 128;
   if (warps > 8) warps = 8;
   return (int)rx::launch(S == 1 ? moe_swiglu_rot_kernel<true> : moe_swiglu_rot_kernel<false>, dim3(pairs_cap, 1), dim3(32 * warps), 0, (cudaStream_t)stream, (const float*)part, S, pairs_cap, F,
@@ -755,6 +1039,10 @@ RX_API int rx_moe_combine(const void* part, int S, int pairs_cap, int M, int d, 
   const CombineDst tp = *(const CombineDst*)desc;
   if (tp.ranks < 1 || tp.ranks > TP_MAX || M > tp.rows_cap) return (int)cudaErrorInvalidValue;
   const int blocks = d / 128;
+  if (S == 1 && tp.dst_flag[0] == nullptr && moe_rows_form(M, blocks, COMBINE_ROWS_MIN))
+    return (int)rx::launch(moe_combine_rows_kernel, dim3(moe_rows_grid(M, blocks)), dim3(256), 0, (cudaStream_t)stream, (const float*)part, M, d, topk,
+                           (const int*)ids, (const float*)w, (const int*)pos_of_pair, (const __half*)svh_down, (const float*)shared,
+                           tp.dst[0] + (size_t)tp.rank * tp.rows_cap * d);
   int gy;
   if (M <= LL_MAX_ROWS) {              // packet mode: many small CTAs (a chain of dependent loads and R remote stores per block)
     gy = (592 + M - 1) / M;
