@@ -366,7 +366,10 @@ class MoEGPU(DenseGPU):
         if cls == "decode":
             tile_rows, max_tiles = (16 if M <= 16 else 32), self.max_tiles_decode
         else:
-            tile_rows, max_tiles = 128, self.max_tiles_prefill
+            # tiles of 256 rows decode an expert's weights once where 128 rows would have them twice: from 80 rows per expert on (128 experts, 2048 -> 1536 and
+            # 768 -> 2048: 16,800 pairs 248 -> 190 and 164 -> 135 us, 10,400 pairs 158 -> 156 and 98 -> 90; 8,800 pairs, uneven, 158 -> 162)
+            tall = pairs >= 80 * cfg.n_experts and all(t.twice in (6, 8) for t in (L["gu"], L["down"]))
+            tile_rows, max_tiles = 256 if tall else 128, self.max_tiles_prefill
         if self.a2a is not None:
             yield from self._ffn_a2a(li, L, M, cls, xn, tile_rows, max_tiles, h, xr_d, next_norm, next_suh)
             return

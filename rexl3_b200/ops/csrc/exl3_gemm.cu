@@ -407,6 +407,14 @@ RX_API int rx_exl3_gemm(const void* xr, int rows, int K, const void* trellis, in
   // Only where both cut K at the same places: a row's bits do not depend on the row count.
   if (twice == 6 && brows == 128 && (long long)(N / STRIP) * splits > 148 && (K / 128) % splits == 0 && gemm_persistent_takes(K, twice, splits, brows))
     return gemm_persistent(xr, rows, K, trellis, 0, N, twice, codebook, part, splits, 128, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
+  // More than 128 rows at 3.0 bpw: tiles of 128 rows where all of them are begun at once (2048 -> 5120, 300 rows 28.7 -> 22.5 us; 4096 -> 2048, 1100 rows
+  // 45.1 -> 34.8), and where tiles of 256 make a CTA more than one item, the persistent kernel over those (2048 -> 5120, 2100 rows 72.5 -> 67.7 us, 8192 rows
+  // 207 -> 188).  In between one item of 256 rows for a CTA is as fast by either kernel (700 rows 28.6 and 29.5 us) and two of 128 slower (38.8).
+  if (twice == 6 && brows == 256 && splits == 1) {
+    const int prow = (long long)(N / STRIP) * ((rows + 127) / 128) <= 148 ? 128 : (long long)(N / STRIP) * row_tiles > 148 ? 256 : 0;
+    if (prow != 0 && gemm_persistent_takes(K, twice, splits, prow))
+      return gemm_persistent(xr, rows, K, trellis, 0, N, twice, codebook, part, splits, 128, nullptr, (rows + prow - 1) / prow, prow, status, (cudaStream_t)stream);
+  }
   CUtensorMap tm;
   int e = make_tmap_f16_2d(&tm, xr, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
   if (e != 0) return e;

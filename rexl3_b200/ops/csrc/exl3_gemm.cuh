@@ -4,7 +4,7 @@
 
 namespace rx {
 
-// Whether gemm_persistent takes the product: widths with a column decoder (twice the bits: 6 or 8), up to 128 rows a tile, splits of 128 k and more.
+// Whether gemm_persistent takes the product: widths with a column decoder (twice the bits: 6 or 8), up to 128 rows a tile or 256 without splits, splits of 128 k and more.
 bool gemm_persistent_takes(int K, int twice, int splits, int brows);
 
 // part[split][row][n]; `cut`: K is split at multiples of 64 or 128.  tile_tab: device int32 [max_tiles][3] = {expert, first row, rows}, nullptr: the

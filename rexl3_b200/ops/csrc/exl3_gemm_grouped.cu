@@ -12,6 +12,11 @@
 // 146 us here; one row 83 and 26 us.  What is left is the decode's own: the integer pipe is 70 % busy.  (Fetching the next item's table entry
 // ahead costs registers that the decode groups do not have: 5 % slower.)
 //
+// Tiles of up to 256 rows (TALL, for prompt slices): both accumulators hold rows of one item, a unit of 128 rows each, so that its weights are decoded once.
+// The activations then come in boxes of 64 rows, no more of them than the tile has rows, and a unit is written out by two groups, half each: with one
+// group a unit the next item waited for them (128 experts, 16,800 pairs, 2048 -> 1536: 229 us by tiles of 128, 211 with one group a unit, 190 so).  What is left
+// of it is the L2's: every strip reads the activations again, 6 TB/s at 65,536 pairs (678 -> 510 us).
+//
 // Warp roles: 0 weight producer (one bulk copy per k-tile row), 1 TMEM owner + MMA issuer, 2 activation producer, then NG decode groups of 4 warps.
 // Group e % NG writes out item e, after its first chunk of a later item: the accumulator of item e is needed again by item e + 2 only, whose
 // first MMA waits for it.  No circle of waits: that chunk's A stage was last read by a chunk of item e or before.  Every wait is bounded.
@@ -27,7 +32,10 @@ constexpr int GR_ROLE_WARPS = 3;
 // A decode group waits for "the MMA that last read this stage": sound while no group can run two phases ahead, i.e. with as many stages as groups.
 __host__ __device__ constexpr int gr_a_stages(int ng) { return ng; }
 __host__ __device__ constexpr int gr_acc_cols(int brows) { return brows < 32 ? 32 : brows; }
-__host__ __device__ inline int gr_smem_bytes(int brows, int twice) { return GR_OP_STAGES * brows * 256 + GR_RAW_STAGES * 1024 * twice + 512; }
+constexpr int GR_TALL_ROWS = 256, GR_UNIT_ROWS = 128, GR_TALL_OPS = 5, GR_BOX_ROWS = 64;
+__host__ __device__ inline int gr_smem_bytes(int brows, int twice) {
+  return (brows > GR_UNIT_ROWS ? GR_TALL_OPS * GR_UNIT_ROWS : GR_OP_STAGES * brows) * 256 + GR_RAW_STAGES * 1024 * twice + 512;
+}
 
 // One k-tile (16 k) of a thread's column: 8 packed pairs, regs[m] = k (2m, 2m + 1), regs[4 + m] = k (8 + 2m, 9 + 2m).
 // w[0] = the word before the thread's eighth of the tile, w[1..] = the eighth's words (see exl3_decode.cuh); b2: which of its two columns.
@@ -75,27 +83,29 @@ __device__ __forceinline__ void decode_column(const uint32_t (&w)[TWICE / 2 + 1]
 }
 
 // HALVES: the last chunk of a split may be half a chunk (its checks cost the MMA issuer and the producers 1 % of a window of 80 rows).
-template <int TWICE, int CB, int NG, bool HALVES>
+template <int TWICE, int CB, int NG, bool HALVES, bool TALL>
 __global__ void __launch_bounds__(GR_ROLE_WARPS * 32 + NG * 128, (NG <= 3 ? 2 : 1))
 exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __restrict__ trellis, size_t expert_words,
                          float* __restrict__ part, int rows, int K, int N, int splits, int cut, int brows, const int* tile_tab, int max_tiles,
                          int* status) {
   pdl_launch();
   constexpr int SA = gr_a_stages(NG), EW = TWICE / 2;            // EW: words of an eighth of a tile
+  constexpr int OPS = TALL ? GR_TALL_OPS : GR_OP_STAGES;
+  const int urows = TALL ? GR_UNIT_ROWS : brows;                 // rows of a unit: one accumulator, one B stage
   // Quarters of a chunk unrolled: short items keep to the instruction cache, long ones gain 5 % (86 experts 2048 -> 1536 in 4 splits 96.7 us with one, 93.2 with
   // two or four; 79 experts 768 -> 2048 in 3 splits 52.0, 52.0, 54.8).
   constexpr int QT = NG <= 3 ? 2 : 4;
   constexpr int TILE_WORDS = 4 * TWICE, ROW_BYTES = 8 * TILE_WORDS * 4, RAW_STAGE = 8 * ROW_BYTES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int b_half = brows * 128, b_stage = 2 * b_half;          // one [brows x 64] swizzled sub-tile
+  const int b_half = urows * 128, b_stage = 2 * b_half;          // one [urows x 64] swizzled sub-tile
   uint8_t* b_base = smem;
-  uint8_t* raw_base = smem + GR_OP_STAGES * b_stage;
+  uint8_t* raw_base = smem + OPS * b_stage;
   uint64_t* a_full = (uint64_t*)(raw_base + GR_RAW_STAGES * RAW_STAGE);   // [SA] 4 decode warps
   uint64_t* a_empty = a_full + SA;                   // [SA] tcgen05.commit
   uint64_t* b_full = a_empty + SA;                   // [OP] activation producer expect_tx
-  uint64_t* b_empty = b_full + GR_OP_STAGES;         // [OP] tcgen05.commit
-  uint64_t* raw_full = b_empty + GR_OP_STAGES;       // [RAW] weight producer expect_tx
+  uint64_t* b_empty = b_full + OPS;         // [OP] tcgen05.commit
+  uint64_t* raw_full = b_empty + OPS;       // [RAW] weight producer expect_tx
   uint64_t* raw_empty = raw_full + GR_RAW_STAGES;    // [RAW] 4 decode warps
   // A parity wait tells a phase from the next one only.  A group may ask for item e before item e - 2 is complete, but its own last write-out was
   // item e - NG, so e - 4 is: four barriers in turn for two accumulators.
@@ -111,15 +121,15 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
   int* split_c0 = (int*)(n_sent + 2);                 // [splits + 1] where each split begins, in halves of a chunk
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strips = N / GR_STRIP, per_tile = strips * splits, nt_total = N / 16;
-  const int acc_cols = gr_acc_cols(brows);
+  const int acc_cols = gr_acc_cols(urows);
   uint32_t ncols = 32;
   while ((int)ncols < 2 * acc_cols + SA * GR_A_COLS) ncols <<= 1;
   if (threadIdx.x == 0) {
     for (int i = 0; i < SA; ++i) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
-    for (int i = 0; i < GR_OP_STAGES; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+    for (int i = 0; i < OPS; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
     for (int i = 0; i < GR_RAW_STAGES; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
     for (int i = 0; i < 4; ++i) mbar_init(&acc_full[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], 4);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], TALL ? 8 : 4);
     mbar_init(drained, 1);
     *abort_flag = *last_flag = 0;
     *tile_end = -1;
@@ -169,6 +179,7 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     for (int i = 0; i < (1 << 20) && (end = *tile_end) < 0; ++i) {}
     return w.tile < end;
   };
+  auto units_of = [&](const Item& i) { return TALL && i.nrows > GR_UNIT_ROWS ? 2 : 1; };
   Item it;
   Walk at = walk_of(blockIdx.x);
   const Walk stride = walk_of(gridDim.x);
@@ -198,13 +209,27 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
       int gc = 0;
       for (; ok && tile_of(at, it); step(at, stride)) {
         const int c0 = split_c0[at.split], halves = split_c0[at.split + 1] - c0, n = (halves + 1) >> 1;
-        for (int c = 0; c < n; ++c, ++gc) {
-          const int s = gc % GR_OP_STAGES, x = c0 * GR_HALF + c * GR_KCH;
+        const int units = units_of(it);
+        for (int c = 0; c < n && ok; ++c) {
+          const int x = c0 * GR_HALF + c * GR_KCH;
           const bool half = HALVES && 2 * c + 2 > halves;
-          if (gc >= GR_OP_STAGES && !mbar_wait(&b_empty[s], ((gc / GR_OP_STAGES) - 1) & 1, abort_flag, status, 211, 250)) { ok = false; break; }
-          mbar_arrive_expect_tx(&b_full[s], (uint32_t)(half ? b_half : b_stage));
-          tma_load_2d(b_base + s * b_stage, &tmap_x, x, it.row0, &b_full[s]);
-          if (!half) tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + GR_HALF, it.row0, &b_full[s]);
+          for (int u = 0; u < units; ++u, ++gc) {
+            const int s = gc % OPS;
+            if (gc >= OPS && !mbar_wait(&b_empty[s], ((gc / OPS) - 1) & 1, abort_flag, status, 211, 250)) { ok = false; break; }
+            uint8_t* dst = b_base + s * b_stage;
+            if constexpr (TALL) {                      // only as many boxes as the unit has rows for: its other columns are neither multiplied nor written
+              const int row0 = it.row0 + u * GR_UNIT_ROWS, boxes = min(it.nrows - u * GR_UNIT_ROWS, GR_UNIT_ROWS) > GR_BOX_ROWS ? 2 : 1;
+              mbar_arrive_expect_tx(&b_full[s], (uint32_t)(boxes * GR_BOX_ROWS * 128 * (half ? 1 : 2)));
+              for (int b = 0; b < boxes; ++b) {
+                tma_load_2d(dst + b * GR_BOX_ROWS * 128, &tmap_x, x, row0 + b * GR_BOX_ROWS, &b_full[s]);
+                if (!half) tma_load_2d(dst + b_half + b * GR_BOX_ROWS * 128, &tmap_x, x + GR_HALF, row0 + b * GR_BOX_ROWS, &b_full[s]);
+              }
+            } else {
+              mbar_arrive_expect_tx(&b_full[s], (uint32_t)(half ? b_half : b_stage));
+              tma_load_2d(dst, &tmap_x, x, it.row0, &b_full[s]);
+              if (!half) tma_load_2d(dst + b_half, &tmap_x, x + GR_HALF, it.row0, &b_full[s]);
+            }
+          }
         }
       }
       n_sent[1] = gc;
@@ -224,27 +249,34 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(b_base));
       const uint32_t half_units = (uint32_t)b_half >> 4, stage_units = (uint32_t)b_stage >> 4;
       bool ok = true;
-      int gc = 0;
-      for (int e = 0; ok && tile_of(at, it); ++e, step(at, stride)) {
+      int gc = 0, gb = 0;
+      for (int e = 0, units = 0; ok && tile_of(at, it); e += units, step(at, stride)) {       // e: the item's first unit
         const int halves = split_c0[at.split + 1] - split_c0[at.split], n = (halves + 1) >> 1;
-        if (e >= 2 && !mbar_wait(&acc_empty[e & 1], ((e >> 1) - 1) & 1, abort_flag, status, 222)) break;
+        units = units_of(it);
+        for (int u = 0; u < units && ok; ++u)
+          if (e + u >= 2) ok = mbar_wait(&acc_empty[(e + u) & 1], (((e + u) >> 1) - 1) & 1, abort_flag, status, 222);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t idesc = umma_idesc_f16(GR_STRIP, max(16, (it.nrows + 15) & ~15), 0, 0);
-        const uint32_t acc = tmem_base + (e & 1) * acc_cols;
-        for (int c = 0; c < n; ++c, ++gc) {
-          const int s = gc % GR_OP_STAGES, sa = gc % SA;
-          if (!mbar_wait(&b_full[s], (gc / GR_OP_STAGES) & 1, abort_flag, status, 220) ||
-              !mbar_wait(&a_full[sa], (gc / SA) & 1, abort_flag, status, 221, 100)) { ok = false; break; }
-          tc_fence_after();
-          const uint64_t bd = desc0 + (uint64_t)(s * stage_units);
+        for (int c = 0; c < n && ok; ++c, ++gc) {
+          const int sa = gc % SA;
           const uint32_t a_at = a_tmem0 + sa * GR_A_COLS;
+          for (int u = 0; u < units; ++u, ++gb) {
+            const int s = gb % OPS;
+            if (!mbar_wait(&b_full[s], (gb / OPS) & 1, abort_flag, status, 220) ||
+                (u == 0 && !mbar_wait(&a_full[sa], (gc / SA) & 1, abort_flag, status, 221, 100))) { ok = false; break; }
+            tc_fence_after();
+            const int nrows = TALL ? min(it.nrows - u * GR_UNIT_ROWS, GR_UNIT_ROWS) : it.nrows;
+            const uint32_t idesc = umma_idesc_f16(GR_STRIP, max(16, (nrows + 15) & ~15), 0, 0);
+            const uint32_t acc = tmem_base + ((e + u) & 1) * acc_cols;
+            const uint64_t bd = desc0 + (uint64_t)(s * stage_units);
 #pragma unroll
-          for (int k = 0; k < GR_KCH / 16; ++k)
-            if (!HALVES || k < GR_HALF / 16 || 2 * c + 2 <= halves) tc_mma_f16_ts(acc, a_at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
-          tc_commit(&a_empty[sa]);
-          tc_commit(&b_empty[s]);
+            for (int k = 0; k < GR_KCH / 16; ++k)
+              if (!HALVES || k < GR_HALF / 16 || 2 * c + 2 <= halves) tc_mma_f16_ts(acc, a_at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, (c | k) != 0);
+            tc_commit(&b_empty[s]);
+          }
+          if (ok) tc_commit(&a_empty[sa]);
         }
-        if (ok) tc_commit(&acc_full[e & 3]);
+        for (int u = 0; u < units && ok; ++u) tc_commit(&acc_full[(e + u) & 3]);
       }
       tc_commit(drained);
     }
@@ -258,31 +290,43 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t my_words = (uint32_t)(nt * TILE_WORDS + g * EW) * 4u;     // byte offset of this thread's eighth inside a k-tile row
     bool ok = true;
-    int next_out = grp;                           // the next item this group writes out, and where it stands
-    Walk out_at = walk_of(blockIdx.x + (unsigned)grp * gridDim.x);
+    int next_out = grp;                           // the next unit (TALL: half of one) that this group writes out, and where it stands
+    Walk out_at = walk_of(blockIdx.x + (TALL ? 0u : (unsigned)grp * gridDim.x));
     const Walk out_stride = walk_of((unsigned)NG * gridDim.x);
-    auto write_out = [&](int e) {
+    int out_first = 0;                            // TALL: the first unit of the item at out_at
+    auto write_out = [&](int job) {
+      const int e = TALL ? job >> 1 : job, from = TALL ? (job & 1) * (GR_UNIT_ROWS / 2) : 0;
       Item o;
       tile_of(out_at, o);
+      if constexpr (TALL) {
+        for (int u; (u = units_of(o)) <= e - out_first;) {
+          out_first += u;
+          step(out_at, stride);
+          tile_of(out_at, o);
+        }
+        o.row0 += (e - out_first) * GR_UNIT_ROWS;
+        o.nrows = min(GR_UNIT_ROWS, o.nrows - (e - out_first) * GR_UNIT_ROWS);
+      }
       if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[e & 3], (e >> 2) & 1, abort_flag, status, 240))) return false;
       tc_fence_after();
       float* out = part + ((size_t)out_at.split * rows + o.row0) * N + out_at.strip * GR_STRIP + n;
-      for (int cb = 0; cb < o.nrows; cb += 16) {
+      const int to = TALL ? min(o.nrows, from + GR_UNIT_ROWS / 2) : o.nrows;
+      for (int cb = from; cb < to; cb += 16) {
         uint32_t r[16];
         tc_ld_32x32b_x16(tmem_base + (e & 1) * acc_cols + lane_addr + cb, r);
         tc_wait_ld();
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (cb + i < o.nrows) out[(size_t)(cb + i) * N] = __uint_as_float(r[i]);
+          if (cb + i < to) out[(size_t)(cb + i) * N] = __uint_as_float(r[i]);
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[e & 1]);
-      step(out_at, out_stride);
+      if constexpr (!TALL) step(out_at, out_stride);
       return true;
     };
-    int gc0 = 0, e = 0;                           // chunks up to the end of item e
-    for (int gc = grp; ok && tile_of(at, it); ++e, step(at, stride)) {
+    int gc0 = 0, e = 0;                           // chunks up to the end of this item, units before it
+    for (int gc = grp; ok && tile_of(at, it); e += units_of(it), step(at, stride)) {
       gc0 += (split_c0[at.split + 1] - split_c0[at.split] + 1) >> 1;
       for (; gc < gc0 && ok; gc += NG) {
         const int rs = gc % GR_RAW_STAGES, os = gc % SA;
@@ -323,16 +367,16 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&a_full[os]);
-        for (; next_out < e && ok; next_out += NG) ok = write_out(next_out);
+        for (; (TALL ? next_out >> 1 : next_out) < e && ok; next_out += NG) ok = write_out(next_out);
       }
     }
-    for (; next_out < e && ok; next_out += NG) ok = write_out(next_out);
+    for (; (TALL ? next_out >> 1 : next_out) < e && ok; next_out += NG) ok = write_out(next_out);
   }
   tc_fence_before();
   __syncthreads();
   if (*abort_flag != 0 && lane == 0) {                // consumers that gave up have not seen the last copies arrive
     if (warp == 0) ring_landed(raw_full, GR_RAW_STAGES, n_sent[0]);
-    if (warp == 2) ring_landed(b_full, GR_OP_STAGES, n_sent[1]);
+    if (warp == 2) ring_landed(b_full, OPS, n_sent[1]);
   }
   if (warp == 1) {
     if (lane == 0) mbar_wait(drained, 0, last_flag, status, 241);      // nothing may still write the tensor memory that is freed
@@ -343,12 +387,12 @@ exl3_gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint3
 
 int make_tmap_f16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
-template <int TWICE, int CB, int NG, bool HALVES>
+template <int TWICE, int CB, int NG, bool HALVES, bool TALL>
 static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t expert_words, float* part, int rows, int K, int N, int splits, int cut, int brows,
                           const int* tile_tab, int max_tiles, int* status, cudaStream_t st) {
   int smem = gr_smem_bytes(brows, TWICE) + 1024;
   if (NG <= 3 && smem < 80 * 1024) smem = 80 * 1024;   // at most two CTAs per SM: each allocates 256 TMEM columns
-  auto kern = exl3_gemm_grouped_kernel<TWICE, CB, NG, HALVES>;
+  auto kern = exl3_gemm_grouped_kernel<TWICE, CB, NG, HALVES, TALL>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
@@ -366,18 +410,18 @@ static int launch_grouped(const CUtensorMap& tm, const uint32_t* trellis, size_t
 // Whether gemm_persistent takes the product: widths with a column decoder, tiles whose two accumulators fit beside the A stages, splits of a chunk
 // and more and no more of them than its table of their bounds holds.
 bool gemm_persistent_takes(int K, int twice, int splits, int brows) {
-  return (twice == 6 || twice == 8) && brows <= 128 && splits <= K / GR_KCH && splits < 32;
+  return (twice == 6 || twice == 8) && (brows <= GR_UNIT_ROWS || (brows == GR_TALL_ROWS && splits == 1)) && splits <= K / GR_KCH && splits < 32;
 }
 
 int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t expert_words, int N, int twice, int codebook, void* part, int splits, int cut,
                     const int* tile_tab, int max_tiles, int brows, int* status, cudaStream_t st) {
   CUtensorMap tm;
-  int e = make_tmap_f16_2d(&tm, xs, (uint64_t)rows, (uint64_t)K, (uint32_t)brows);
+  int e = make_tmap_f16_2d(&tm, xs, (uint64_t)rows, (uint64_t)K, (uint32_t)(brows > GR_UNIT_ROWS ? GR_BOX_ROWS : brows));
   if (e != 0) return e;
   const uint32_t* tr = (const uint32_t*)trellis;
   const bool halves = cut == GR_HALF && (K / GR_KCH) % splits != 0;
-#define RX_GR_H(T, CBV, H) (brows > 32 ? launch_grouped<T, CBV, 4, H>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st) \
-                                       : launch_grouped<T, CBV, 3, H>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st))
+#define RX_GR_L(T, CBV, NGV, H, TL) launch_grouped<T, CBV, NGV, H, TL>(tm, tr, expert_words, (float*)part, rows, K, N, splits, cut, brows, tile_tab, max_tiles, status, st)
+#define RX_GR_H(T, CBV, H) (brows > GR_UNIT_ROWS ? RX_GR_L(T, CBV, 4, false, true) : brows > 32 ? RX_GR_L(T, CBV, 4, H, false) : RX_GR_L(T, CBV, 3, H, false))
 #define RX_GR(T, CBV) (halves ? RX_GR_H(T, CBV, true) : RX_GR_H(T, CBV, false))
   switch (codebook) {
     case CB_3INST: return twice == 6 ? RX_GR(6, CB_3INST) : RX_GR(8, CB_3INST);
@@ -387,6 +431,7 @@ int gemm_persistent(const void* xs, int rows, int K, const void* trellis, size_t
   }
 #undef RX_GR
 #undef RX_GR_H
+#undef RX_GR_L
 }
 
 }  // namespace rx
