@@ -518,6 +518,13 @@ class HybridGPU(DenseGPU):
         return sum(t.numel() * 4 for t in self.conv_pool.values()) + sum(t.numel() * 4 for t in self.ssm_pool.values())
 
     # ------------------------------------------------------------------ forward
+    def _in_proj(self, xr, w, M, cls, name, proj):
+        K, work = self.K, self.wide if cls == "prefill" else None
+        if work is not None and isinstance(w, K.Exl3Weight) and self.splits[(cls, name)] == 1 and K.wide_takes(w, M) and work.numel() >= K.wide_bytes(w.K, w.N):
+            K.exl3_gemm_store(xr, w, proj, work, self.status)
+        else:
+            K.finish_store(self.part, self._linear(xr, w, M, cls, name), M, w, proj)
+
     def _mixer(self, li, L, M, cls, xr_d, xr_a, q, positions, slots, row_seq, ctx_len, block_table, prefill, max_ctx, scale):
         if L["kind"] == "A":
             return super()._mixer(li, L, M, cls, xr_d, xr_a, q, positions, slots, row_seq, ctx_len, block_table, prefill, max_ctx, scale)
@@ -531,18 +538,16 @@ class HybridGPU(DenseGPU):
         if L["kind"] in "GK":
             kda = L["kind"] == "K"
             wp = cfg.delta_proj_width(L["kind"])
-            s = self._linear(xr_d, L["in_proj"], M, cls, "kda_in" if kda else "gdn_in")
             proj = self.rec_proj[li][:M] if rec else self.ssm_proj[:M * wp].view(M, wp)
-            K.finish_store(self.part, s, M, L["in_proj"], proj)
+            self._in_proj(xr_d, L["in_proj"], M, cls, "kda_in" if kda else "gdn_in", proj)
             out = self.ssm_out[:M * cfg.gdn_inner].view(M, cfg.gdn_inner)
             K.gdn_mixer(proj, M, cfg.gdn_k_heads, cfg.gdn_v_heads, 128, row_seq, positions, seg_s, seg_l, nseg, L["conv_w"], L["conv_b"], L["dt_bias"],
                         L["a_neg"], L["norm_w"], cfg.eps, self.conv_pool[li], self.ssm_pool[li], xbc, out, kda=kda, mode=mode, y32=self.ssm_y)
             xr_g = self.xr[:M * cfg.gdn_inner].view(M, cfg.gdn_inner)
             K.norm_rot_in(out, None, cfg.eps, L["out_proj"].suh, xr_g)
             return self._linear(xr_g, L["out_proj"], M, cls, "gdn_out")
-        s = self._linear(xr_d, L["in_proj"], M, cls, "in_proj")
         proj = self.rec_proj[li][:M] if rec else self.ssm_proj[:M * cfg.in_proj_width].view(M, cfg.in_proj_width)
-        K.finish_store(self.part, s, M, L["in_proj"], proj)
+        self._in_proj(xr_d, L["in_proj"], M, cls, "in_proj", proj)
         out = self.ssm_out[:M * cfg.d_inner].view(M, cfg.d_inner)
         K.ssm_mixer(proj, M, cfg.ssm_heads, cfg.ssm_head_dim, cfg.ssm_groups, cfg.ssm_state, row_seq, positions, seg_s, seg_l, nseg, L["conv_w"], L["conv_b"],
                     L["dt_bias"], L["a_neg"], L["d_skip"], L["norm_w"], cfg.eps, self.conv_pool[li], self.ssm_pool[li], xbc, self.ssm_y, out, mode=mode)

@@ -34,7 +34,7 @@ constexpr long long WD_FRONT = WD_COUNTERS * 4ll + WD_PAIRS * WD_HAND * 4;
 constexpr int WD_OUT = 2 * 32 * 128;               // bytes of an epilogue warp's staging: two boxes of 32 rows x 128 bytes, swizzled
 constexpr int WD_SMEM = WD_STAGES * 2 * WD_HALF + 4 * WD_OUT + 256 + 1024;
 
-enum : int { WD_PLAIN = 0, WD_SWIGLU = 1 };
+enum : int { WD_PLAIN = 0, WD_SWIGLU = 1, WD_STORE = 2 };
 
 struct WideArgs {
   const __half* svh;
@@ -391,6 +391,47 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
+      } else if constexpr (MODE == WD_STORE) {
+        if (row0 < a.rows)
+#pragma unroll 1
+          for (int b = 0; b < w.width; b += 128) {
+            const int c0 = w.col + b;
+            const float* bias = a.bias == nullptr ? nullptr : a.bias + c0;
+            transform_block(src + b, [&](int c, uint32_t(&lo)[16], uint32_t(&hi)[16]) {
+              float scale[2][16];
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const uint4* sv = reinterpret_cast<const uint4*>(a.svh + c0 + 64 * h + c);
+                const uint4 v[2] = {__ldg(sv), __ldg(sv + 1)};
+                const __half2* x = reinterpret_cast<const __half2*>(v);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  const float2 f = __half22float2(x[i]);
+                  scale[h][2 * i] = f.x, scale[h][2 * i + 1] = f.y;
+                }
+              }
+              scale16(lo, scale[0], bias == nullptr ? nullptr : bias + c);
+              scale16(hi, scale[1], bias == nullptr ? nullptr : bias + 64 + c);
+              if ((c & 16) == 0) {
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the copies before have read the boxes
+                __syncwarp();
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                st_box(box0, lane, (c & 16) / 4 + j, lo[4 * j], lo[4 * j + 1], lo[4 * j + 2], lo[4 * j + 3]);
+                st_box(box0 + WD_OUT / 2, lane, (c & 16) / 4 + j, hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
+              }
+              if (c & 16) {
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                  tma_store_2d(&tmap_out, box0, c0 + c - 16, row0);
+                  tma_store_2d(&tmap_out, box0 + WD_OUT / 2, c0 + 64 + c - 16, row0);
+                  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+              }
+            });
+          }
       } else if (row0 < a.rows) {
         const int c0 = w.ct * 128;
         const bool live = row0 + lane < a.rows;    // the zeros of rows past the end would send the division down its slow path
@@ -443,7 +484,7 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[acc]), 0));
       if (GROUPS == 2 && n + 2 == last) take(last);
     }
-    if (MODE == WD_PLAIN && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (MODE != WD_SWIGLU && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   } else {
     // ---- expansion: a piece is 32 columns x 256 k, in the order in which the tiles need them.  The words of a piece are loaded as those of the piece
     // before are used up, and the piece after it is claimed meanwhile.
@@ -564,6 +605,7 @@ RX_API long long rx_exl3_wide_bytes(int K, int N) { return WD_FRONT + 2ll * K * 
 static int gemm_wide(WideArgs a, const void* xr, int codebook, int mode, void* out, void* work, long long work_bytes, cudaStream_t st) {
   if (a.rows <= 0 || a.K % 128 != 0 || a.K < WD_PIECE_K || a.N % (mode == WD_SWIGLU ? 256 : 128) != 0 || a.N <= 0) return (int)cudaErrorInvalidValue;
   if (work == nullptr || work_bytes < rx_exl3_wide_bytes(a.K, a.N) || wide_counters(a.K, a.N) > WD_COUNTERS) return (int)cudaErrorInvalidValue;
+  if (mode == WD_STORE && ((((uintptr_t)a.svh) & 15) || (((uintptr_t)a.bias) & 15))) return (int)cudaErrorMisalignedAddress;
   if ((((uintptr_t)xr) & 15) || (((uintptr_t)out) & 31) || (((uintptr_t)a.trellis) & 15) || (((uintptr_t)work) & 127)) return (int)cudaErrorMisalignedAddress;
   a.count = (int*)work;
   a.hand = (float*)((char*)work + WD_COUNTERS * 4);
@@ -581,9 +623,10 @@ static int gemm_wide(WideArgs a, const void* xr, int codebook, int mode, void* o
   if (e == 0) e = make_tmap_f16_2d(&tw, a.w, (uint64_t)a.N * (a.K / 64), 64, 128);
   if (e == 0) e = make_tmap_f16_2d(&tw64, a.w, (uint64_t)a.N * (a.K / 64), 64, 64);
   to = tx;
-  if (e == 0 && mode == WD_PLAIN) e = make_tmap_f32_2d(&to, out, (uint64_t)a.rows, (uint64_t)a.N, 32);
+  if (e == 0 && mode != WD_SWIGLU) e = make_tmap_f32_2d(&to, out, (uint64_t)a.rows, (uint64_t)a.N, 32);
   if (e != 0) return e;
-#define RX_WD(CBV) (mode == WD_SWIGLU ? launch_wide<CBV, WD_SWIGLU>(tx, tw, tw64, to, a, st) : launch_wide<CBV, WD_PLAIN>(tx, tw, tw64, to, a, st))
+#define RX_WD(CBV) (mode == WD_SWIGLU ? launch_wide<CBV, WD_SWIGLU>(tx, tw, tw64, to, a, st) \
+                    : mode == WD_STORE ? launch_wide<CBV, WD_STORE>(tx, tw, tw64, to, a, st) : launch_wide<CBV, WD_PLAIN>(tx, tw, tw64, to, a, st))
   switch (codebook) {
     case CB_3INST: return RX_WD(CB_3INST);
     case CB_MCG: return RX_WD(CB_MCG);
@@ -610,4 +653,14 @@ RX_API int rx_exl3_gemm_wide_swiglu(const void* xr, int rows, int K, const void*
   a.trellis = (const uint32_t*)trellis, a.status = status;
   a.rows = rows, a.K = K, a.N = 2 * F;
   return gemm_wide(a, xr, codebook, WD_SWIGLU, act, work, work_bytes, (cudaStream_t)stream);
+}
+
+// The same with rx_finish_store of fp32 rows in its epilogue.
+RX_API int rx_exl3_gemm_wide_store(const void* xr, int rows, int K, const void* trellis, int N, int codebook, const void* svh, const void* bias, void* out,
+                                   void* work, long long work_bytes, int* status, void* stream) {
+  WideArgs a = {};
+  a.svh = (const __half*)svh, a.bias = (const float*)bias;
+  a.trellis = (const uint32_t*)trellis, a.status = status;
+  a.rows = rows, a.K = K, a.N = N;
+  return gemm_wide(a, xr, codebook, WD_STORE, out, work, work_bytes, (cudaStream_t)stream);
 }

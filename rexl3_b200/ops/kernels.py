@@ -107,6 +107,17 @@ def exl3_gemm_swiglu_rot(xr: torch.Tensor, w: Exl3Weight, suh_down: torch.Tensor
     _lib.count()
 
 
+def exl3_gemm_store(xr: torch.Tensor, w: Exl3Weight, out: torch.Tensor, work: torch.Tensor, status: torch.Tensor) -> None:
+    """`exl3_gemm` and `finish_store` in one kernel for the rows of a prompt slice (where `wide_takes`): out fp32 [rows, N]."""
+    rows, K = xr.shape
+    assert xr.dtype == torch.float16 and xr.is_contiguous() and K == w.K and w.twice == 8
+    assert out.dtype == torch.float32 and out.is_contiguous() and out.numel() >= rows * w.N
+    _lib.check(_lib.load().rx_exl3_gemm_wide_store(xr.data_ptr(), rows, K, w.trellis.data_ptr(), w.N, CB_ID[w.codebook], w.svh.data_ptr(), _lib.ptr(w.bias),
+                                                   out.data_ptr(), work.data_ptr(), work.numel(), status.data_ptr(), _lib.stream_ptr()),
+               "rx_exl3_gemm_wide_store")
+    _lib.count()
+
+
 def exl3_gemm(xr: torch.Tensor, w: Exl3Weight, part: torch.Tensor, splits: int, status: torch.Tensor, force_generic: bool = False,
               work: "torch.Tensor | None" = None, flags: "torch.Tensor | None" = None) -> None:
     """part[s, row, n] = partial sums of xr @ W_q over split s.  xr: fp16 [rows, K] contiguous; part: fp32 >= splits*rows*N.  `work` (uint8, see

@@ -50,6 +50,7 @@ def _declare(lib):
         "rx_exl3_wide_takes": (c_int, [c_int, c_int, c_int, c_int]),
         "rx_exl3_wide_bytes": (c_ll, [c_int, c_int]),
         "rx_exl3_gemm_wide": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_void, c_void, c_ll, c_void, c_void]),
+        "rx_exl3_gemm_wide_store": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_void, c_void, c_void, c_void, c_ll, c_void, c_void]),
         "rx_exl3_gemm_wide_swiglu": (c_int, [c_void, c_int, c_int, c_void, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_ll, c_void, c_void]),
         "rx_tp_bump_epoch": (c_int, [c_void, c_void]),
         "rx_tp_finish_rs": (c_int, [c_void, c_int, c_int, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_void]),

@@ -67,6 +67,23 @@ def test_wide_swiglu_has_the_bits_of_gemm_and_finish(rows, K, F, bias):
     assert torch.equal(a, b[:rows]) and bool(b[rows].isnan().all())
 
 
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("rows,K,N", [(1, 256, 128), (257, 384, 640), (2304, 512, 2176), (2100, 1152, 5120), (1184, 1024, 3840)])
+def test_wide_store_has_the_bits_of_gemm_and_finish(rows, K, N, bias):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    KK, w, x, work, st, g = _problem(rows, K, N, "mcg")
+    w.bias = torch.randn(N, device="cuda", generator=g) if bias else None
+    part, a = torch.empty(rows, N, device="cuda"), torch.full((rows, N), float("nan"), device="cuda")
+    b = torch.full((rows + 1, N), float("nan"), device="cuda")
+    KK.exl3_gemm(x, w, part, 1, st)
+    KK.finish_store(part, 1, rows, w, a)
+    for _ in range(2):
+        KK.exl3_gemm_store(x, w, b, work, st)
+        KK.check_status(st)
+        assert torch.equal(a, b[:rows]) and bool(b[rows].isnan().all())
+
+
 def test_prompt_slice_through_either_gemm_gives_the_same_logits():
     """A model whose slice of 1100 rows takes the wide kernel, against the same model without its workspace."""
     if not torch.cuda.is_available():
