@@ -541,16 +541,19 @@ class HybridGPU(DenseGPU):
             proj = self.rec_proj[li][:M] if rec else self.ssm_proj[:M * wp].view(M, wp)
             self._in_proj(xr_d, L["in_proj"], M, cls, "kda_in" if kda else "gdn_in", proj)
             out = self.ssm_out[:M * cfg.gdn_inner].view(M, cfg.gdn_inner)
-            K.gdn_mixer(proj, M, cfg.gdn_k_heads, cfg.gdn_v_heads, 128, row_seq, positions, seg_s, seg_l, nseg, L["conv_w"], L["conv_b"], L["dt_bias"],
-                        L["a_neg"], L["norm_w"], cfg.eps, self.conv_pool[li], self.ssm_pool[li], xbc, out, kda=kda, mode=mode, y32=self.ssm_y)
             xr_g = self.xr[:M * cfg.gdn_inner].view(M, cfg.gdn_inner)
-            K.norm_rot_in(out, None, cfg.eps, L["out_proj"].suh, xr_g)
+            K.gdn_mixer(proj, M, cfg.gdn_k_heads, cfg.gdn_v_heads, 128, row_seq, positions, seg_s, seg_l, nseg, L["conv_w"], L["conv_b"], L["dt_bias"],
+                        L["a_neg"], L["norm_w"], cfg.eps, self.conv_pool[li], self.ssm_pool[li], xbc, out, kda=kda, mode=mode, y32=self.ssm_y,
+                        rot=(L["out_proj"].suh, xr_g))
             return self._linear(xr_g, L["out_proj"], M, cls, "gdn_out")
         proj = self.rec_proj[li][:M] if rec else self.ssm_proj[:M * cfg.in_proj_width].view(M, cfg.in_proj_width)
         self._in_proj(xr_d, L["in_proj"], M, cls, "in_proj", proj)
         out = self.ssm_out[:M * cfg.d_inner].view(M, cfg.d_inner)
-        K.ssm_mixer(proj, M, cfg.ssm_heads, cfg.ssm_head_dim, cfg.ssm_groups, cfg.ssm_state, row_seq, positions, seg_s, seg_l, nseg, L["conv_w"], L["conv_b"],
-                    L["dt_bias"], L["a_neg"], L["d_skip"], L["norm_w"], cfg.eps, self.conv_pool[li], self.ssm_pool[li], xbc, self.ssm_y, out, mode=mode)
         xr_m = self.xr[:M * cfg.d_inner].view(M, cfg.d_inner)
-        K.norm_rot_in(out, None, cfg.eps, L["out_proj"].suh, xr_m)
+        rot = (L["out_proj"].suh, xr_m) if K.ssm_rotates(cfg.d_inner, cfg.ssm_groups) else None
+        K.ssm_mixer(proj, M, cfg.ssm_heads, cfg.ssm_head_dim, cfg.ssm_groups, cfg.ssm_state, row_seq, positions, seg_s, seg_l, nseg, L["conv_w"], L["conv_b"],
+                    L["dt_bias"], L["a_neg"], L["d_skip"], L["norm_w"], cfg.eps, self.conv_pool[li], self.ssm_pool[li], xbc, self.ssm_y, out, mode=mode,
+                    rot=rot)
+        if rot is None:
+            K.norm_rot_in(out, None, cfg.eps, L["out_proj"].suh, xr_m)
         return self._linear(xr_m, L["out_proj"], M, cls, "out_proj")

@@ -168,34 +168,48 @@ def norm_rot_in(x: torch.Tensor, norm_w, eps: float, suh: torch.Tensor, xr: torc
 SCAN_RECORD, SCAN_COMMIT, SCAN_FINAL = 1, 2, 3
 
 
+def _rot_ptrs(rot):
+    if rot is None:
+        return None, None
+    suh, xr = rot
+    assert suh.dtype == torch.float16 and xr.dtype == torch.float16 and xr.is_contiguous()
+    return suh.data_ptr(), xr.data_ptr()
+
+
+def ssm_rotates(d_inner: int, groups: int) -> bool:
+    return d_inner // groups % 128 == 0 and d_inner // groups <= 16384
+
+
 def ssm_mixer(proj: torch.Tensor, M: int, H: int, P: int, G: int, N: int, row_seq, positions, seg_start, seg_len, nseg: int, conv_w, conv_b, dt_bias,
-              a_neg, d_skip, norm_w, eps: float, conv_pool, ssm_pool, xbc, y, out, mode: int = SCAN_FINAL) -> None:
+              a_neg, d_skip, norm_w, eps: float, conv_pool, ssm_pool, xbc, y, out, mode: int = SCAN_FINAL, rot=None) -> None:
     """Mamba2 mixer between in_proj and out_proj: `proj` f32 [M, ldp] (z | x | B | C | dt | pad) -> `out` bf16 [M, H*P] (gated, normed);
     the conv and state pools of the rows' sequences advance.  seg_start / seg_len: device int32 segment table or None (found on the device).
     Three launches (conv, recurrence, gated norm).  mode: SCAN_FINAL = rows are final (outputs and pools written); SCAN_RECORD = a window
     whose rows may be rejected (pools only read; the caller keeps `proj` and `xbc` as the record); SCAN_COMMIT = the recurrence again over
-    the recorded rows of the segments given (seg_len = rows kept), pools written, one launch."""
+    the recorded rows of the segments given (seg_len = rows kept), pools written, one launch.  `rot` = (suh, xr): `norm_rot_in` of the rows
+    without a norm, fp16 to xr, in place of `out` (groups of whole 128-blocks, see `ssm_rotates`)."""
     L = _lib.load()
     assert proj.dtype == torch.float32 and proj.stride(-1) == 1 and out.dtype == torch.bfloat16
     _lib.check(L.rx_ssm_mixer(proj.data_ptr(), proj.stride(0), M, H, P, G, N, row_seq.data_ptr(), positions.data_ptr(), _lib.ptr(seg_start),
                               _lib.ptr(seg_len), nseg, conv_w.data_ptr(), conv_b.data_ptr(), dt_bias.data_ptr(), a_neg.data_ptr(), d_skip.data_ptr(),
                               norm_w.data_ptr(), eps, conv_pool.data_ptr(), ssm_pool.data_ptr(), xbc.data_ptr(), y.data_ptr(), out.data_ptr(),
-                              _lib.stream_ptr(), mode), "rx_ssm_mixer")
+                              _lib.stream_ptr(), mode, *_rot_ptrs(rot)), "rx_ssm_mixer")
     _lib.count(1 if mode == SCAN_COMMIT else 3)
 
 
 def gdn_mixer(proj: torch.Tensor, M: int, Hk: int, Hv: int, D: int, row_seq, positions, seg_start, seg_len, nseg: int, conv_w, conv_b, dt_bias, a_neg,
-              norm_w, eps: float, conv_pool, s_pool, xbc, out, kda: bool = False, mode: int = SCAN_FINAL, y32=None) -> None:
+              norm_w, eps: float, conv_pool, s_pool, xbc, out, kda: bool = False, mode: int = SCAN_FINAL, y32=None, rot=None) -> None:
     """Gated delta net mixer between in_proj and out_proj: `proj` f32 [M, ldp] (z | q | k | v | b | a | pad) -> `out` bf16 [M, Hv*D]
     (per-head normed and gated); the conv and state pools of the rows' sequences advance.  Two launches (conv; recurrence + norm).
     `kda`: per-key-channel decay (a and dt_bias have Hv*D entries) and a sigmoid output gate.  `mode` as in `ssm_mixer`.  `y32` (f32 scratch
-    of M * Hv * D values) with a segment table: the recurrence runs split over a head's value columns and the norm as its own launch (same bits)."""
+    of M * Hv * D values) with a segment table: the recurrence runs split over a head's value columns and the norm as its own launch (same bits).
+    `rot` as in `ssm_mixer`."""
     L = _lib.load()
     assert proj.dtype == torch.float32 and proj.stride(-1) == 1 and out.dtype == torch.bfloat16
     _lib.check(L.rx_gdn_mixer(proj.data_ptr(), proj.stride(0), M, Hk, Hv, D, row_seq.data_ptr(), positions.data_ptr(), _lib.ptr(seg_start),
                               _lib.ptr(seg_len), nseg, conv_w.data_ptr(), conv_b.data_ptr(), dt_bias.data_ptr(), a_neg.data_ptr(), norm_w.data_ptr(),
                               eps, conv_pool.data_ptr(), s_pool.data_ptr(), xbc.data_ptr(), out.data_ptr(), _lib.stream_ptr(), 1 if kda else 0,
-                              mode, _lib.ptr(y32)), "rx_gdn_mixer")
+                              mode, _lib.ptr(y32), *_rot_ptrs(rot)), "rx_gdn_mixer")
     split = seg_start is not None and y32 is not None
     _lib.count(1 if mode == SCAN_COMMIT else (3 if split else 2))
 
