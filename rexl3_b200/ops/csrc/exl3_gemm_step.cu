@@ -1,4 +1,4 @@
-// EXL3 4.0 bpw GEMM of decode windows of up to 64 rows (sm_100a): one persistent CTA per SM, each with an equal share of the weights.
+// EXL3 4.0 bpw GEMM of decode windows of up to 96 rows (sm_100a): one persistent CTA per SM, each with an equal share of the weights.
 //
 // Contract, decode and data path of exl3_gemm_tm.cu (weights decoded into tensor memory, part[split][row][n]), another schedule.  There a CTA has one (strip,
 // split) and two CTAs share an SM: 272 items on 296 places leave an SM in six half idle, 224 one in two.  Here the strips' chunks of 128 k stand in a row that is cut
@@ -10,6 +10,9 @@
 //
 // What bounds it: the decode's integer work (18 of the 20 weights a clock that its loop reaches alone) and 8 us that no weight is decoded in: the start, the last
 // MMAs, and CTAs that begin late because their SM's last one ended late.
+//
+// Up to 32 rows tensor memory holds two accumulators beside the six A stages.  More rows (TALL) have one, which 96 rows still leave room for: what its write-out
+// costs is kept short by giving each 16 rows of it to another decode group, and up to six chunks are decoded meanwhile.
 //
 // Warp roles: 0 weight producer, 1 TMEM owner + MMA issuer, 2 activation producer, then six decode groups of four warps; group g takes every sixth chunk and
 // writes out every sixth piece, after its first chunk of a later one.  Every wait is bounded.
@@ -23,17 +26,21 @@ constexpr int ST_CTAS = 148, ST_NG = 6, ST_ROLE_WARPS = 3, ST_THREADS = ST_ROLE_
 constexpr int ST_KCH = 128, ST_A_COLS = ST_KCH / 2;
 // Operand stages, A in tensor memory and B in shared memory.  Two chunks stand behind one pair of barriers: the MMA issuer's waits and commits, instructions that
 // have to win their issue slots from 24 busy decode warps, come once in 256 k.
-constexpr int ST_STAGES = ST_NG, ST_PAIRS = ST_STAGES / 2;
-constexpr int ST_RAW = 12, ST_RAW_BYTES = 8 * 8 * 128;
-constexpr int ST_ACC = 64;                         // columns of one of two accumulators
+// (TALL has one chunk behind a barrier: its last chunk of a piece must not wait for a chunk of the next one, which may wait for the accumulator.)
+constexpr int ST_STAGES = ST_NG;
+__host__ __device__ constexpr int st_per(bool tall) { return tall ? 1 : 2; }
+__host__ __device__ constexpr int st_raw(bool tall) { return tall ? 8 : 12; }
+constexpr int ST_RAW_BYTES = 8 * 8 * 128;
+constexpr int ST_ACC = 64;                         // columns of one of two accumulators; TALL: one of up to 96
+constexpr int ST_FLAT_ROWS = 32, ST_TALL_ROWS = 96;
 constexpr int ST_PIECES = 32;                      // of a share, at most
 constexpr int ST_OUT = 8;                          // barriers of finished pieces (a group asks for piece f when piece f - 6 is complete)
 static_assert(2 * ST_ACC + ST_STAGES * ST_A_COLS <= 512, "tensor memory");
-__host__ __device__ inline int st_smem_bytes(int brows) { return ST_STAGES * brows * 256 + ST_RAW * ST_RAW_BYTES + 512 + ST_PIECES * 16; }
+__host__ __device__ inline int st_smem_bytes(int brows, bool tall) { return ST_STAGES * brows * 256 + st_raw(tall) * ST_RAW_BYTES + 512 + ST_PIECES * 16; }
 
 struct StepArgs {
   float* part;
-  int* flags;                // [0]: CTAs begun, modulo ST_CTAS; [32 + 4 share + quarter]: accumulator handed on.  Zero between calls.
+  int* flags;                // [0]: CTAs begun, modulo ST_CTAS; [32 + 4 share + quarter], TALL [32 + 32 share + 8 quarter + 16-row block]: accumulator handed on.  Zero between calls.
   int* status;
   int rows, K, N, splits, brows;
 };
@@ -61,22 +68,24 @@ __device__ __forceinline__ int step_pieces(const StepArgs& a, int share, int lan
   return count;
 }
 
-template <int CB>
+template <int CB, bool TALL>
 __global__ void __launch_bounds__(ST_THREADS, 1)
 exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ StepArgs a) {
+  constexpr int PER = st_per(TALL), LOG = PER - 1, ST_BARS = ST_STAGES / PER, ST_RAW = st_raw(TALL);
+  const int nb = a.brows / 16;                                     // TALL: blocks of 16 rows, each written out by another group
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int b_half = a.brows * 128, b_stage = 2 * b_half;          // one [brows x 64] swizzled sub-tile
   uint8_t* b_base = smem;
   uint8_t* raw_base = smem + ST_STAGES * b_stage;
   int4* table = (int4*)(raw_base + ST_RAW * ST_RAW_BYTES);
-  uint64_t* full = (uint64_t*)(table + ST_PIECES);                 // [pairs of stages] eight decode warps and the copies of the activations
-  uint64_t* empty = full + ST_PAIRS;                               // [pairs] commit
-  uint64_t* raw_full = empty + ST_PAIRS;                           // [RAW] weight producer
+  uint64_t* full = (uint64_t*)(table + ST_PIECES);                 // [PER stages each] their decode warps and the copies of the activations
+  uint64_t* empty = full + ST_BARS;                                // commit
+  uint64_t* raw_full = empty + ST_BARS;                            // [RAW] weight producer
   uint64_t* raw_empty = raw_full + ST_RAW;                         // [RAW] four decode warps
   uint64_t* acc_full = raw_empty + ST_RAW;                         // [8] commit
-  uint64_t* acc_empty = acc_full + ST_OUT;                         // [2] four decode warps
-  uint64_t* acc_taken = acc_empty + 2;                             // four decode warps
+  uint64_t* acc_empty = acc_full + ST_OUT;                         // [2] the decode warps that write out
+  uint64_t* acc_taken = acc_empty + 2;                             // the decode warps that take in
   uint64_t* drained = acc_taken + 1;                               // every MMA of this CTA has completed
   uint32_t* tmem_slot = (uint32_t*)(drained + 1);
   volatile int* share_slot = (volatile int*)(tmem_slot + 1);       // [3]: share, pieces, chunks
@@ -86,11 +95,11 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < ST_PAIRS; ++i) { mbar_init(&full[i], 9); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < ST_BARS; ++i) { mbar_init(&full[i], 4 * PER + 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < ST_RAW; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
     for (int i = 0; i < ST_OUT; ++i) mbar_init(&acc_full[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], 4);
-    mbar_init(acc_taken, 4);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], TALL ? 4 * nb : 4);
+    mbar_init(acc_taken, TALL ? 4 * nb : 4);
     mbar_init(drained, 1);
     *abort_flag = *last_flag = 0;
     n_sent[0] = n_sent[1] = 0;
@@ -150,10 +159,10 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         const StepPiece p = piece(f);
         for (int c = 0; c < p.n; ++c, ++gc) {
           const int s = gc % ST_STAGES, x = (p.c0 + c) * ST_KCH;
-          uint64_t* bar = &full[s >> 1];
-          if ((gc & 1) == 0) {
-            if (gc >= ST_STAGES && !(ok = mbar_wait(&empty[s >> 1], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 171, 100))) break;
-            mbar_arrive_expect_tx(bar, (uint32_t)b_stage * (gc + 1 < total ? 2 : 1));
+          uint64_t* bar = &full[s >> LOG];
+          if ((gc & (PER - 1)) == 0) {
+            if (gc >= ST_STAGES && !(ok = mbar_wait(&empty[s >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 171, 100))) break;
+            mbar_arrive_expect_tx(bar, (uint32_t)b_stage * (PER == 2 && gc + 1 < total ? 2 : 1));
           }
           tma_load_2d(b_base + s * b_stage, &tmap_x, x, 0, bar);
           tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + 64, 0, bar);
@@ -171,22 +180,23 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       bool ok = true;
       StepPiece p = piece(0);
       uint32_t acc = 0, accumulate = 0;
-      for (int gc = 0; gc < total; gc += 2) {
+      for (int gc = 0; gc < total; gc += PER) {
         if (!(ok = mbar_wait(&full[ps], parity, abort_flag, a.status, 173))) break;
         tc_fence_after();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 1 && gc + 1 >= total) break;
+        for (int h = 0; h < PER; ++h) {
+          if (PER == 2 && h == 1 && gc + 1 >= total) break;
           if (c == 0) {
             if (p.take) ok = mbar_wait(acc_taken, 0, abort_flag, a.status, 174);
-            if (ok && f >= 2) ok = mbar_wait(&acc_empty[f & 1], ((f >> 1) - 1) & 1, abort_flag, a.status, 172);
+            if (TALL && ok && f >= 1) ok = mbar_wait(&acc_empty[0], (f - 1) & 1, abort_flag, a.status, 172);
+            if (!TALL && ok && f >= 2) ok = mbar_wait(&acc_empty[f & 1], ((f >> 1) - 1) & 1, abort_flag, a.status, 172);
             if (!ok) break;
             tc_fence_after();
-            acc = tmem_base + (f & 1) * ST_ACC;
+            acc = tmem_base + (TALL ? 0 : (f & 1) * ST_ACC);
             accumulate = p.take;
           }
-          const uint64_t bd = desc0 + (uint64_t)((2 * ps + h) * stage_units);
-          const uint32_t at = a_tmem0 + (2 * ps + h) * ST_A_COLS;
+          const uint64_t bd = desc0 + (uint64_t)((PER * ps + h) * stage_units);
+          const uint32_t at = a_tmem0 + (PER * ps + h) * ST_A_COLS;
 #pragma unroll
           for (int k = 0; k < ST_KCH / 16; ++k)
             tc_mma_f16_ts(acc, at + k * 8, bd + (uint64_t)((k >> 2) * half_units + (k & 3) * 2), idesc, k == 0 ? accumulate : 1u);
@@ -199,7 +209,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         }
         if (!ok) break;
         tc_commit(&empty[ps]);
-        if (++ps == ST_PAIRS) ps = 0, parity ^= 1;
+        if (++ps == ST_BARS) ps = 0, parity ^= 1;
       }
       tc_commit(drained);
     }
@@ -212,21 +222,22 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t my_words = (uint32_t)((n >> 4) * 8 + (n & 7)) * 16u;
     const int share = *share_slot;
-    int* flag_out = a.flags + 32 + share * 4 + q;
+    constexpr int FLAGS = TALL ? 32 : 4;          // of a share: a quarter's blocks of 16 rows, or all rows
+    int* flag_out = a.flags + 32 + share * FLAGS + q * (FLAGS / 4);
     bool ok = true, waited = false;
     auto kernel_before = [&]() {                  // `part` and the flags may be in use until it has ended
       if (!waited) pdl_wait();
       waited = true;
     };
     auto place = [&](const StepPiece& o) { return a.part + ((size_t)o.split * a.rows) * a.N + o.strip * 128 + n; };
-    // piece f has had its last MMA: its accumulator goes to its place
-    auto write_out = [&](const StepPiece& o, int f) {
+    // piece f has had its last MMA: its accumulator (TALL: block b of it) goes to its place
+    auto write_out = [&](const StepPiece& o, int f, int b) {
       kernel_before();
       tc_fence_after();
       float* out = place(o);
-      for (int cb = 0; cb < a.rows; cb += 16) {
+      for (int cb = 16 * b; cb < (TALL ? 16 * b + 1 : a.rows); cb += 16) {
         uint32_t r[16];
-        tc_ld_32x32b_x16(tmem_base + (f & 1) * ST_ACC + lane_addr + cb, r);
+        tc_ld_32x32b_x16(tmem_base + (TALL ? 0 : (f & 1) * ST_ACC) + lane_addr + cb, r);
         tc_wait_ld();
 #pragma unroll
         for (int i = 0; i < 16; ++i)
@@ -236,38 +247,46 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       if (o.hand) __threadfence();
       __syncwarp();
       if (lane == 0) {
-        if (o.hand) atomicExch(flag_out, 1);
-        mbar_arrive(&acc_empty[f & 1]);
+        if (o.hand) atomicExch(flag_out + b, 1);
+        mbar_arrive(&acc_empty[TALL ? 0 : f & 1]);
       }
     };
-    // The accumulator of the last piece f, as the CTA before left it.  The group that writes out piece f - 2, whose place it takes, brings it in: a wait of another
-    // group could miss two phases of that buffer's barrier.
-    auto take_in = [&](const StepPiece& o, int f) {
+    // The accumulator of the last piece f, as the CTA before left it.  The group that writes out piece f - 2 (TALL: block b of piece f - 1), whose place it takes,
+    // brings it in: a wait of another group could miss two phases of that buffer's barrier.
+    auto take_in = [&](const StepPiece& o, int f, int b) {
       kernel_before();
-      if (!__all_sync(0xffffffffu, wait_count(flag_out - 4, 1, abort_flag, a.status, 178))) return false;
+      if (!__all_sync(0xffffffffu, wait_count(flag_out - FLAGS + b, 1, abort_flag, a.status, 178))) return false;
       const float* in = place(o);
-      for (int cb = 0; cb < a.rows; cb += 16) {
+      for (int cb = 16 * b; cb < (TALL ? 16 * b + 1 : a.rows); cb += 16) {
         uint32_t r[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) r[i] = cb + i < a.rows ? __float_as_uint(__ldcg(in + (size_t)(cb + i) * a.N)) : 0u;
-        tc_st_32x32b_x16(tmem_base + (f & 1) * ST_ACC + lane_addr + cb, r);
+        tc_st_32x32b_x16(tmem_base + (TALL ? 0 : (f & 1) * ST_ACC) + lane_addr + cb, r);
       }
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        atomicExch(flag_out - 4, 0);
+        atomicExch(flag_out - FLAGS + b, 0);
         mbar_arrive(acc_taken);
       }
       return true;
     };
-    int next_out = grp, f = 0;                    // the next piece that this group writes out; the piece it is in
+    int next_out = TALL ? 0 : grp, f = 0;         // the next piece that this group writes out (TALL: or looks at); the piece it is in
+    // TALL: the block of piece f that this group writes out; nb and more: none.  Over the pieces the blocks go round the groups.
+    auto block_of = [&](int f) { return (int)((unsigned)(grp + ST_NG * ST_PIECES - f * nb) % (unsigned)ST_NG); };
     // Writes out this group's pieces before piece `end`.  (Left for later when the last MMA is still to come, a group could wait for an operand stage whose MMA
     // waits for that very accumulator.)
     auto write_before = [&](int end) {
-      for (; ok && next_out < end; next_out += ST_NG) {
+      for (; ok && next_out < end; next_out += TALL ? 1 : ST_NG) {
+        const int b = TALL ? block_of(next_out) : 0;
+        if (TALL && b >= nb) continue;
         ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[next_out % ST_OUT], (next_out / ST_OUT) & 1, abort_flag, a.status, 176));
-        if (ok) write_out(piece(next_out), next_out);
+        if (ok) write_out(piece(next_out), next_out, b);
+        if (TALL && ok && next_out + 1 < pieces) {
+          const StepPiece p = piece(next_out + 1);
+          if (p.take) ok = take_in(p, next_out + 1, b);
+        }
       }
     };
     int gc0 = 0;                                  // chunks up to the end of piece f
@@ -275,9 +294,11 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       const StepPiece p = piece(f);
       gc0 += p.n;
       // (not before: the CTA before may still be at it)
-      if (p.take && grp == (f < 2 ? f : (f - 2) % ST_NG)) {
+      if (TALL) {
+        if (p.take && f == 0 && grp < nb) ok = take_in(p, 0, grp);
+      } else if (p.take && grp == (f < 2 ? f : (f - 2) % ST_NG)) {
         write_before(f - 1);
-        if (ok) ok = take_in(p, f);
+        if (ok) ok = take_in(p, f, 0);
       }
       for (; gc < gc0 && ok; gc += ST_NG) {
         const int rs = gc % ST_RAW, os = gc % ST_STAGES;
@@ -308,7 +329,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             }
           }
           if (qt == 0) {
-            if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty[os >> 1], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 180));
+            if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty[os >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 180));
             if (!ok) break;
             tc_fence_after();
           }
@@ -318,14 +339,14 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full[os >> 1]);
+        if (lane == 0) mbar_arrive(&full[os >> LOG]);
         write_before(f);
       }
-      if (f == pieces - 1 && gc == total && (total & 1) != 0 && ok) {
+      if (PER == 2 && f == pieces - 1 && gc == total && (total & 1) != 0 && ok) {
         // the last pair has one chunk: the arrivals of the other
         const int os = gc % ST_STAGES;
-        if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty[os >> 1], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 180));
-        if (ok && lane == 0) mbar_arrive(&full[os >> 1]);
+        if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty[os >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 180));
+        if (ok && lane == 0) mbar_arrive(&full[os >> LOG]);
       }
     }
     write_before(f);
@@ -347,16 +368,16 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
 int make_tmap_f16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 int make_tmap_trellis(CUtensorMap* out, const void* base, uint64_t kt_rows, uint64_t row_words, uint32_t box_words, uint32_t box_rows);
 
-template <int CB>
+template <int CB, bool TALL>
 static int launch_step(const CUtensorMap& tx, const CUtensorMap& tw, const StepArgs& a, cudaStream_t st) {
-  auto kern = exl3_gemm_step_kernel<CB>;
+  auto kern = exl3_gemm_step_kernel<CB, TALL>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  int smem = st_smem_bytes(a.brows) + 1024;
+  int smem = st_smem_bytes(a.brows, TALL) + 1024;
   if (smem < 120 * 1024) smem = 120 * 1024;        // one CTA per SM: it allocates all 512 TMEM columns
   return (int)rx::launch(kern, dim3(ST_CTAS), dim3(ST_THREADS), smem, st, tx, tw, a);
 }
@@ -367,23 +388,30 @@ using namespace rx;
 
 RX_API int rx_exl3_tile_rows(int rows);
 
-RX_API int rx_exl3_step_flags() { return 32 + ST_CTAS * 4; }
+RX_API int rx_exl3_step_flags() { return 32 + ST_CTAS * 32; }
 
 // At least one item for every CTA, no more pieces than the table holds.
 static bool step_fits(int rows, int K, int N, int splits) {
-  if (rows < 1 || rows > 64 || K % ST_KCH != 0 || N % 128 != 0 || splits < 1 || splits > K / ST_KCH) return false;
+  if (rows < 1 || rows > ST_TALL_ROWS || K % ST_KCH != 0 || N % 128 != 0 || splits < 1 || splits > K / ST_KCH) return false;
   const long long items = (long long)(N / 128) * splits, chunks = (long long)(N / 128) * (K / ST_KCH);
   return items >= ST_CTAS && items / ST_CTAS + 3 <= ST_PIECES && chunks < (1 << 24);
 }
 
 // Whether the call below is faster than exl3_gemm_tm.cu: that one takes 0.527 us a chunk on the SMs with two items and 3 us, this one 0.48 us a chunk of an equal
 // share and 8.5 us (its start, and the spread of CTAs that wait for one another's accumulators).  One row, us: 4096 -> 28,672 36.1 and 30.6; 5120 ->
-// 32,768 44.9 and 41.2; 5120 -> 34,816 45.1 and 43.1; 17,408 -> 5120 in seven splits 23.6 and 25.0; 5120 -> 5120 in seven 9.1 and 13.2.  The write-outs of 33 rows and
-// more cost more than the shares gain.
+// 32,768 44.9 and 41.2; 5120 -> 34,816 45.1 and 43.1; 17,408 -> 5120 in seven splits 23.6 and 25.0; 5120 -> 5120 in seven 9.1 and 13.2.  From 33 to 64 rows
+// that one still has two CTAs to an SM and the gains are below 5 % (5120 -> 34,816 45.1 and 49.4; 4096 -> 28,672 36.3 and 34.8).
+// Verify windows of 65 to 96 rows, one CTA per SM either way: the persistent kernel of whole items (exl3_gemm_grouped.cu) takes 0.78 us a chunk of the CTAs with
+// most of them and 5 us, this one, with half as many decode warps more, 0.514 us a chunk of an equal share and 11.5 us.  80 rows, us: 5120 -> 34,816 65.0
+// and 49.4; 4096 -> 28,672 50.8 and 36.0; 5120 -> 151,936 283 and 221; 17,408 -> 5120 34.0 and 30.5; 5120 -> 8192 in four splits 21.2 and 19.9; 6144 -> 5120 in
+// seven 17.1 and 17.7; 5120 -> 5120 14.5 and 16.8.
 RX_API int rx_exl3_step_takes(int rows, int K, int N, int splits) {
-  if (!step_fits(rows, K, N, splits) || rows > 32 || (long long)(N / 128) * splits > 2 * ST_CTAS) return 0;
-  const int item = (K / ST_KCH + splits - 1) / splits;
-  return 2 * item * 0.527 + 3.0 > (N / 128) * (K / ST_KCH) / (double)ST_CTAS * 0.48 + (rows <= 16 ? 8.5 : 9.5);
+  if (!step_fits(rows, K, N, splits) || (rows > ST_FLAT_ROWS && rows <= 64)) return 0;
+  const int item = (K / ST_KCH + splits - 1) / splits, items = (N / 128) * splits;
+  const double share = (N / 128) * (K / ST_KCH) / (double)ST_CTAS;
+  if (rows > 64) return (items + ST_CTAS - 1) / ST_CTAS * item * 0.78 + 5.0 > share * 0.514 + 11.5;
+  if (items > 2 * ST_CTAS) return 0;
+  return 2 * item * 0.527 + 3.0 > share * 0.48 + (rows <= 16 ? 8.5 : 9.5);
 }
 
 // rx_exl3_gemm_b4 for decode windows; flags: int32 [rx_exl3_step_flags()], zero before the first call, one buffer for calls that may overlap.
@@ -393,15 +421,17 @@ RX_API int rx_exl3_gemm_step(const void* xr, int rows, int K, const void* trelli
   if ((((uintptr_t)xr) & 15) != 0 || (((uintptr_t)trellis) & 15) != 0) return (int)cudaErrorMisalignedAddress;
   StepArgs a = {};
   a.part = (float*)part, a.flags = (int*)flags, a.status = status;
-  a.rows = rows, a.K = K, a.N = N, a.splits = splits, a.brows = rx_exl3_tile_rows(rows);
+  a.rows = rows, a.K = K, a.N = N, a.splits = splits, a.brows = rows <= ST_FLAT_ROWS ? rx_exl3_tile_rows(rows) : (rows + 15) & ~15;
   CUtensorMap tx, tw;
   int e = make_tmap_f16_2d(&tx, xr, (uint64_t)rows, (uint64_t)K, (uint32_t)a.brows);
   if (e == 0) e = make_tmap_trellis(&tw, trellis, (uint64_t)(K / 16), (uint64_t)(N / 16) * 32, 256, 8);
   if (e != 0) return e;
+#define RX_STEP(CBV) (rows <= ST_FLAT_ROWS ? launch_step<CBV, false>(tx, tw, a, (cudaStream_t)stream) : launch_step<CBV, true>(tx, tw, a, (cudaStream_t)stream))
   switch (codebook) {
-    case CB_3INST: return launch_step<CB_3INST>(tx, tw, a, (cudaStream_t)stream);
-    case CB_MCG: return launch_step<CB_MCG>(tx, tw, a, (cudaStream_t)stream);
-    case CB_MUL1: return launch_step<CB_MUL1>(tx, tw, a, (cudaStream_t)stream);
+    case CB_3INST: return RX_STEP(CB_3INST);
+    case CB_MCG: return RX_STEP(CB_MCG);
+    case CB_MUL1: return RX_STEP(CB_MUL1);
     default: return (int)cudaErrorInvalidValue;
   }
+#undef RX_STEP
 }
