@@ -124,6 +124,29 @@ __global__ void __launch_bounds__(1024) norm_rot_in_kernel(const uint16_t* __res
   }
 }
 
+// The plain rotation of many rows: eight lanes to a 128-block.  x and xr of [rows * nb] blocks, suh of nb.
+__global__ void __launch_bounds__(256) rot_in_rows_kernel(const uint16_t* __restrict__ x, const __half* __restrict__ suh, __half* __restrict__ xr, long long blocks,
+                                                          int nb) {
+  pdl_launch();
+  pdl_wait();
+  const long long at = ((long long)blockIdx.x * 256 + threadIdx.x) >> 3, item = min(at, blocks - 1);
+  const int l4 = (threadIdx.x & 7) * 4, n0 = (int)(item % nb) * 128 + l4;
+  float v[4][4], s[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    load4_bf16(x + item * 128 + l4 + 32 * j, v[j]);
+    load4_f16(suh + n0 + 32 * j, s[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[j][e] *= s[j][e];        // exact: 8 and 11 bits
+  fwht128_oct(v);
+  if (at >= blocks) return;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) store4_f16(xr + item * 128 + l4 + 32 * j, v[j]);
+}
+
 // ------------------------------------------------------------------------------------------------ finish kernels
 // y[row][n] = H_N( sum_s part[s][row][:] )[n] * svh[n] + bias[n] for one 128-block, lane holds 4 consecutive n.
 // ONE: a single plane, known at compile time.  The loop over planes keeps eight loads in registers; a kernel that carries it for nothing holds a
@@ -301,50 +324,58 @@ __global__ void __cluster_dims__(FEW_CTAS, 1, 1) __launch_bounds__(FEW_WARPS * 3
   store4_f16(xr + (size_t)row * N + n0, v);
 }
 
-// The same for the many rows of a prompt slice (one plane, rows of up to ROWS_NB * 1024 elements), bound by memory: a CTA of eight warps per row, a warp's
-// blocks (one in eight) stay in registers between the sum of squares and the scaling, all of them loaded before the first is used.
-// 8192 rows of 5120: 125 us, 165 before (blocks one after the other, the row through shared memory).
-constexpr int ROWS_NB = 5;
-__global__ void __launch_bounds__(256) finish_add_norm_rot_rows_kernel(const float* __restrict__ part, int N, const __half* __restrict__ svh,
+// The same for the many rows of a prompt slice (one plane, rows of up to ROWS_MAX elements): a CTA per row, eight lanes to a 128-block and ROWS_NB blocks to a
+// lane, which stay in registers between the sum of squares and the scaling, all of them loaded before the first is used.  By warps, a block each, it was
+// bound by the shuffles of its two transforms: 8192 rows of 5120 122 us, 96 now; 900 rows of 4096 24.6 -> 16.4.
+constexpr int ROWS_NB = 2, ROWS_MAX = 5120;
+__global__ void __launch_bounds__(ROWS_MAX / 16 / ROWS_NB) finish_add_norm_rot_rows_kernel(const float* __restrict__ part, int N, const __half* __restrict__ svh,
                                                                       const float* __restrict__ bias, uint16_t* __restrict__ h,
                                                                       const uint16_t* __restrict__ norm_w, float eps, const __half* __restrict__ suh_next,
                                                                       __half* __restrict__ xr, uint16_t* __restrict__ xn_out) {
   pdl_launch();
   pdl_wait();
-  __shared__ float blk_ss[8 * ROWS_NB];
-  const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = N / 128;
-  const size_t base = (size_t)row * N + lane * 4;
-  float v[ROWS_NB][4], r[ROWS_NB][4];
+  __shared__ float blk_ss[ROWS_MAX / 128];
+  const int row = blockIdx.x, nb = N / 128, groups = blockDim.x / 8, grp = threadIdx.x >> 3, l4 = (threadIdx.x & 7) * 4;
+  const size_t base = (size_t)row * N + l4;
+  float v[ROWS_NB][4][4], r[ROWS_NB][4][4];
 #pragma unroll
   for (int i = 0; i < ROWS_NB; ++i) {
-    const int b = warp + 8 * i;
-    if (b < nb) {
-      const float4 p = __ldg(reinterpret_cast<const float4*>(part + base + b * 128));
-      v[i][0] = p.x, v[i][1] = p.y, v[i][2] = p.z, v[i][3] = p.w;
-      load4_bf16(h + base + b * 128, r[i]);
+    const int b = min(grp + groups * i, nb - 1);          // (past the end the last block again: nothing of it is stored)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 p = __ldg(reinterpret_cast<const float4*>(part + base + b * 128 + 32 * j));
+      v[i][j][0] = p.x, v[i][j][1] = p.y, v[i][j][2] = p.z, v[i][j][3] = p.w;
+      load4_bf16(h + base + b * 128 + 32 * j, r[i][j]);
     }
   }
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < ROWS_NB; ++i) {
-    const int b = warp + 8 * i, n0 = b * 128 + lane * 4;
-    if (b >= nb) break;
-    fwht128_warp(v[i]);
-    float sv[4], ss = 0.f;
-    load4_f16(svh + n0, sv);
+    const int b = grp + groups * i, n0 = min(b, nb - 1) * 128 + l4;
+    fwht128_oct(v[i]);
+    float ss[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[i][e] = __fmul_rn(v[i][e], sv[e]);
-    if (bias != nullptr) {
-      const float4 bb = *reinterpret_cast<const float4*>(bias + n0);
-      v[i][0] += bb.x, v[i][1] += bb.y, v[i][2] += bb.z, v[i][3] += bb.w;
-    }
+    for (int j = 0; j < 4; ++j) {
+      float sv[4];
+      load4_f16(svh + n0 + 32 * j, sv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      v[i][e] = bf16_to_f(f_to_bf16(r[i][e] + v[i][e]));
-      ss = __fmaf_rn(v[i][e], v[i][e], ss);
+      for (int e = 0; e < 4; ++e) v[i][j][e] = __fmul_rn(v[i][j][e], sv[e]);
+      if (bias != nullptr) {
+        const float4 bb = *reinterpret_cast<const float4*>(bias + n0 + 32 * j);
+        v[i][j][0] += bb.x, v[i][j][1] += bb.y, v[i][j][2] += bb.z, v[i][j][3] += bb.w;
+      }
+      ss[j] = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[i][j][e] = bf16_to_f(f_to_bf16(r[i][j][e] + v[i][j][e]));
+        ss[j] = __fmaf_rn(v[i][j][e], v[i][j][e], ss[j]);
+      }
+      if (b < nb) store4_bf16(h + base + b * 128 + 32 * j, v[i][j]);
     }
-    store4_bf16(h + base + b * 128, v[i]);
-    ss = warp_sum(ss);
-    if (lane == 0) blk_ss[b] = ss;
+    float sum = (ss[0] + ss[2]) + (ss[1] + ss[3]);         // warp_sum's order over the 32 fours of a block
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (l4 == 0 && b < nb) blk_ss[b] = sum;
   }
   if (suh_next == nullptr && xn_out == nullptr) return;
   float rinv = 1.f;
@@ -356,22 +387,29 @@ __global__ void __launch_bounds__(256) finish_add_norm_rot_rows_kernel(const flo
   }
 #pragma unroll
   for (int i = 0; i < ROWS_NB; ++i) {
-    const int b = warp + 8 * i, n0 = b * 128 + lane * 4;
-    if (b >= nb) break;
-    if (norm_w != nullptr) {
-      float w[4];
-      load4_bf16(norm_w + n0, w);
+    const int b = grp + groups * i, n0 = min(b, nb - 1) * 128 + l4;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[i][e] = __fmul_rn(bf16_to_f(f_to_bf16(v[i][e] * rinv)), w[e]);
+    for (int j = 0; j < 4; ++j) {
+      if (norm_w != nullptr) {
+        float w[4];
+        load4_bf16(norm_w + n0 + 32 * j, w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[i][j][e] = __fmul_rn(bf16_to_f(f_to_bf16(v[i][j][e] * rinv)), w[e]);
+      }
+      if (xn_out != nullptr && b < nb) store4_bf16(xn_out + base + b * 128 + 32 * j, v[i][j]);
     }
-    if (xn_out != nullptr) store4_bf16(xn_out + base + b * 128, v[i]);
     if (suh_next == nullptr) continue;
-    float s[4];
-    load4_f16(suh_next + n0, s);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[i][e] *= s[e];
-    fwht128_warp(v[i]);
-    store4_f16(xr + base + b * 128, v[i]);
+    for (int j = 0; j < 4; ++j) {
+      float s[4];
+      load4_f16(suh_next + n0 + 32 * j, s);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[i][j][e] *= s[e];
+    }
+    fwht128_oct(v[i]);
+    if (b < nb)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) store4_f16(xr + base + b * 128 + 32 * j, v[i][j]);
   }
 }
 
@@ -426,8 +464,17 @@ RX_API int rx_embed(const void* ids, const void* table, void* h, int rows, int d
   return (int)cudaGetLastError();
 }
 
+// Eight lanes a block from 8192 blocks on (8192 rows of 8192 67.6 -> 57.3 us, 300 rows of 4096 9.1 -> 8.2, 128 of 8192 level); a few rows are level or, 128 of 2048,
+// 0.8 us slower.
+constexpr long long ROT_ROWS_MIN = 8192;
 RX_API int rx_norm_rot_in(const void* x_bf16, const void* norm_w_bf16, float eps, const void* suh, void* xr, int rows, int K, void* stream) {
   if (K % 128 || K / 128 > 512) return (int)cudaErrorInvalidValue;
+  const long long blocks = (long long)rows * (K / 128);
+  if (norm_w_bf16 == nullptr && blocks >= ROT_ROWS_MIN) {
+    rx::launch(rot_in_rows_kernel, dim3((unsigned)((blocks + 31) / 32)), dim3(256), 0, (cudaStream_t)stream, (const uint16_t*)x_bf16, (const __half*)suh, (__half*)xr,
+               blocks, K / 128);
+    return (int)cudaGetLastError();
+  }
   rx::launch(norm_rot_in_kernel, dim3(rows), dim3(rows >= 512 ? 256 : 1024), 0, (cudaStream_t)stream, (const uint16_t*)x_bf16, (const uint16_t*)norm_w_bf16, eps, (const __half*)suh,
                                                             (__half*)xr, K);
   return (int)cudaGetLastError();
@@ -455,11 +502,10 @@ RX_API int rx_finish_store(const void* part, int S, int M, int N, const void* sv
 RX_API int rx_finish_add_norm_rot(const void* part, int S, int M, int N, const void* svh, const void* bias, void* h_bf16, const void* norm_w,
                                   float eps, const void* suh_next, void* xr, void* stream, void* xn_out) {
   if (N % 128 || N * 4 > 200 * 1024 || N / 128 > 512) return (int)cudaErrorInvalidValue;
-  // Up to 592 rows the form below is two waves of two 32-warp CTAs per SM at most and the faster one (592 rows of 5120: 10.8 us, 13.9 by the row form; 593
-  // rows 14.4 and 13.9, 1500 rows 25.4 and 23.4); for shorter rows, of which an SM holds more, longer (1184 rows of 2048 9.3 and 10.1, 2100
-  // level, 8192 66.5 and 61.9; rows of 1024 always).
-  if (S == 1 && N > 1024 && N <= ROWS_NB * 1024 && M > (N >= 3072 ? 592 : 2048)) {
-    rx::launch(finish_add_norm_rot_rows_kernel, dim3(M), dim3(256), 0, (cudaStream_t)stream, (const float*)part, N, (const __half*)svh, (const float*)bias,
+  // More rows than SMs: 150 rows of 5120 16.3 us by the form below, 12.3 by the row form; 150 of 4096, 3072 or 2048 level, 300 16.4 and 12.3, 14.3 and 12.3, 14.3 and
+  // 12.3; 74 rows 9.1 and 12.2.  (Just below 592 short rows are 2 us faster below: two whole waves of its CTAs.)
+  if (S == 1 && N > 1024 && N <= ROWS_MAX && M > 148) {
+    rx::launch(finish_add_norm_rot_rows_kernel, dim3(M), dim3((N / 128 + 4 * ROWS_NB - 1) / (4 * ROWS_NB) * 32), 0, (cudaStream_t)stream, (const float*)part, N, (const __half*)svh, (const float*)bias,
                (uint16_t*)h_bf16, (const uint16_t*)norm_w, eps, (const __half*)suh_next, (__half*)xr, (uint16_t*)xn_out);
     return (int)cudaGetLastError();
   }

@@ -396,34 +396,6 @@ __global__ void moe_gather_rot_kernel(const uint16_t* __restrict__ x, const int*
   }
 }
 
-// The 128-point transform of fwht128_warp by eight lanes: element j * 32 + (lane & 7) * 4 + i of the block is v[j][i].  The strides come in the same order
-// (1, 2 in the lane, 4, 8, 16 across lanes, 32, 64 in the lane), so the sums are the same to the bit; a block costs 12 shuffles of a warp, not 20, and a lane
-// has four times the loads in flight.
-__device__ __forceinline__ void fwht128_oct(float (&v)[4][4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float a0 = v[j][0] + v[j][1], a1 = v[j][0] - v[j][1], a2 = v[j][2] + v[j][3], a3 = v[j][2] - v[j][3];
-    v[j][0] = a0 + a2; v[j][1] = a1 + a3; v[j][2] = a0 - a2; v[j][3] = a1 - a3;
-  }
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    const float sgn = (lane & o) ? -1.f : 1.f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float other = __shfl_xor_sync(0xffffffffu, v[j][i], o);
-        v[j][i] = fmaf(sgn, v[j][i], other);
-      }
-  }
-  const float s = 0.08838834764831845f;  // 1/sqrt(128)
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float a0 = v[0][i] + v[1][i], a1 = v[0][i] - v[1][i], a2 = v[2][i] + v[3][i], a3 = v[2][i] - v[3][i];
-    v[0][i] = (a0 + a2) * s; v[1][i] = (a1 + a3) * s; v[2][i] = (a0 - a2) * s; v[3][i] = (a1 - a3) * s;
-  }
-}
 __device__ __forceinline__ void moe_half4(const uint2 u, float (&f)[4]) {
   const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
