@@ -162,6 +162,108 @@ __global__ void __launch_bounds__(256) finish_qkv_rope_kernel(const float* __res
   }
 }
 
+// The same for the many rows of a prompt slice with heads of 128, one plane and a bf16 cache: a CTA per row, eight lanes to a block and two blocks of a lane in
+// flight.  An element's partner in the rotation is in the same lane, a transform costs 12 shuffles and not 20.  The sums run in the other form's order.
+__global__ void __launch_bounds__(160, 4) finish_qkv_rope_rows_kernel(const float* __restrict__ part, int n_q, int n_kv, const __half* __restrict__ svh,
+                                       const float* __restrict__ bias, const uint16_t* __restrict__ q_norm, const uint16_t* __restrict__ k_norm,
+                                       float eps, const int* __restrict__ positions, const float* __restrict__ inv_freq,
+                                       const int* __restrict__ slot, uint16_t* __restrict__ q_out, uint16_t* __restrict__ k_cache,
+                                       uint16_t* __restrict__ v_cache, const int* __restrict__ pos3, int lim_h, int lim_w) {
+  pdl_launch();
+  pdl_wait();
+  constexpr int HD = 128, NB = 2;
+  const int row = blockIdx.x, nb = n_q + 2 * n_kv, groups = blockDim.x / 8, grp = threadIdx.x >> 3, l4 = (threadIdx.x & 7) * 4;
+  const float* src = part + (size_t)row * nb * HD + l4;
+  float y[NB][4][4];
+  auto load = [&](int c) {
+#pragma unroll
+    for (int t = 0; t < NB; ++t) {
+      const int b = min(c + grp + t * groups, nb - 1);         // (past the end the last block again: nothing of it is stored)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 p = __ldg(reinterpret_cast<const float4*>(src + (size_t)b * HD + 32 * j));
+        y[t][j][0] = p.x, y[t][j][1] = p.y, y[t][j][2] = p.z, y[t][j][3] = p.w;
+      }
+    }
+  };
+  load(0);
+  const int sl = slot[row];
+  __shared__ float2 rot[HD / 2];
+  for (int fi = threadIdx.x; fi < HD / 2; fi += blockDim.x) {
+    float p = (float)positions[row];
+    if (pos3 != nullptr) {
+      const int axis = (fi % 3 == 1 && fi < lim_h) ? 1 : ((fi % 3 == 2 && fi < lim_w) ? 2 : 0);
+      p = (float)pos3[row * 3 + axis];
+    }
+    float sn, cs;
+    sincosf(p * inv_freq[fi], &sn, &cs);
+    rot[fi] = make_float2(sn, cs);
+  }
+  __syncthreads();
+  float2 sc[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sc[j][i] = rot[32 * j + l4 + i];
+  for (int c = 0; c < nb; c += NB * groups) {
+    if (c > 0) load(c);
+#pragma unroll
+    for (int t = 0; t < NB; ++t) {
+      const int b = c + grp + t * groups, head = min(b, nb - 1), n0 = head * HD + l4;
+      fwht128_oct(y[t]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint2 su = *reinterpret_cast<const uint2*>(svh + n0 + 32 * j);
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&su.x)), d = __half22float2(*reinterpret_cast<const __half2*>(&su.y));
+        y[t][j][0] *= a.x; y[t][j][1] *= a.y; y[t][j][2] *= d.x; y[t][j][3] *= d.y;
+        if (bias != nullptr) {
+          const float4 bb = *reinterpret_cast<const float4*>(bias + n0 + 32 * j);
+          y[t][j][0] += bb.x; y[t][j][1] += bb.y; y[t][j][2] += bb.z; y[t][j][3] += bb.w;
+        }
+      }
+      const bool is_q = head < n_q, is_k = !is_q && head < n_q + n_kv;
+      if (q_norm != nullptr || k_norm != nullptr) {
+        float ss[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float* v = y[t][j];
+          ss[j] = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+#pragma unroll
+          for (int o = 1; o < 8; o <<= 1) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], o);
+        }
+        const uint16_t* nw_ptr = is_q ? q_norm : is_k ? k_norm : nullptr;
+        if (nw_ptr != nullptr) {
+          const float rinv = rsqrtf(((ss[0] + ss[1]) + (ss[2] + ss[3])) / (float)HD + eps);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[t][j][i] = y[t][j][i] * rinv * g_bf16_to_f(nw_ptr[32 * j + l4 + i]);
+        }
+      }
+      if (is_q || is_k) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float sn = sc[j][i].x, cs = sc[j][i].y, lo = y[t][j][i], hi = y[t][j + 2][i];
+            y[t][j][i] = lo * cs - hi * sn;
+            y[t][j + 2][i] = hi * cs + lo * sn;
+          }
+      }
+      if (b >= nb || (!is_q && sl < 0)) continue;
+      uint16_t* out = is_q ? q_out + ((size_t)row * n_q + head) * HD
+                           : (is_k ? k_cache : v_cache) + (((size_t)(sl / 64) * n_kv + (is_k ? head - n_q : head - n_q - n_kv)) * 64 + (sl % 64)) * HD;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint2 u;
+        u.x = (uint32_t)g_f_to_bf16(y[t][j][0]) | ((uint32_t)g_f_to_bf16(y[t][j][1]) << 16);
+        u.y = (uint32_t)g_f_to_bf16(y[t][j][2]) | ((uint32_t)g_f_to_bf16(y[t][j][3]) << 16);
+        *reinterpret_cast<uint2*>(out + 32 * j + l4) = u;
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ exact top-k
 // key = (order-preserving bits of the float) << 32 | ~id : bigger key = bigger value, then lower id.
 __device__ __forceinline__ uint64_t topk_key(float v, uint32_t id) {
@@ -299,6 +401,9 @@ __global__ void __launch_bounds__(TOPK_THREADS) topk_stage2_kernel(const uint64_
 
 using namespace rx;
 
+// Rows for the form of eight lanes a block: 40 heads and 8 of K and V, 600 rows 18.4 -> 15.2 us, 2100 38.9 -> 33.6, 8192 111.6 -> 92.2; 300 rows 13.1 and 16.3 (in CTAs of
+// 224 threads), 64 rows 8.2 and 10.2.  CTAs of up to 160 threads: of 224, in one pass, an SM holds too few (8192 rows 118.8).
+constexpr int QKV_ROWS_MIN = 593;
 RX_API int rx_finish_qkv_rope(const void* part, int S, int M, int n_q, int n_kv, int hd, const void* svh, const void* bias, const void* q_norm,
                               const void* k_norm, float eps, const void* positions, const void* inv_freq, const void* slot, void* q_out,
                               void* k_cache, void* v_cache, void* stream, const void* kv_scale, void* kv_amax, const void* pos3, int section_h,
@@ -313,7 +418,12 @@ RX_API int rx_finish_qkv_rope(const void* part, int S, int M, int n_q, int n_kv,
 #define RX_ARGS (const float*)part, S, M, n_q, n_kv, (const __half*)svh, (const float*)bias, (const uint16_t*)q_norm, (const uint16_t*)k_norm, eps, \
                 (const int*)positions, (const float*)inv_freq, (const int*)slot, (uint16_t*)q_out, (uint16_t*)k_cache, (uint16_t*)v_cache, \
                 (const float*)kv_scale, (float*)kv_amax, (const int*)pos3, 3 * section_h, 3 * section_w, (float*)k_tscale, (float*)v_tscale, q4
-  if (hd == 128) rx::launch(S == 1 ? finish_qkv_rope_kernel<128, true> : finish_qkv_rope_kernel<128, false>, dim3(grid), dim3(256), 0, st, RX_ARGS);
+  if (hd == 128 && S == 1 && M >= QKV_ROWS_MIN && kv_scale == nullptr && kv_amax == nullptr && k_tscale == nullptr && n_q > 0) {
+    const int nb = n_q + 2 * n_kv, passes = (nb + 39) / 40, threads = (nb + 8 * passes - 1) / (8 * passes) * 32;
+    rx::launch(finish_qkv_rope_rows_kernel, dim3(M), dim3(threads), 0, st, (const float*)part, n_q, n_kv, (const __half*)svh, (const float*)bias,
+               (const uint16_t*)q_norm, (const uint16_t*)k_norm, eps, (const int*)positions, (const float*)inv_freq, (const int*)slot, (uint16_t*)q_out,
+               (uint16_t*)k_cache, (uint16_t*)v_cache, (const int*)pos3, 3 * section_h, 3 * section_w);
+  } else if (hd == 128) rx::launch(S == 1 ? finish_qkv_rope_kernel<128, true> : finish_qkv_rope_kernel<128, false>, dim3(grid), dim3(256), 0, st, RX_ARGS);
   else if (hd == 64) rx::launch(S == 1 ? finish_qkv_rope_kernel<64, true> : finish_qkv_rope_kernel<64, false>, dim3(grid), dim3(256), 0, st, RX_ARGS);
   else return (int)cudaErrorInvalidValue;
 #undef RX_ARGS

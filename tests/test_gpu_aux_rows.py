@@ -40,3 +40,30 @@ def test_rotation_of_a_slice_equals_its_windows(M, N):
     for r in range(0, M, 64):
         K.norm_rot_in(x[r:r + 64], None, 1e-6, suh, b[r:])
     assert a.abs().max() > 0 and torch.isfinite(a.float()).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("nq,nkv", [(1, 1), (6, 2), (32, 4), (40, 8), (80, 16)])           # 3 to 112 blocks a row: one to three passes
+@pytest.mark.parametrize("qn,kn,bias,axes", [(True, True, False, False), (False, False, True, False), (True, False, True, True), (False, True, False, False)])
+def test_rope_of_a_slice_equals_its_windows(nq, nkv, qn, kn, bias, axes):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from rexl3_b200.ops import lib
+    M, N, pages = 601, (nq + 2 * nkv) * 128, 11
+    g = torch.Generator(device="cuda").manual_seed(N)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    part, svh, b, wq, wk, inv = r(M, N), r(N).half(), r(N), (1 + 0.1 * r(128)).bfloat16(), (1 + 0.1 * r(128)).bfloat16(), torch.rand(64, device="cuda", generator=g)
+    pos, pos3 = torch.arange(7, 7 + M, device="cuda").int(), torch.randint(0, 900, (M, 3), device="cuda", generator=g).int()
+    slot = torch.randperm(pages * 64, device="cuda", generator=g)[:M].int()
+    slot[::5] = -1                                                                          # rows that are not cached
+    p = lambda t, on=True: t.data_ptr() if on else None  # noqa: E731
+    got = []
+    for step in (M, 100):
+        q, kc, vc = (torch.zeros(*s, dtype=torch.bfloat16, device="cuda") for s in ((M + 1, nq * 128), (pages, nkv, 64, 128), (pages, nkv, 64, 128)))
+        for r0 in range(0, M, step):
+            sec = 16 if axes else 0
+            lib.check(lib.load().rx_finish_qkv_rope(p(part[r0:]), 1, min(step, M - r0), nq, nkv, 128, p(svh), p(b, bias), p(wq, qn), p(wk, kn), 1e-6, p(pos[r0:]),
+                                                    p(inv), p(slot[r0:]), p(q[r0:]), p(kc), p(vc), lib.stream_ptr(), None, None, p(pos3[r0:], axes), sec, sec, None,
+                                                    None, 0), "rx_finish_qkv_rope")
+        got.append((q, kc, vc))
+    for x, y in zip(*got):
+        assert x.abs().max() > 0 and torch.isfinite(x.float()).all() and torch.equal(x, y)
