@@ -12,10 +12,11 @@
 // Warps: 0 = TMA producer, 1 and 10 = MMA issuers of tile 0 and 1 (1 also owns the tensor memory), 2..5 / 6..9 = softmax of tile 0 / 1 (thread = query
 // row = TMEM lane).  An issuer runs QK two pages ahead of PV, so a tile's next scores are there when its softmax has finished a page, and two softmax warps
 // per scheduler hide each other's latencies.
-// What bounds it is the issue of the MMAs: an MMA of 128 x 64 x 16 keeps its thread for 66 cycles, one of 128 x 128 x 16 for 78 (32 and 64 of the tensor
-// core), a wait that is already over for 80.  8192 rows, 40 heads: 776 us (0.89 PFLOP/s); 1089 with one issuer for both tiles, 1173 with its
-// waits for pages between P and the MMAs, 1242 with one S buffer beside Q in tensor memory.  Whole-warp issue by a predicate (1248) and the
-// two tiles' QK and PV issued in turn (1372) were slower.
+// What bounded it was the issue of the MMAs: entered by a lane comparison, an MMA of 128 x 64 x 16 kept its thread for 66 cycles, one of 128 x 128 x 16 for 78
+// (32 and 64 of the tensor core), a wait that was already over for 80; entered by elect.sync an MMA takes 12, and what is left is the chain of scores,
+// softmax and products of a page.  8192 rows, 40 heads: 726 us (0.95 PFLOP/s), 755 before elect.sync.  Forms before that, inside a slice:
+// 776 with two issuers, 1089 with one for both tiles, 1173 with its waits for pages between P and the MMAs, 1242 with one S buffer beside Q in tensor
+// memory.  Whole-warp issue by a predicate (1248) and the two tiles' QK and PV issued in turn (1372) were slower.
 //
 // The running maximum of a row moves only when it grows by more than 2^8 (the probabilities then stay below 2^8, harmless in fp32
 // sums and bf16 products); O is rescaled only in those steps.  Every such decision is per row, so a row's bits never depend on its

@@ -9,13 +9,13 @@
 // and the accumulator is double buffered, its epilogue done by one decode group while the others go on.  One CTA per item in exl3_gemm.cu
 // spent most of its life in its prologue and on shared-memory traffic of the decoded tile: 16 rows x 8 picks of 128 experts (2048 -> 1536 and
 // 768 -> 2048, 3.0 bpw) took 235 us for both products,
-// 146 us here; one row 83 and 26 us.  What is left is the decode's own: the integer pipe is 70 % busy.  (Fetching the next item's table entry
+// 141 us here; one row 83 and 26 us.  What is left is the decode's own: the integer pipe is 70 % busy.  (Fetching the next item's table entry
 // ahead costs registers that the decode groups do not have: 5 % slower.)
 //
 // Tiles of up to 256 rows (TALL, for prompt slices): both accumulators hold rows of one item, a unit of 128 rows each, so that its weights are decoded once.
 // The activations then come in boxes of 64 rows, no more of them than the tile has rows, and a unit is written out by two groups, half each: with one
-// group a unit the next item waited for them (128 experts, 16,800 pairs, 2048 -> 1536: 229 us by tiles of 128, 211 with one group a unit, 190 so).  What is left
-// of it is the L2's: every strip reads the activations again, 6 TB/s at 65,536 pairs (678 -> 510 us).
+// group a unit the next item waited for them (4.0 bpw, 128 experts, 16,800 pairs, 2048 -> 1536: 229 us by tiles of 128, 211 with one group a unit, 190 so).  What is left
+// of it is the L2's: every strip reads the activations again, 6 TB/s at 65,536 pairs (3.0 bpw, 678 -> 510 us).
 //
 // Warp roles: 0 weight producer (one bulk copy per k-tile row), 1 TMEM owner + MMA issuer, 2 activation producer, then NG decode groups of 4 warps.
 // Group e % NG writes out item e, after its first chunk of a later item: the accumulator of item e is needed again by item e + 2 only, whose

@@ -293,8 +293,9 @@ static int gemm_b4(const void* xr, int rows, int K, const void* trellis, int N, 
   if ((((uintptr_t)xr) & 15) != 0 || (((uintptr_t)trellis) & 15) != 0) return (int)cudaErrorMisalignedAddress;
   const int brows = rx_exl3_tile_rows(rows);
   const int row_tiles = (rows + brows - 1) / brows;
-  // 65 to 128 rows on one rank: one CTA per SM either way, and a CTA that walks several items spares each its prologue and tail (verify window of 80
-  // rows on eight layers 2165 -> 2120 us; up to 64 rows two CTAs per SM hide the prologue and this form is the better one: step of 64 rows 2130, 2290 us).
+  // 65 to 128 rows on one rank (of decode windows those that exl3_gemm_step.cu does not take): one CTA per SM either way, and a CTA that walks several items
+  // spares each its prologue and tail (verify window of 80 rows on eight layers, every product so, 2165 -> 2120 us; up to 64 rows two CTAs per SM hide the
+  // prologue and this form is the better one: step of 64 rows 2130, 2290 us).
   // With one item for a CTA there is nothing to spare (2048 -> 1536, 80 rows, 96 items: 5.8 us by this form, 7.0 by the persistent one).
   if (brows == 128 && (long long)(N / 128) * splits > 148 && tp.strips_per_rank == 0 && tp.in_flag == nullptr && gemm_persistent_takes(K, 8, splits, brows))
     return gemm_persistent(xr, rows, K, trellis, 0, N, 8, codebook, part, splits, 128, nullptr, row_tiles, brows, status, (cudaStream_t)stream);
