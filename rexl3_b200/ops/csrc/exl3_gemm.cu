@@ -87,6 +87,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
   uint64_t* acc_full = raw_empty + RAW_STAGES;    // [1]
   uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  volatile int* n_sent = abort_flag + 1;          // [2] chunks that the producer has issued: weights, activations
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strip = blockIdx.x;
@@ -116,6 +117,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
   tc_fence_after();
   // The weights were not written by the previous kernel, everything else may have been: the first weights come and are decoded while it still runs.
   const uint32_t tmem_base = *tmem_slot;
+  int c_next = nchunks;                           // decode warps, lane 0: the first chunk of theirs that was not announced
 
   if (warp == 0) {
     // ------------------------------------------------ producer
@@ -125,6 +127,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
       // decode warps release a raw stage before they wait for an operand stage.
       constexpr int AHEAD = 4;
       bool ok = true;
+      int n_raw = 0, n_op = 0;
       for (int i = 0; i < nchunks + AHEAD && ok; ++i) {
         if (i < nchunks) {
           const int c = i, s = c % RAW_STAGES;
@@ -137,6 +140,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
             const uint32_t* src = trellis + ((size_t)(kt0 + r) * nt_total + (size_t)strip * 8) * TILE_WORDS;
             bulk_g2s(smem + L.raw_off + s * RAW_STAGE + r * ROW_BYTES, src, ROW_BYTES, &raw_full[s]);
           }
+          ++n_raw;
         }
         if (i == AHEAD) pdl_wait();
         if (i >= AHEAD) {
@@ -145,8 +149,11 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
           if (!ok) break;
           mbar_arrive_expect_tx(&op_full[s], (uint32_t)b_stage);
           tma_load_2d(smem + L.b_off + s * b_stage, &tmap_x, (c_begin + c) * KCH, g_row0, &op_full[s]);
+          ++n_op;
         }
       }
+      n_sent[0] = n_raw;
+      n_sent[1] = n_op;
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
@@ -175,6 +182,8 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     const int t = (dw % (NDEC_WARPS / NDEC_GROUPS)) * 32 + lane;  // 0..127 inside the group
     const int h = t & 3, ktl = (t >> 2) & 3, nt = t >> 4;
     bool ok = true;
+    c_next = grp;
+    // A wait that gives up does not end the loop, the chunks are void then: lanes that left it one by one would be missed by the others' shuffles.
     if constexpr (TWICE == 8) {
       // ---- 4.0 bpw fast path.  A thread owns the two eighths 2h and 2h+1 of its tile (two 16-byte loads, conflict free
       // because odd k-tiles take them in the other order), gets the one word before each from its own other eighth or from
@@ -185,18 +194,16 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
       const int o1 = (n1 >> 3) * 1024 + (n1 & 7) * 128 + (((2 * ktl) ^ (g1 & 7)) << 4);
       const int o2 = (n2 >> 3) * 1024 + (n2 & 7) * 128 + (((2 * ktl) ^ (g2 & 7)) << 4);
       const int src = (lane & ~3) | ((h + 3) & 3);
-      for (int c = grp; c < nchunks && ok; c += NDEC_GROUPS) {
+      for (int c = grp; c < nchunks; c += NDEC_GROUPS) {
         const int rs = c % RAW_STAGES, os = c % OP_STAGES;
-        ok = mbar_wait(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, status, 30);
-        if (!ok) break;
+        ok = ok && mbar_wait(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, status, 30);
         const uint4* tile4 = reinterpret_cast<const uint4*>(smem + L.raw_off + rs * RAW_STAGE) + (ktl * 8 + nt) * 8;
         const uint4 first = tile4[g1], second = tile4[g2];
         const uint32_t sh_second = __shfl_sync(0xffffffffu, second.w, src), sh_first = __shfl_sync(0xffffffffu, first.w, src);
         const uint32_t w1[5] = {x ? second.w : sh_second, first.x, first.y, first.z, first.w};
         const uint32_t w2[5] = {x ? sh_first : first.w, second.x, second.y, second.z, second.w};
         release_read_stage(&raw_empty[rs], lane);      // generic-proxy reads, async-proxy refill: proxy fence before the release
-        if (c >= OP_STAGES) ok = mbar_wait(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 31);
-        if (!ok) break;
+        if (c >= OP_STAGES) ok = ok && mbar_wait(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 31);
         uint8_t* a_tile = smem + L.a_off + os * A_STAGE;
         {
           uint32_t h2[16];
@@ -218,16 +225,17 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&op_full[os]);
+        if (lane == 0 && ok) {
+          mbar_arrive(&op_full[os]);
+          c_next = c + NDEC_GROUPS;
+        }
       }
     } else
-    for (int c = grp; c < nchunks && ok; c += NDEC_GROUPS) {
+    for (int c = grp; c < nchunks; c += NDEC_GROUPS) {
       const int rs = c % RAW_STAGES, os = c % OP_STAGES;
-      ok = mbar_wait(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, status, 30);
-      if (!ok) break;
+      ok = ok && mbar_wait(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, status, 30);
       const uint32_t* tile = (const uint32_t*)(smem + L.raw_off + rs * RAW_STAGE) + (ktl * 8 + nt) * TILE_WORDS;
-      if (c >= OP_STAGES) ok = mbar_wait(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 31);
-      if (!ok) break;
+      if (c >= OP_STAGES) ok = ok && mbar_wait(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 31);
       uint8_t* a_tile = smem + L.a_off + os * A_STAGE;
       if constexpr (TWICE % 2 == 0) {
         // two word-aligned eighths per thread; odd k-tiles take them in the other order, which makes the 8 threads
@@ -259,14 +267,17 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
       }
       release_read_stage(&raw_empty[rs], lane);        // (the fence also covers the operand tile written above)
       __syncwarp();
-      if (lane == 0) mbar_arrive(&op_full[os]);
+      if (lane == 0 && ok) {
+        mbar_arrive(&op_full[os]);
+        c_next = c + NDEC_GROUPS;
+      }
     }
     // ------------------------------------------------ epilogue (warps 2..5 cover TMEM lane quarters 2,3,0,1)
     if (dw < 4) {
       pdl_wait();
-      const bool done = mbar_wait(acc_full, 0, abort_flag, status, 40);
+      const bool done = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, status, 40) && *abort_flag == 0);
       tc_fence_after();
-      if (done && *abort_flag == 0) {
+      if (done) {
         const int q = warp & 3;
         const int n = strip * STRIP + q * 32 + lane;
         float* out = part + ((size_t)split * rows) * N + n;
@@ -287,11 +298,18 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
   // ------------------------------------------------ teardown: every role falls through to here
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
-    if (*abort_flag != 0 && lane == 0) {
-      // make sure no MMA is still writing TMEM before it is freed (bounded)
-      mbar_wait(acc_full, 0, abort_flag, nullptr, 41);
+  if (*abort_flag != 0 && lane == 0) {
+    // Consumers that gave up have seen neither the last copies arrive nor the last MMA end.  A stage of operands is complete with the arrivals of its decode
+    // warps, too: those that are missing are made up for.
+    if (warp >= 2)
+      for (; c_next < n_sent[1]; c_next += NDEC_GROUPS) mbar_arrive(&op_full[c_next % OP_STAGES]);
+    if (warp == 0) {
+      ring_landed(raw_full, RAW_STAGES, n_sent[0]);
+      ring_landed(op_full, OP_STAGES, n_sent[1]);
     }
+    if (warp == 1) ring_landed(acc_full, 1, 1);
+  }
+  if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tmem_base, ncols);
   }

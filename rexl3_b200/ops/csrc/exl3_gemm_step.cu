@@ -133,6 +133,8 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     return StepPiece{v.x, v.y & 0xffff, v.z, v.w, (v.y >> 16 & 1) != 0, (v.y >> 17 & 1) != 0};
   };
 
+  int gc_next = total + ST_NG;                      // decode warps: the first chunk of theirs that they have not announced
+
   if (warp == 0) {
     // ---- weight producer: ONE 2-D tiled copy per chunk (8 k-tile rows x 1 KB of the strip)
     if (elect_one()) {
@@ -289,8 +291,8 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         }
       }
     };
-    int gc0 = 0;                                  // chunks up to the end of piece f
-    for (int gc = grp; ok && f < pieces; ++f) {
+    int gc = grp, gc0 = 0;                        // chunks up to the end of piece f
+    for (; ok && f < pieces; ++f) {
       const StepPiece p = piece(f);
       gc0 += p.n;
       // (not before: the CTA before may still be at it)
@@ -346,17 +348,25 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         // the last pair has one chunk: the arrivals of the other
         const int os = gc % ST_STAGES;
         if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty[os >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 180));
-        if (ok && lane == 0) mbar_arrive(&full[os >> LOG]);
+        if (ok) {
+          if (lane == 0) mbar_arrive(&full[os >> LOG]);
+          gc += ST_NG;
+        }
       }
     }
+    gc_next = gc;
     write_before(f);
   }
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag != 0 && lane == 0) {                // consumers that gave up have not seen the last copies arrive
+  if (*abort_flag != 0 && lane == 0) {
+    // Consumers that gave up have not seen the last copies arrive.  A barrier of operands is complete with the arrivals of its decode warps, too: those that
+    // are missing are made up for.
+    const int begun = (n_sent[1] + PER - 1) / PER;
+    if (warp >= ST_ROLE_WARPS)
+      for (; gc_next < begun * PER; gc_next += ST_NG) mbar_arrive(&full[(gc_next % ST_STAGES) >> LOG]);
     if (warp == 0) ring_landed(raw_full, ST_RAW, n_sent[0]);
-    if (warp == 2)
-      for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    if (warp == 2) ring_landed(full, ST_BARS, begun);
   }
   if (warp == 1) {
     if (lane == 0) mbar_wait(drained, 0, last_flag, a.status, 181);      // nothing may still write the tensor memory that is freed

@@ -62,6 +62,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   uint64_t* acc_full = raw_empty + TM_RAW_STAGES;
   uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  volatile int* n_sent = abort_flag + 1;             // [2] chunks that the producers have issued: weights, activations
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strip = blockIdx.x, split = blockIdx.y, row_tile = blockIdx.z;
@@ -103,23 +104,24 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   if (warp == 0) {
     // ---- weight producer: ONE 2-D tiled copy per chunk (8 k-tile rows x 1 KB of this strip)
     if (elect_one()) {
-      int y = (c_begin + TM_RAW_STAGES) * 8;
+      int y = (c_begin + TM_RAW_STAGES) * 8, c = TM_RAW_STAGES;
       const int x = strip * 256;
-      for (int c = TM_RAW_STAGES; c < nchunks; ++c, y += 8) {   // the first ring's worth was issued in the prologue
+      for (; c < nchunks; ++c, y += 8) {                        // the first ring's worth was issued in the prologue
         const int s = c % TM_RAW_STAGES;
         if (!mbar_wait(&raw_empty[s], ((c / TM_RAW_STAGES) - 1) & 1, abort_flag, status, 110, 1000)) break;
         mbar_arrive_expect_tx(&raw_full[s], TM_RAW_STAGE_BYTES);
         tma_load_2d(raw_base + s * TM_RAW_STAGE_BYTES, &tmap_w, x, y, &raw_full[s]);
       }
+      n_sent[0] = min(c, nchunks);
     }
   } else if (warp == 2) {
     // ---- activation producer: two [brows x 64] swizzled boxes per chunk
     if (elect_one()) {
-      int x = c_begin * TM_KCH;
+      int x = c_begin * TM_KCH, c = 0;
       const int y = row_tile * brows;
       int waited_src = -1;
       const unsigned ticket = (tp.in_flag != nullptr) ? tp_ticket(tp.epoch, tp.use_index) : 0u;
-      for (int c = 0; c < nchunks; ++c, x += TM_KCH) {
+      for (; c < nchunks; ++c, x += TM_KCH) {
         const int s = c % TM_OP_STAGES;
         if (tp.in_flag != nullptr) {
           // all-gather -> GEMM: this K chunk was pushed into the local buffer by rank `src`; consume it as soon as it has landed
@@ -134,6 +136,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         tma_load_2d(b_base + s * b_stage, &tmap_x, x, y, &b_full[s]);
         tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + 64, y, &b_full[s]);
       }
+      n_sent[1] = c;
     }
   } else if (warp == 1) {
     // ---- MMA issuer: A from tensor memory, B from shared memory
@@ -166,11 +169,10 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     const int prev_lane = (lane & ~7) | ((lane + 7) & 7);
     const uint32_t st_addr = a_tmem0 + ((uint32_t)(q * 32) << 16);
     const int tile_off = nt * 8 + g;              // uint4 index of this thread's eighth inside a k-tile row
-    bool ok = true;
-    for (int c = grp; c < nchunks && ok; c += NG) {
+    // A wait that gives up does not end the loop, the chunks are void then: lanes that left it one by one would be missed by the others' shuffles.
+    for (int c = grp; c < nchunks; c += NG) {
       const int rs = c % TM_RAW_STAGES, os = c % SA;
-      ok = mbar_wait(&raw_full[rs], (c / TM_RAW_STAGES) & 1, abort_flag, status, 130, 200);
-      if (!ok) break;
+      mbar_wait(&raw_full[rs], (c / TM_RAW_STAGES) & 1, abort_flag, status, 130, 200);
       const uint32_t raw4 = smem_u32(raw_base + rs * TM_RAW_STAGE_BYTES) + (uint32_t)tile_off * 16u;
       bool waited = false;
 #pragma unroll
@@ -200,14 +202,12 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           }
         }
         if (!waited) {
-          if (c >= SA) ok = mbar_wait(&a_empty[os], ((c / SA) - 1) & 1, abort_flag, status, 131, NG == 4 ? 64 : 0);   // prefill class: the tensor core sets the pace
+          if (c >= SA) mbar_wait(&a_empty[os], ((c / SA) - 1) & 1, abort_flag, status, 131, NG == 4 ? 64 : 0);   // prefill class: the tensor core sets the pace
           waited = true;
-          if (!ok) break;
           tc_fence_after();
         }
         tc_st_32x32b_x16(st_addr + os * TM_A_COLS + qt * 16, regs);
       }
-      if (!ok) break;
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -215,9 +215,9 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     }
     if (dw < 4) {
       pdl_wait();
-      const bool done = mbar_wait(acc_full, 0, abort_flag, status, 140, 100);
+      const bool done = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, status, 140, 100) && *abort_flag == 0);
       tc_fence_after();
-      if (done && *abort_flag == 0) {
+      if (done) {
         float* out;
         size_t ld;
         if (tp.strips_per_rank > 0) {
@@ -252,8 +252,12 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   }
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0 && lane == 0) {                // consumers that gave up have seen neither the last copies arrive nor the last MMA end
+    if (warp == 0) ring_landed(raw_full, TM_RAW_STAGES, n_sent[0]);
+    if (warp == 1) ring_landed(acc_full, 1, 1);
+    if (warp == 2) ring_landed(b_full, TM_OP_STAGES, n_sent[1]);
+  }
   if (warp == 1) {
-    if (*abort_flag != 0 && lane == 0) mbar_wait(acc_full, 0, abort_flag, nullptr, 141);
     __syncwarp();
     tmem_dealloc(tmem_base, ncols);
   }

@@ -57,6 +57,9 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {      // as a copy of that many bytes does
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
@@ -219,9 +222,12 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   uint64_t* acc_full = empty + WD_STAGES;                         // [2] commit
   uint64_t* acc_empty = acc_full + 2;                             // [2] of the first CTA: eight epilogue warps
   uint64_t* acc_taken = acc_empty + 2;                            // of the first CTA: eight epilogue warps have put the handed accumulator in place
-  uint32_t* tmem_slot = (uint32_t*)(acc_taken + 1);
+  uint64_t* drained = acc_taken + 1;                              // every MMA of the pair has completed
+  uint32_t* tmem_slot = (uint32_t*)(drained + 1);
   int* pair_slot = (int*)(tmem_slot + 1);
   volatile int* abort_flag = (volatile int*)(pair_slot + 1);
+  int* n_sent = pair_slot + 2;                                    // stages that this CTA's copies were issued for
+  int* sent = n_sent + 1;                                         // [stages] their bytes
   constexpr int GROUPS = MODE == WD_SWIGLU ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
@@ -232,6 +238,7 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     for (int i = 0; i < WD_STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
     mbar_init(acc_taken, 8);
+    mbar_init(drained, 1);
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
@@ -281,12 +288,15 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
           if (it >= WD_STAGES) ok = mbar_wait(&empty[s], ((it / WD_STAGES) - 1) & 1, abort_flag, a.status, 161, 20);
           if (!ok) break;
           uint8_t* st = smem + s * 2 * WD_HALF;
-          if (rank == 0) mbar_arrive_expect_tx(&full[s], 2u * (WD_HALF + (uint32_t)half * 128u));
+          const uint32_t bytes = WD_HALF + (uint32_t)half * 128u;
+          sent[s] = (int)bytes;
+          if (rank == 0) mbar_arrive_expect_tx(&full[s], 2u * bytes);
           const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
           tma_load_2d_pair(st, &tmap_x, kb * 64, xrow, bar);
           tma_load_2d_pair(st + WD_HALF, half == 128 ? &tmap_w : &tmap_w64, 0, wrow + kb * 128, bar);
         }
       }
+      *n_sent = it;
     }
   } else if (warp == 1) {
     // ---- MMA issuer of the pair
@@ -315,6 +325,9 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         }
         if (ok) tc_commit_pair(&acc_full[acc]);
       }
+      // nothing may still write the tensor memory that is freed, after a wait that gave up either
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(drained)) : "memory");
+      ring_landed(drained, 1, 1);
     }
   } else if (warp >= 4 && warp < 4 + 4 * GROUPS) {
     // ---- epilogue: lane = row of this CTA's 128; with two groups of warps, each takes every other tile
@@ -552,12 +565,23 @@ exl3_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       now = nx;
     }
   }
-  __syncwarp();
-  if (*abort_flag != 0 && threadIdx.x == 0)
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);   // copies in flight land before their memory is left
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0 && threadIdx.x == 0)
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_u32(smem_u32((const void*)abort_flag), rank ^ 1)), "r"(1) : "memory");
+  __syncwarp();
   cluster_sync();
+  if (*abort_flag != 0) {
+    // Either CTA has given up, and the last copies may be under way.  A stage that only one CTA has issued its copies for gets the other's bytes here.
+    if (rank == 0 && threadIdx.x == 0) {
+      const int n0 = *n_sent, n1 = ld_cluster(n_sent, 1);
+      for (int i = n1; i < n0; ++i) mbar_complete_tx(&full[i % WD_STAGES], (uint32_t)sent[i % WD_STAGES]);
+      for (int i = n0; i < n1; ++i) mbar_arrive_expect_tx(&full[i % WD_STAGES], (uint32_t)ld_cluster(sent + i % WD_STAGES, 1));
+      ring_landed(full, WD_STAGES, max(n0, n1));
+    }
+    __syncwarp();
+    cluster_sync();
+  }
   if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   if (warp == 0) {
     // the last CTA leaves the counters as it found them
