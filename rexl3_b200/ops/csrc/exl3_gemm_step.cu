@@ -40,7 +40,9 @@ __host__ __device__ inline int st_smem_bytes(int brows, bool tall) { return ST_S
 
 struct StepArgs {
   float* part;
-  int* flags;                // [0]: CTAs begun, modulo ST_CTAS; [32 + 4 share + quarter], TALL [32 + 32 share + 8 quarter + 16-row block]: accumulator handed on.  Zero between calls.
+  // [0]: CTAs begun, modulo ST_CTAS; [32 + 4 share + quarter], TALL [32 + 32 share + 8 quarter + 16-row block]: accumulator handed on.  Zero between calls, those that
+  // gave up among them: in every call the CTA that hands on sets a flag once and the one that takes clears it once, as its last act if it has given up.
+  int* flags;
   int* status;
   int rows, K, N, splits, brows;
 };
@@ -67,6 +69,9 @@ __device__ __forceinline__ int step_pieces(const StepArgs& a, int share, int lan
   }
   return count;
 }
+
+// TALL: the block of piece f, of nb, that a group writes out; nb and more: none.  Over the pieces the blocks go round the groups.
+__device__ __forceinline__ int step_block(int grp, int f, int nb) { return (int)((unsigned)(grp + ST_NG * ST_PIECES - f * nb) % (unsigned)ST_NG); }
 
 template <int CB, bool TALL>
 __global__ void __launch_bounds__(ST_THREADS, 1)
@@ -128,12 +133,14 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t a_tmem0 = tmem_base + 2 * ST_ACC;
   const int pieces = share_slot[1], total = share_slot[2];
+  constexpr int FLAGS = TALL ? 32 : 4, QFLAGS = FLAGS / 4;         // of a share: a quarter's blocks of 16 rows, or all rows
   auto piece = [&](int f) {
     const int4 v = table[f];
     return StepPiece{v.x, v.y & 0xffff, v.z, v.w, (v.y >> 16 & 1) != 0, (v.y >> 17 & 1) != 0};
   };
 
   int gc_next = total + ST_NG;                      // decode warps: the first chunk of theirs that they have not announced
+  int passed = 0;                                   // decode warps, bits: the kernel before has ended; this warp has handed on; it has taken
 
   if (warp == 0) {
     // ---- weight producer: ONE 2-D tiled copy per chunk (8 k-tile rows x 1 KB of the strip)
@@ -224,12 +231,11 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t my_words = (uint32_t)((n >> 4) * 8 + (n & 7)) * 16u;
     const int share = *share_slot;
-    constexpr int FLAGS = TALL ? 32 : 4;          // of a share: a quarter's blocks of 16 rows, or all rows
-    int* flag_out = a.flags + 32 + share * FLAGS + q * (FLAGS / 4);
-    bool ok = true, waited = false;
+    int* flag_out = a.flags + 32 + share * FLAGS + q * QFLAGS;
+    bool ok = true;
     auto kernel_before = [&]() {                  // `part` and the flags may be in use until it has ended
-      if (!waited) pdl_wait();
-      waited = true;
+      if (passed == 0) pdl_wait();
+      passed |= 1;
     };
     auto place = [&](const StepPiece& o) { return a.part + ((size_t)o.split * a.rows) * a.N + o.strip * 128 + n; };
     // piece f has had its last MMA: its accumulator (TALL: block b of it) goes to its place
@@ -252,6 +258,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         if (o.hand) atomicExch(flag_out + b, 1);
         mbar_arrive(&acc_empty[TALL ? 0 : f & 1]);
       }
+      if (o.hand) passed |= 2;
     };
     // The accumulator of the last piece f, as the CTA before left it.  The group that writes out piece f - 2 (TALL: block b of piece f - 1), whose place it takes,
     // brings it in: a wait of another group could miss two phases of that buffer's barrier.
@@ -272,16 +279,15 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         atomicExch(flag_out - FLAGS + b, 0);
         mbar_arrive(acc_taken);
       }
+      passed |= 4;
       return true;
     };
     int next_out = TALL ? 0 : grp, f = 0;         // the next piece that this group writes out (TALL: or looks at); the piece it is in
-    // TALL: the block of piece f that this group writes out; nb and more: none.  Over the pieces the blocks go round the groups.
-    auto block_of = [&](int f) { return (int)((unsigned)(grp + ST_NG * ST_PIECES - f * nb) % (unsigned)ST_NG); };
     // Writes out this group's pieces before piece `end`.  (Left for later when the last MMA is still to come, a group could wait for an operand stage whose MMA
     // waits for that very accumulator.)
     auto write_before = [&](int end) {
       for (; ok && next_out < end; next_out += TALL ? 1 : ST_NG) {
-        const int b = TALL ? block_of(next_out) : 0;
+        const int b = TALL ? step_block(grp, next_out, nb) : 0;
         if (TALL && b >= nb) continue;
         ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[next_out % ST_OUT], (next_out / ST_OUT) & 1, abort_flag, a.status, 176));
         if (ok) write_out(piece(next_out), next_out, b);
@@ -368,6 +374,24 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     if (warp == 0) ring_landed(raw_full, ST_RAW, n_sent[0]);
     if (warp == 2) ring_landed(full, ST_BARS, begun);
   }
+  if (*abort_flag != 0 && warp >= ST_ROLE_WARPS && lane == 0) {
+    // the next CTA gets its flags all the same, and those of the CTA before, which has begun and whose own waits are bounded, are cleared
+    const int grp = (warp - ST_ROLE_WARPS) >> 2;
+    int* flag = a.flags + 32 + *share_slot * FLAGS + (warp & 3) * QFLAGS;
+    pdl_wait();
+    for (int f = 0; f < share_slot[1]; ++f) {
+      const StepPiece p = piece(f);
+      const int b = TALL ? step_block(grp, f, nb) : 0;
+      if (p.hand && (TALL ? b < nb : grp == f % ST_NG) && !(passed & 2)) atomicExch(flag + b, 1);
+    }
+    for (int f = 0; f < share_slot[1]; ++f) {
+      const StepPiece p = piece(f);
+      const int b = !TALL ? 0 : f == 0 ? grp : step_block(grp, f - 1, nb);
+      if (p.take && (TALL ? b < nb : grp == (f < 2 ? f : (f - 2) % ST_NG)) && !(passed & 4))
+        for (int i = 0; i < (1 << 22) && atomicExch(flag - FLAGS + b, 0) == 0; ++i) __nanosleep(100);
+    }
+  }
+  __syncwarp();
   if (warp == 1) {
     if (lane == 0) mbar_wait(drained, 0, last_flag, a.status, 181);      // nothing may still write the tensor memory that is freed
     __syncwarp();
@@ -424,7 +448,7 @@ RX_API int rx_exl3_step_takes(int rows, int K, int N, int splits) {
   return 2 * item * 0.527 + 3.0 > share * 0.48 + (rows <= 16 ? 8.5 : 9.5);
 }
 
-// rx_exl3_gemm_b4 for decode windows; flags: int32 [rx_exl3_step_flags()], zero before the first call, one buffer for calls that may overlap.
+// rx_exl3_gemm_b4 for decode windows; flags: int32 [rx_exl3_step_flags()], zero before the first call; calls that may overlap need one each.
 RX_API int rx_exl3_gemm_step(const void* xr, int rows, int K, const void* trellis, int N, int codebook, void* part, int splits, void* flags, int* status,
                              void* stream) {
   if (!step_fits(rows, K, N, splits) || flags == nullptr) return (int)cudaErrorInvalidValue;

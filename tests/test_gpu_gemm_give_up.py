@@ -70,17 +70,22 @@ def test_item_gemm_behind_a_long_kernel(long_kernel, rows, words):
     (80, 2048, 224 * 128, 1),     # one accumulator, blocks of 16 rows
     (96, 4096, 40 * 128, 7),      # short items, pieces on both ends
 ])
-def test_step_gemm(rows, K, N, splits):
+@pytest.mark.parametrize("kept", [False, True])
+def test_step_gemm(rows, K, N, splits, kept):
+    """kept: all calls use one flags buffer, as an executor's do; one that gave up leaves it as it found it, too."""
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
     from rexl3_b200.ops import lib
     KK, w, g = _weights(K, N)
     x = torch.randn(rows, K, device="cuda", generator=g).half()
 
+    one = torch.zeros(KK.step_flags(), dtype=torch.int32, device="cuda")
+
     def call(out, st):
-        flags = torch.zeros(KK.step_flags(), dtype=torch.int32, device="cuda")
+        flags = one if kept else torch.zeros_like(one)
         lib.check(lib.load().rx_exl3_gemm_step(x.data_ptr(), rows, K, w.trellis.data_ptr(), N, KK.CB_ID[w.codebook], out.data_ptr(), splits, flags.data_ptr(),
                                                st.data_ptr(), lib.stream_ptr()), "rx_exl3_gemm_step")
+        assert int(flags.abs().sum()) == 0
     assert _check(call, torch.empty(splits, rows, N, device="cuda")) > 0
 
 
