@@ -135,6 +135,34 @@ __device__ __forceinline__ bool wait_count(const int* count, int want, volatile 
   return true;
 }
 
+// mbar_wait of a role that does not wait for the kernel before, while that may still run.  `ended` (CTA-shared, 0 at first): the role that has waited for it stores
+// kernel_ended_at() there, and the limit counts from then on.
+__device__ __forceinline__ int kernel_ended_at() { return (int)(globaltimer_ns() / 1000 & 0x3FFFFFFF) + 1; }      // microseconds modulo 2^30, not 0
+__device__ __forceinline__ bool mbar_wait_early(uint64_t* bar, uint32_t parity, volatile int* abort_flag, volatile int* ended, int* status, int site,
+                                                uint32_t sleep_ns = 0) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = globaltimer_ns();
+  const uint64_t limit = wait_limit_ns(status);
+  uint32_t polls = 0;
+  while (true) {
+    if (sleep_ns != 0) __nanosleep(sleep_ns);
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((++polls & 15u) == 0) {
+      if (*abort_flag != 0) return false;
+      int code = host_abort(status) ? ST_ABORTED : ST_OK;
+      if (globaltimer_ns() - t0 > limit) {
+        const int at = *ended;
+        if (at != 0 && (uint64_t)((kernel_ended_at() - at) & 0x3FFFFFFF) * 1000 > limit) code = ST_TIMEOUT;
+      }
+      if (code != ST_OK) {
+        *abort_flag = 1;
+        set_status(status, code, site, (int)parity);
+        return false;
+      }
+    }
+  }
+}
+
 // Waits (bounded, and not cut short by an abort) until the copies of the last of `issued` phases of a ring of `stages` barriers have landed: a consumer whose
 // wait gave up does not, and a copy must not arrive in memory that its CTA has left.
 __device__ __forceinline__ void ring_landed(uint64_t* bars, int stages, int issued) {

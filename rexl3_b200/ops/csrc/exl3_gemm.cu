@@ -88,6 +88,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
   uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   volatile int* n_sent = abort_flag + 1;          // [2] chunks that the producer has issued: weights, activations
+  volatile int* ended = n_sent + 2;               // when the kernel before had ended
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strip = blockIdx.x;
@@ -104,7 +105,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     for (int i = 0; i < OP_STAGES; ++i) { mbar_init(&op_full[i], NDEC_WARPS / NDEC_GROUPS + 1); mbar_init(&op_empty[i], 1); }
     for (int i = 0; i < RAW_STAGES; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], NDEC_WARPS / NDEC_GROUPS); }
     mbar_init(acc_full, 1);
-    *abort_flag = 0;
+    *abort_flag = *ended = 0;
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
   }
@@ -142,7 +143,10 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
           }
           ++n_raw;
         }
-        if (i == AHEAD) pdl_wait();
+        if (i == AHEAD) {
+          pdl_wait();
+          *ended = kernel_ended_at();
+        }
         if (i >= AHEAD) {
           const int c = i - AHEAD, s = c % OP_STAGES;
           if (c >= OP_STAGES) ok = mbar_wait(&op_empty[s], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 11);
@@ -162,7 +166,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
       bool ok = true;
       for (int c = 0; c < nchunks && ok; ++c) {
         const int s = c % OP_STAGES;
-        ok = mbar_wait(&op_full[s], (c / OP_STAGES) & 1, abort_flag, status, 20);
+        ok = mbar_wait_early(&op_full[s], (c / OP_STAGES) & 1, abort_flag, ended, status, 20);
         if (!ok) break;
         tc_fence_after();
         const uint32_t a_addr = smem_u32(smem + L.a_off + s * A_STAGE);
@@ -196,14 +200,14 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
       const int src = (lane & ~3) | ((h + 3) & 3);
       for (int c = grp; c < nchunks; c += NDEC_GROUPS) {
         const int rs = c % RAW_STAGES, os = c % OP_STAGES;
-        ok = ok && mbar_wait(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, status, 30);
+        ok = ok && mbar_wait_early(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, ended, status, 30);
         const uint4* tile4 = reinterpret_cast<const uint4*>(smem + L.raw_off + rs * RAW_STAGE) + (ktl * 8 + nt) * 8;
         const uint4 first = tile4[g1], second = tile4[g2];
         const uint32_t sh_second = __shfl_sync(0xffffffffu, second.w, src), sh_first = __shfl_sync(0xffffffffu, first.w, src);
         const uint32_t w1[5] = {x ? second.w : sh_second, first.x, first.y, first.z, first.w};
         const uint32_t w2[5] = {x ? sh_first : first.w, second.x, second.y, second.z, second.w};
         release_read_stage(&raw_empty[rs], lane);      // generic-proxy reads, async-proxy refill: proxy fence before the release
-        if (c >= OP_STAGES) ok = ok && mbar_wait(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 31);
+        if (c >= OP_STAGES) ok = ok && mbar_wait_early(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, ended, status, 31);
         uint8_t* a_tile = smem + L.a_off + os * A_STAGE;
         {
           uint32_t h2[16];
@@ -233,9 +237,9 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     } else
     for (int c = grp; c < nchunks; c += NDEC_GROUPS) {
       const int rs = c % RAW_STAGES, os = c % OP_STAGES;
-      ok = ok && mbar_wait(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, status, 30);
+      ok = ok && mbar_wait_early(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, ended, status, 30);
       const uint32_t* tile = (const uint32_t*)(smem + L.raw_off + rs * RAW_STAGE) + (ktl * 8 + nt) * TILE_WORDS;
-      if (c >= OP_STAGES) ok = ok && mbar_wait(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 31);
+      if (c >= OP_STAGES) ok = ok && mbar_wait_early(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, ended, status, 31);
       uint8_t* a_tile = smem + L.a_off + os * A_STAGE;
       if constexpr (TWICE % 2 == 0) {
         // two word-aligned eighths per thread; odd k-tiles take them in the other order, which makes the 8 threads

@@ -97,6 +97,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   volatile int* abort_flag = share_slot + 3;
   volatile int* last_flag = abort_flag + 1;                        // of the wait before the tensor memory is freed, which an abort does not cut short
   volatile int* n_sent = last_flag + 1;                            // [2] chunks that the producers have issued: weights, activations
+  volatile int* ended = n_sent + 2;                                // when the kernel before had ended
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -106,7 +107,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     for (int i = 0; i < 2; ++i) mbar_init(&acc_empty[i], TALL ? 4 * nb : 4);
     mbar_init(acc_taken, TALL ? 4 * nb : 4);
     mbar_init(drained, 1);
-    *abort_flag = *last_flag = 0;
+    *abort_flag = *last_flag = *ended = 0;
     n_sent[0] = n_sent[1] = 0;
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
@@ -151,7 +152,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
         const StepPiece p = piece(f);
         for (int c = 0; c < p.n; ++c, ++gc) {
           const int s = gc % ST_RAW;
-          if (gc >= ST_RAW && !(ok = mbar_wait(&raw_empty[s], ((gc / ST_RAW) - 1) & 1, abort_flag, a.status, 170, 300))) break;
+          if (gc >= ST_RAW && !(ok = mbar_wait_early(&raw_empty[s], ((gc / ST_RAW) - 1) & 1, abort_flag, ended, a.status, 170, 300))) break;
           mbar_arrive_expect_tx(&raw_full[s], ST_RAW_BYTES);
           tma_load_2d(raw_base + s * ST_RAW_BYTES, &tmap_w, p.strip * 256, (p.c0 + c) * 8, &raw_full[s]);
         }
@@ -175,6 +176,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
           }
           tma_load_2d(b_base + s * b_stage, &tmap_x, x, 0, bar);
           tma_load_2d(b_base + s * b_stage + b_half, &tmap_x, x + 64, 0, bar);
+          if (gc == 0) *ended = kernel_ended_at();
         }
       }
       n_sent[1] = gc;
@@ -190,7 +192,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       StepPiece p = piece(0);
       uint32_t acc = 0, accumulate = 0;
       for (int gc = 0; gc < total; gc += PER) {
-        if (!(ok = mbar_wait(&full[ps], parity, abort_flag, a.status, 173))) break;
+        if (!(ok = mbar_wait_early(&full[ps], parity, abort_flag, ended, a.status, 173))) break;
         tc_fence_after();
 #pragma unroll
         for (int h = 0; h < PER; ++h) {
@@ -289,7 +291,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       for (; ok && next_out < end; next_out += TALL ? 1 : ST_NG) {
         const int b = TALL ? step_block(grp, next_out, nb) : 0;
         if (TALL && b >= nb) continue;
-        ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[next_out % ST_OUT], (next_out / ST_OUT) & 1, abort_flag, a.status, 176));
+        ok = __all_sync(0xffffffffu, mbar_wait_early(&acc_full[next_out % ST_OUT], (next_out / ST_OUT) & 1, abort_flag, ended, a.status, 176));
         if (ok) write_out(piece(next_out), next_out, b);
         if (TALL && ok && next_out + 1 < pieces) {
           const StepPiece p = piece(next_out + 1);
@@ -310,7 +312,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       }
       for (; gc < gc0 && ok; gc += ST_NG) {
         const int rs = gc % ST_RAW, os = gc % ST_STAGES;
-        ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[rs], (gc / ST_RAW) & 1, abort_flag, a.status, 179, 100));
+        ok = __all_sync(0xffffffffu, mbar_wait_early(&raw_full[rs], (gc / ST_RAW) & 1, abort_flag, ended, a.status, 179, 100));
         if (!ok) break;
         const uint32_t raw4 = smem_u32(raw_base + rs * ST_RAW_BYTES) + my_words;
 #pragma unroll
@@ -337,7 +339,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             }
           }
           if (qt == 0) {
-            if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty[os >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 180));
+            if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait_early(&empty[os >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, ended, a.status, 180));
             if (!ok) break;
             tc_fence_after();
           }
@@ -353,7 +355,7 @@ exl3_gemm_step_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
       if (PER == 2 && f == pieces - 1 && gc == total && (total & 1) != 0 && ok) {
         // the last pair has one chunk: the arrivals of the other
         const int os = gc % ST_STAGES;
-        if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(&empty[os >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, a.status, 180));
+        if (gc >= ST_STAGES) ok = __all_sync(0xffffffffu, mbar_wait_early(&empty[os >> LOG], ((gc / ST_STAGES) - 1) & 1, abort_flag, ended, a.status, 180));
         if (ok) {
           if (lane == 0) mbar_arrive(&full[os >> LOG]);
           gc += ST_NG;

@@ -63,6 +63,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   volatile int* n_sent = abort_flag + 1;             // [2] chunks that the producers have issued: weights, activations
+  volatile int* ended = n_sent + 2;                  // when the kernel before had ended
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int strip = blockIdx.x, split = blockIdx.y, row_tile = blockIdx.z;
@@ -79,7 +80,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     for (int i = 0; i < TM_OP_STAGES; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
     for (int i = 0; i < TM_RAW_STAGES; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
     mbar_init(acc_full, 1);
-    *abort_flag = 0;
+    *abort_flag = *ended = 0;
     fence_barrier_init();
     prefetch_tmap(&tmap_x);
     prefetch_tmap(&tmap_w);
@@ -104,6 +105,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   if (warp == 0) {
     // ---- weight producer: ONE 2-D tiled copy per chunk (8 k-tile rows x 1 KB of this strip)
     if (elect_one()) {
+      *ended = kernel_ended_at();
       int y = (c_begin + TM_RAW_STAGES) * 8, c = TM_RAW_STAGES;
       const int x = strip * 256;
       for (; c < nchunks; ++c, y += 8) {                        // the first ring's worth was issued in the prologue
@@ -172,7 +174,9 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     // A wait that gives up does not end the loop, the chunks are void then: lanes that left it one by one would be missed by the others' shuffles.
     for (int c = grp; c < nchunks; c += NG) {
       const int rs = c % TM_RAW_STAGES, os = c % SA;
-      mbar_wait(&raw_full[rs], (c / TM_RAW_STAGES) & 1, abort_flag, status, 130, 200);
+      // (with more raw stages than A stages a refill follows a product that this group has waited for)
+      if constexpr (TM_RAW_STAGES > SA) mbar_wait(&raw_full[rs], (c / TM_RAW_STAGES) & 1, abort_flag, status, 130, 200);
+      else mbar_wait_early(&raw_full[rs], (c / TM_RAW_STAGES) & 1, abort_flag, ended, status, 130, 200);
       const uint32_t raw4 = smem_u32(raw_base + rs * TM_RAW_STAGE_BYTES) + (uint32_t)tile_off * 16u;
       bool waited = false;
 #pragma unroll
@@ -202,7 +206,7 @@ exl3_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           }
         }
         if (!waited) {
-          if (c >= SA) mbar_wait(&a_empty[os], ((c / SA) - 1) & 1, abort_flag, status, 131, NG == 4 ? 64 : 0);   // prefill class: the tensor core sets the pace
+          if (c >= SA) mbar_wait_early(&a_empty[os], ((c / SA) - 1) & 1, abort_flag, ended, status, 131, NG == 4 ? 64 : 0);   // prefill class: the tensor core sets the pace
           waited = true;
           tc_fence_after();
         }

@@ -64,6 +64,26 @@ def test_item_gemm_behind_a_long_kernel(long_kernel, rows, words):
     _check(call, torch.empty(rows, N, device="cuda"))
 
 
+@pytest.mark.parametrize("rows,words,step", [(1, 64, False), (100, 64, False), (20, 32, False), (20, 40, False), (20, 64, None), (20, 96, False), (1, 64, True),
+                                             (80, 64, True)])
+def test_the_time_of_the_kernel_before_does_not_count(long_kernel, rows, words, step):
+    """A GEMM that begins under a kernel of some 300 us, with a limit that is below that and above each of its own waits.  step None: the general kernel."""
+    from rexl3_b200.ops import lib
+    K, N = 4096, 224 * 128 if step else 1152
+    KK, w, g = _weights(K, N, words, "mul1" if words == 40 else "3inst")
+    x, part = torch.randn(rows, K, device="cuda", generator=g).half(), torch.empty(rows, N, device="cuda")
+    flags, st = torch.zeros(KK.step_flags(), dtype=torch.int32, device="cuda"), KK.new_status()
+    KK.set_wait_limit(st, 100)
+    for _ in range(5):
+        long_kernel()
+        if step:
+            lib.check(lib.load().rx_exl3_gemm_step(x.data_ptr(), rows, K, w.trellis.data_ptr(), N, KK.CB_ID[w.codebook], part.data_ptr(), 1, flags.data_ptr(),
+                                                   st.data_ptr(), lib.stream_ptr()), "rx_exl3_gemm_step")
+        else:
+            KK.exl3_gemm(x, w, part, 1, st, force_generic=step is None)
+        KK.check_status(st)
+
+
 @pytest.mark.parametrize("rows,K,N,splits", [
     (1, 2048, 224 * 128, 1),      # shares of one item and a half
     (17, 1664, 75 * 128, 2),      # odd shares
