@@ -1091,7 +1091,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float*
 // twice the chunks in flight, and there are four times the warps; the rotation follows in the CTA's first warp.  A sum meets the chunks in the same order.
 constexpr int MERGE_FEW_LOADS = 32;
 template <int HD>
-__global__ void __launch_bounds__(128) attn_merge_few_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const int* __restrict__ ctx_len,
+__global__ void __launch_bounds__(128) attn_merge_few_kernel(const float* part_o, const float* part_ml, const int* ctx_len,
                                                              int n_q, int max_chunks, const __half* __restrict__ suh, __half* __restrict__ xr,
                                                              uint16_t* __restrict__ out_bf16) {
   pdl_launch();

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(1024) norm_rot_in_kernel(const uint16_t* __res
 }
 
 // The plain rotation of many rows: eight lanes to a 128-block.  x and xr of [rows * nb] blocks, suh of nb.
-__global__ void __launch_bounds__(256) rot_in_rows_kernel(const uint16_t* __restrict__ x, const __half* __restrict__ suh, __half* __restrict__ xr, long long blocks,
+__global__ void __launch_bounds__(256) rot_in_rows_kernel(const uint16_t* x, const __half* __restrict__ suh, __half* __restrict__ xr, long long blocks,
                                                           int nb) {
   pdl_launch();
   pdl_wait();
@@ -328,8 +328,8 @@ __global__ void __cluster_dims__(FEW_CTAS, 1, 1) __launch_bounds__(FEW_WARPS * 3
 // lane, which stay in registers between the sum of squares and the scaling, all of them loaded before the first is used.  By warps, a block each, it was
 // bound by the shuffles of its two transforms: 8192 rows of 5120 122 us, 96 now; 900 rows of 4096 24.6 -> 16.4.
 constexpr int ROWS_NB = 2, ROWS_MAX = 5120;
-__global__ void __launch_bounds__(ROWS_MAX / 16 / ROWS_NB) finish_add_norm_rot_rows_kernel(const float* __restrict__ part, int N, const __half* __restrict__ svh,
-                                                                      const float* __restrict__ bias, uint16_t* __restrict__ h,
+__global__ void __launch_bounds__(ROWS_MAX / 16 / ROWS_NB) finish_add_norm_rot_rows_kernel(const float* part, int N, const __half* __restrict__ svh,
+                                                                      const float* __restrict__ bias, uint16_t* h,
                                                                       const uint16_t* __restrict__ norm_w, float eps, const __half* __restrict__ suh_next,
                                                                       __half* __restrict__ xr, uint16_t* __restrict__ xn_out) {
   pdl_launch();
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(ROWS_MAX / 16 / ROWS_NB) finish_add_norm_rot_r
     const int b = min(grp + groups * i, nb - 1);          // (past the end the last block again: nothing of it is stored)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float4 p = __ldg(reinterpret_cast<const float4*>(part + base + b * 128 + 32 * j));
+      const float4 p = *reinterpret_cast<const float4*>(part + base + b * 128 + 32 * j);
       v[i][j][0] = p.x, v[i][j][1] = p.y, v[i][j][2] = p.z, v[i][j][3] = p.w;
       load4_bf16(h + base + b * 128 + 32 * j, r[i][j]);
     }

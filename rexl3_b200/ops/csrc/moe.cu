@@ -407,7 +407,7 @@ __device__ __forceinline__ uint2 moe_to_half4(const float (&f)[4]) {
 
 // The same rows for a prompt slice: eight lanes take one 128-block of a row and write it for all the experts that the row picked, so that the row is read once
 // and four experts' rotations are in flight.
-__global__ void __launch_bounds__(256) moe_gather_rot_rows_kernel(const uint16_t* __restrict__ x, const int* __restrict__ ids, const int* __restrict__ pos_of_pair,
+__global__ void __launch_bounds__(256) moe_gather_rot_rows_kernel(const uint16_t* x, const int* ids, const int* pos_of_pair,
                                                                   int pairs, int topk, int d, const __half* __restrict__ suh, __half* __restrict__ xs) {
   pdl_launch();
   pdl_wait();
@@ -699,9 +699,9 @@ __global__ void __launch_bounds__(PLANES > 0 ? 256 : 1024) moe_combine_kernel(co
 }
 
 // The same sum of a single plane on one rank for a prompt slice: eight lanes take one 128-block of a row through its slots, four slots' loads at a time.
-__global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* __restrict__ part, int M, int d, int topk, const int* __restrict__ ids,
-                                                               const float* __restrict__ w, const int* __restrict__ pos_of_pair,
-                                                               const __half* __restrict__ svh_down, const float* __restrict__ shared, float* __restrict__ dst) {
+__global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* part, int M, int d, int topk, const int* ids,
+                                                               const float* w, const int* pos_of_pair,
+                                                               const __half* __restrict__ svh_down, const float* shared, float* __restrict__ dst) {
   pdl_launch();
   pdl_wait();
   constexpr int SLOTS = 4;
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* __re
       pos[t] = live && j0 + t < topk ? pos_of_pair[row * topk + j0 + t] : -1;
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        p[t][j] = pos[t] >= 0 ? __ldg(reinterpret_cast<const float4*>(part + (size_t)pos[t] * d + n0 + 32 * j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        p[t][j] = pos[t] >= 0 ? *reinterpret_cast<const float4*>(part + (size_t)pos[t] * d + n0 + 32 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int t = 0; t < SLOTS; ++t) {
