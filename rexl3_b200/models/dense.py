@@ -369,10 +369,12 @@ class DenseGPU:
     """
 
     def __init__(self, w: "HostWeights | DenseConfig", num_pages: int, max_rows: int = 256, max_seqs: int = 64, max_blocks_per_seq: int = 256,
-                 device="cuda", max_prefill_rows: int = 8192, seed: int = 0, kv_dtype: str = "bf16"):
+                 device="cuda", max_prefill_rows: int = 8192, seed: int = 0, kv_dtype: str = "bf16", prefill_workspace: bool = True):
         """`w` is either host weights (uploaded as stored) or a bare config (random-init EXL3 weights are then generated on the
-        device: any random bit ring is a valid trellis, which is how benchmark models of tens of GB are made in seconds)."""
+        device: any random bit ring is a valid trellis, which is how benchmark models of tens of GB are made in seconds).
+        `prefill_workspace` False: without the memory of `prefill_workspace_bytes`; prompt slices then decode a matrix once per tile of rows."""
         from ..ops import kernels as K
+        self.prefill_workspace = prefill_workspace
         self.K = K
         self.window_seq_rows = 1       # the most adjacent rows one sequence has in the next decode / verify window (set by the backend)
         self.attn_plan = None          # device plan of the current window for the attention kernel (allocated with the scratch)
@@ -515,8 +517,8 @@ class DenseGPU:
         self._part_split = torch.empty(part_elems, dtype=torch.float32, device=dev) if split else None
         self.step_flags = torch.zeros(K.step_flags(), dtype=torch.int32, device=dev)
         # prompt slices of many rows: the decoded fp16 tiles of the largest matrix that goes that way
-        wide = [w for L in self.layers for n, w in L.items() if n in ("qkv", "o", "gate_up", "down") and self.splits.get(("prefill", n), 1) == 1 and
-                (K.wide_takes(w, R) or K.wide_takes(w, R, n == "gate_up"))]
+        wide = [w for L in self.layers for n, w in L.items() if self.prefill_workspace and n in ("qkv", "o", "gate_up", "down") and
+                self.splits.get(("prefill", n), 1) == 1 and (K.wide_takes(w, R) or K.wide_takes(w, R, n == "gate_up"))]
         self.wide = g("wide", max(K.wide_bytes(w.K, w.N) for w in wide), torch.uint8, zero=True) if wide else None
         kmax = max(k for k, _ in shapes.values())
         self.xr = g("xr", R * kmax, torch.float16)
@@ -536,8 +538,26 @@ class DenseGPU:
         self.cand_vals = torch.empty(min(R, 256), 64, dtype=torch.float32, device=dev)
 
     def _gemm_shapes(self) -> dict:
+        return self.gemm_shapes(self.cfg)
+
+    @classmethod
+    def prefill_workspace_bytes(cls, w: "HostWeights | DenseConfig", rows: int) -> int:
+        """Bytes that an executor of these host weights (or of a bare config) keeps for prompt slices of up to `rows` rows to decode a matrix into; 0 where
+        no matrix goes that way."""
+        from ..ops import kernels as K
+        if isinstance(w, DenseConfig):
+            four = exl3.Bits.of(w.bits).tile_words == 64
+            mats = [(n, *s) for n, s in cls.gemm_shapes(w).items() if four and n not in ("lm_head", "eh_proj") + cls.routed]
+        else:
+            mats = [(n, l.trellis.shape[0] * 16, l.trellis.shape[1] * 16) for lay in w.layers for n, l in vars(lay).items()
+                    if isinstance(l, HostLinear) and l.trellis.shape[2] == 64]
+        return max((K.wide_bytes(k, m) for n, k, m in mats if K.wide_takes_shape(rows, k, m) or K.wide_takes_shape(rows, k, m, n == "gate_up")), default=0)
+
+    routed = ()            # names of `gemm_shapes` that are routed experts here
+
+    @classmethod
+    def gemm_shapes(cls, cfg) -> dict:
         """name -> (K, N) of every EXL3 GEMM this executor launches through `_linear` (sizes the split plans and the scratch)."""
-        cfg = self.cfg
         return dict(qkv=(cfg.d_model, cfg.qkv_width), o=(cfg.n_q * cfg.head_dim, cfg.d_model), gate_up=(cfg.d_model, 2 * cfg.ffn_padded),
                     down=(cfg.ffn_padded, cfg.d_model), lm_head=(cfg.d_model, cfg.vocab_padded), eh_proj=(cfg.d_model, cfg.d_model))
 

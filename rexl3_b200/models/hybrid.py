@@ -352,10 +352,10 @@ class HybridGPU(DenseGPU):
     order."""
 
     def __init__(self, w: "HostWeights | HybridConfig", num_pages: int, max_rows: int = 256, max_seqs: int = 64, max_blocks_per_seq: int = 256,
-                 device="cuda", max_prefill_rows: int = 8192, seed: int = 0, kv_dtype: str = "bf16"):
+                 device="cuda", max_prefill_rows: int = 8192, seed: int = 0, kv_dtype: str = "bf16", prefill_workspace: bool = True):
         cfg = w if isinstance(w, HybridConfig) else w.cfg
         cfg.validate()
-        super().__init__(w, num_pages, max_rows, max_seqs, max_blocks_per_seq, device, max_prefill_rows, seed, kv_dtype)
+        super().__init__(w, num_pages, max_rows, max_seqs, max_blocks_per_seq, device, max_prefill_rows, seed, kv_dtype, prefill_workspace)
         if cfg.nope:
             self.inv_freq.zero_()
         H, P, N, C = cfg.ssm_heads, cfg.ssm_head_dim, cfg.ssm_state, cfg.conv_channels
@@ -408,9 +408,9 @@ class HybridGPU(DenseGPU):
     def _kv_layers(self):
         return self.cfg.attn_layers()
 
-    def _gemm_shapes(self) -> dict:
-        cfg = self.cfg
-        s = super()._gemm_shapes()
+    @classmethod
+    def gemm_shapes(cls, cfg) -> dict:
+        s = super().gemm_shapes(cfg)
         if "M" in cfg.pattern:
             s.update(in_proj=(cfg.d_model, cfg.in_proj_width), out_proj=(cfg.d_inner, cfg.d_model))
         if "G" in cfg.pattern:

@@ -199,9 +199,10 @@ class CombineDst(ctypes.Structure):
 class MoEGPU(DenseGPU):
     """sm_100a executor.  `experts=(lo, hi)` keeps only those experts on this GPU (expert parallelism); `ep` is then the object
     that supplies the all-reduce slots (see parallel/ep.py); with all experts local the combine writes a local slot."""
+    routed = ("gate_up", "down")
 
     def __init__(self, w, num_pages, max_rows=256, max_seqs=64, max_blocks_per_seq=256, device="cuda", max_prefill_rows=4096, seed=0,
-                 experts=None, ep=None, a2a=None, expert_paging=None):
+                 experts=None, ep=None, a2a=None, expert_paging=None, prefill_workspace=True):
         """`expert_paging` = dict(path=FILE, budget_bytes=N[, fill_threads, direct]): the routed experts stay in a record file (written there
         from the host weights when FILE does not exist yet) and are paged into a device slab of N bytes as the router asks for them
         (models/expert_paging.py); one rank, weights from host tensors.  Every layer's call then costs a device -> host read of its picks.
@@ -219,7 +220,7 @@ class MoEGPU(DenseGPU):
             raise ValueError("expert paging runs on one rank that owns every expert, over host weights")
         if ctypes.sizeof(CombineDst) != _lib.load().rx_moe_combine_desc_size():
             raise _lib.KernelError("MoE combine descriptor layout mismatch")
-        super().__init__(w, num_pages, max_rows, max_seqs, max_blocks_per_seq, device, max_prefill_rows, seed)
+        super().__init__(w, num_pages, max_rows, max_seqs, max_blocks_per_seq, device, max_prefill_rows, seed, prefill_workspace=prefill_workspace)
 
     # ------------------------------------------------------------------ weights
     def _load_host(self, w: HostWeights) -> None:

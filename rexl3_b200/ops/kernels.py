@@ -83,7 +83,12 @@ def tile_rows(rows: int) -> int:
 def wide_takes(w, rows: int, swiglu: bool = False) -> bool:
     """Whether `rows` rows through `w` in one split (and, with `swiglu`, what `finish_swiglu_rot` does) are faster by the kernel that decodes the matrix
     once into a workspace.  The bits are the same."""
-    return isinstance(w, Exl3Weight) and w.twice == 8 and bool(_lib.load().rx_exl3_wide_takes(rows, w.K, w.N, int(swiglu)))
+    return isinstance(w, Exl3Weight) and w.twice == 8 and wide_takes_shape(rows, w.K, w.N, swiglu)
+
+
+def wide_takes_shape(rows: int, K: int, N: int, swiglu: bool = False) -> bool:
+    """The same of a 4.0 bpw matrix that is not on the device (yet)."""
+    return bool(_lib.load().rx_exl3_wide_takes(rows, K, N, int(swiglu)))
 
 
 def step_flags() -> int:

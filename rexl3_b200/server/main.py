@@ -229,14 +229,15 @@ def build(args):
                     wbytes += (args.expert_cache_mib << 20) - int(cfg.n_layers * cfg.n_experts * 3 * cfg.d_model * cfg.expert_ffn * cfg.bits / 8)
                 if is_mla and args.expert_cache_mib:
                     wbytes += (args.expert_cache_mib << 20) - int((cfg.n_layers - cfg.n_dense) * cfg.n_experts * 3 * cfg.d_model * cfg.expert_ffn * (0.5 + 1 / 32))
-                mm = ModelMemory(wbytes, kvb, activation_reserve=2 << 30)
-                adm = Admission(free, 1 << 30, mm, args.slots).with_max_context(args.max_model_len).with_kv_tokens(kv_tokens)
-                adm.check(min(args.max_model_len, 1))     # fail closed: a plan that can never hold one token is refused at boot
-                if pages * kvb * dense.PAGE > adm.capacity:
-                    raise RuntimeError(f"memory plan refused: {kv_tokens} KV tokens need {pages * kvb * dense.PAGE >> 20} MiB, "
-                                       f"{adm.capacity >> 20} MiB are available after weights and reserve")
                 common = dict(num_pages=pages, max_rows=min(256, args.window_rows), max_seqs=args.slots,
                               max_blocks_per_seq=-(-args.max_model_len // dense.PAGE) + 1, max_prefill_rows=args.prefill_chunk)
+                workspace = 0
+                if not is_mla:
+                    cls = moe_models.MoEGPU if is_moe else hybrid_models.HybridGPU if is_hybrid else dense.DenseGPU
+                    workspace = cls.prefill_workspace_bytes(weights if weights is not None else cfg, max(common["max_rows"], args.prefill_chunk))
+                adm, with_workspace = plan_memory(free, wbytes, kvb, pages * dense.PAGE, workspace, args.slots, args.max_model_len, kv_tokens)
+                if not is_mla:
+                    common["prefill_workspace"] = with_workspace
                 paging = None
                 if args.expert_cache_mib:
                     if not (is_mla or is_moe):
@@ -286,6 +287,21 @@ def build(args):
     info["chat_format"] = fmt.id
     info["reasoning"] = fmt.caps.describe()
     return make, tok, fmt, name, info
+
+
+def plan_memory(free: int, weight_bytes: int, kv_bytes_per_token: int, pool_tokens: int, workspace: int, slots: int, max_context: int, kv_tokens: int):
+    """-> (Admission of the plan, whether it has room for the `workspace` bytes that only make prompt slices faster).  RuntimeError where the KV pool of
+    `pool_tokens` does not fit beside weights and reserve."""
+    for extra in (workspace, 0):
+        mm = ModelMemory(weight_bytes, kv_bytes_per_token, activation_reserve=(2 << 30) + extra)
+        adm = Admission(free, 1 << 30, mm, slots).with_max_context(max_context).with_kv_tokens(kv_tokens)
+        if pool_tokens * kv_bytes_per_token <= adm.capacity:
+            break
+    adm.check(min(max_context, 1))     # fail closed: a plan that can never hold one token is refused at boot
+    if pool_tokens * kv_bytes_per_token > adm.capacity:
+        raise RuntimeError(f"memory plan refused: {kv_tokens} KV tokens need {pool_tokens * kv_bytes_per_token >> 20} MiB, "
+                           f"{adm.capacity >> 20} MiB are available after weights and reserve")
+    return adm, extra == workspace
 
 
 def cache_namespace(name: str, cfg, info: dict, args, model=None) -> bytes:
