@@ -518,7 +518,7 @@ class DenseGPU:
         self.step_flags = torch.zeros(K.step_flags(), dtype=torch.int32, device=dev)
         # prompt slices of many rows: the decoded fp16 tiles of the largest matrix that goes that way
         wide = [w for L in self.layers for n, w in L.items() if self.prefill_workspace and n in ("qkv", "o", "gate_up", "down") and
-                self.splits.get(("prefill", n), 1) == 1 and (K.wide_takes(w, R) or K.wide_takes(w, R, n == "gate_up"))]
+                self.splits.get(("prefill", n), 1) == 1 and (K.wide_takes(w, R) or K.wide_takes(w, R, n == "gate_up", w is L.get("in_proj")))]
         self.wide = g("wide", max(K.wide_bytes(w.K, w.N) for w in wide), torch.uint8, zero=True) if wide else None
         kmax = max(k for k, _ in shapes.values())
         self.xr = g("xr", R * kmax, torch.float16)
@@ -551,9 +551,11 @@ class DenseGPU:
         else:
             mats = [(n, l.trellis.shape[0] * 16, l.trellis.shape[1] * 16) for lay in w.layers for n, l in vars(lay).items()
                     if isinstance(l, HostLinear) and l.trellis.shape[2] == 64]
-        return max((K.wide_bytes(k, m) for n, k, m in mats if K.wide_takes_shape(rows, k, m) or K.wide_takes_shape(rows, k, m, n == "gate_up")), default=0)
+        takes = lambda n, k, m: K.wide_takes_shape(rows, k, m) or K.wide_takes_shape(rows, k, m, n == "gate_up", n in cls.projected)  # noqa: E731
+        return max((K.wide_bytes(k, m) for n, k, m in mats if takes(n, k, m)), default=0)
 
     routed = ()            # names of `gemm_shapes` that are routed experts here
+    projected = ("in_proj", "gdn_in", "kda_in")        # those whose rows `exl3_gemm_store` may write
 
     @classmethod
     def gemm_shapes(cls, cfg) -> dict:

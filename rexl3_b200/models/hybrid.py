@@ -520,7 +520,7 @@ class HybridGPU(DenseGPU):
     # ------------------------------------------------------------------ forward
     def _in_proj(self, xr, w, M, cls, name, proj):
         K, work = self.K, self.wide if cls == "prefill" else None
-        if work is not None and isinstance(w, K.Exl3Weight) and self.splits[(cls, name)] == 1 and K.wide_takes(w, M) and work.numel() >= K.wide_bytes(w.K, w.N):
+        if work is not None and isinstance(w, K.Exl3Weight) and self.splits[(cls, name)] == 1 and K.wide_takes(w, M, store=True) and work.numel() >= K.wide_bytes(w.K, w.N):
             K.exl3_gemm_store(xr, w, proj, work, self.status)
         else:
             K.finish_store(self.part, self._linear(xr, w, M, cls, name), M, w, proj)

@@ -11,8 +11,8 @@
 //
 // What bounds it: the power limit (1.3 GHz in a long loop) and the operands' way through shared memory (each SM copies 32 KB in and reads 32 KB per 512 tensor
 // cycles, all that its 128 bytes a cycle carry: 620 to 650 cycles); beside it the expansion (178 M weights 98 us alone, its stores 3.6 TB/s).  Measured against
-// exl3_gemm_tm.cu, both in turn: 5120 -> 34,816 with its SwiGLU, 8192 rows 3.56 -> 2.41 ms, 2048 rows 936 -> 690 us; 17,408 -> 5120, 2048 rows 441 -> 300
-// us; 5120 -> 5120, 1024 rows 89 -> 73 us.  Tried and slower: rows of W [N][K] instead of tiles (a copy of 128 rows then touches 128 DRAM pages; 17,408 ->
+// exl3_gemm_tm.cu, both in turn, several matrices after one another: 5120 -> 34,816 with its SwiGLU, 8192 rows 3.27 -> 2.31 ms, 2048 rows 850 -> 657 us; 17,408 ->
+// 5120, 2048 rows 391 -> 317 us; 5120 -> 5120, 1024 rows 66 -> 62 us.  Tried and slower: rows of W [N][K] instead of tiles (a copy of 128 rows then touches 128 DRAM pages; 17,408 ->
 // 5120, 1024 rows 233 -> 188 us), f32 rows stored by their threads (150 -> 120 us at 2048 rows of 5120 x 5120), a last wave cut along the columns (narrow
 // tiles are bound by their copies).
 #include <cuda.h>
@@ -613,14 +613,18 @@ static int wide_counters(int K, int N) { return WC_READY + (N + 255) / 256 * ((K
 
 using namespace rx;
 
-// Whether the calls below are faster than exl3_gemm_tm.cu (and, with `swiglu`, the finish kernel after it).  That one takes 8 ns per k and wave of 148 tiles, this
-// one 6.6 per k and share of 74, but it has the expansion and a longer start.  Fitted to 224 (matrix, rows) with both timed in turn: gains from 1.0 to 1.6;
-// where it says no, the other is faster or within 12 %; where it says yes, the worst is 0.97.
-RX_API int rx_exl3_wide_takes(int rows, int K, int N, int swiglu) {
-  if (K % 128 != 0 || K < WD_PIECE_K || N % 128 != 0 || wide_counters(K, N) > WD_COUNTERS) return 0;
+// Whether the calls below are faster than exl3_gemm_tm.cu and, of the forms with one, the finish kernel after it; form: 0 plain, 1 SwiGLU, 2 store.  In units of that
+// kernel's 8 per k and wave of 148 tiles: a share of 74 costs about as much per k here, the expansion and a longer start come on top, a wave's start and the finish
+// kernel's rows fall away.  Fitted to 36 matrices (512 to 28,672 wide) at 19 row counts from 130 to 8192 each, both timed in turn: where it says yes the ratio of
+// the times is 0.985 and more (plain 1.33 at the most, SwiGLU 1.54, store 1.74), where it says no below 1.06 (store 1.10 once).
+RX_API int rx_exl3_wide_takes(int rows, int K, int N, int form) {
+  if (K % 128 != 0 || K < WD_PIECE_K || N % 128 != 0 || wide_counters(K, N) > WD_COUNTERS || form < 0 || form > 2) return 0;
+  static const struct { double wave, unit_k, unit, expand, start, finish; } F[3] = {
+      {11770, 7.94, 30, 4.06e-4, 44750, 0}, {3760, 7.65, 40, 3.78e-4, 48900, 2.84e-3}, {11130, 7.97, 250, 5.98e-4, 46700, 2.97e-3}};
+  const auto& f = F[form];
   const double rt = (rows + 255) / 256, tiles = rt * ((N + 255) / 256), units = tiles < WD_PAIRS ? 1.0 : tiles / WD_PAIRS;
   const double waves = (int)((rt * (N / 128) + 147) / 148);
-  return waves * (K * 8.0 + 4500) > units * (K * 6.6 + 2500) + (double)N * K * 3.4e-4 + (swiglu ? 36e3 - rows * (double)N * 1.7e-3 : 18e3);   // ns
+  return waves * (K * 8.0 + f.wave) + f.finish * rows * (double)N > units * (K * f.unit_k + f.unit) + f.expand * (double)N * K + f.start;
 }
 
 // Bytes of workspace for a matrix; its first WD_COUNTERS * 4 bytes are zero before the first call.

@@ -80,15 +80,15 @@ def tile_rows(rows: int) -> int:
     return _lib.load().rx_exl3_tile_rows(rows)
 
 
-def wide_takes(w, rows: int, swiglu: bool = False) -> bool:
-    """Whether `rows` rows through `w` in one split (and, with `swiglu`, what `finish_swiglu_rot` does) are faster by the kernel that decodes the matrix
-    once into a workspace.  The bits are the same."""
-    return isinstance(w, Exl3Weight) and w.twice == 8 and wide_takes_shape(rows, w.K, w.N, swiglu)
+def wide_takes(w, rows: int, swiglu: bool = False, store: bool = False) -> bool:
+    """Whether `rows` rows through `w` in one split (and, with `swiglu` or `store`, what `finish_swiglu_rot` or `finish_store` does) are faster by the kernel
+    that decodes the matrix once into a workspace.  The bits are the same."""
+    return isinstance(w, Exl3Weight) and w.twice == 8 and wide_takes_shape(rows, w.K, w.N, swiglu, store)
 
 
-def wide_takes_shape(rows: int, K: int, N: int, swiglu: bool = False) -> bool:
+def wide_takes_shape(rows: int, K: int, N: int, swiglu: bool = False, store: bool = False) -> bool:
     """The same of a 4.0 bpw matrix that is not on the device (yet)."""
-    return bool(_lib.load().rx_exl3_wide_takes(rows, K, N, int(swiglu)))
+    return bool(_lib.load().rx_exl3_wide_takes(rows, K, N, 1 if swiglu else 2 if store else 0))
 
 
 def step_flags() -> int:
@@ -102,7 +102,7 @@ def wide_bytes(K: int, N: int) -> int:
 
 
 def exl3_gemm_swiglu_rot(xr: torch.Tensor, w: Exl3Weight, suh_down: torch.Tensor, act: torch.Tensor, work: torch.Tensor, status: torch.Tensor) -> None:
-    """`exl3_gemm` and `finish_swiglu_rot` in one kernel for the rows of a prompt slice (where `wide_takes`): act fp16 [rows, N / 2]."""
+    """`exl3_gemm` and `finish_swiglu_rot` in one kernel for the rows of a prompt slice (where `wide_takes` with `swiglu`): act fp16 [rows, N / 2]."""
     rows, K = xr.shape
     assert xr.dtype == torch.float16 and xr.is_contiguous() and K == w.K and w.twice == 8
     assert act.dtype == torch.float16 and act.is_contiguous() and act.numel() >= rows * w.N // 2
@@ -113,7 +113,7 @@ def exl3_gemm_swiglu_rot(xr: torch.Tensor, w: Exl3Weight, suh_down: torch.Tensor
 
 
 def exl3_gemm_store(xr: torch.Tensor, w: Exl3Weight, out: torch.Tensor, work: torch.Tensor, status: torch.Tensor) -> None:
-    """`exl3_gemm` and `finish_store` in one kernel for the rows of a prompt slice (where `wide_takes`): out fp32 [rows, N]."""
+    """`exl3_gemm` and `finish_store` in one kernel for the rows of a prompt slice (where `wide_takes` with `store`): out fp32 [rows, N]."""
     rows, K = xr.shape
     assert xr.dtype == torch.float16 and xr.is_contiguous() and K == w.K and w.twice == 8
     assert out.dtype == torch.float32 and out.is_contiguous() and out.numel() >= rows * w.N

@@ -39,3 +39,14 @@ def test_plan_counts_the_workspace_or_does_without():
         main.plan_memory(20 * GB, 10 * GB, 1 << 20, 7 * 1024 + 1, GB, 4, 1024, 7 * 1024 + 1)
     adm, kept = main.plan_memory(20 * GB, 10 * GB, 1 << 20, 7 * 1024, 0, 4, 1024, 7 * 1024)        # nothing to keep
     assert kept and adm.capacity == 7 * GB
+
+
+@pytest.mark.parametrize("K,N,rows,form,tile_us,wide_us", [
+    (8192, 8192, 900, "plain", 121, 151), (17408, 5120, 1650, "plain", 273, 322), (4096, 28672, 300, "plain", 119, 138), (17408, 5120, 1650, "swiglu", 299, 335),
+    (12288, 4096, 2048, "store", 194, 222), (512, 6144, 3072, "store", 69, 47), (4096, 18432, 1280, "store", 232, 197), (5120, 34816, 2048, "swiglu", 850, 657),
+    (17408, 5120, 2048, "plain", 391, 317), (1024, 4096, 4096, "store", 75, 57),
+])
+def test_slices_go_where_they_were_measured_faster(K, N, rows, form, tile_us, wide_us):
+    """Times on a B200 of the kernel that decodes a matrix per tile of rows (and the finish kernel of the form) and of the one that decodes it once."""
+    from rexl3_b200.ops import kernels as KK
+    assert KK.wide_takes_shape(rows, K, N, form == "swiglu", form == "store") == (wide_us < tile_us)
