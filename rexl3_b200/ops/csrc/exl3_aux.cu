@@ -499,12 +499,18 @@ RX_API int rx_finish_store(const void* part, int S, int M, int N, const void* sv
   return (int)cudaGetLastError();
 }
 
+// Whether a prompt slice of one plane goes by the row form.  The general form below has up to 296 rows in one wave of two CTAs of 1024 threads per SM, and from 512 on,
+// where its CTAs are smaller, up to 592 in one wave again; rows wider than 4096 take it a second pass.  us, general and row form: 149 rows of 4224 9.5 and 6.9, 296 of
+// 2048 6.0 and 6.4, 297 8.1 and 7.0, 511 10.3 and 7.2, 592 6.4 and 7.6, 593 8.5 and 7.6; 296 of 4096 7.1 and 8.2, 297 9.9 and 7.6, 592 10.3 and 8.5.
+RX_API int rx_add_norm_rot_by_rows(int M, int N) {
+  if (N <= 1024 || N > ROWS_MAX) return 0;
+  return N > 4096 ? M > 148 : M > 296 && (N > 2048 || M < 512 || M > 592);
+}
+
 RX_API int rx_finish_add_norm_rot(const void* part, int S, int M, int N, const void* svh, const void* bias, void* h_bf16, const void* norm_w,
                                   float eps, const void* suh_next, void* xr, void* stream, void* xn_out) {
   if (N % 128 || N * 4 > 200 * 1024 || N / 128 > 512) return (int)cudaErrorInvalidValue;
-  // More rows than SMs: 150 rows of 5120 16.3 us by the form below, 12.3 by the row form; 150 of 4096, 3072 or 2048 level, 300 16.4 and 12.3, 14.3 and 12.3, 14.3 and
-  // 12.3; 74 rows 9.1 and 12.2.  (Just below 592 short rows are 2 us faster below: two whole waves of its CTAs.)
-  if (S == 1 && N > 1024 && N <= ROWS_MAX && M > 148) {
+  if (S == 1 && rx_add_norm_rot_by_rows(M, N)) {
     rx::launch(finish_add_norm_rot_rows_kernel, dim3(M), dim3((N / 128 + 4 * ROWS_NB - 1) / (4 * ROWS_NB) * 32), 0, (cudaStream_t)stream, (const float*)part, N, (const __half*)svh, (const float*)bias,
                (uint16_t*)h_bf16, (const uint16_t*)norm_w, eps, (const __half*)suh_next, (__half*)xr, (uint16_t*)xn_out);
     return (int)cudaGetLastError();

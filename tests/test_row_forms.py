@@ -1,0 +1,11 @@
+"""Where the row kernels of prompt slices (eight lanes a 128-block) take over from the forms of few rows: measured points, us on a B200 (few rows' form, slices' form)."""
+import pytest
+
+from rexl3_b200.ops import lib
+
+
+@pytest.mark.parametrize("M,N,few,rows", [(149, 4224, 9.5, 6.9), (149, 1152, 5.5, 6.0), (296, 2048, 6.0, 6.4), (297, 2048, 8.1, 7.0), (511, 2048, 10.3, 7.2),
+                                          (512, 1152, 5.7, 6.9), (592, 2048, 6.4, 7.6), (593, 2048, 8.5, 7.6), (296, 4096, 7.1, 8.2), (592, 4096, 10.3, 8.5),
+                                          (8192, 5120, 152.5, 89.9)])
+def test_residual_finish(M, N, few, rows):
+    assert lib.load().rx_add_norm_rot_by_rows(M, N) == (rows < few)
