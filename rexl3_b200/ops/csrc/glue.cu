@@ -402,8 +402,10 @@ __global__ void __launch_bounds__(TOPK_THREADS) topk_stage2_kernel(const uint64_
 using namespace rx;
 
 // Rows for the form of eight lanes a block: 40 heads and 8 of K and V, 600 rows 18.4 -> 15.2 us, 2100 38.9 -> 33.6, 8192 111.6 -> 92.2; 300 rows 13.1 and 16.3 (in CTAs of
-// 224 threads), 64 rows 8.2 and 10.2.  CTAs of up to 160 threads: of 224, in one pass, an SM holds too few (8192 rows 118.8).
-constexpr int QKV_ROWS_MIN = 593;
+// 224 threads), 64 rows 8.2 and 10.2.  CTAs of up to 160 threads: of 224, in one pass, an SM holds too few (8192 rows 118.8).  Up to eight blocks a row make a
+// CTA of one warp, and six for an SM are wanted: four heads and one of K and V, 800 rows 3.7 us by the other form and 4.3, 900 rows 4.6 and 4.4.
+RX_API int rx_qkv_rope_by_lanes(int M, int n_q, int n_kv) { return n_q > 0 && M >= (n_q + 2 * n_kv <= 8 ? 900 : 593); }
+
 RX_API int rx_finish_qkv_rope(const void* part, int S, int M, int n_q, int n_kv, int hd, const void* svh, const void* bias, const void* q_norm,
                               const void* k_norm, float eps, const void* positions, const void* inv_freq, const void* slot, void* q_out,
                               void* k_cache, void* v_cache, void* stream, const void* kv_scale, void* kv_amax, const void* pos3, int section_h,
@@ -418,7 +420,7 @@ RX_API int rx_finish_qkv_rope(const void* part, int S, int M, int n_q, int n_kv,
 #define RX_ARGS (const float*)part, S, M, n_q, n_kv, (const __half*)svh, (const float*)bias, (const uint16_t*)q_norm, (const uint16_t*)k_norm, eps, \
                 (const int*)positions, (const float*)inv_freq, (const int*)slot, (uint16_t*)q_out, (uint16_t*)k_cache, (uint16_t*)v_cache, \
                 (const float*)kv_scale, (float*)kv_amax, (const int*)pos3, 3 * section_h, 3 * section_w, (float*)k_tscale, (float*)v_tscale, q4
-  if (hd == 128 && S == 1 && M >= QKV_ROWS_MIN && kv_scale == nullptr && kv_amax == nullptr && k_tscale == nullptr && n_q > 0) {
+  if (hd == 128 && S == 1 && kv_scale == nullptr && kv_amax == nullptr && k_tscale == nullptr && rx_qkv_rope_by_lanes(M, n_q, n_kv)) {
     const int nb = n_q + 2 * n_kv, passes = (nb + 39) / 40, threads = (nb + 8 * passes - 1) / (8 * passes) * 32;
     rx::launch(finish_qkv_rope_rows_kernel, dim3(M), dim3(threads), 0, st, (const float*)part, n_q, n_kv, (const __half*)svh, (const float*)bias,
                (const uint16_t*)q_norm, (const uint16_t*)k_norm, eps, (const int*)positions, (const float*)inv_freq, (const int*)slot, (uint16_t*)q_out,

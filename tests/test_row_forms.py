@@ -9,3 +9,9 @@ from rexl3_b200.ops import lib
                                           (8192, 5120, 152.5, 89.9)])
 def test_residual_finish(M, N, few, rows):
     assert lib.load().rx_add_norm_rot_by_rows(M, N) == (rows < few)
+
+
+@pytest.mark.parametrize("M,n_q,n_kv,few,lanes", [(593, 1, 1, 3.2, 3.9), (800, 4, 1, 3.7, 4.3), (900, 4, 1, 4.6, 4.4), (593, 8, 2, 4.8, 4.4), (593, 40, 8, 11.1, 8.3),
+                                                  (300, 40, 8, 13.1, 16.3), (800, 4, 2, 4.0, 4.4), (8192, 1, 1, 13.1, 12.1)])
+def test_qkv_finish(M, n_q, n_kv, few, lanes):
+    assert lib.load().rx_qkv_rope_by_lanes(M, n_q, n_kv) == (lanes < few)
