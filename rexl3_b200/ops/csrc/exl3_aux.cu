@@ -464,13 +464,16 @@ RX_API int rx_embed(const void* ids, const void* table, void* h, int rows, int d
   return (int)cudaGetLastError();
 }
 
-// Eight lanes a block from 8192 blocks on (8192 rows of 8192 67.6 -> 57.3 us, 300 rows of 4096 9.1 -> 8.2, 128 of 8192 level); a few rows are level or, 128 of 2048,
-// 0.8 us slower.
-constexpr long long ROT_ROWS_MIN = 8192;
+// Eight lanes a block from 8192 blocks on (8192 rows of 4096 32.9 -> 27.3 us, 512 rows of 8192 7.0 -> 5.3), of rows of up to 1024 from 16,384 (1500 of 1024 level, 1024
+// 3.1 us by a warp a block and 3.3).  Not from 149 to 296 rows of up to 8192, which the form below has in one wave of two CTAs per SM (256 of 4096 2.5 and 3.4 us).
+RX_API int rx_rot_in_by_lanes(int rows, int K) {
+  return (long long)rows * (K / 128) >= (K <= 1024 ? 16384 : 8192) && (rows <= 148 || rows > 296 || K > 8192);
+}
+
 RX_API int rx_norm_rot_in(const void* x_bf16, const void* norm_w_bf16, float eps, const void* suh, void* xr, int rows, int K, void* stream) {
   if (K % 128 || K / 128 > 512) return (int)cudaErrorInvalidValue;
   const long long blocks = (long long)rows * (K / 128);
-  if (norm_w_bf16 == nullptr && blocks >= ROT_ROWS_MIN) {
+  if (norm_w_bf16 == nullptr && rx_rot_in_by_lanes(rows, K)) {
     rx::launch(rot_in_rows_kernel, dim3((unsigned)((blocks + 31) / 32)), dim3(256), 0, (cudaStream_t)stream, (const uint16_t*)x_bf16, (const __half*)suh, (__half*)xr,
                blocks, K / 128);
     return (int)cudaGetLastError();

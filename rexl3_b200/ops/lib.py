@@ -117,6 +117,7 @@ def _declare(lib):
         "rx_set_pdl": (c_int, [c_int]),
         "rx_embed": (c_int, [c_void, c_void, c_void, c_int, c_int, c_int, c_void]),
         "rx_norm_rot_in": (c_int, [c_void, c_void, c_f, c_void, c_void, c_int, c_int, c_void]),
+        "rx_rot_in_by_lanes": (c_int, [c_int, c_int]),
         "rx_add_norm_rot_by_rows": (c_int, [c_int, c_int]),
         "rx_qkv_rope_by_lanes": (c_int, [c_int, c_int, c_int]),
         "rx_finish_store": (c_int, [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_int, c_void]),

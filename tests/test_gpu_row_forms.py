@@ -33,3 +33,8 @@ def test_qkv_finish_of_narrow_rows(nq, nkv):
         got.append((q, kc, vc))
     for x, y in zip(*got):
         assert x.abs().max() > 0 and torch.isfinite(x.float()).all() and torch.equal(x, y)
+
+
+@pytest.mark.parametrize("M,N", [(16385, 128), (5462, 384), (297, 4096)])
+def test_plain_rotation(M, N):
+    aux.test_rotation_of_a_slice_equals_its_windows(M, N)

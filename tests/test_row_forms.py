@@ -15,3 +15,9 @@ def test_residual_finish(M, N, few, rows):
                                                   (300, 40, 8, 13.1, 16.3), (800, 4, 2, 4.0, 4.4), (8192, 1, 1, 13.1, 12.1)])
 def test_qkv_finish(M, n_q, n_kv, few, lanes):
     assert lib.load().rx_qkv_rope_by_lanes(M, n_q, n_kv) == (lanes < few)
+
+
+@pytest.mark.parametrize("rows,K,few,lanes", [(1024, 1024, 3.1, 3.3), (256, 4096, 2.5, 3.4), (296, 5120, 3.0, 3.6), (297, 5120, 4.7, 3.6), (128, 8192, 3.6, 3.4),
+                                              (2048, 1024, 4.3, 4.1), (8192, 4096, 32.9, 27.3), (200, 16384, 5.8, 4.9)])
+def test_plain_rotation(rows, K, few, lanes):
+    assert lib.load().rx_rot_in_by_lanes(rows, K) == (lanes < few)
