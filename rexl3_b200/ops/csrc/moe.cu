@@ -965,15 +965,23 @@ RX_API int rx_moe_plan(const void* ids, int pairs, int E, int e_lo, int e_hi, in
 // The forms of eight lanes a block take 32 blocks a CTA: bound by the shuffles and the issue of the transform (L1 85 % busy, its data pipe carries both), where
 // a warp a block spent two thirds more shuffles and waited for one block's loads at a time.  2100 rows x 8 picks, 2048 wide, experts of 768, with the
 // launch: gather 45 -> 33 us, SwiGLU 55 -> 48, combine 76 -> 49; 8192 rows: 154 -> 95, 176 -> 150, 242 -> 138.  A window leaves their fewer warps idle, so each
-// begins where it is the faster one, in 128-blocks of its input: gather 4096 blocks 11.1 -> 10.2 us, 2048 blocks 9.0 -> 10.2; SwiGLU 12,288 blocks
-// 14.3 -> 14.2, 6144 blocks 10.2 -> 12.2; combine 640 blocks 16.4 -> 12.2, 528 blocks 12.3 -> 13.1.
-constexpr long long GATHER_ROWS_MIN = 2560, SWIGLU_ROWS_MIN = 12288, COMBINE_ROWS_MIN = 640;
-static int moe_rows_grid(int rows, int blocks) { return (int)(((long long)rows * blocks + 31) / 32); }
+// begins where it is the faster one, in 128-blocks of its input.  Gather, us: 2048 wide, 8 picks, 256 rows 6.6 by the other
+// form and 9.8, 450 rows (7200 blocks) 9.5 and 11.2, 600 rows (9600) level, 800 rows 15.1 and 12.0; 4096 wide, 3 picks, 160 rows (5120) 4.6 and 5.1, 200 rows
+// (6400) 5.1 and 4.2; where the other form, a CTA a pair, has few of them, sooner: 6144 wide, 2 picks, 64 rows 5.0 and 3.6; 7168 wide, 1 pick, 64 rows
+// 5.9 and 2.9, 400 rows 7.2 and 6.3, 700 rows 8.0 and 8.3.  SwiGLU 12,288 blocks
+// 14.3 -> 14.2, 6144 blocks 10.2 -> 12.2.
+// Combine: 640 blocks 16.4 -> 12.2 us, 528 blocks 12.3 -> 13.1.
 static bool moe_rows_form(int rows, int blocks, long long least) { return (long long)rows * blocks >= least && (long long)rows * blocks < (1ll << 28); }
+RX_API int rx_moe_gather_by_rows(int pairs, int topk, int d) {
+  if (topk < 1 || (topk == 1 && pairs > 512)) return 0;
+  return moe_rows_form((pairs + topk - 1) / topk, d / 128, topk == 1 || (topk == 2 && pairs <= 320) ? 2560 : topk < 4 ? 6400 : 9600);
+}
+constexpr long long SWIGLU_ROWS_MIN = 12288, COMBINE_ROWS_MIN = 640;
+static int moe_rows_grid(int rows, int blocks) { return (int)(((long long)rows * blocks + 31) / 32); }
 
 RX_API int rx_moe_gather_rot(const void* x, const void* ids, const void* pos_of_pair, int pairs, int topk, int d, const void* suh, void* xs, void* stream) {
   if (pairs < 1 || d % 128 != 0) return (int)cudaErrorInvalidValue;
-  if (topk > 0 && moe_rows_form((pairs + topk - 1) / topk, d / 128, GATHER_ROWS_MIN))
+  if (rx_moe_gather_by_rows(pairs, topk, d))
     return (int)rx::launch(moe_gather_rot_rows_kernel, dim3(moe_rows_grid((pairs + topk - 1) / topk, d / 128)), dim3(256), 0, (cudaStream_t)stream,
                            (const uint16_t*)x, (const int*)ids, (const int*)pos_of_pair, pairs, topk, d, (const __half*)suh, (__half*)xs);
   int warps = d / 128;

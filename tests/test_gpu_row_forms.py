@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import test_gpu_aux_rows as aux
+import test_gpu_moe_rows as moe
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,9 @@ def test_qkv_finish_of_narrow_rows(nq, nkv):
 @pytest.mark.parametrize("M,N", [(16385, 128), (5462, 384), (297, 4096)])
 def test_plain_rotation(M, N):
     aux.test_rotation_of_a_slice_equals_its_windows(M, N)
+
+
+@pytest.mark.parametrize("M,topk,d", [(433, 1, 768), (3201, 2, 256), (1601, 3, 512), (801, 10, 1536), (601, 7, 2048)])
+@pytest.mark.parametrize("rotated", [True, False])
+def test_routed_gather(M, topk, d, rotated):
+    moe.test_gather_of_a_slice_equals_its_windows(M, topk, d, rotated)

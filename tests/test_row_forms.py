@@ -21,3 +21,10 @@ def test_qkv_finish(M, n_q, n_kv, few, lanes):
                                               (2048, 1024, 4.3, 4.1), (8192, 4096, 32.9, 27.3), (200, 16384, 5.8, 4.9)])
 def test_plain_rotation(rows, K, few, lanes):
     assert lib.load().rx_rot_in_by_lanes(rows, K) == (lanes < few)
+
+
+@pytest.mark.parametrize("rows,topk,d,few,lanes", [(256, 8, 2048, 6.6, 9.8), (450, 8, 2048, 9.5, 11.2), (800, 8, 2048, 15.1, 12.0), (160, 3, 4096, 4.6, 5.1),
+                                                   (200, 3, 4096, 5.1, 4.2), (64, 2, 6144, 5.0, 3.6), (64, 1, 7168, 5.9, 2.9), (700, 1, 7168, 8.0, 8.3),
+                                                   (3000, 1, 4096, 13.6, 16.1), (74, 4, 5120, 4.4, 5.0), (3000, 8, 2048, 56.2, 37.1)])
+def test_routed_gather(rows, topk, d, few, lanes):
+    assert lib.load().rx_moe_gather_by_rows(rows * topk, topk, d) == (lanes < few)
