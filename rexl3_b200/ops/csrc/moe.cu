@@ -968,15 +968,19 @@ RX_API int rx_moe_plan(const void* ids, int pairs, int E, int e_lo, int e_hi, in
 // begins where it is the faster one, in 128-blocks of its input.  Gather, us: 2048 wide, 8 picks, 256 rows 6.6 by the other
 // form and 9.8, 450 rows (7200 blocks) 9.5 and 11.2, 600 rows (9600) level, 800 rows 15.1 and 12.0; 4096 wide, 3 picks, 160 rows (5120) 4.6 and 5.1, 200 rows
 // (6400) 5.1 and 4.2; where the other form, a CTA a pair, has few of them, sooner: 6144 wide, 2 picks, 64 rows 5.0 and 3.6; 7168 wide, 1 pick, 64 rows
-// 5.9 and 2.9, 400 rows 7.2 and 6.3, 700 rows 8.0 and 8.3.  SwiGLU 12,288 blocks
-// 14.3 -> 14.2, 6144 blocks 10.2 -> 12.2.
+// 5.9 and 2.9, 400 rows 7.2 and 6.3, 700 rows 8.0 and 8.3.  SwiGLU: 12,288 blocks; rows of up to 1024, which a CTA of the other form has in one pass, lose between
+// a wave of three CTAs per SM and 18,000 blocks (768 wide, 2048 pairs 8.2 and 7.6, 2400 pairs 8.6 and 9.4, 4800 pairs 14.5 and 14.3).
 // Combine: 640 blocks 16.4 -> 12.2 us, 528 blocks 12.3 -> 13.1.
 static bool moe_rows_form(int rows, int blocks, long long least) { return (long long)rows * blocks >= least && (long long)rows * blocks < (1ll << 28); }
 RX_API int rx_moe_gather_by_rows(int pairs, int topk, int d) {
   if (topk < 1 || (topk == 1 && pairs > 512)) return 0;
   return moe_rows_form((pairs + topk - 1) / topk, d / 128, topk == 1 || (topk == 2 && pairs <= 320) ? 2560 : topk < 4 ? 6400 : 9600);
 }
-constexpr long long SWIGLU_ROWS_MIN = 12288, COMBINE_ROWS_MIN = 640;
+RX_API int rx_moe_swiglu_by_rows(int pairs, int F) {
+  const long long blocks = (long long)pairs * (F / 128);
+  return moe_rows_form(pairs, F / 128, 12288) && (F > 1024 || blocks <= 444 * 32 || blocks >= 18000);
+}
+constexpr long long COMBINE_ROWS_MIN = 640;
 static int moe_rows_grid(int rows, int blocks) { return (int)(((long long)rows * blocks + 31) / 32); }
 
 RX_API int rx_moe_gather_rot(const void* x, const void* ids, const void* pos_of_pair, int pairs, int topk, int d, const void* suh, void* xs, void* stream) {
@@ -993,7 +997,7 @@ RX_API int rx_moe_gather_rot(const void* x, const void* ids, const void* pos_of_
 RX_API int rx_moe_swiglu_rot(const void* part, int S, int pairs_cap, int F, const void* expert_of_pos, const void* total, const void* svh_gu,
                              const void* suh_down, void* xs2, void* stream) {
   if (pairs_cap < 1 || F % 128 != 0 || S < 1) return (int)cudaErrorInvalidValue;
-  if (S == 1 && moe_rows_form(pairs_cap, F / 128, SWIGLU_ROWS_MIN))
+  if (S == 1 && rx_moe_swiglu_by_rows(pairs_cap, F))
     return (int)rx::launch(moe_swiglu_rot_rows_kernel, dim3(moe_rows_grid(pairs_cap, F / 128)), dim3(256), 0, (cudaStream_t)stream, (const float*)part, F,
                            (const int*)expert_of_pos, (const int*)total, (const __half*)svh_gu, (const __half*)suh_down, (__half*)xs2);
   int warps = F / 128;

@@ -74,6 +74,7 @@ def _declare(lib):
         "rx_moe_plan": (c_int, [c_void, c_int, c_int, c_int, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_void, c_void]),
         "rx_moe_gather_rot": (c_int, [c_void, c_void, c_void, c_int, c_int, c_int, c_void, c_void, c_void]),
         "rx_moe_gather_by_rows": (c_int, [c_int, c_int, c_int]),
+        "rx_moe_swiglu_by_rows": (c_int, [c_int, c_int]),
         "rx_moe_swiglu_rot": (c_int, [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_void]),
         "rx_moe_relu2_rot": (c_int, [c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void, c_void, c_void]),
         "rx_moe_combine_desc_size": (c_int, []),

@@ -28,3 +28,9 @@ def test_plain_rotation(rows, K, few, lanes):
                                                    (3000, 1, 4096, 13.6, 16.1), (74, 4, 5120, 4.4, 5.0), (3000, 8, 2048, 56.2, 37.1)])
 def test_routed_gather(rows, topk, d, few, lanes):
     assert lib.load().rx_moe_gather_by_rows(rows * topk, topk, d) == (lanes < few)
+
+
+@pytest.mark.parametrize("pairs,F,few,lanes", [(2048, 768, 8.2, 7.6), (2400, 768, 8.6, 9.4), (1800, 1024, 8.5, 9.4), (4800, 768, 14.5, 14.3), (24000, 768, 63.8, 56.3),
+                                               (1200, 1408, 11.6, 7.6)])
+def test_routed_swiglu(pairs, F, few, lanes):
+    assert lib.load().rx_moe_swiglu_by_rows(pairs, F) == (lanes < few)
