@@ -433,10 +433,13 @@ static bool step_fits(int rows, int K, int N, int splits) {
   return items >= ST_CTAS && items / ST_CTAS + 3 <= ST_PIECES && chunks < (1 << 24);
 }
 
-// Whether the call below is faster than exl3_gemm_tm.cu: that one takes 0.527 us a chunk on the SMs with two items and 3 us, this one 0.48 us a chunk of an equal
-// share and 8.5 us (its start, and the spread of CTAs that wait for one another's accumulators).  One row, us: 4096 -> 28,672 36.1 and 30.6; 5120 ->
-// 32,768 44.9 and 41.2; 5120 -> 34,816 45.1 and 43.1; 17,408 -> 5120 in seven splits 23.6 and 25.0; 5120 -> 5120 in seven 9.1 and 13.2.  From 33 to 64 rows
-// that one still has two CTAs to an SM and the gains are below 5 % (5120 -> 34,816 45.1 and 49.4; 4096 -> 28,672 36.3 and 34.8).
+// Whether the call below is faster than exl3_gemm_tm.cu: that one takes 0.527 us a chunk on the SMs with two items and 3 us, this one 0.505 us a chunk of an equal
+// share and 9.5 us (its start, and the spread of CTAs that wait for one another's accumulators), 11.5 from 17 rows on.  What an accumulator takes from one CTA to the next
+// is hidden by the chunks that a share is longer than an item: with fewer than 4 of them, from 5 rows on 8 and from 17 rows on 10, the CTAs wait.  Layers of dense
+// models, us by that one and this one, every other product the same: 4608 -> 24,576 (share 47, item 36) one row 93.6 and 85.5, 32 rows 102.2 and 100.9; 4096 ->
+// 28,672 (48, 32) 88.1 and 84.9, 100.8 and 100.3; 4096 -> 22,016 (37, 32) 89.4 and 84.5, 113.0 and 118.9; 2560 -> 19,456 (20.5, 20) 60.0 and 66.0, 74.3 and 86.6;
+// 5120 -> 34,816 (73.5, 40) 108.7 and 109.6, 124.3 and 124.9; 7168 -> 36,864 (109, 56) 149.9 and 151.9.  From 33 to 64 rows that one still has two CTAs to an SM
+// and the gains are below 5 % (5120 -> 34,816 45.1 and 49.4; 4096 -> 28,672 36.3 and 34.8).
 // Verify windows of 65 to 96 rows, one CTA per SM either way: the persistent kernel of whole items (exl3_gemm_grouped.cu) takes 0.78 us a chunk of the CTAs with
 // most of them and 5 us, this one, with half as many decode warps more, 0.514 us a chunk of an equal share and 11.5 us.  80 rows, us: 5120 -> 34,816 65.0
 // and 49.4; 4096 -> 28,672 50.8 and 36.0; 5120 -> 151,936 283 and 221; 17,408 -> 5120 34.0 and 30.5; 5120 -> 8192 in four splits 21.2 and 19.9; 6144 -> 5120 in
@@ -446,8 +449,8 @@ RX_API int rx_exl3_step_takes(int rows, int K, int N, int splits) {
   const int item = (K / ST_KCH + splits - 1) / splits, items = (N / 128) * splits;
   const double share = (N / 128) * (K / ST_KCH) / (double)ST_CTAS;
   if (rows > 64) return (items + ST_CTAS - 1) / ST_CTAS * item * 0.78 + 5.0 > share * 0.514 + 11.5;
-  if (items > 2 * ST_CTAS) return 0;
-  return 2 * item * 0.527 + 3.0 > share * 0.48 + (rows <= 16 ? 8.5 : 9.5);
+  if (items > 2 * ST_CTAS || share - item < (rows <= 4 ? 4 : rows <= 16 ? 8 : 10)) return 0;
+  return 2 * item * 0.527 + 3.0 > share * 0.505 + (rows <= 16 ? 9.5 : 11.5);
 }
 
 // rx_exl3_gemm_b4 for decode windows; flags: int32 [rx_exl3_step_flags()], zero before the first call; calls that may overlap need one each.
