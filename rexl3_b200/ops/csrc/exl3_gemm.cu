@@ -188,6 +188,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     bool ok = true;
     c_next = grp;
     // A wait that gives up does not end the loop, the chunks are void then: lanes that left it one by one would be missed by the others' shuffles.
+    // (The waits after it are made all the same, a branch around each costs 0.5 % of a step at 2, 5 and 6 bpw; they end by the abort flag.)
     if constexpr (TWICE == 8) {
       // ---- 4.0 bpw fast path.  A thread owns the two eighths 2h and 2h+1 of its tile (two 16-byte loads, conflict free
       // because odd k-tiles take them in the other order), gets the one word before each from its own other eighth or from
@@ -200,14 +201,14 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
       const int src = (lane & ~3) | ((h + 3) & 3);
       for (int c = grp; c < nchunks; c += NDEC_GROUPS) {
         const int rs = c % RAW_STAGES, os = c % OP_STAGES;
-        ok = ok && mbar_wait_early(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, ended, status, 30);
+        ok = mbar_wait_early(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, ended, status, 30) && ok;
         const uint4* tile4 = reinterpret_cast<const uint4*>(smem + L.raw_off + rs * RAW_STAGE) + (ktl * 8 + nt) * 8;
         const uint4 first = tile4[g1], second = tile4[g2];
         const uint32_t sh_second = __shfl_sync(0xffffffffu, second.w, src), sh_first = __shfl_sync(0xffffffffu, first.w, src);
         const uint32_t w1[5] = {x ? second.w : sh_second, first.x, first.y, first.z, first.w};
         const uint32_t w2[5] = {x ? sh_first : first.w, second.x, second.y, second.z, second.w};
         release_read_stage(&raw_empty[rs], lane);      // generic-proxy reads, async-proxy refill: proxy fence before the release
-        if (c >= OP_STAGES) ok = ok && mbar_wait_early(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, ended, status, 31);
+        if (c >= OP_STAGES) ok = mbar_wait_early(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, ended, status, 31) && ok;
         uint8_t* a_tile = smem + L.a_off + os * A_STAGE;
         {
           uint32_t h2[16];
@@ -237,9 +238,9 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     } else
     for (int c = grp; c < nchunks; c += NDEC_GROUPS) {
       const int rs = c % RAW_STAGES, os = c % OP_STAGES;
-      ok = ok && mbar_wait_early(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, ended, status, 30);
+      ok = mbar_wait_early(&raw_full[rs], (c / RAW_STAGES) & 1, abort_flag, ended, status, 30) && ok;
       const uint32_t* tile = (const uint32_t*)(smem + L.raw_off + rs * RAW_STAGE) + (ktl * 8 + nt) * TILE_WORDS;
-      if (c >= OP_STAGES) ok = ok && mbar_wait_early(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, ended, status, 31);
+      if (c >= OP_STAGES) ok = mbar_wait_early(&op_empty[os], ((c / OP_STAGES) - 1) & 1, abort_flag, ended, status, 31) && ok;
       uint8_t* a_tile = smem + L.a_off + os * A_STAGE;
       if constexpr (TWICE % 2 == 0) {
         // two word-aligned eighths per thread; odd k-tiles take them in the other order, which makes the 8 threads
