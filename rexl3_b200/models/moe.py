@@ -191,6 +191,13 @@ class _ExpertStack:
         return _ExpertStack(tr, suh, svh, lins[0].codebook)
 
 
+def tall_tiles(pairs: int, experts: int, N: int) -> bool:
+    """Whether a prompt slice's expert tiles have 256 rows, which decode an expert's weights once where 128 rows would have them twice: from 80 rows per expert
+    on (128 experts, 2048 -> 1536 and 768 -> 2048: 16,800 pairs 248 -> 190 and 164 -> 135 us, 10,400 pairs 158 -> 156 and 98 -> 90; 8,800 pairs, uneven, 158 -> 162),
+    and where tiles of 128 rows are more than the SMs have at once (8 experts, 1024 -> 1024: 1600 pairs 14 us by 128 rows and 18, 2400 pairs 23 and 18)."""
+    return pairs >= 80 * experts and experts * -(-pairs // (128 * experts)) * (N // 128) > 148
+
+
 class CombineDst(ctypes.Structure):
     _fields_ = [("ranks", ctypes.c_int), ("rank", ctypes.c_int), ("dst", ctypes.c_void_p * TP_MAX), ("dst_flag", ctypes.c_void_p * TP_MAX),
                 ("local_count", ctypes.c_void_p), ("epoch", ctypes.c_void_p), ("use_index", ctypes.c_uint), ("rows_cap", ctypes.c_int)]
@@ -367,9 +374,7 @@ class MoEGPU(DenseGPU):
         if cls == "decode":
             tile_rows, max_tiles = (16 if M <= 16 else 32), self.max_tiles_decode
         else:
-            # tiles of 256 rows decode an expert's weights once where 128 rows would have them twice: from 80 rows per expert on (128 experts, 2048 -> 1536 and
-            # 768 -> 2048: 16,800 pairs 248 -> 190 and 164 -> 135 us, 10,400 pairs 158 -> 156 and 98 -> 90; 8,800 pairs, uneven, 158 -> 162)
-            tall = pairs >= 80 * cfg.n_experts and all(t.twice in (6, 8) for t in (L["gu"], L["down"]))
+            tall = tall_tiles(pairs, cfg.n_experts, L["gu"].N) and all(t.twice in (6, 8) for t in (L["gu"], L["down"]))
             tile_rows, max_tiles = 256 if tall else 128, self.max_tiles_prefill
         if self.a2a is not None:
             yield from self._ffn_a2a(li, L, M, cls, xn, tile_rows, max_tiles, h, xr_d, next_norm, next_suh)

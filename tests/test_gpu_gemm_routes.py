@@ -73,7 +73,7 @@ def test_routed_slice_by_tall_tiles():
     if not torch.cuda.is_available():
         pytest.skip("needs a CUDA device")
     from rexl3_b200.models import moe
-    cfg = moe.MoEConfig(n_layers=2, d_model=512, n_q=4, n_kv=2, head_dim=128, ffn=128, vocab=512, bits=3.0, n_experts=8, top_k=4, expert_ffn=256)
+    cfg = moe.MoEConfig(n_layers=2, d_model=512, n_q=4, n_kv=2, head_dim=128, ffn=128, vocab=512, bits=3.0, n_experts=8, top_k=4, expert_ffn=1280)
     T, pages = 400, 7
     m = moe.MoEGPU(cfg, num_pages=pages, max_rows=64, max_seqs=1, max_blocks_per_seq=pages, max_prefill_rows=T)
     tiles, grouped = [], m._grouped_shifted

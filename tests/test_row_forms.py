@@ -34,3 +34,10 @@ def test_routed_gather(rows, topk, d, few, lanes):
                                                (1200, 1408, 11.6, 7.6)])
 def test_routed_swiglu(pairs, F, few, lanes):
     assert lib.load().rx_moe_swiglu_by_rows(pairs, F) == (lanes < few)
+
+
+@pytest.mark.parametrize("pairs,experts,N,low,tall", [(1600, 8, 1024, 14, 18), (1024, 8, 1024, 13, 17), (2400, 8, 1024, 23, 18), (800, 8, 28672, 421, 344), (1600, 16, 2048, 50, 44),
+                                                      (16800, 128, 1536, 248, 190), (8800, 128, 1536, 158, 162), (10400, 128, 1536, 158, 156)])
+def test_expert_tiles(pairs, experts, N, low, tall):
+    from rexl3_b200.models.moe import tall_tiles
+    assert tall_tiles(pairs, experts, N) == (tall < low)
