@@ -5,11 +5,12 @@
 // into 148 equal shares.  A share begins and ends inside an item (a strip's split): the first k of an item are the end of a share, the last k the beginning of
 // the next one.  A CTA takes its first-k piece first and hands its accumulator on through the item's place in `part`; it takes whole items next and its last-k
 // piece, with the accumulator of the CTA before, at the end.  So an accumulator meets its k in the one order that a single CTA would, and the bits are those of
-// exl3_gemm_tm.cu.  The CTA that waits has long got what it waits for: it is numbered after one that was running when it began, and shares are no shorter
-// than items.
+// exl3_gemm_tm.cu.  No circle of waits: a CTA waits for one that was numbered before it and was running when it began, and no piece is both taken and handed on.
+// (That would be a share strictly inside an item, which is then two chunks longer at least.  But with no fewer items than CTAs a share has at least as many whole
+// chunks as the mean item, and the longest item is at most one more.)
 //
-// What bounds it: the decode's integer work (18 of the 20 weights a clock that its loop reaches alone) and 8 us that no weight is decoded in: the start, the last
-// MMAs, and CTAs that begin late because their SM's last one ended late.
+// What bounds it: the decode's integer work (18 of the 20 weights a clock that its loop reaches alone) and 9 us that no weight is decoded in: the start, the last
+// MMAs, and CTAs that begin late because their SM's last one ended late; and, where shares are hardly longer than items, the accumulators that CTAs wait for.
 //
 // Up to 32 rows tensor memory holds two accumulators beside the six A stages.  More rows (TALL) have one, which 96 rows still leave room for: what its write-out
 // costs is kept short by giving each 16 rows of it to another decode group, and up to six chunks are decoded meanwhile.

@@ -11,8 +11,8 @@
 //
 // What bounds it: the power limit (1.3 GHz in a long loop) and the operands' way through shared memory (each SM copies 32 KB in and reads 32 KB per 512 tensor
 // cycles, all that its 128 bytes a cycle carry: 620 to 650 cycles); beside it the expansion (178 M weights 98 us alone, its stores 3.6 TB/s).  Measured against
-// exl3_gemm_tm.cu, both in turn, several matrices after one another: 5120 -> 34,816 with its SwiGLU, 8192 rows 3.27 -> 2.31 ms, 2048 rows 850 -> 657 us; 17,408 ->
-// 5120, 2048 rows 391 -> 317 us; 5120 -> 5120, 1024 rows 66 -> 62 us.  Tried and slower: rows of W [N][K] instead of tiles (a copy of 128 rows then touches 128 DRAM pages; 17,408 ->
+// exl3_gemm_tm.cu, four matrices after one another: 5120 -> 34,816 with its SwiGLU, 8192 rows 3.30 -> 2.07 ms (2.31 once the power limit holds the clock), 2048 rows 832 ->
+// 649 us; 17,408 -> 5120, 2048 rows 405 -> 325 us; 5120 -> 5120, 1024 rows 66 -> 62 us.  Tried and slower: rows of W [N][K] instead of tiles (a copy of 128 rows then touches 128 DRAM pages; 17,408 ->
 // 5120, 1024 rows 233 -> 188 us), f32 rows stored by their threads (150 -> 120 us at 2048 rows of 5120 x 5120), a last wave cut along the columns (narrow
 // tiles are bound by their copies).
 #include <cuda.h>
