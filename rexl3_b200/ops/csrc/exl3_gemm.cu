@@ -143,10 +143,7 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
           }
           ++n_raw;
         }
-        if (i == AHEAD) {
-          pdl_wait();
-          *ended = kernel_ended_at();
-        }
+        if (i == AHEAD) pdl_wait();
         if (i >= AHEAD) {
           const int c = i - AHEAD, s = c % OP_STAGES;
           if (c >= OP_STAGES) ok = mbar_wait(&op_empty[s], ((c / OP_STAGES) - 1) & 1, abort_flag, status, 11);
@@ -164,9 +161,11 @@ exl3_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint32_t* __r
     if (elect_one()) {
       const uint32_t idesc = umma_idesc_f16(STRIP, brows, 0, 0);
       bool ok = true;
+      pdl_wait();                                  // (its first operands come after that anyway, and the producer has no time to read a clock)
+      *ended = kernel_ended_at();
       for (int c = 0; c < nchunks && ok; ++c) {
         const int s = c % OP_STAGES;
-        ok = mbar_wait_early(&op_full[s], (c / OP_STAGES) & 1, abort_flag, ended, status, 20);
+        ok = mbar_wait(&op_full[s], (c / OP_STAGES) & 1, abort_flag, status, 20);
         if (!ok) break;
         tc_fence_after();
         const uint32_t a_addr = smem_u32(smem + L.a_off + s * A_STAGE);
